@@ -42,7 +42,6 @@ FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0}
 # dram__bytes_read.sum + dram__bytes_write.sum per step of the dominant kernel, from the ncu captures summarised under
 # profiles/ (workload, kernel) -> bytes; anything not listed is reported as null
 DRAM_TRAFFIC = {
-    ("default", "gdn_chain_t_kernel"): 358.0e6,      # 307.1 MB read + 50.9 MB written by the one split launch
     ("default", "gdn_chain_kernel"): 361.8e6,
     ("default", "gdn_coop_kernel"): 328.7e6,
 }
@@ -772,13 +771,13 @@ def main():
     single_launch = args.path == "coop" or (args.path == "auto" and w.S <= 2048 and 4 * B_local * w.Hv <= n_sm)
     transposed = args.path == "twopass_t" or (args.path == "auto" and not single_launch)
     kernels = ("gdn_coop_kernel (one launch)" if single_launch else
-               "gdn_prepare_pair_kernel + gdn_chain_t_kernel (few long sequences are split into warmed-up segments on the device)"
+               "gdn_prepare_lean_kernel + gdn_chain_r_kernel (few long sequences are split into warmed-up segments on the device)"
                if transposed else
                "gdn_prepare_kernel + gdn_chain_kernel" if args.path in ("twopass_nv32", "twopass_nv64") else args.path)
     if transposed or args.path in ("twopass_nv32", "twopass_nv64"):
         per_kernel = {}
         step()                                            # leaves a valid workspace for the chain-only launches
-        for key, name in (("prepare_only", "prepare_only_t" if transposed else "prepare_only"),
+        for key, name in (("prepare_only", "prepare_only_r" if transposed else "prepare_only"),
                           ("chain_only", "chain_only_t" if transposed else "chain_only")):
             times = []
             for _ in range(max(3, min(args.steps, 10))):
@@ -826,8 +825,8 @@ def main():
         k_s = per_kernel["chain_only"] * 1e-3
         tf = fl_chain / k_s / 1e12
         # DRAM bytes of one chain launch on the default workload, from an ncu capture (profiles/): read + write
-        traffic = DRAM_TRAFFIC.get((args.workload, "gdn_chain_t_kernel" if transposed else "gdn_chain_kernel")) if world == 1 else None
-        roofline = {"kernel": "gdn_chain_t_kernel" if transposed else "gdn_chain_kernel", "bound": "tensor", "achieved": tf, "peak": peaks["bf16_tflops"],
+        traffic = DRAM_TRAFFIC.get((args.workload, "gdn_chain_r_kernel" if transposed else "gdn_chain_kernel")) if world == 1 else None
+        roofline = {"kernel": "gdn_chain_r_kernel" if transposed else "gdn_chain_kernel", "bound": "tensor", "achieved": tf, "peak": peaks["bf16_tflops"],
                     "unit": "TFLOP/s", "frac": tf / peaks["bf16_tflops"], "traffic": traffic,
                     "peak_kind": f"{peak_kind} (burst cuBLAS bf16)", "algorithmic_flops_per_launch": fl_chain,
                     "kernel_ms": per_kernel["chain_only"],

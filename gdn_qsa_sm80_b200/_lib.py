@@ -36,7 +36,7 @@ FLAG_GATE_ACTIVATIONS = 2
 PATHS = {"auto": PATH_AUTO, "simt": PATH_SIMT, 
          "twopass_nv64": PATH_TWOPASS_NV64, "twopass_nv32": PATH_TWOPASS_NV32,
          "prepare_only": PATH_PREPARE_ONLY, "chain_only": PATH_CHAIN_ONLY, "coop": PATH_COOP, "coop_chain_only": PATH_COOP_CHAIN_ONLY, "decode": 11, "twopass_t": 12,
-         "prepare_only_t": 13, "chain_only_t": 14}
+         "prepare_only_t": 13, "chain_only_t": 14, "prepare_only_r": 15}
 
 # Every symbol the public header declares (checked by the CPU tests).
 EXPORTS = (

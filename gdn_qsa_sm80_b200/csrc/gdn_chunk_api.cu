@@ -94,6 +94,14 @@ int encode_workspace_maps(const Problem& p, const Workspace& ws, void* tw, void*
     return 0;
 }
 
+int encode_tile_maps(const Problem& p, const Workspace& ws, void* tp, void* tt2) {
+    const unsigned long long tiles = p.pk_chunk ? static_cast<unsigned long long>(p.pk_chunks) * p.Hv
+                                                : static_cast<unsigned long long>(p.B) * p.Hv * ((p.S + kChunk - 1) / kChunk);
+    const unsigned long long d[2] = {64, tiles * kChunk}, s[1] = {128};
+    const unsigned box[2] = {64, 64};
+    return encode_tma(tp, ws.P, 2, 2, d, s, box, 128) || encode_tma(tt2, ws.U, 2, 2, d, s, box, 128);
+}
+
 int sm_count() {
     static int cached[64] = {0};
     int dev = 0;
@@ -121,18 +129,21 @@ static size_t tiles_of(int B, int S, int Hv) {
     return static_cast<size_t>(B) * Hv * ((S + kChunk - 1) / kChunk);
 }
 
+// the residual-form chain, or the prepare kernels that write what it reads
+static bool transposed_path(int path) {
+    return path == GDN_PATH_TWOPASS_T || path == GDN_PATH_PREPARE_ONLY_T || path == GDN_PATH_CHAIN_ONLY_T || path == GDN_PATH_PREPARE_ONLY_R;
+}
+
 static bool path_uses_workspace(int path) {
     return path == GDN_PATH_AUTO || path == GDN_PATH_TWOPASS_NV64 || path == GDN_PATH_TWOPASS_NV32 ||
            path == GDN_PATH_PREPARE_ONLY || path == GDN_PATH_CHAIN_ONLY || path == GDN_PATH_COOP ||
-           path == GDN_PATH_COOP_CHAIN_ONLY || path == GDN_PATH_TWOPASS_T ||
-           path == GDN_PATH_PREPARE_ONLY_T || path == GDN_PATH_CHAIN_ONLY_T;
+           path == GDN_PATH_COOP_CHAIN_ONLY || transposed_path(path);
 }
 
-// segments the path cuts every sequence into (only the transposed chain splits sequences; 1 = not split)
+// the most segments the path cuts every sequence into (only the transposed chain splits sequences; 1 = not split)
 static int segments_of(int B, int S, int Hv, int path) {
-    if (path != GDN_PATH_TWOPASS_T && path != GDN_PATH_AUTO && path != GDN_PATH_PREPARE_ONLY_T && path != GDN_PATH_CHAIN_ONLY_T)
-        return 1;
-    return chain_segments(B, Hv, S, sm_count());
+    if (path != GDN_PATH_AUTO && !transposed_path(path)) return 1;
+    return chain_segments(static_cast<long long>(B) * Hv, S, 2 * sm_count());   // two CTAs per SM
 }
 
 size_t gdn_chunk_scratch_bytes(int B, int S, int Hq, int Hv, int path) {
@@ -185,7 +196,7 @@ int forward_device(const void* q, const void* k, const void* v, const void* g, c
     if (flags & ~static_cast<unsigned>(GDN_FLAG_QK_L2NORM | GDN_FLAG_GATE_ACTIVATIONS)) return GDN_ERR_BAD_ARGUMENT;
     if (B <= 0 || S < 0 || Hq <= 0 || Hv <= 0 || Hv % Hq != 0) return GDN_ERR_BAD_ARGUMENT;
     if (gate_dtype != GDN_GATE_BF16 && gate_dtype != GDN_GATE_F32) return GDN_ERR_BAD_ARGUMENT;
-    if (path < GDN_PATH_AUTO || path > GDN_PATH_CHAIN_ONLY_T || path == 2 || path == 3 || path == 10) return GDN_ERR_BAD_ARGUMENT;
+    if (path < GDN_PATH_AUTO || path > GDN_PATH_PREPARE_ONLY_R || path == 2 || path == 3 || path == 10) return GDN_ERR_BAD_ARGUMENT;
     // the least a path needs; gdn_chunk_scratch_bytes may ask for more (room to split long sequences), which is used
     // when it is there
     const size_t need = path_uses_workspace(path) ? workspace_layout(tiles_of(B, S, Hv)).total : 256;
@@ -204,7 +215,7 @@ int forward_device(const void* q, const void* k, const void* v, const void* g, c
     if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(out) || !aligned16(h0) || !aligned16(hT))
         return GDN_ERR_BAD_ARGUMENT;
 
-    Problem p;
+    Problem p = {};
     p.q = static_cast<const __nv_bfloat16*>(q);
     p.k = static_cast<const __nv_bfloat16*>(k);
     p.v = static_cast<const __nv_bfloat16*>(v);
@@ -248,8 +259,8 @@ int forward_device(const void* q, const void* k, const void* v, const void* g, c
     else nv = 64;
     // the transposed chain splits sequences when the scratch buffer has room for the per-tile scalars its decision
     // reads (a caller that sized it for an unsplit run, like the fixed-array entry point, gets the unsplit run)
-    const bool transposed = path == GDN_PATH_TWOPASS_T || path == GDN_PATH_PREPARE_ONLY_T || path == GDN_PATH_CHAIN_ONLY_T;
-    int n_seg = transposed ? segments_of(B, S, Hv, path) : 1;
+    const bool transposed = transposed_path(path);
+    int n_seg = segments_of(B, S, Hv, path);
     if (n_seg > 1 && scratch_bytes < workspace_layout(tiles_of(B, S, Hv), true).total) n_seg = 1;
     const WorkspaceLayout l = workspace_layout(tiles_of(B, S, Hv), n_seg > 1);
     uint8_t* base = static_cast<uint8_t*>(scratch);
@@ -270,13 +281,18 @@ int forward_device(const void* q, const void* k, const void* v, const void* g, c
         if (!(automatic && st == GDN_ERR_CUDA)) return then_gate(st);
         (void)cudaGetLastError();
         path = GDN_PATH_TWOPASS_T;
+        ws.n_seg = 1;
+    }
+    if (path == GDN_PATH_CHAIN_ONLY_T) return then_gate(launch_chain_r(p, ws, stream));
+    if (path == GDN_PATH_TWOPASS_T || path == GDN_PATH_PREPARE_ONLY_R) {
+        const int st = launch_prepare_lean(p, ws, stream);
+        if (st != GDN_OK || path == GDN_PATH_PREPARE_ONLY_R) return st;
+        return then_gate(launch_chain_r(p, ws, stream));
     }
     if (path == GDN_PATH_CHAIN_ONLY) return then_gate(launch_chain(p, ws, nv, stream));   // workspace left by an earlier call
-    if (path == GDN_PATH_CHAIN_ONLY_T) return then_gate(launch_chain_t(p, ws, stream));
     const bool pairs = transposed && (Hv / Hq) % 2 == 0 && p.dbg != 3;
     const int st = pairs ? launch_prepare_pair(p, ws, stream) : launch_prepare(p, ws, stream, !transposed);
     if (st != GDN_OK || path == GDN_PATH_PREPARE_ONLY || path == GDN_PATH_PREPARE_ONLY_T) return st;
-    if (path == GDN_PATH_TWOPASS_T) return then_gate(launch_chain_t(p, ws, stream));
     return then_gate(launch_chain(p, ws, nv, stream));
 }
 }  // namespace gdn

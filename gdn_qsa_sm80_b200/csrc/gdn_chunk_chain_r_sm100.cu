@@ -1,0 +1,586 @@
+// "chain", residual form: one CTA per (sequence, value head[, segment]) runs the serial state recurrence and the outputs
+// of all 128 value columns.  Instead of W = T (beta e^gamma K), formed per chunk by the prepare step and read back here, it
+// applies T'' = T diag(beta) to both parts of the chunk's residual V - e^gamma K S (notation of gdn_qsa_sm80/reference/gdn_chunk_ref.py:90-94;
+// v_new = U - W S = T'' V - T'' diag(e^gamma) K S), all products transposed so that what the recurrence rewrites are A
+// operands in tensor memory and every B operand is a tile as TMA loaded it:
+//   E1   KS     = S^T K^T              (A = bf16 S^T)
+//   E1'  O      = S^T Q^T              (same A)           O <- scale e^gamma_i O  (column factors, by the output warps)
+//   E0   v_new  = V^T T''^T            (A = the raw V tile, MN-major)
+//        X      = e^gamma_j KS         (column factors, bf16)
+//   ER   v_new -= X^T T''^T            (A = bf16 X^T, negated)                                              (ref :91)
+//   E2   ACC_S  = v~^T K               (A = bf16 v~^T, v~ = e^(gamma_C - gamma_i) v_new)
+//        S^T   <- e^gamma_C S^T + ACC_S                                                                    (ref :94)
+//   E3   O     += v_new^T P^T                                                                           (ref :92-93)
+// Against the form with W (this library's chain before) a chunk has one hand-off more on its critical path, but reads 16 KB
+// less and needs 256 tensor-memory columns, 100 KB of shared memory and 32 K registers, so TWO CTAs share an SM and
+// each fills the other's waits: what counts here is the time of a chunk step per SM, not its latency.
+//
+// Tensor memory of a CTA (columns; each operand is written over an accumulator that is dead by then - UMMAs of one thread
+// execute in order):
+//   0..127    ACC_S; the state epilogue packs the bf16 state over columns it has read: the warps of half h own the blocks
+//             32 h and 64 + 32 h of 32 columns and pack them into 32 h, so that A_S lies in 0..63, its k order permuted,
+//             and 64..127 are free for v_new (E0, ER) while E1 and E1' read A_S
+//   128..191  KS; X packed over it (128..143, 160..175); then v~ (128..159) and v_new (160..191) once ER has read X
+//   192..255  O
+// Order of issue: E1, E0, ER, E1', E2, E3 - E0 runs during the X epilogue and E1' during the v_new epilogue, so of the two
+// products nothing on the critical path waits for, neither delays one that is on it.
+// Shared memory: K, V and T'' in two slots, Q and P in one: every tile is used once (K twice, a few thousand cycles
+// apart), and its slot is reloaded as soon as the UMMA that read it has completed.
+//
+// Roles (16 warps): 0-7 critical (warp w: TMEM lane quadrant w % 4, column half w / 4): X, v_new and state epilogues,
+// fp32 state in registers; 8-11 output; 12 TMA producer; 13 issues every UMMA.  Registers are moved from the last two
+// groups of four warps to the first two (64 each at launch -> 88, 88, 48, 24).
+//
+// Sequences are split into segments when there are too few of them (gdn_segment_plan.cuh).
+// Stands in for the reference's gdn_recurrence_kernel (csrc/gdn_chunk/gdn_kernel.cu:1027-1271).
+#include <cuda.h>
+
+#include "../../include/gdn_chunk_sm100.h"
+#include "gdn_common.cuh"
+#include "gdn_segment_plan.cuh"
+#include "ptx_sm100.cuh"
+
+namespace gdn {
+namespace {
+
+constexpr int kRThreads = 512;
+constexpr uint32_t R_K = 0, R_V = 32768, R_Q = 65536, R_T2 = 81920, R_P = 98304, R_VEC = 106496, kRBytes = R_VEC + 2048;
+constexpr uint32_t kRDynamic = kRBytes + 1024;
+constexpr uint32_t C_S = 0, C_VN = 64, C_KS = 128, C_VS = 128, C_VP = 160, C_O = 192, kRTmemCols = 256;
+constexpr int kRTimeout = 0x500;   // + the barrier's index
+
+// barriers
+enum : uint32_t { R_KFULL = 0, R_VFULL = 2, R_VEMPTY = 4, R_TFULL = 6, R_QFULL = 8, R_PFULL, R_KS, R_QS, R_X, R_VACC, R_VN, R_S, R_STATE,
+                  R_QSC, R_O, R_ODONE, kRBars };
+
+// Byte offset, in a [64 tokens][128 dk] tile of two 64-column halves, of the 16 dk that k step `ks` of A_S holds (half ks / 4
+// of the warps packed the column blocks 32 h .. and 64 + 32 h ..).
+__device__ constexpr uint32_t dk_bytes(int ks) { return ((ks >> 1) & 1) * 8192 + (ks >> 2) * 64 + (ks & 1) * 32; }
+
+// What a CTA runs, in shared memory (the roles re-read what they need instead of holding it in registers): `steps` chunks
+// of the sequence from chunk t0 on, outputs stored from step `store_from` on.
+struct RWork {
+    int t0, steps, store_from, len;        // len: tokens of the sequence
+    int b, s_first;                        // TMA coordinates of the sequence's first token
+    size_t tok0, tile0;                    // first token and first workspace tile of the sequence and head
+    const float* s_in;                     // state it starts from (null: zeros) and where the one it ends with goes
+    float* s_out;
+    int* status;
+    int abort;
+};
+
+// Shared-memory descriptor of this file's operands: 1024 bytes between 8-row groups and the 128-byte swizzle throughout, so
+// the upper word is a constant and only the lower one (address and, MN-major, the distance of 64-column groups) varies.
+__device__ __forceinline__ uint64_t r_desc(uint32_t lo) {
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"((1024u >> 4) | (1u << 14) | (SWZ_128B << 29)));
+    return d;
+}
+constexpr uint32_t kLoK = (16u >> 4) << 16, kLoMN = (8192u >> 4) << 16;
+
+// Bounded, abortable wait (see mbar_wait_abortable_a) that holds next to nothing in registers: what only its slow path
+// needs (the status word's address, the CTA's abort flag) is read from shared memory there.
+__device__ __forceinline__ bool r_wait(uint32_t bar, uint32_t parity, int code, RWork& work) {
+#pragma unroll 1
+    for (int i = 0; i < 128; ++i)
+        if (mbar_try_wait_a(bar, parity)) return true;
+    uint32_t t0;
+    asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(t0));
+#pragma unroll 1
+    while (true) {
+#pragma unroll 1
+        for (int i = 0; i < 256; ++i)
+            if (mbar_try_wait_a(bar, parity)) return true;
+        if (*const_cast<volatile int*>(&work.abort)) return false;
+        uint32_t now;
+        asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(now));
+        if (now - t0 > static_cast<uint32_t>(WAIT_LIMIT_NS)) {
+            atomicCAS(*const_cast<int* volatile*>(&work.status), 0, code);
+            *const_cast<volatile int*>(&work.abort) = 1;
+            return false;
+        }
+    }
+}
+
+// Row stores of the output warps; opaque to the compiler, which would otherwise keep dozens of precomputed addresses.
+__device__ __forceinline__ void next_row(unsigned long long& a, unsigned long long stride) {
+    asm volatile("add.u64 %0, %0, %1;" : "+l"(a) : "l"(stride));
+}
+__device__ __forceinline__ void store_lo(unsigned long long a, uint32_t x) {
+    asm volatile("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %1;\n\tst.global.b16 [%0], lo;\n\t}" ::"l"(a), "r"(x) : "memory");
+}
+__device__ __forceinline__ void store_hi(unsigned long long a, uint32_t x) {
+    asm volatile("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %1;\n\tst.global.b16 [%0], hi;\n\t}" ::"l"(a), "r"(x) : "memory");
+}
+
+template <int N>
+__device__ __forceinline__ void set_max_registers_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void set_max_registers_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
+template <bool SPLIT>
+__global__ void __launch_bounds__(kRThreads, 2)
+gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_p,
+                   const __grid_constant__ CUtensorMap tm_t2, const __grid_constant__ Problem p,
+                   const __grid_constant__ Workspace ws) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    const uint32_t sm_u32 = warp_uniform(smem_u32(sm));
+    __shared__ __align__(8) uint64_t bars[kRBars];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int plan_best;
+    __shared__ SegmentPlan plan;
+    __shared__ RWork work;
+
+    const int tid = threadIdx.x, warp = static_cast<int>(warp_uniform(tid >> 5)), lane = tid & 31;
+    const int hv = blockIdx.x, hq = hv / (p.Hv / p.Hq);
+    const uint32_t bar0 = smem_u32(bars);
+    auto cb = [&](uint32_t i) { return bar0 + 8u * i; };
+
+    if (tid == 0) {
+        for (uint32_t i = 0; i < kRBars; ++i) {
+            const uint32_t count = i == R_VEMPTY || i == R_VEMPTY + 1 ? 12
+                                   : i == R_X || i == R_VN || i == R_STATE ? 8 : i == R_QSC || i == R_ODONE ? 4 : 1;
+            mbar_init(&bars[i], count);
+        }
+        work.abort = 0;
+        work.status = p.status;
+        fence_mbar_init();
+    }
+    if (warp == 0) {
+        tmem_alloc(&tmem_slot, kRTmemCols);
+        tmem_relinquish();
+    }
+    grid_dependency_wait();   // launched ahead of the end of the prepare kernel: nothing of the workspace is read above
+
+    if (tid == 0) {   // which sequence: its tokens, chunks and workspace tiles
+        int seq;
+        if (p.pk_chunk) {
+            const int2 o = p.pk_order[blockIdx.y];
+            seq = o.x;
+            work.b = 0;
+            work.s_first = p.pk_cu[seq];
+            work.len = p.pk_cu[seq + 1] - work.s_first;
+            work.tok0 = work.s_first;
+            work.tile0 = static_cast<size_t>(o.y) * p.Hv + static_cast<size_t>(hv) * ((work.len + kChunk - 1) / kChunk);
+        } else {
+            seq = work.b = blockIdx.y;
+            work.s_first = 0;
+            work.len = p.S;
+            work.tok0 = static_cast<size_t>(seq) * p.S;
+            work.tile0 = (static_cast<size_t>(seq) * p.Hv + hv) * ((p.S + kChunk - 1) / kChunk);
+        }
+        const size_t state_off = (static_cast<size_t>(seq) * p.Hv + hv) * kD * kD;
+        work.t0 = work.store_from = 0;
+        work.steps = (work.len + kChunk - 1) / kChunk;
+        work.s_in = p.h0 ? p.h0 + state_off : nullptr;
+        work.s_out = p.hT ? p.hT + state_off : nullptr;
+    }
+    if (SPLIT) {
+        __syncthreads();
+        const int nt = work.steps;
+        plan_segments<kRThreads>(ws.meta + 2 * work.tile0, nt, ws.n_seg, reinterpret_cast<float*>(sm), plan, &plan_best);
+        if (tid == 0) {
+            const int seg = static_cast<int>(blockIdx.z), g = plan.g;
+            if (g > 1) {
+                const int a = seg == 0 ? 0 : plan.L0 + (seg - 1) * plan.L1;
+                const int e = min(nt, seg == 0 ? plan.L0 : a + plan.L1);
+                if (seg >= g || a >= nt) {
+                    work.steps = 0;
+                } else {
+                    work.store_from = seg == 0 ? 0 : plan.warm[seg];
+                    work.t0 = a - work.store_from;
+                    work.steps = e - work.t0;
+                    if (seg > 0) work.s_in = nullptr;
+                    if (e < nt) work.s_out = nullptr;
+                }
+            } else if (seg > 0) {
+                work.steps = 0;
+            }
+        }
+        fence_proxy_async_smem();   // the prefix sums lie where the ring's loads go
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem = warp_uniform(tmem_slot);
+    const bool prof_cta = GDN_DIAG(p.prof != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0);
+    const int steps = work.steps;
+    auto wait = [&](uint32_t bar, uint32_t parity) {
+        return r_wait(cb(bar), parity & 1, kRTimeout + static_cast<int>(bar), work);
+    };
+
+    if (steps == 0) {
+    } else if (warp >= 12) {
+        set_max_registers_down<24>();
+        if (warp == 12) {
+            // ------------------------------- TMA producer ----------------------------------------------------------
+            auto load_k = [&](int n) {
+                const uint32_t s = n & 1, fb = cb(R_KFULL + s), d = sm_u32 + R_K + s * 16384;
+                const int s0 = work.s_first + (work.t0 + n) * kChunk;
+                const int b = work.b;
+                if (elect_one()) {
+                    mbar_arrive_expect_tx_a(fb, 16384);
+                    tma_load_4d_a(d, &tm_k, fb, 0, hq, s0, b);
+                    tma_load_4d_a(d + 8192, &tm_k, fb, 64, hq, s0, b);
+                }
+            };
+            auto load_v = [&](int n) {
+                const uint32_t s = n & 1, fb = cb(R_VFULL + s);
+                const int t = work.t0 + n, s0 = work.s_first + t * kChunk, b = work.b;
+                const float* vec = ws.vec + (work.tile0 + t) * 256;
+                if (elect_one()) {
+                    mbar_arrive_expect_tx_a(fb, 16384 + 1024);
+                    tma_load_4d_a(sm_u32 + R_V + s * 16384, &tm_v, fb, 0, hv, s0, b);
+                    tma_load_4d_a(sm_u32 + R_V + s * 16384 + 8192, &tm_v, fb, 64, hv, s0, b);
+                    bulk_load_1d_a(sm_u32 + R_VEC + s * 1024, vec, 1024, fb);
+                }
+            };
+            auto load_t2 = [&](int n) {
+                const uint32_t s = n & 1, fb = cb(R_TFULL + s);
+                const int row0 = static_cast<int>((work.tile0 + work.t0 + n) * kChunk);
+                if (elect_one()) {
+                    mbar_arrive_expect_tx_a(fb, 8192);
+                    tma_load_2d_a(sm_u32 + R_T2 + s * 8192, &tm_t2, fb, 0, row0);
+                }
+            };
+            load_k(0);
+            load_t2(0);
+            load_v(0);
+            // A slot's reload waits for the UMMA (or the epilogue) that read it.  The waits of one iteration are in the
+            // order in which those complete, and none of them can be overtaken by the next completion of the same
+            // barrier: that one needs a tile loaded later in the iteration.
+            for (int n = 0; n < steps; ++n) {
+                if (n + 1 < steps) {
+                    if (n > 0 && !wait(R_VEMPTY + ((n + 1) & 1), ((n + 1) >> 1) - 1)) break;
+                    load_v(n + 1);
+                }
+                if (n > 0 && !wait(R_S, n - 1)) break;          // E2, hence also ER and E1', of chunk n - 1
+                if (n + 1 < steps) {
+                    load_k(n + 1);
+                    load_t2(n + 1);
+                }
+                const int s0 = work.s_first + (work.t0 + n) * kChunk, b = work.b;
+                const int row0 = static_cast<int>((work.tile0 + work.t0 + n) * kChunk);
+                if (elect_one()) {
+                    mbar_arrive_expect_tx_a(cb(R_QFULL), 16384);
+                    tma_load_4d_a(sm_u32 + R_Q, &tm_q, cb(R_QFULL), 0, hq, s0, b);
+                    tma_load_4d_a(sm_u32 + R_Q + 8192, &tm_q, cb(R_QFULL), 64, hq, s0, b);
+                }
+                if (n > 0 && !wait(R_O, n - 1)) break;
+                if (elect_one()) {
+                    mbar_arrive_expect_tx_a(cb(R_PFULL), 8192);
+                    tma_load_2d_a(sm_u32 + R_P, &tm_p, cb(R_PFULL), 0, row0);
+                }
+            }
+        } else if (warp == 13) {
+            // ------------------------------- UMMA issuer ------------------------------------------------------------
+            constexpr uint32_t idesc_n64 = umma_idesc_bf16(128, 64, MAJOR_K, MAJOR_K);
+            constexpr uint32_t idesc_e0 = umma_idesc_bf16(128, 64, MAJOR_MN, MAJOR_K);
+            constexpr uint32_t idesc_neg = umma_idesc_bf16(128, 64, MAJOR_K, MAJOR_K, 1);   // negated A
+            constexpr uint32_t idesc_e2 = umma_idesc_bf16(128, 128, MAJOR_K, MAJOR_MN);
+            const uint32_t base = (sm_u32 & 0x3FFFFu) >> 4;   // (a cluster CTA's window address has bits above)
+            for (int n = 0; n < steps; ++n) {
+                const uint32_t s = n & 1;
+                if (!wait(R_KFULL + s, n >> 1)) break;
+                if (!wait(R_STATE, n)) break;
+                tc_fence_after_sync();
+                if (elect_one()) {
+#pragma unroll
+                    for (int ks = 0; ks < 8; ++ks)               // E1
+                        umma_bf16_ts(tmem + C_KS, tmem + C_S + ks * 8, r_desc(base + s * (16384 >> 4) + kLoK + ((R_K + dk_bytes(ks)) >> 4)), idesc_n64, ks > 0);
+                    umma_commit_a(cb(R_KS));
+                }
+                if (!wait(R_TFULL + s, n >> 1)) break;
+                if (!wait(R_VFULL + s, n >> 1)) break;
+                if (elect_one()) {
+#pragma unroll
+                    for (int ks = 0; ks < 4; ++ks)               // E0
+                        umma_bf16_ss(tmem + C_VN, r_desc(base + s * (16384 >> 4) + kLoMN + ((R_V + ks * 2048) >> 4)),
+                                     r_desc(base + s * (8192 >> 4) + kLoK + ((R_T2 + ks * 32) >> 4)), idesc_e0, ks > 0);
+                }
+                if (!wait(R_X, n)) break;
+                tc_fence_after_sync();
+                if (elect_one()) {
+#pragma unroll
+                    for (int ks = 0; ks < 4; ++ks)               // ER
+                        umma_bf16_ts(tmem + C_VN, tmem + C_KS + (ks >> 1) * 32 + (ks & 1) * 8,
+                                     r_desc(base + s * (8192 >> 4) + kLoK + ((R_T2 + ks * 32) >> 4)), idesc_neg, 1);
+                    umma_commit_a(cb(R_VACC));
+                }
+                if (!wait(R_QFULL, n)) break;
+                if (n > 0 && !wait(R_ODONE, n - 1)) break;   // chunk n - 1's outputs have been read
+                tc_fence_after_sync();
+                if (elect_one()) {
+#pragma unroll
+                    for (int ks = 0; ks < 8; ++ks)               // E1'
+                        umma_bf16_ts(tmem + C_O, tmem + C_S + ks * 8, r_desc(base + kLoK + ((R_Q + dk_bytes(ks)) >> 4)), idesc_n64, ks > 0);
+                    umma_commit_a(cb(R_QS));
+                }
+                if (!wait(R_VN, n)) break;
+                tc_fence_after_sync();
+                if (elect_one()) {
+#pragma unroll
+                    for (int ks = 0; ks < 4; ++ks)               // E2
+                        umma_bf16_ts(tmem + C_S, tmem + C_VS + ks * 8, r_desc(base + s * (16384 >> 4) + kLoMN + ((R_K + ks * 2048) >> 4)), idesc_e2, ks > 0);
+                    umma_commit_a(cb(R_S));
+                }
+                if (!wait(R_PFULL, n)) break;
+                if (!wait(R_QSC, n)) break;
+                tc_fence_after_sync();
+                if (elect_one()) {
+#pragma unroll
+                    for (int ks = 0; ks < 4; ++ks)               // E3
+                        umma_bf16_ts(tmem + C_O, tmem + C_VP + ks * 8, r_desc(base + kLoK + ((R_P + ks * 32) >> 4)), idesc_n64, 1);
+                    umma_commit_a(cb(R_O));
+                }
+            }
+        }
+    } else if (warp >= 8) {
+        // ------------------------------- output warps ----------------------------------------------------------------
+        set_max_registers_down<48>();
+        const uint32_t lane_base = static_cast<uint32_t>(warp & 3) * 32u;
+        const int dv = (warp & 3) * 32 + lane;                // the value column (= TMEM lane) this thread owns
+        const uint32_t o_addr = tmem_addr(tmem, lane_base, C_O);
+        const unsigned long long row_bytes = static_cast<unsigned long long>(p.Hv) * kD * 2;
+        unsigned long long dst = reinterpret_cast<unsigned long long>(p.out) + ((work.tok0 + static_cast<size_t>(work.t0) * kChunk) * p.Hv + hv) * (kD * 2) + dv * 2;
+        for (int n = 0; n < steps; ++n) {
+            const uint32_t s = n & 1;
+            if (!wait(R_VFULL + s, n >> 1)) break;            // the factors
+            if (!wait(R_QS, n)) break;
+            tc_fence_after_sync();
+            const float* qf = reinterpret_cast<const float*>(sm + R_VEC + s * 1024) + kChunk;   // scale e^gamma_j
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                uint32_t x[8];
+                tmem_ld_x8(o_addr + 8 * u, x);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 8; j += 4) {
+                    const float4 f = *reinterpret_cast<const float4*>(qf + 8 * u + j);
+                    x[j] = __float_as_uint(__uint_as_float(x[j]) * f.x);
+                    x[j + 1] = __float_as_uint(__uint_as_float(x[j + 1]) * f.y);
+                    x[j + 2] = __float_as_uint(__uint_as_float(x[j + 2]) * f.z);
+                    x[j + 3] = __float_as_uint(__uint_as_float(x[j + 3]) * f.w);
+                }
+                tmem_st_x8(o_addr + 8 * u, x);
+            }
+            tmem_st_wait();
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive_a(cb(R_QSC));
+                mbar_arrive_a(cb(R_VEMPTY + s));
+            }
+            if (!wait(R_O, n)) break;
+            tc_fence_after_sync();
+            // O^T[dv][j]: a warp stores 64 contiguous bytes of row j; warm-up chunks store nothing
+            const int valid = n >= work.store_from ? min(kChunk, work.len - (work.t0 + n) * kChunk) : 0;
+#pragma unroll
+            for (int h2 = 0; h2 < 2; ++h2) {                  // 32 tokens at a time through packed registers
+                uint32_t pk[16];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    uint32_t x[8];
+                    tmem_ld_x8(o_addr + 32 * h2 + 8 * u, x);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) pk[4 * u + c] = pack_bf16x2(__uint_as_float(x[2 * c]), __uint_as_float(x[2 * c + 1]));
+                }
+                if (h2 == 1) {                                // the accumulator has been read
+                    tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_a(cb(R_ODONE));
+                }
+                if (valid == kChunk) {
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) {
+                        store_lo(dst, pk[c]);
+                        next_row(dst, row_bytes);
+                        store_hi(dst, pk[c]);
+                        next_row(dst, row_bytes);
+                    }
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) {
+                        if (32 * h2 + 2 * c < valid) store_lo(dst, pk[c]);
+                        next_row(dst, row_bytes);
+                        if (32 * h2 + 2 * c + 1 < valid) store_hi(dst, pk[c]);
+                        next_row(dst, row_bytes);
+                    }
+                }
+            }
+        }
+    } else {
+        // ------------------------------- critical warps ----------------------------------------------------------------
+        set_max_registers_up<88>();
+        const uint32_t lane_base = static_cast<uint32_t>(warp & 3) * 32u;
+        const int dv = (warp & 3) * 32 + lane;
+        const int hf = warp >> 2;                             // which half of the columns of each accumulator
+        const uint32_t a_s = tmem_addr(tmem, lane_base, C_S + 32 * hf);
+        const uint32_t a_ks = tmem_addr(tmem, lane_base, C_KS + 32 * hf);
+        float st[64];                                         // S^T[dv][dk], dk = 32 hf + c (c < 32), 64 + 32 hf + c - 32
+        const float* s_in = work.s_in ? work.s_in + 32 * hf * kD + dv : nullptr;
+#pragma unroll
+        for (int c = 0; c < 64; ++c) st[c] = s_in ? s_in[(c + (c & 32)) * kD] : 0.f;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            uint32_t pk[8];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) pk[c] = pack_bf16x2(st[16 * u + 2 * c], st[16 * u + 2 * c + 1]);
+            tmem_st_x8(a_s + 8 * u, pk);
+        }
+        // The last tiles of a packed sequence hold the next sequence's first tokens below its own: beta and the gates are
+        // zero there, but what the tiles hold (an infinity) must not reach this sequence, so those rows of K and V are
+        // cleared before the step's first product.
+        auto clear_tail = [&](int n) {
+            const int valid = work.len - (work.t0 + n) * kChunk;
+            if (!p.pk_chunk || valid >= kChunk) return;
+            if (!wait(R_KFULL + (n & 1), n >> 1) || !wait(R_VFULL + (n & 1), n >> 1)) return;
+            uint8_t* tile = sm + (n & 1) * 16384;
+            for (int e = tid; e < (kChunk - valid) * 16; e += 256) {
+                const uint32_t off = ((e >> 3) & 1) * 8192 + (valid + (e >> 4)) * 128 + (e & 7) * 16;
+                *reinterpret_cast<uint4*>(tile + R_K + off) = make_uint4(0, 0, 0, 0);
+                *reinterpret_cast<uint4*>(tile + R_V + off) = make_uint4(0, 0, 0, 0);
+            }
+            fence_proxy_async_smem();
+        };
+        if (steps == 1) clear_tail(0);
+        tmem_st_wait();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_a(cb(R_STATE));
+        bool ok = true;
+        for (int n = 0; n < steps; ++n) {
+            const uint32_t s = n & 1;
+            ok = wait(R_VFULL + s, n >> 1) && wait(R_KS, n);
+            if (!ok) break;
+            tc_fence_after_sync();
+            const float* vec = reinterpret_cast<const float*>(sm + R_VEC + s * 1024);
+            const float dC = vec[2 * kChunk];                 // exp(gamma_C); read now, the slot is released below
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {                     // X of tokens [32 hf + 8 u, +8)
+                uint32_t x[8], pk[4];
+                tmem_ld_x8(a_ks + 8 * u, x);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 8; j += 4) {
+                    const float4 f = *reinterpret_cast<const float4*>(vec + 3 * kChunk + 32 * hf + 8 * u + j);
+                    pk[j / 2] = pack_bf16x2(__uint_as_float(x[j]) * f.x, __uint_as_float(x[j + 1]) * f.y);
+                    pk[j / 2 + 1] = pack_bf16x2(__uint_as_float(x[j + 2]) * f.z, __uint_as_float(x[j + 3]) * f.w);
+                }
+                tmem_st_x4(a_ks + 4 * u, pk);
+            }
+            tmem_st_wait();
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_a(cb(R_X));
+            ok = wait(R_VACC, n);
+            if (!ok) break;
+            tc_fence_after_sync();
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {                     // v_new and v~ of tokens [32 hf + 8 u, +8)
+                uint32_t x[8], pk[4];
+                tmem_ld_x8(tmem_addr(tmem, lane_base, C_VN + 32 * hf + 8 * u), x);
+                tmem_ld_wait();
+#pragma unroll
+                for (int c = 0; c < 4; ++c) pk[c] = pack_bf16x2(__uint_as_float(x[2 * c]), __uint_as_float(x[2 * c + 1]));
+                tmem_st_x4(tmem_addr(tmem, lane_base, C_VP + 16 * hf + 4 * u), pk);
+#pragma unroll
+                for (int c = 0; c < 4; c += 2) {
+                    const float4 f = *reinterpret_cast<const float4*>(vec + 32 * hf + 8 * u + 2 * c);   // exp(gamma_C - gamma_j)
+                    pk[c] = pack_bf16x2(__uint_as_float(x[2 * c]) * f.x, __uint_as_float(x[2 * c + 1]) * f.y);
+                    pk[c + 1] = pack_bf16x2(__uint_as_float(x[2 * c + 2]) * f.z, __uint_as_float(x[2 * c + 3]) * f.w);
+                }
+                tmem_st_x4(tmem_addr(tmem, lane_base, C_VS + 16 * hf + 4 * u), pk);
+            }
+            tmem_st_wait();
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive_a(cb(R_VN));
+                mbar_arrive_a(cb(R_VEMPTY + s));
+            }
+            ok = wait(R_S, n);
+            if (!ok) break;
+            tc_fence_after_sync();
+            const bool more = n + 1 < steps;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {                     // S^T <- exp(gamma_C) S^T + v~^T K, 16 columns at a time
+                uint32_t x[16];
+                tmem_ld_x16(a_s + (u >> 1) * 64 + (u & 1) * 16, x);
+                tmem_ld_wait();
+#pragma unroll
+                for (int c = 0; c < 16; ++c) st[16 * u + c] = fmaf(dC, st[16 * u + c], __uint_as_float(x[c]));
+                if (more) {
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) x[c] = pack_bf16x2(st[16 * u + 2 * c], st[16 * u + 2 * c + 1]);
+                    tmem_st_x8(a_s + 8 * u, reinterpret_cast<const uint32_t (&)[8]>(x));
+                }
+            }
+            if (more) {
+                if (n + 2 == steps) clear_tail(n + 1);
+                tmem_st_wait();
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_a(cb(R_STATE));
+            }
+        }
+        if (ok && work.s_out) {
+            float* s_out = work.s_out + 32 * hf * kD + dv;
+#pragma unroll
+            for (int c = 0; c < 64; ++c) s_out[(c + (c & 32)) * kD] = st[c];
+        }
+    }
+
+    tc_fence_before_sync();
+    __syncthreads();
+    if (work.abort) {   // let copies that may still be in flight land before the CTA's memory is released
+        const unsigned long long w0 = globaltimer_ns();
+        while (globaltimer_ns() - w0 < 100000ull) {}
+        __syncthreads();
+    }
+    if (warp == 0) tmem_dealloc(tmem, kRTmemCols);
+    (void)prof_cta;
+}
+
+}  // namespace
+
+int launch_chain_r(const Problem& p, const Workspace& ws, cudaStream_t stream) {
+    alignas(64) CUtensorMap tq, tk, tv, tp, tt2;
+    if (encode_qkv_maps(p, &tq, &tk, &tv, 64)) return GDN_ERR_DRIVER;
+    if (encode_tile_maps(p, ws, &tp, &tt2)) return GDN_ERR_DRIVER;
+    auto go = [&](auto kernel, unsigned gz) -> int {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRDynamic) != cudaSuccess) return GDN_ERR_CUDA;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(p.Hv, p.pk_chunk ? p.pk_n : p.B, gz);
+        cfg.blockDim = dim3(kRThreads);
+        cfg.dynamicSmemBytes = kRDynamic;
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // CTAs set up while the prepare kernel drains
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        // The value heads that share a qk head read the same K and Q tiles: as a cluster of two CTAs they start together
+        // and run in step, so the second read of a tile finds it in L2 (nothing else of the cluster is used).
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = 2;
+        attr[1].val.clusterDim.y = 1;
+        attr[1].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = (p.Hv / p.Hq) % 2 == 0 ? 2 : 1;
+        cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tq, tk, tv, tp, tt2, p, ws);
+        if (e != cudaSuccess) {             // a context without dependent launches or clusters: an ordinary one (the kernel's wait is a no-op then)
+            (void)cudaGetLastError();
+            cfg.numAttrs = 0;
+            e = cudaLaunchKernelEx(&cfg, kernel, tq, tk, tv, tp, tt2, p, ws);
+        }
+        count_launch();
+        return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? GDN_OK : GDN_ERR_CUDA;
+    };
+    const int G = ws.n_seg;
+    if (G <= 1 || G > kMaxSegments || !ws.meta) return go(gdn_chain_r_kernel<false>, 1);
+    return go(gdn_chain_r_kernel<true>, static_cast<unsigned>(G));
+}
+
+}  // namespace gdn

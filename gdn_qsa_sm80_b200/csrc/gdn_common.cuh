@@ -37,6 +37,11 @@ struct Problem {
     int gate_act;          // 1: g and beta hold raw values; the kernels apply g = -softplus(.), beta = sigmoid(.)
     int l2norm;            // 1: q and k are L2-normalised per head vector inside the kernels
     int dbg;               // experiment switch (environment variable GDN_CHUNK_DBG); 0 in production
+    // Packed batch (residual-form kernels only; null / 0 otherwise): B = 1, S = all tokens, sequences laid end to end
+    const int* pk_cu;      // [pk_n + 1] first token of each sequence
+    const int2* pk_chunk;  // [pk_chunks] (sequence, chunk within it), sequences in order
+    const int2* pk_order;  // [pk_n] (sequence, its first entry in pk_chunk), longest sequence first
+    int pk_n, pk_chunks;
 };
 
 // Workspace of the two-kernel path (device pointers into the caller's scratch buffer).
@@ -45,7 +50,7 @@ struct Workspace {
     __nv_bfloat16* W;   // [tiles][64][128]  W = T (beta e^gamma K)
     __nv_bfloat16* P;   // [tiles][64][64]   masked, scaled Q K^T
     __nv_bfloat16* U;   // [tiles][64][128]  U = T (beta V); the transposed chain's T'' = T diag(beta), [tiles][64][64], instead
-    float* vec;         // [tiles][256]      exp(gamma_C-gamma_i) | scale exp(gamma_i) | exp(gamma_C) | pad
+    float* vec;         // [tiles][256]      exp(gamma_C-gamma_i) | scale exp(gamma_i) | exp(gamma_C), pad | exp(gamma_i)
     float* meta;        // [tiles][2]        sum of g over the chunk | max_j beta_j |k_j|^2 (+inf if a gate is out of range);
                         //                   null when sequences are not split
     int n_seg;          // segments a sequence is split into by the transposed chain (1 = not split)
@@ -68,16 +73,16 @@ inline WorkspaceLayout workspace_layout(size_t tiles, bool with_meta = false) {
     l.total = l.meta + (with_meta ? (tiles * 8 + 1023) / 1024 * 1024 : 0);
     return l;
 }
-// Into how many contiguous segments the transposed chain splits every sequence (1 = not at all): only when there are
-// too few sequences to fill the GPU, segments of at least 16 chunks, at most 8 of them.  A function of the shape and
-// of the SM count alone.
-inline int chain_segments(int B, int Hv, int S, int sms) {
-    const long long seqs = static_cast<long long>(B) * Hv;
+// The most segments the transposed chains may cut every sequence into (1 = not at all; how many a head uses is decided on
+// the device, gdn_segment_plan.cuh): as many CTAs as the GPU holds at once, segments of at least four chunks on average.
+// `slots`: CTAs the GPU holds at once.  A function of the shape and of the SM count alone.
+constexpr int kMaxSegments = 15;
+inline int chain_segments(long long seqs, int S, int slots) {
     const int NT = (S + kChunk - 1) / kChunk;
-    if (seqs * 2 > sms) return 1;
-    int g = static_cast<int>(sms / seqs);
-    if (g > 8) g = 8;
-    if (g > NT / 16) g = NT / 16;
+    if (seqs * 2 > slots || NT > 24000) return 1;    // (the prefix sums of a head have to fit the ring's shared memory)
+    int g = static_cast<int>(slots / seqs);
+    if (g > kMaxSegments) g = kMaxSegments;
+    if (g > NT / 4) g = NT / 4;
     return g < 2 ? 1 : g;
 }
 constexpr float kForgetLn = -115.f;   // exp(-115) < 2^-149: a transfer matrix bounded by it is zero in fp32
@@ -100,11 +105,11 @@ int launch_prepare(const Problem& p, const Workspace& ws, cudaStream_t stream, b
 // products, one product for both W); needs an even number of value heads per qk head.
 int launch_prepare_pair(const Problem& p, const Workspace& ws, cudaStream_t stream);
 int launch_chain(const Problem& p, const Workspace& ws, int nv, cudaStream_t stream);
-// The chain in transposed form: one CTA per (batch, value head), all 128 value columns (gdn_chain_t_device.cuh).
-// With ws.n_seg > 1 every sequence is cut into ws.n_seg segments that run as independent chains of one launch, each
-// warmed up from a zero state over the chunks before it that make the state forget its past - for the heads whose
-// gates allow that (decided on the device from ws.meta); the other heads run as one serial chain.  Exact in both cases.
-int launch_chain_t(const Problem& p, const Workspace& ws, cudaStream_t stream);
+// The two kernels of the automatic path: "lean" prepare (P, T'', factors; no W) and the transposed chain that applies T'' to
+// the residual V - exp(gamma) K S, one CTA per (sequence, value head[, segment]); with ws.n_seg > 1 sequences may be cut
+// into up to that many segments (gdn_segment_plan.cuh).
+int launch_prepare_lean(const Problem& p, const Workspace& ws, cudaStream_t stream);
+int launch_chain_r(const Problem& p, const Workspace& ws, cudaStream_t stream);
 // Single-launch variant (prepare shared among the four column CTAs of a head, chain in the same kernel);
 // only when all CTAs fit on the GPU at once.
 bool coop_supported(const Problem& p);
@@ -125,6 +130,8 @@ inline int encode_tma_bf16(void* tmap_out, const void* base, int rank, const uns
 // stores and the chain side loads for W and P), and U as nv x 64 boxes (swizzle span 2*nv bytes) for the chain's
 // column slice.  tu_load may be null.
 int encode_workspace_maps(const Problem& p, const Workspace& ws, void* tw, void* tp, void* tu_store, void* tu_load, int nv);
+// TMA descriptors of P and T'' (at the start of the U array) as 64x64 bf16 boxes.
+int encode_tile_maps(const Problem& p, const Workspace& ws, void* tp, void* tt2);
 // Number of SMs of the current device (cached per device).
 cudaError_t launch_decode(const Problem& p, cudaStream_t stream);
 int sm_count();

@@ -74,7 +74,8 @@ __device__ __forceinline__ void prep_activate_gates(float& gv, float& bv) {
 // Gate cumsum over the chunk by warp shuffles (threads 0-63 hold one token each: gv, bv) and the decay tables.
 // Contains two barriers of the group; a third one is needed before the tables are read.
 // If vec_out != nullptr, also writes the per-token factors a later kernel needs:
-//   vec_out[i] = exp(gamma_C - gamma_i), vec_out[64+i] = scale * exp(gamma_i), vec_out[128] = exp(gamma_C).
+//   vec_out[i] = exp(gamma_C - gamma_i), vec_out[64+i] = scale * exp(gamma_i), vec_out[128] = exp(gamma_C),
+//   vec_out[192+i] = exp(gamma_i).
 // tables = false skips the block decay tables (ctab) for callers whose mask epilogue does not use them.
 __device__ __forceinline__ void prep_gates(PrepScratch& ps, float gv, float bv, float scale, float* vec_out,
                                            PrepCtx ctx = PrepCtx::whole_cta(), bool tables = true) {
@@ -103,6 +104,7 @@ __device__ __forceinline__ void prep_gates(PrepScratch& ps, float gv, float bv, 
         if (vec_out) {
             vec_out[tid] = exp2f(gC - gi);
             vec_out[kChunk + tid] = scale * e;
+            vec_out[3 * kChunk + tid] = e;
             if (tid == 0) vec_out[2 * kChunk] = exp2f(gC);
         }
     }
@@ -172,6 +174,7 @@ __device__ __forceinline__ void prep_l2norm_fold(PrepScratch& ps, const uint8_t*
         if (vec_out) {
             vec_out[tid] *= ps.rn[tid];
             vec_out[kChunk + tid] *= ps.rn[kChunk + tid];
+            vec_out[3 * kChunk + tid] *= ps.rn[tid];
         }
     }
     if (tid < 96) {
