@@ -11,6 +11,7 @@ import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "lib", "libgdn_chunk_sm100.so")
+FRONTEND_PATH = os.path.join(_HERE, "lib", "_gdn_frontend.so")
 
 GDN_OK = 0
 GDN_ERR_BAD_ARGUMENT = 1
@@ -114,6 +115,27 @@ def load() -> ctypes.CDLL:
     lib.gdn_umma_probe.restype = ci
     _lib = lib
     return lib
+
+
+_frontend = None
+
+
+def frontend():
+    """The native front end (csrc/gdn_frontend.cpp), loaded once; raises if it has not been built."""
+    global _frontend
+    if _frontend is None:
+        load()
+        if not os.path.exists(FRONTEND_PATH):
+            raise GdnLibraryError(f"{FRONTEND_PATH} is missing: build it with `python -m gdn_qsa_sm80_b200.build`")
+        import importlib.machinery
+        import importlib.util
+
+        import torch  # noqa: F401  (the extension links its libraries)
+        loader = importlib.machinery.ExtensionFileLoader("_gdn_frontend", FRONTEND_PATH)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_gdn_frontend", loader))
+        loader.exec_module(module)
+        _frontend = module
+    return _frontend
 
 
 def error_string(status: int) -> str:

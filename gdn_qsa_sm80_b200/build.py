@@ -3,7 +3,8 @@
     python -m gdn_qsa_sm80_b200.build [--force] [--verbose]
 
 Compiles every ``csrc/*.cu`` with nvcc (``-gencode arch=compute_100a,code=sm_100a -lineinfo``)
-and links ``lib/libgdn_chunk_sm100.so`` next to this file.  nvcc cross-compiles, so no GPU is
+and links ``lib/libgdn_chunk_sm100.so`` next to this file, and the native front end of the Python
+wrapper (``csrc/gdn_frontend.cpp``, a CPython extension) as ``lib/_gdn_frontend.so`` beside it.  nvcc cross-compiles, so no GPU is
 needed to build.  There is no other architecture, no JIT cache and no fallback target.
 """
 
@@ -20,6 +21,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libgdn_chunk_sm100.so")
+FRONTEND_PATH = os.path.join(LIB_DIR, "_gdn_frontend.so")
 OBJ_DIR = os.path.join(HERE, "build")
 
 NVCC_FLAGS = [
@@ -49,7 +51,24 @@ def _deps_mtime() -> float:
 
 
 def needs_build() -> bool:
-    return (not os.path.exists(LIB_PATH)) or os.path.getmtime(LIB_PATH) < _deps_mtime()
+    return any(not os.path.exists(p) or os.path.getmtime(p) < _deps_mtime() for p in (LIB_PATH, FRONTEND_PATH))
+
+
+def _build_frontend() -> None:
+    import sysconfig
+    import torch
+    torch_dir = os.path.dirname(torch.__file__)
+    torch_lib = os.path.join(torch_dir, "lib")
+    include = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
+               sysconfig.get_paths()["include"], os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *[f"-I{d}" for d in include], os.path.join(CSRC, "gdn_frontend.cpp"), "-o", FRONTEND_PATH,
+           f"-L{LIB_DIR}", "-lgdn_chunk_sm100", f"-L{torch_lib}", "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_cuda",
+           "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError("g++ failed on gdn_frontend.cpp")
 
 
 def build(force: bool = False, verbose: bool = False, diagnostics: bool | None = None) -> str:
@@ -86,6 +105,7 @@ def build(force: bool = False, verbose: bool = False, diagnostics: bool | None =
     if r.returncode != 0:
         sys.stderr.write(r.stdout + r.stderr)
         raise RuntimeError("link failed")
+    _build_frontend()
     return LIB_PATH
 
 

@@ -89,7 +89,22 @@ def _scratch_for(device, nbytes):
     if buf is None or buf.numel() < nbytes:
         buf = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
         _scratch[key] = buf
+        _lib.frontend().note_scratch(*key, buf)
     return buf
+
+
+_native_forward = None
+
+
+def _native():
+    """The front end's forward(): the plain call (CUDA tensors of the current device, contiguous, in the kernels' dtypes)
+    without this module's interpreter time; it returns None for everything else, which then takes _forward()."""
+    global _native_forward
+    if _native_forward is None:
+        front = _lib.frontend()
+        front.set_grow_scratch(lambda index, nbytes: _scratch_for(torch.device("cuda", index), nbytes))
+        _native_forward = front.forward
+    return _native_forward
 
 
 def _flags(l2norm, gate_act):
@@ -187,6 +202,10 @@ def gdn_chunk(q, k, v, g, beta, output_final_state=True, initial_state=None, pat
     Returns:
         out [B, S, Hv, D] bf16, and final_state [B, Hv, D, D] fp32 (None when not requested).
     """
+    done = (_native_forward or _native())(q, k, v, g, beta, output_final_state, initial_state, _lib.PATHS[path],
+                                          _flags(use_qk_l2norm_in_kernel, gate_activations), output_gate)
+    if done is not None:
+        return done
     return _forward(q, k, v, g, beta, output_final_state, initial_state, path, bool(use_qk_l2norm_in_kernel),
                     bool(gate_activations), output_gate)
 
