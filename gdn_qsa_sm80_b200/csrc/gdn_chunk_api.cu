@@ -9,6 +9,7 @@
 
 #include "../../include/gdn_chunk_sm100.h"
 #include "gdn_common.cuh"
+#include "gdn_launch.cuh"
 
 namespace gdn {
 
@@ -114,6 +115,23 @@ int sm_count() {
     return cached[dev];
 }
 
+int allow_smem(const void* kernel, size_t bytes) {
+    struct Set { const void* kernel; int dev; size_t bytes; };
+    static Set set[64];
+    static int n = 0;
+    static std::mutex mutex;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 1;
+    std::lock_guard<std::mutex> lock(mutex);
+    int i = 0;
+    while (i < n && (set[i].kernel != kernel || set[i].dev != dev)) ++i;
+    if (i < n && set[i].bytes >= bytes) return 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)) != cudaSuccess) return 1;
+    if (i == n && n < 64) set[n++] = Set{kernel, dev, 0};
+    if (i < n) set[i].bytes = bytes;
+    return 0;
+}
+
 static long long* g_phase_profile = nullptr;
 constexpr int kDecodeMaxTokens = 8;   // sequences this short take the decode kernel under GDN_PATH_AUTO
 
@@ -201,8 +219,12 @@ int forward_device(const void* q, const void* k, const void* v, const void* g, c
     // when it is there
     const size_t need = path_uses_workspace(path) ? workspace_layout(tiles_of(B, S, Hv)).total : 256;
     if (!scratch || (reinterpret_cast<uintptr_t>(scratch) & 255u) || scratch_bytes < need) return GDN_ERR_SCRATCH;
-    if (clear_status && cudaMemsetAsync(scratch, 0, 256, stream) != cudaSuccess) return GDN_ERR_CUDA;
+    // the decode and lean prepare kernels clear the status word themselves (a memset costs a launch); its first writer could
+    // come two seconds later, when a bounded wait runs out
+    const bool decode = path == GDN_PATH_DECODE || (path == GDN_PATH_AUTO && S <= kDecodeMaxTokens);
+    auto clear = [&]() { return !clear_status || cudaMemsetAsync(scratch, 0, 256, stream) == cudaSuccess; };
     if (S == 0) {   // nothing to scan: the final state is the initial state
+        if (!clear()) return GDN_ERR_CUDA;
         if (hT) {
             const size_t bytes = static_cast<size_t>(B) * Hv * kD * kD * sizeof(float);
             const cudaError_t e = h0 ? cudaMemcpyAsync(hT, h0, bytes, cudaMemcpyDeviceToDevice, stream)
@@ -226,6 +248,7 @@ int forward_device(const void* q, const void* k, const void* v, const void* g, c
     p.hT = hT;
     p.status = static_cast<int*>(scratch);
     p.prof = g_phase_profile;
+    p.clear_status = clear_status;
     p.B = B; p.S = S; p.Hq = Hq; p.Hv = Hv;
     p.gate_f32 = gate_dtype == GDN_GATE_F32;
     p.l2norm = (flags & GDN_FLAG_QK_L2NORM) ? 1 : 0;
@@ -244,8 +267,8 @@ int forward_device(const void* q, const void* k, const void* v, const void* g, c
 
     // a few new tokens: the state read and write is all there is, and the decode kernel streams it (measured on
     // 2048 states: 55 us at one token = 4.8 TB/s, against 238 us through the chunk kernels; the two meet near 16 tokens)
-    if (path == GDN_PATH_DECODE || (path == GDN_PATH_AUTO && S <= kDecodeMaxTokens))
-        return then_gate(launch_decode(p, stream) == cudaSuccess ? GDN_OK : GDN_ERR_CUDA);
+    if (decode) return launch_decode(p, gate, stream);
+    if (path == GDN_PATH_SIMT && !clear()) return GDN_ERR_CUDA;
     if (path == GDN_PATH_SIMT) return then_gate(launch_simt(p, stream) == cudaSuccess ? GDN_OK : GDN_ERR_CUDA);
     // Automatic choice, by shape alone.  Few short sequences (up to 1024 tokens): the single-launch kernel whose four
     // 32-column CTAs per head share the prepare work.  Everything else: the prepare kernel and the transposed chain
@@ -271,6 +294,7 @@ int forward_device(const void* q, const void* k, const void* v, const void* g, c
     ws.vec = reinterpret_cast<float*>(base + l.vec);
     ws.meta = n_seg > 1 ? reinterpret_cast<float*>(base + l.meta) : nullptr;
     ws.n_seg = n_seg;
+    if (path != GDN_PATH_TWOPASS_T && path != GDN_PATH_PREPARE_ONLY_R && !clear()) return GDN_ERR_CUDA;
     if (path == GDN_PATH_COOP_CHAIN_ONLY)
         return then_gate(launch_coop(p, ws, reinterpret_cast<int*>(base + l.flags), l.flag_bytes, stream, true));
     if (path == GDN_PATH_COOP) {

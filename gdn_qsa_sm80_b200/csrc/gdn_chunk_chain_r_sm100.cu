@@ -37,6 +37,7 @@
 
 #include "../../include/gdn_chunk_sm100.h"
 #include "gdn_common.cuh"
+#include "gdn_launch.cuh"
 #include "gdn_segment_plan.cuh"
 #include "ptx_sm100.cuh"
 
@@ -552,31 +553,12 @@ int launch_chain_r(const Problem& p, const Workspace& ws, cudaStream_t stream) {
     if (encode_qkv_maps(p, &tq, &tk, &tv, 64)) return GDN_ERR_DRIVER;
     if (encode_tile_maps(p, ws, &tp, &tt2)) return GDN_ERR_DRIVER;
     auto go = [&](auto kernel, unsigned gz) -> int {
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRDynamic) != cudaSuccess) return GDN_ERR_CUDA;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(p.Hv, p.pk_chunk ? p.pk_n : p.B, gz);
-        cfg.blockDim = dim3(kRThreads);
-        cfg.dynamicSmemBytes = kRDynamic;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[2];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // CTAs set up while the prepare kernel drains
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        if (allow_smem(reinterpret_cast<const void*>(kernel), kRDynamic)) return GDN_ERR_CUDA;
         // The value heads that share a qk head read the same K and Q tiles: as a cluster of two CTAs they start together
         // and run in step, so the second read of a tile finds it in L2 (nothing else of the cluster is used).
-        attr[1].id = cudaLaunchAttributeClusterDimension;
-        attr[1].val.clusterDim.x = 2;
-        attr[1].val.clusterDim.y = 1;
-        attr[1].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = (p.Hv / p.Hq) % 2 == 0 ? 2 : 1;
-        cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tq, tk, tv, tp, tt2, p, ws);
-        if (e != cudaSuccess) {             // a context without dependent launches or clusters: an ordinary one (the kernel's wait is a no-op then)
-            (void)cudaGetLastError();
-            cfg.numAttrs = 0;
-            e = cudaLaunchKernelEx(&cfg, kernel, tq, tk, tv, tp, tt2, p, ws);
-        }
-        count_launch();
-        return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? GDN_OK : GDN_ERR_CUDA;
+        const cudaError_t e = launch_dependent(kernel, dim3(p.Hv, p.pk_chunk ? p.pk_n : p.B, gz), dim3(kRThreads), kRDynamic, stream,
+                                               (p.Hv / p.Hq) % 2 == 0, tq, tk, tv, tp, tt2, p, ws);
+        return e == cudaSuccess ? GDN_OK : GDN_ERR_CUDA;
     };
     const int G = ws.n_seg;
     if (G <= 1 || G > kMaxSegments || !ws.meta) return go(gdn_chain_r_kernel<false>, 1);

@@ -19,6 +19,7 @@
 
 #include "../../include/gdn_chunk_sm100.h"
 #include "gdn_common.cuh"
+#include "gdn_launch.cuh"
 #include "gdn_prep_lean_device.cuh"
 #include "ptx_sm100.cuh"
 
@@ -128,19 +129,23 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         prof_t = now_;                                 \
     }
 
-    unsigned n = blockIdx.x;
-    Item cur = decode(n);
     if (tid == 0) {
         mbar_init(&bar_tma, 1);
         mbar_init(&bar_mma, 1);
         fence_mbar_init();
-        load_k(cur);
-        load_q_half(cur, 0);
-        load_q_half(cur, 1);
     }
     if (warp == 0) {
         tmem_alloc(&tmem_slot, kLeanTmemCols);
         tmem_relinquish();
+    }
+    grid_dependency_wait();   // launched ahead of the end of the kernel before: no memory is touched above
+    unsigned n = blockIdx.x;
+    Item cur = decode(n);
+    if (tid == 0) {
+        if (p.clear_status && n == 0) *p.status = 0;
+        load_k(cur);
+        load_q_half(cur, 0);
+        load_q_half(cur, 1);
     }
     LaneGates gates{0.f, 0.f, 0.f, 0.f};
     if (hwarp == 0) gates = lean_load_gates<GATE_F32>(p, cur.tok0, cur.hv, cur.valid, lane);
@@ -265,10 +270,10 @@ int launch_prepare_lean(const Problem& p, const Workspace& ws, cudaStream_t stre
         if (items >= (1ll << 31)) return GDN_ERR_BAD_ARGUMENT;
         const long long max_ctas = static_cast<long long>(per_sm) * sm_count();
         const unsigned grid = static_cast<unsigned>(items < max_ctas ? items : max_ctas);
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return GDN_ERR_CUDA;
-        kernel<<<grid, 128 * heads, smem, stream>>>(tq, tk, tp, tt2, p, ws, static_cast<unsigned>(NT), static_cast<unsigned>(items));
-        count_launch();
-        return cudaGetLastError() == cudaSuccess ? GDN_OK : GDN_ERR_CUDA;
+        if (allow_smem(reinterpret_cast<const void*>(kernel), smem)) return GDN_ERR_CUDA;
+        const cudaError_t e = launch_dependent(kernel, dim3(grid), dim3(128 * heads), smem, stream, false, tq, tk, tp, tt2, p, ws,
+                                               static_cast<unsigned>(NT), static_cast<unsigned>(items));
+        return e == cudaSuccess ? GDN_OK : GDN_ERR_CUDA;
     };
     if ((p.Hv / p.Hq) % 2 == 0) {
         return p.gate_f32 ? go(gdn_prepare_lean_kernel<2, true>, 2, LeanSmem<2>::kDynamic, kLeanCtasPerSm<2>)

@@ -36,6 +36,7 @@ struct Problem {
     int gate_f32;          // 0: g/beta are bf16, 1: fp32
     int gate_act;          // 1: g and beta hold raw values; the kernels apply g = -softplus(.), beta = sigmoid(.)
     int l2norm;            // 1: q and k are L2-normalised per head vector inside the kernels
+    int clear_status;      // 1: the launch's first kernel clears the status word
     int dbg;               // experiment switch (environment variable GDN_CHUNK_DBG); 0 in production
     // Packed batch (residual-form kernels only; null / 0 otherwise): B = 1, S = all tokens, sequences laid end to end
     const int* pk_cu;      // [pk_n + 1] first token of each sequence
@@ -133,7 +134,6 @@ int encode_workspace_maps(const Problem& p, const Workspace& ws, void* tw, void*
 // TMA descriptors of P and T'' (at the start of the U array) as 64x64 bf16 boxes.
 int encode_tile_maps(const Problem& p, const Workspace& ws, void* tp, void* tt2);
 // Number of SMs of the current device (cached per device).
-cudaError_t launch_decode(const Problem& p, cudaStream_t stream);
 int sm_count();
 cudaError_t launch_rmsnorm_gated(const void* y, const void* z, const void* weight, void* out, long long n_rows,
                                  float eps, cudaStream_t stream);
@@ -146,6 +146,8 @@ struct OutputGate {
     const void* weight;
     float eps;
 };
+// Token-by-token kernel for a few new tokens on stored states; og: gated normalisation of its rows in the same launch.
+int launch_decode(const Problem& p, const OutputGate* og, cudaStream_t stream);
 int forward_device(const void* q, const void* k, const void* v, const void* g, const void* beta, const float* h0,
                    void* out, float* hT, void* scratch, size_t scratch_bytes, int B, int S, int Hq, int Hv,
                    int gate_dtype, int path, unsigned flags, cudaStream_t stream, bool clear_status,

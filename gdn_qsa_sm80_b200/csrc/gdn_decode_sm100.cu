@@ -2,130 +2,295 @@
 // of a stored state).  Same recurrence as the reference's recurrent torch definition
 // (gdn_qsa_sm80/reference/gdn_chunk_ref.py:133-141), fp32 throughout:
 //     S <- exp(g) S ;  delta = beta (v - S^T k) ;  S <- S + k delta^T ;  o = S^T q / sqrt(D)
-// With one token the operator is nothing but a read and a write of the 64 KB state per (batch, value head), so
-// the kernel is laid out for HBM: a CTA of 256 threads owns one state; warp w holds rows w, w+8, ... (16 rows),
-// lane l the four columns 4l..4l+3 of each, so every load and store is a whole 512-byte row per warp and a thread
-// keeps 16 independent 16-byte loads in flight; two CTAs per SM.  The two column sums a token needs (S^T k and
-// S^T q) are partial per warp and meet in shared memory.
+// With one token the operator is nothing but a read and a write of the 64 KB state per (batch, value head), so the
+// kernel is laid out for HBM.  The value columns of a state are independent, so the unit of work is a tile of
+// [128 rows][32 columns] (16 KB): two warps own one, 64 values per thread, and a persistent CTA streams tiles through a
+// ring of three TMA stages - the loads of the next tiles are in flight while this one is computed and the one before
+// leaves by TMA store, which the load-compute-store phases of one CTA per state could not do (75 % of the copy bandwidth).
+// The tile is 128-byte swizzled and lane l owns rows = l mod 8 and the four columns of chunk l / 8, so a 16-byte access
+// of eight lanes covers all banks, and the column sums a token needs (S^T k, S^T q) are three shuffles: no barrier.
+//   GROUPS = 1: a CTA of two compute warps and a producer warp, four per SM; 32 states give 128 CTAs.
+//   GROUPS = 4: the four tiles of a state in one CTA, for the gated normalisation of the output rows (their sum of squares
+//   needs all 128 columns: one barrier a token), which then costs no launch and no pass over the rows of its own.
+#include <cuda.h>
+
+#include "../../include/gdn_chunk_sm100.h"
 #include "gdn_common.cuh"
+#include "gdn_launch.cuh"
+#include "ptx_sm100.cuh"
 
 namespace gdn {
 namespace {
 
-constexpr int kDecThreads = 256, kDecWarps = 8, kRowsPerWarp = kD / kDecWarps;
+constexpr int kDecStages = 3, kDecTokens = 8;      // tokens whose vectors travel through the ring (later ones: global loads)
+constexpr int kDecTimeoutFull = 0x601, kDecTimeoutEmpty = 0x602;
+
+struct DecodeGate {                                // gated normalisation of the output rows (z null: none)
+    const __nv_bfloat16* z;
+    const __nv_bfloat16* weight;
+    float eps;
+};
 
 template <bool GATE_F32>
 __device__ __forceinline__ float dec_gate(const void* p, size_t idx) {
     if (GATE_F32) return static_cast<const float*>(p)[idx];
     return __bfloat162float(static_cast<const __nv_bfloat16*>(p)[idx]);
 }
+__device__ __forceinline__ float bf16_bits(unsigned short x) { return __uint_as_float(static_cast<uint32_t>(x) << 16); }
+__device__ __forceinline__ float sum_rows(float x) {   // over the eight lanes that share a column
+    x += __shfl_xor_sync(0xffffffffu, x, 1);
+    x += __shfl_xor_sync(0xffffffffu, x, 2);
+    x += __shfl_xor_sync(0xffffffffu, x, 4);
+    return x;
+}
 
-template <bool GATE_F32>
-__global__ void __launch_bounds__(kDecThreads, 2) gdn_decode_kernel(Problem p) {
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int b = blockIdx.x / p.Hv, h = blockIdx.x % p.Hv;
-    const int hq = h / (p.Hv / p.Hq);
-    const float scale = rsqrtf(static_cast<float>(kD));
-    __shared__ float ks[kD], qs[kD];
-    __shared__ __align__(16) float part[2][kDecWarps][kD];
+// bytes of the token area of one stage: k, q rows, 32 columns of v, g and beta
+__host__ __device__ constexpr uint32_t dec_token_bytes(int nt) { return nt * (256 + 256 + 64) + 2 * kDecTokens * 4; }
 
-    const size_t st_base = (static_cast<size_t>(b) * p.Hv + h) * kD * kD;
-    float4 st[kRowsPerWarp];
-#pragma unroll
-    for (int i = 0; i < kRowsPerWarp; ++i) {
-        const int r = warp + kDecWarps * i;
-        st[i] = p.h0 ? *reinterpret_cast<const float4*>(p.h0 + st_base + static_cast<size_t>(r) * kD + 4 * lane)
-                     : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    for (int s = 0; s < p.S; ++s) {
-        const size_t tok = static_cast<size_t>(b) * p.S + s;
-        if (tid < kD) ks[tid] = __bfloat162float(p.k[(tok * p.Hq + hq) * kD + tid]);
-        else qs[tid - kD] = __bfloat162float(p.q[(tok * p.Hq + hq) * kD + tid - kD]) * scale;
-        float gt = dec_gate<GATE_F32>(p.g, tok * p.Hv + h), bt = dec_gate<GATE_F32>(p.beta, tok * p.Hv + h);
-        if (p.gate_act) {   // raw gates: g = -softplus(.), beta = sigmoid(.)
-            gt = gt > 20.f ? -gt : -log1pf(__expf(gt));
-            bt = 1.f / (1.f + __expf(-bt));
-        }
-        const float dec = __expf(gt);
-        const uint2 vraw = *reinterpret_cast<const uint2*>(p.v + (tok * p.Hv + h) * kD + 4 * lane);
-        __syncthreads();
-        float rk = 1.f, rq = 1.f;
-        if (p.l2norm) {   // every warp sums the squares itself: the vectors are in shared memory anyway
-            const float4 k4 = *reinterpret_cast<const float4*>(ks + 4 * lane), q4 = *reinterpret_cast<const float4*>(qs + 4 * lane);
-            float kk = k4.x * k4.x + k4.y * k4.y + k4.z * k4.z + k4.w * k4.w;
-            float qq = q4.x * q4.x + q4.y * q4.y + q4.z * q4.z + q4.w * q4.w;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                kk += __shfl_xor_sync(0xffffffffu, kk, o);
-                qq += __shfl_xor_sync(0xffffffffu, qq, o);
+template <int GROUPS, bool GATE_F32>
+__global__ void __launch_bounds__(GROUPS * 64 + 32, GROUPS == 1 ? 4 : 1)
+gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_out,
+                  const __grid_constant__ Problem p, const __grid_constant__ DecodeGate gate, int items, int nt) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    __shared__ __align__(8) uint64_t full[GROUPS][kDecStages], empty[GROUPS][kDecStages];
+    __shared__ float ssq[2][GROUPS * 2];
+    __shared__ int failed;
+
+    const int tid = threadIdx.x, warp = static_cast<int>(warp_uniform(tid >> 5)), lane = tid & 31;
+    const uint32_t tok_bytes = dec_token_bytes(nt);
+    // stage s of group g: the tile at (g * kDecStages + s) * 16 KB; the token areas behind all tiles
+    auto tile_of = [&](int g, int s) { return sm + (g * kDecStages + s) * 16384; };
+    auto tok_of = [&](int g, int s) { return sm + GROUPS * kDecStages * 16384 + (g * kDecStages + s) * tok_bytes; };
+    const int rep = p.Hv / p.Hq;
+
+    if (tid == 0) {
+        for (int g = 0; g < GROUPS; ++g)
+            for (int s = 0; s < kDecStages; ++s) {
+                mbar_init(&full[g][s], 2);       // the copies (bytes) and the gates (written by the producer warp)
+                mbar_init(&empty[g][s], 1);
             }
-            rk = rsqrtf(kk + 1e-6f);
-            rq = rsqrtf(qq / (scale * scale) + 1e-6f);   // qs holds q * scale
-        }
-        // S^T k, this warp's rows
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int i = 0; i < kRowsPerWarp; ++i) {
-            const float kr = ks[warp + kDecWarps * i];
-            acc.x = fmaf(st[i].x, kr, acc.x); acc.y = fmaf(st[i].y, kr, acc.y);
-            acc.z = fmaf(st[i].z, kr, acc.z); acc.w = fmaf(st[i].w, kr, acc.w);
-        }
-        *reinterpret_cast<float4*>(&part[0][warp][4 * lane]) = acc;
-        __syncthreads();
-        float4 kv = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int w = 0; w < kDecWarps; ++w) {
-            const float4 x = *reinterpret_cast<const float4*>(&part[0][w][4 * lane]);
-            kv.x += x.x; kv.y += x.y; kv.z += x.z; kv.w += x.w;
-        }
-        const float f = dec * rk, bk = bt * rk;
-        float4 dl;   // delta = beta (v - (decayed S)^T k), with the key's norm folded in
-        dl.x = (__uint_as_float(vraw.x << 16) - kv.x * f) * bk;
-        dl.y = (__uint_as_float(vraw.x & 0xffff0000u) - kv.y * f) * bk;
-        dl.z = (__uint_as_float(vraw.y << 16) - kv.z * f) * bk;
-        dl.w = (__uint_as_float(vraw.y & 0xffff0000u) - kv.w * f) * bk;
-        float4 oa = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int i = 0; i < kRowsPerWarp; ++i) {
-            const float kr = ks[warp + kDecWarps * i], qr = qs[warp + kDecWarps * i];
-            st[i].x = fmaf(kr, dl.x, dec * st[i].x); st[i].y = fmaf(kr, dl.y, dec * st[i].y);
-            st[i].z = fmaf(kr, dl.z, dec * st[i].z); st[i].w = fmaf(kr, dl.w, dec * st[i].w);
-            oa.x = fmaf(st[i].x, qr, oa.x); oa.y = fmaf(st[i].y, qr, oa.y);
-            oa.z = fmaf(st[i].z, qr, oa.z); oa.w = fmaf(st[i].w, qr, oa.w);
-        }
-        *reinterpret_cast<float4*>(&part[1][warp][4 * lane]) = oa;
-        __syncthreads();
-        if (warp == 0) {
-            float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int w = 0; w < kDecWarps; ++w) {
-                const float4 x = *reinterpret_cast<const float4*>(&part[1][w][4 * lane]);
-                o.x += x.x; o.y += x.y; o.z += x.z; o.w += x.w;
-            }
-            const __nv_bfloat162 lo = __floats2bfloat162_rn(o.x * rq, o.y * rq), hi = __floats2bfloat162_rn(o.z * rq, o.w * rq);
-            uint2 pk;
-            pk.x = *reinterpret_cast<const uint32_t*>(&lo);
-            pk.y = *reinterpret_cast<const uint32_t*>(&hi);
-            *reinterpret_cast<uint2*>(p.out + (tok * p.Hv + h) * kD + 4 * lane) = pk;
-        }
+        failed = 0;
+        fence_mbar_init();
     }
-    if (p.hT) {
-#pragma unroll
-        for (int i = 0; i < kRowsPerWarp; ++i) {
-            const int r = warp + kDecWarps * i;
-            *reinterpret_cast<float4*>(p.hT + st_base + static_cast<size_t>(r) * kD + 4 * lane) = st[i];
+    __syncthreads();
+    grid_dependency_wait();
+    grid_launch_dependents();
+    if (p.clear_status && blockIdx.x == 0 && tid == 0) *p.status = 0;
+
+    // work items: GROUPS = 1: a tile (state, quarter); GROUPS = 4: a state
+    const int first = blockIdx.x, step = gridDim.x;
+    if (warp == GROUPS * 2) {
+        // ------------------------------- producer ---------------------------------------------------------------------
+        int n = 0;
+        for (int it = first; it < items; it += step, ++n) {
+            const int s = n % kDecStages;
+            const int state = GROUPS == 1 ? it >> 2 : it;
+            const int b = state / p.Hv, h = state - b * p.Hv, hq = h / rep;
+            const size_t tok0 = static_cast<size_t>(b) * p.S;
+            bool ok = true;
+            for (int g = 0; g < GROUPS && ok; ++g) {
+                if (n >= kDecStages) ok = mbar_wait(&empty[g][s], ((n / kDecStages) - 1) & 1, p.status, kDecTimeoutEmpty);
+                const int quarter = GROUPS == 1 ? it & 3 : g;
+                if (ok && elect_one()) {
+                    uint8_t* tk = tok_of(g, s);
+                    mbar_arrive_expect_tx(&full[g][s], (p.h0 ? 16384 : 0) + nt * (256 + 256 + 64));
+                    if (p.h0) tma_load_2d(tile_of(g, s), &tm_in, &full[g][s], quarter * 32, state * kD);
+                    for (int t = 0; t < nt; ++t) {
+                        const size_t row = (tok0 + t) * p.Hq + hq;
+                        bulk_load_1d(tk + t * 256, p.k + row * kD, 256, &full[g][s]);
+                        bulk_load_1d(tk + (nt + t) * 256, p.q + row * kD, 256, &full[g][s]);
+                        bulk_load_1d(tk + nt * 512 + t * 64, p.v + ((tok0 + t) * p.Hv + h) * kD + quarter * 32, 64, &full[g][s]);
+                    }
+                }
+                __syncwarp();
+            }
+            if (!ok) {   // the compute warps then stop waiting as well
+                *const_cast<volatile int*>(&failed) = 1;
+                break;
+            }
+            float x = 0.f;
+            if (lane < 2 * kDecTokens && (lane & 7) < nt)
+                x = dec_gate<GATE_F32>(lane < kDecTokens ? p.g : p.beta, (tok0 + (lane & 7)) * p.Hv + h);
+            for (int g = 0; g < GROUPS; ++g) {
+                if (lane < 2 * kDecTokens) *reinterpret_cast<float*>(tok_of(g, s) + nt * (256 + 256 + 64) + lane * 4) = x;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full[g][s]);
+            }
         }
+    } else {
+        // ------------------------------- compute: two warps per tile ------------------------------------------------------
+        const int g = warp >> 1, half = warp & 1;             // half: which 16 of the tile's 32 columns
+        const int rg = lane & 7, ch = half * 4 + (lane >> 3); // rows rg, rg + 8, ...; 16-byte chunk of a 128-byte row
+        const uint32_t off0 = rg * 128 + ((ch ^ rg) << 4);    // the same chunk in every row = rg mod 8
+        const float scale = rsqrtf(static_cast<float>(kD));
+        int n = 0;
+        for (int it = first; it < items; it += step, ++n) {
+            const int s = n % kDecStages;
+            const int state = GROUPS == 1 ? it >> 2 : it, quarter = GROUPS == 1 ? it & 3 : g;
+            const int b = state / p.Hv, h = state - b * p.Hv, hq = h / rep;
+            const size_t tok0 = static_cast<size_t>(b) * p.S;
+            // after a wait that ran out nobody waits again, but every warp keeps to the loop: its barriers count all of them
+            const bool ok = !*const_cast<volatile int*>(&failed) &&
+                            mbar_wait(&full[g][s], (n / kDecStages) & 1, p.status, kDecTimeoutFull);
+            if (!ok) *const_cast<volatile int*>(&failed) = 1;
+            uint8_t* tile = tile_of(g, s) + off0;
+            const uint8_t* tk = tok_of(g, s);
+            float4 st[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                st[i] = p.h0 ? *reinterpret_cast<const float4*>(tile + i * 1024) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float* gates = reinterpret_cast<const float*>(tk + nt * (256 + 256 + 64));
+            for (int t = 0; t < p.S; ++t) {
+                const size_t tok = tok0 + t;
+                // this lane's rows of k and q (fp32), its four values, the gates
+                const unsigned short *kr, *qr;
+                uint2 vraw;
+                float gt, bt;
+                if (t < nt) {
+                    kr = reinterpret_cast<const unsigned short*>(tk + t * 256);
+                    qr = reinterpret_cast<const unsigned short*>(tk + (nt + t) * 256);
+                    vraw = *reinterpret_cast<const uint2*>(tk + nt * 512 + t * 64 + ch * 8);
+                    gt = gates[t];
+                    bt = gates[kDecTokens + t];
+                } else {
+                    kr = reinterpret_cast<const unsigned short*>(p.k + (tok * p.Hq + hq) * kD);
+                    qr = reinterpret_cast<const unsigned short*>(p.q + (tok * p.Hq + hq) * kD);
+                    vraw = *reinterpret_cast<const uint2*>(p.v + (tok * p.Hv + h) * kD + quarter * 32 + ch * 4);
+                    gt = dec_gate<GATE_F32>(p.g, tok * p.Hv + h);
+                    bt = dec_gate<GATE_F32>(p.beta, tok * p.Hv + h);
+                }
+                if (p.gate_act) {   // raw gates: g = -softplus(.), beta = sigmoid(.)
+                    gt = gt > 20.f ? -gt : -log1pf(__expf(gt));
+                    bt = 1.f / (1.f + __expf(-bt));
+                }
+                const float dec = __expf(gt);
+                float kf[16], qf[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    kf[i] = bf16_bits(kr[rg + 8 * i]);
+                    qf[i] = bf16_bits(qr[rg + 8 * i]) * scale;
+                }
+                float rk = 1.f, rq = 1.f;
+                if (p.l2norm) {
+                    float kk = 0.f, qq = 0.f;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        kk = fmaf(kf[i], kf[i], kk);
+                        qq = fmaf(qf[i], qf[i], qq);
+                    }
+                    rk = rsqrtf(sum_rows(kk) + 1e-6f);
+                    rq = rsqrtf(sum_rows(qq) / (scale * scale) + 1e-6f);   // qf holds q * scale
+                }
+                float4 kv = make_float4(0.f, 0.f, 0.f, 0.f);              // S^T k
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    kv.x = fmaf(st[i].x, kf[i], kv.x); kv.y = fmaf(st[i].y, kf[i], kv.y);
+                    kv.z = fmaf(st[i].z, kf[i], kv.z); kv.w = fmaf(st[i].w, kf[i], kv.w);
+                }
+                kv.x = sum_rows(kv.x); kv.y = sum_rows(kv.y); kv.z = sum_rows(kv.z); kv.w = sum_rows(kv.w);
+                const float f = dec * rk, bk = bt * rk;
+                float4 dl;   // delta = beta (v - (decayed S)^T k), with the key's norm folded in
+                dl.x = (__uint_as_float(vraw.x << 16) - kv.x * f) * bk;
+                dl.y = (__uint_as_float(vraw.x & 0xffff0000u) - kv.y * f) * bk;
+                dl.z = (__uint_as_float(vraw.y << 16) - kv.z * f) * bk;
+                dl.w = (__uint_as_float(vraw.y & 0xffff0000u) - kv.w * f) * bk;
+                float4 oa = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    st[i].x = fmaf(kf[i], dl.x, dec * st[i].x); st[i].y = fmaf(kf[i], dl.y, dec * st[i].y);
+                    st[i].z = fmaf(kf[i], dl.z, dec * st[i].z); st[i].w = fmaf(kf[i], dl.w, dec * st[i].w);
+                    oa.x = fmaf(st[i].x, qf[i], oa.x); oa.y = fmaf(st[i].y, qf[i], oa.y);
+                    oa.z = fmaf(st[i].z, qf[i], oa.z); oa.w = fmaf(st[i].w, qf[i], oa.w);
+                }
+                oa.x = sum_rows(oa.x) * rq; oa.y = sum_rows(oa.y) * rq; oa.z = sum_rows(oa.z) * rq; oa.w = sum_rows(oa.w) * rq;
+                const size_t o_at = (tok * p.Hv + h) * kD + quarter * 32 + ch * 4;
+                uint2 pk;
+                pk.x = pack_bf16x2(oa.x, oa.y);
+                pk.y = pack_bf16x2(oa.z, oa.w);
+                if (GROUPS == 4 && gate.z) {
+                    // the row as bf16, normalised and gated (the arithmetic of gdn_output_gate_sm100.cu on the rounded row)
+                    const float a[4] = {__uint_as_float(pk.x << 16), __uint_as_float(pk.x & 0xffff0000u),
+                                        __uint_as_float(pk.y << 16), __uint_as_float(pk.y & 0xffff0000u)};
+                    const uint2 zr = *reinterpret_cast<const uint2*>(gate.z + o_at);
+                    const uint2 wr = *reinterpret_cast<const uint2*>(gate.weight + quarter * 32 + ch * 4);
+                    float ss = a[0] * a[0];
+                    ss = fmaf(a[1], a[1], ss); ss = fmaf(a[2], a[2], ss); ss = fmaf(a[3], a[3], ss);
+                    ss += __shfl_xor_sync(0xffffffffu, ss, 8);
+                    ss += __shfl_xor_sync(0xffffffffu, ss, 16);
+                    if (lane == 0) ssq[t & 1][warp] = ss;
+                    named_bar_sync(1, GROUPS * 64);       // (the next token writes the other slot)
+                    float tot = 0.f;
+#pragma unroll
+                    for (int w = 0; w < GROUPS * 2; ++w) tot += ssq[t & 1][w];
+                    const float rstd = rsqrtf(tot * (1.f / 128.f) + gate.eps);
+                    const float z4[4] = {__uint_as_float(zr.x << 16), __uint_as_float(zr.x & 0xffff0000u),
+                                         __uint_as_float(zr.y << 16), __uint_as_float(zr.y & 0xffff0000u)};
+                    const float w4[4] = {__uint_as_float(wr.x << 16), __uint_as_float(wr.x & 0xffff0000u),
+                                         __uint_as_float(wr.y << 16), __uint_as_float(wr.y & 0xffff0000u)};
+                    float o4[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) o4[e] = a[e] * (rstd * w4[e]) * __fdividef(z4[e], 1.f + __expf(-z4[e]));
+                    pk.x = pack_bf16x2(o4[0], o4[1]);
+                    pk.y = pack_bf16x2(o4[2], o4[3]);
+                }
+                if (rg == 0) *reinterpret_cast<uint2*>(p.out + o_at) = pk;
+            }
+            // the tile goes back into its stage and leaves by TMA; the stage before it is free once its store has been read
+            if (p.hT) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) *reinterpret_cast<float4*>(tile + i * 1024) = st[i];
+                fence_proxy_async_smem();
+            }
+            named_bar_sync(2 + g, 64);
+            if (half == 0 && elect_one()) {
+                if (p.hT) {
+                    tma_store_wait_read();                // tile n - 1's store has read its stage
+                    if (n > 0) mbar_arrive(&empty[g][(n - 1) % kDecStages]);
+                    if (ok) tma_store_2d(&tm_out, tile_of(g, s), quarter * 32, state * kD);
+                    tma_store_commit();
+                } else {
+                    mbar_arrive(&empty[g][s]);
+                }
+            }
+            __syncwarp();
+        }
+        if (p.hT && half == 0 && elect_one()) tma_store_wait_all();
     }
 }
 
 }  // namespace
 
-cudaError_t launch_decode(const Problem& p, cudaStream_t stream) {
-    const dim3 grid(p.B * p.Hv), block(kDecThreads);
-    if (p.gate_f32) gdn_decode_kernel<true><<<grid, block, 0, stream>>>(p);
-    else gdn_decode_kernel<false><<<grid, block, 0, stream>>>(p);
-    count_launch();
-    return cudaGetLastError();
+// `og`: gated normalisation applied to the output rows by the same kernel (null: none).
+int launch_decode(const Problem& p, const OutputGate* og, cudaStream_t stream) {
+    const long long states = static_cast<long long>(p.B) * p.Hv;
+    if (states * kD >= (1ll << 31)) return GDN_ERR_BAD_ARGUMENT;
+    alignas(64) CUtensorMap tin, tout;
+    const unsigned long long d[2] = {kD, static_cast<unsigned long long>(states) * kD}, sb[1] = {kD * 4};
+    const unsigned box[2] = {32, kD};
+    const float* any = p.h0 ? p.h0 : p.hT;
+    if (any) {   // a map nobody uses still has to be a valid one
+        if (encode_tma(&tin, any, 4, 2, d, sb, box, 128)) return GDN_ERR_DRIVER;
+        if (encode_tma(&tout, p.hT ? p.hT : any, 4, 2, d, sb, box, 128)) return GDN_ERR_DRIVER;
+    } else {
+        tin = tout = CUtensorMap{};
+    }
+    DecodeGate gate{};
+    if (og) gate = DecodeGate{static_cast<const __nv_bfloat16*>(og->z), static_cast<const __nv_bfloat16*>(og->weight), og->eps};
+    auto go = [&](auto kernel, int groups, long long items) -> int {
+        const int most = groups == 4 ? 4 : kDecTokens;            // tokens whose vectors fit the ring of four groups
+        const int nt = p.S < most ? p.S : most;
+        const uint32_t smem = groups * kDecStages * (16384 + dec_token_bytes(nt)) + 1024;
+        if (allow_smem(reinterpret_cast<const void*>(kernel), smem)) return GDN_ERR_CUDA;
+        const int fit = static_cast<int>(228 * 1024 / (smem + 1536)), per_sm = fit > 4 ? 4 : fit;
+        const long long cap = static_cast<long long>(sm_count()) * per_sm;
+        const unsigned grid = static_cast<unsigned>(items < cap ? items : cap);
+        const cudaError_t e = launch_dependent(kernel, dim3(grid), dim3(groups * 64 + 32), smem, stream, false, tin, tout, p,
+                                               gate, static_cast<int>(items), nt);
+        return e == cudaSuccess ? GDN_OK : GDN_ERR_CUDA;
+    };
+    if (og) return p.gate_f32 ? go(gdn_decode_kernel<4, true>, 4, states) : go(gdn_decode_kernel<4, false>, 4, states);
+    return p.gate_f32 ? go(gdn_decode_kernel<1, true>, 1, states * 4) : go(gdn_decode_kernel<1, false>, 1, states * 4);
 }
 
 }  // namespace gdn

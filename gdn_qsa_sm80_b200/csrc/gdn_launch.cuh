@@ -1,0 +1,44 @@
+// Host side of a kernel launch: the dynamic shared-memory limit (set once per kernel and device, not on every call) and
+// the launch as a programmatic dependent of the kernel before it in the stream.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stddef.h>
+
+#include "gdn_common.cuh"
+
+namespace gdn {
+
+// Lets `kernel` use `bytes` of dynamic shared memory on the current device; 0 on success.
+int allow_smem(const void* kernel, size_t bytes);
+
+// Launches with the programmatic-stream-serialization attribute: the CTAs may set up while the kernel before this one in the
+// stream drains (the kernel waits for it with grid_dependency_wait before it touches memory).  `pairs`: clusters of two CTAs
+// along x.  Where the context has neither, an ordinary launch, in which that wait is a no-op.
+template <typename Kernel, typename... Args>
+inline cudaError_t launch_dependent(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool pairs, const Args&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 2;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pairs ? 2 : 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        cfg.numAttrs = 0;
+        e = cudaLaunchKernelEx(&cfg, kernel, args...);
+    }
+    count_launch();
+    return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+}  // namespace gdn
