@@ -52,6 +52,8 @@ EXPORTS = (
     "gdn_chunk_fwd_gated_sm100",
     "gdn_chunk_fwd_host_sm100",
     "gdn_chunk_fwd_sm100_noalloc",
+    "gdn_chunk_varlen_scratch_bytes",
+    "gdn_chunk_fwd_varlen_sm100",
     "gdn_chunk_scan_transfers",
     "gdn_chunk_read_status",
     "gdn_chunk_error_string",
@@ -101,6 +103,10 @@ def load() -> ctypes.CDLL:
     lib.gdn_chunk_fwd_gated_sm100.restype = ci
     lib.gdn_chunk_fwd_sm100_noalloc.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, ci, ci, ci, ci, ci, vp]
     lib.gdn_chunk_fwd_sm100_noalloc.restype = ci
+    lib.gdn_chunk_varlen_scratch_bytes.argtypes = [ctypes.POINTER(ci), ci, ci]
+    lib.gdn_chunk_varlen_scratch_bytes.restype = sz
+    lib.gdn_chunk_fwd_varlen_sm100.argtypes = [vp] * 9 + [sz, ctypes.POINTER(ci), ci, ci, ci, ci, ctypes.c_uint, vp]
+    lib.gdn_chunk_fwd_varlen_sm100.restype = ci
     lib.gdn_chunk_scan_transfers.argtypes = [vp, vp, vp, vp, vp, ci, ci, vp]
     lib.gdn_chunk_scan_transfers.restype = ci
     lib.gdn_chunk_read_status.argtypes = [vp, vp, ctypes.POINTER(ci)]

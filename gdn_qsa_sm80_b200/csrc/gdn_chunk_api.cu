@@ -95,12 +95,13 @@ int encode_workspace_maps(const Problem& p, const Workspace& ws, void* tw, void*
     return 0;
 }
 
-int encode_tile_maps(const Problem& p, const Workspace& ws, void* tp, void* tt2) {
+int encode_tile_maps(const Problem& p, const Workspace& ws, TileMaps& maps) {
+    if (encode_qkv_maps(p, maps.q, maps.k, maps.v, 64)) return 1;
     const unsigned long long tiles = p.pk_chunk ? static_cast<unsigned long long>(p.pk_chunks) * p.Hv
                                                 : static_cast<unsigned long long>(p.B) * p.Hv * ((p.S + kChunk - 1) / kChunk);
     const unsigned long long d[2] = {64, tiles * kChunk}, s[1] = {128};
     const unsigned box[2] = {64, 64};
-    return encode_tma(tp, ws.P, 2, 2, d, s, box, 128) || encode_tma(tt2, ws.U, 2, 2, d, s, box, 128);
+    return encode_tma(maps.p, ws.P, 2, 2, d, s, box, 128) || encode_tma(maps.t2, ws.U, 2, 2, d, s, box, 128);
 }
 
 int sm_count() {
@@ -133,7 +134,6 @@ int allow_smem(const void* kernel, size_t bytes) {
 }
 
 static long long* g_phase_profile = nullptr;
-constexpr int kDecodeMaxTokens = 8;   // sequences this short take the decode kernel under GDN_PATH_AUTO
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
@@ -270,13 +270,11 @@ int forward_device(const void* q, const void* k, const void* v, const void* g, c
     if (decode) return launch_decode(p, gate, stream);
     if (path == GDN_PATH_SIMT && !clear()) return GDN_ERR_CUDA;
     if (path == GDN_PATH_SIMT) return then_gate(launch_simt(p, stream) == cudaSuccess ? GDN_OK : GDN_ERR_CUDA);
-    // Automatic choice, by shape alone.  Few short sequences (up to 1024 tokens): the single-launch kernel whose four
-    // 32-column CTAs per head share the prepare work.  Everything else: the prepare kernel and the transposed chain
-    // (one CTA per head, state-dependent operands in tensor memory), which splits long sequences into segments when
-    // there are too few of them to fill the GPU.  Measured on one B200, 32 sequences, single launch against the two
-    // kernels: 512 tokens 0.036 / 0.037 ms, 1024 tokens 0.050 / 0.057, 2048 tokens 0.084 / 0.074.
-    const bool automatic = path == GDN_PATH_AUTO;
-    if (automatic) path = (S <= 1024 && coop_supported(p)) ? GDN_PATH_COOP : GDN_PATH_TWOPASS_T;
+    // Automatic choice beyond the decode lengths: the prepare kernel and the transposed chain.  The single-launch kernel is an
+    // explicit path only: its serial step is longer (32 sequences of 300 / 700 / 1000 tokens, decay 0.5: 30.7 / 41.0 / 49.2 us
+    // against 26.6 / 35.6 / 38.9 us for the two kernels; with decay 0.05, where no sequence is split, 41.0 / 49.2 against
+    // 41.0 / 50.3 us at 700 / 1000 tokens) and it needs two memsets.
+    if (path == GDN_PATH_AUTO) path = GDN_PATH_TWOPASS_T;
     int nv;
     if (path == GDN_PATH_TWOPASS_NV32) nv = 32;
     else nv = 64;
@@ -297,21 +295,13 @@ int forward_device(const void* q, const void* k, const void* v, const void* g, c
     if (path != GDN_PATH_TWOPASS_T && path != GDN_PATH_PREPARE_ONLY_R && !clear()) return GDN_ERR_CUDA;
     if (path == GDN_PATH_COOP_CHAIN_ONLY)
         return then_gate(launch_coop(p, ws, reinterpret_cast<int*>(base + l.flags), l.flag_bytes, stream, true));
-    if (path == GDN_PATH_COOP) {
-        const int st = launch_coop(p, ws, reinterpret_cast<int*>(base + l.flags), l.flag_bytes, stream);
-        // the single-launch kernel is a cooperative launch: when its grid cannot be resident all at once on this
-        // context (fewer SMs than the device reports, a limited partition) the launch is refused and nothing has
-        // run; the automatic path then takes the two-kernel route, which waits for nothing inside a launch
-        if (!(automatic && st == GDN_ERR_CUDA)) return then_gate(st);
-        (void)cudaGetLastError();
-        path = GDN_PATH_TWOPASS_T;
-        ws.n_seg = 1;
-    }
-    if (path == GDN_PATH_CHAIN_ONLY_T) return then_gate(launch_chain_r(p, ws, stream));
-    if (path == GDN_PATH_TWOPASS_T || path == GDN_PATH_PREPARE_ONLY_R) {
-        const int st = launch_prepare_lean(p, ws, stream);
+    if (path == GDN_PATH_COOP) return then_gate(launch_coop(p, ws, reinterpret_cast<int*>(base + l.flags), l.flag_bytes, stream));
+    if (path == GDN_PATH_TWOPASS_T || path == GDN_PATH_PREPARE_ONLY_R || path == GDN_PATH_CHAIN_ONLY_T) {
+        TileMaps maps;
+        if (encode_tile_maps(p, ws, maps)) return GDN_ERR_DRIVER;
+        int st = path == GDN_PATH_CHAIN_ONLY_T ? GDN_OK : launch_prepare_lean(p, ws, maps, stream);
         if (st != GDN_OK || path == GDN_PATH_PREPARE_ONLY_R) return st;
-        return then_gate(launch_chain_r(p, ws, stream));
+        return then_gate(launch_chain_r(p, ws, maps, stream));
     }
     if (path == GDN_PATH_CHAIN_ONLY) return then_gate(launch_chain(p, ws, nv, stream));   // workspace left by an earlier call
     const bool pairs = transposed && (Hv / Hq) % 2 == 0 && p.dbg != 3;

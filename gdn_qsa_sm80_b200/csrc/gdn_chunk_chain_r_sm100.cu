@@ -548,16 +548,14 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 
 }  // namespace
 
-int launch_chain_r(const Problem& p, const Workspace& ws, cudaStream_t stream) {
-    alignas(64) CUtensorMap tq, tk, tv, tp, tt2;
-    if (encode_qkv_maps(p, &tq, &tk, &tv, 64)) return GDN_ERR_DRIVER;
-    if (encode_tile_maps(p, ws, &tp, &tt2)) return GDN_ERR_DRIVER;
+int launch_chain_r(const Problem& p, const Workspace& ws, const TileMaps& maps, cudaStream_t stream) {
+    auto map = [](const unsigned char* m) -> const CUtensorMap& { return *reinterpret_cast<const CUtensorMap*>(m); };
     auto go = [&](auto kernel, unsigned gz) -> int {
         if (allow_smem(reinterpret_cast<const void*>(kernel), kRDynamic)) return GDN_ERR_CUDA;
         // The value heads that share a qk head read the same K and Q tiles: as a cluster of two CTAs they start together
         // and run in step, so the second read of a tile finds it in L2 (nothing else of the cluster is used).
         const cudaError_t e = launch_dependent(kernel, dim3(p.Hv, p.pk_chunk ? p.pk_n : p.B, gz), dim3(kRThreads), kRDynamic, stream,
-                                               (p.Hv / p.Hq) % 2 == 0, tq, tk, tv, tp, tt2, p, ws);
+                                               (p.Hv / p.Hq) % 2 == 0, map(maps.q), map(maps.k), map(maps.v), map(maps.p), map(maps.t2), p, ws);
         return e == cudaSuccess ? GDN_OK : GDN_ERR_CUDA;
     };
     const int G = ws.n_seg;

@@ -259,10 +259,8 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
 
 }  // namespace
 
-int launch_prepare_lean(const Problem& p, const Workspace& ws, cudaStream_t stream) {
-    alignas(64) CUtensorMap tq, tk, tv, tp, tt2;
-    if (encode_qkv_maps(p, &tq, &tk, &tv, 64)) return GDN_ERR_DRIVER;
-    if (encode_tile_maps(p, ws, &tp, &tt2)) return GDN_ERR_DRIVER;
+int launch_prepare_lean(const Problem& p, const Workspace& ws, const TileMaps& maps, cudaStream_t stream) {
+    auto map = [](const unsigned char* m) -> const CUtensorMap& { return *reinterpret_cast<const CUtensorMap*>(m); };
     const int NT = (p.S + kChunk - 1) / kChunk;
     const long long chunks = p.pk_chunk ? p.pk_chunks : static_cast<long long>(p.B) * NT;
     auto go = [&](auto kernel, int heads, uint32_t smem, int per_sm) -> int {
@@ -271,7 +269,7 @@ int launch_prepare_lean(const Problem& p, const Workspace& ws, cudaStream_t stre
         const long long max_ctas = static_cast<long long>(per_sm) * sm_count();
         const unsigned grid = static_cast<unsigned>(items < max_ctas ? items : max_ctas);
         if (allow_smem(reinterpret_cast<const void*>(kernel), smem)) return GDN_ERR_CUDA;
-        const cudaError_t e = launch_dependent(kernel, dim3(grid), dim3(128 * heads), smem, stream, false, tq, tk, tp, tt2, p, ws,
+        const cudaError_t e = launch_dependent(kernel, dim3(grid), dim3(128 * heads), smem, stream, false, map(maps.q), map(maps.k), map(maps.p), map(maps.t2), p, ws,
                                                static_cast<unsigned>(NT), static_cast<unsigned>(items));
         return e == cudaSuccess ? GDN_OK : GDN_ERR_CUDA;
     };

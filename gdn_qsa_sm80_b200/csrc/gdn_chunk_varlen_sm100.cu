@@ -1,0 +1,191 @@
+// Packed batch: sequences of different lengths laid end to end in [1, T, H, .] tensors, in one pass of the two-kernel path.
+//
+// The kernels find a chunk's sequence through three small tables (first token of each sequence; (sequence, chunk) per 64-token
+// chunk; (sequence, first chunk) longest first, so that the last CTAs of the chain's grid are the short ones), written to the
+// scratch buffer by a kernel whose parameters carry the lengths: no copy from the host, and a captured graph keeps them.
+// The last tile of a sequence also holds the next one's first tokens; gates and beta count as zero there, and the kernels
+// mask those rows (prepare) or clear them in the tile (chain), so no sequence ever sees another's values.
+// Sequences of at most kDecodeMaxTokens tokens take the decode kernel, neighbours of equal length in one launch.
+//
+// Without this a packed batch was gathered into a padded one and scattered back (torch indexing: two passes over all
+// tensors, and the padding's share of the work), or ran sequence by sequence.
+#include <algorithm>
+#include <numeric>
+#include <vector>
+
+#include "../../include/gdn_chunk_sm100.h"
+#include "gdn_common.cuh"
+#include "gdn_launch.cuh"
+#include "ptx_sm100.cuh"
+
+namespace gdn {
+namespace {
+
+constexpr int kPiece = 1024;          // sequences per launch of the table kernel (kernel parameters: 32 KB at most)
+struct TablePiece {
+    int first;                        // sequence of entry 0
+    int start[kPiece], len[kPiece];
+    int chunk0[kPiece];               // its first entry in the chunk table; -1: a short sequence, in no table but cu
+    int rank[kPiece];                 // its place in the longest-first order
+};
+
+__global__ void __launch_bounds__(64) gdn_pack_tables_kernel(const __grid_constant__ TablePiece piece, int* cu, int2* chunk, int2* order,
+                                                             int* status) {
+    grid_dependency_wait();           // earlier kernels of the stream may still read the tables of their own call
+    grid_launch_dependents();
+    const int i = blockIdx.x, seq = piece.first + i, c0 = piece.chunk0[i];
+    if (threadIdx.x == 0) {
+        cu[seq] = piece.start[i];
+        cu[seq + 1] = piece.start[i] + piece.len[i];   // (the next sequence's block writes the same value)
+        if (c0 >= 0) order[piece.rank[i]] = make_int2(seq, c0);
+        if (seq == 0 && status) *status = 0;
+    }
+    if (c0 < 0) return;
+    const int nt = (piece.len[i] + kChunk - 1) / kChunk;
+    for (int t = threadIdx.x; t < nt; t += blockDim.x) chunk[c0 + t] = make_int2(seq, t);
+}
+
+struct PackedLayout {
+    WorkspaceLayout ws;
+    size_t cu, chunk, order, total;
+    size_t chunks;                    // 64-token chunks of the sequences that take the two-kernel path
+    int longs;                        // how many those are
+    int max_len;
+};
+PackedLayout packed_layout(const int* cu, int n_seq, int Hv) {
+    PackedLayout l{};
+    for (int i = 0; i < n_seq; ++i) {
+        const int n = cu[i + 1] - cu[i];
+        if (n > l.max_len) l.max_len = n;
+        if (n <= kDecodeMaxTokens) continue;
+        l.chunks += (n + kChunk - 1) / kChunk;
+        ++l.longs;
+    }
+    l.ws = workspace_layout(l.chunks * Hv, true);
+    auto up = [](size_t x) { return (x + 255) & ~static_cast<size_t>(255); };
+    l.cu = up(l.ws.total);
+    l.chunk = up(l.cu + (static_cast<size_t>(n_seq) + 1) * 4);
+    l.order = up(l.chunk + l.chunks * 8);
+    l.total = up(l.order + static_cast<size_t>(l.longs) * 8);
+    return l;
+}
+bool bounds_rise(const int* cu, int n_seq) {
+    if (!cu || n_seq <= 0 || cu[0] != 0) return false;
+    for (int i = 0; i < n_seq; ++i)
+        if (cu[i + 1] <= cu[i]) return false;
+    return true;
+}
+
+}  // namespace
+}  // namespace gdn
+
+using namespace gdn;
+
+extern "C" {
+
+size_t gdn_chunk_varlen_scratch_bytes(const int* cu_seqlens, int n_seq, int Hv) {
+    return bounds_rise(cu_seqlens, n_seq) && Hv > 0 ? packed_layout(cu_seqlens, n_seq, Hv).total : 0;
+}
+
+int gdn_chunk_fwd_varlen_sm100(const void* q, const void* k, const void* v, const void* g, const void* beta, const float* h0,
+                               void* out, float* hT, void* scratch, size_t scratch_bytes, const int* cu_seqlens, int n_seq,
+                               int Hq, int Hv, int gate_dtype, unsigned flags, void* stream_) {
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    if (!bounds_rise(cu_seqlens, n_seq) || Hq <= 0 || Hv <= 0 || Hv % Hq != 0) return GDN_ERR_BAD_ARGUMENT;
+    if (gate_dtype != GDN_GATE_BF16 && gate_dtype != GDN_GATE_F32) return GDN_ERR_BAD_ARGUMENT;
+    if (flags & ~static_cast<unsigned>(GDN_FLAG_QK_L2NORM | GDN_FLAG_GATE_ACTIVATIONS)) return GDN_ERR_BAD_ARGUMENT;
+    if (!q || !k || !v || !g || !beta || !out) return GDN_ERR_BAD_ARGUMENT;
+    const uintptr_t bits = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
+                           reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(h0) | reinterpret_cast<uintptr_t>(hT);
+    if (bits & 15u) return GDN_ERR_BAD_ARGUMENT;
+    const PackedLayout l = packed_layout(cu_seqlens, n_seq, Hv);
+    if (!scratch || (reinterpret_cast<uintptr_t>(scratch) & 255u) || scratch_bytes < l.total) return GDN_ERR_SCRATCH;
+    uint8_t* base = static_cast<uint8_t*>(scratch);
+    bool clear = true;                // whichever kernel comes first clears the status word
+
+    if (l.longs > 0) {
+        std::vector<int> rank(n_seq), order;
+        order.reserve(l.longs);
+        for (int i = 0; i < n_seq; ++i)
+            if (cu_seqlens[i + 1] - cu_seqlens[i] > kDecodeMaxTokens) order.push_back(i);
+        std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+            return cu_seqlens[a + 1] - cu_seqlens[a] > cu_seqlens[b + 1] - cu_seqlens[b];
+        });
+        for (int r = 0; r < l.longs; ++r) rank[order[r]] = r;
+        int* d_cu = reinterpret_cast<int*>(base + l.cu);
+        int2* d_chunk = reinterpret_cast<int2*>(base + l.chunk);
+        int2* d_order = reinterpret_cast<int2*>(base + l.order);
+        int c = 0;
+        for (int i0 = 0; i0 < n_seq; i0 += kPiece) {
+            TablePiece piece;
+            piece.first = i0;
+            const int n = std::min(kPiece, n_seq - i0);
+            for (int i = 0; i < n; ++i) {
+                const int s = i0 + i, len = cu_seqlens[s + 1] - cu_seqlens[s];
+                piece.start[i] = cu_seqlens[s];
+                piece.len[i] = len;
+                piece.rank[i] = rank[s];
+                piece.chunk0[i] = len > kDecodeMaxTokens ? c : -1;
+                if (len > kDecodeMaxTokens) c += (len + kChunk - 1) / kChunk;
+            }
+            const cudaError_t e = launch_dependent(gdn_pack_tables_kernel, dim3(n), dim3(64), 0, stream, false, piece, d_cu, d_chunk, d_order,
+                                                   i0 == 0 ? static_cast<int*>(scratch) : static_cast<int*>(nullptr));
+            if (e != cudaSuccess) return GDN_ERR_CUDA;
+        }
+        clear = false;
+        Problem p = {};
+        p.q = static_cast<const __nv_bfloat16*>(q);
+        p.k = static_cast<const __nv_bfloat16*>(k);
+        p.v = static_cast<const __nv_bfloat16*>(v);
+        p.g = g;
+        p.beta = beta;
+        p.h0 = h0;
+        p.out = static_cast<__nv_bfloat16*>(out);
+        p.hT = hT;
+        p.status = static_cast<int*>(scratch);
+        p.B = 1;
+        p.S = cu_seqlens[n_seq];
+        p.Hq = Hq;
+        p.Hv = Hv;
+        p.gate_f32 = gate_dtype == GDN_GATE_F32;
+        p.l2norm = (flags & GDN_FLAG_QK_L2NORM) ? 1 : 0;
+        p.gate_act = (flags & GDN_FLAG_GATE_ACTIVATIONS) ? 1 : 0;
+        p.pk_cu = d_cu;
+        p.pk_chunk = d_chunk;
+        p.pk_order = d_order;
+        p.pk_n = l.longs;
+        p.pk_chunks = static_cast<int>(l.chunks);
+        Workspace ws = {};
+        ws.P = reinterpret_cast<__nv_bfloat16*>(base + l.ws.P);
+        ws.U = reinterpret_cast<__nv_bfloat16*>(base + l.ws.U);
+        ws.vec = reinterpret_cast<float*>(base + l.ws.vec);
+        ws.n_seg = chain_segments(static_cast<long long>(l.longs) * Hv, l.max_len, 2 * sm_count());
+        ws.meta = ws.n_seg > 1 ? reinterpret_cast<float*>(base + l.ws.meta) : nullptr;
+        TileMaps maps;
+        if (encode_tile_maps(p, ws, maps)) return GDN_ERR_DRIVER;
+        int st = launch_prepare_lean(p, ws, maps, stream);
+        if (st == GDN_OK) st = launch_chain_r(p, ws, maps, stream);
+        if (st != GDN_OK) return st;
+    }
+    // short sequences: the decode kernel, neighbours of equal length in one launch
+    const size_t gate_bytes = gate_dtype == GDN_GATE_F32 ? 4 : 2;
+    for (int i = 0; i < n_seq;) {
+        const int n = cu_seqlens[i + 1] - cu_seqlens[i];
+        int j = i + 1;
+        if (n <= kDecodeMaxTokens) {
+            while (j < n_seq && cu_seqlens[j + 1] - cu_seqlens[j] == n) ++j;
+            const size_t tok = cu_seqlens[i], state = static_cast<size_t>(i) * Hv * kD * kD;
+            auto at = [](const void* x, size_t bytes) -> const void* { return static_cast<const char*>(x) + bytes; };
+            const int st = forward_device(at(q, tok * Hq * kD * 2), at(k, tok * Hq * kD * 2), at(v, tok * Hv * kD * 2),
+                                          at(g, tok * Hv * gate_bytes), at(beta, tok * Hv * gate_bytes), h0 ? h0 + state : nullptr,
+                                          static_cast<char*>(out) + tok * Hv * kD * 2, hT ? hT + state : nullptr, scratch, scratch_bytes,
+                                          j - i, n, Hq, Hv, gate_dtype, GDN_PATH_DECODE, flags, stream, clear);
+            if (st != GDN_OK) return st;
+            clear = false;
+        }
+        i = j;
+    }
+    return GDN_OK;
+}
+
+}  // extern "C"

@@ -86,6 +86,7 @@ inline int chain_segments(long long seqs, int S, int slots) {
     if (g > NT / 4) g = NT / 4;
     return g < 2 ? 1 : g;
 }
+constexpr int kDecodeMaxTokens = 8;   // sequences this short take the decode kernel under GDN_PATH_AUTO
 constexpr float kForgetLn = -115.f;   // exp(-115) < 2^-149: a transfer matrix bounded by it is zero in fp32
 
 // Device status codes written by kernels (0 = fine).  The low byte says which wait gave up.
@@ -109,8 +110,14 @@ int launch_chain(const Problem& p, const Workspace& ws, int nv, cudaStream_t str
 // The two kernels of the automatic path: "lean" prepare (P, T'', factors; no W) and the transposed chain that applies T'' to
 // the residual V - exp(gamma) K S, one CTA per (sequence, value head[, segment]); with ws.n_seg > 1 sequences may be cut
 // into up to that many segments (gdn_segment_plan.cuh).
-int launch_prepare_lean(const Problem& p, const Workspace& ws, cudaStream_t stream);
-int launch_chain_r(const Problem& p, const Workspace& ws, cudaStream_t stream);
+// TMA descriptors both of them read (128 bytes each, CUtensorMap): q, k, v as 64 x 64 boxes, P and T'' (at the start of the
+// U array) as 64 x 64 boxes.  Encoded once per call: each encoding costs the host 0.1-0.2 microseconds.
+struct alignas(64) TileMaps {
+    unsigned char q[128], k[128], v[128], p[128], t2[128];
+};
+int encode_tile_maps(const Problem& p, const Workspace& ws, TileMaps& maps);
+int launch_prepare_lean(const Problem& p, const Workspace& ws, const TileMaps& maps, cudaStream_t stream);
+int launch_chain_r(const Problem& p, const Workspace& ws, const TileMaps& maps, cudaStream_t stream);
 // Single-launch variant (prepare shared among the four column CTAs of a head, chain in the same kernel);
 // only when all CTAs fit on the GPU at once.
 bool coop_supported(const Problem& p);
@@ -131,8 +138,6 @@ inline int encode_tma_bf16(void* tmap_out, const void* base, int rank, const uns
 // stores and the chain side loads for W and P), and U as nv x 64 boxes (swizzle span 2*nv bytes) for the chain's
 // column slice.  tu_load may be null.
 int encode_workspace_maps(const Problem& p, const Workspace& ws, void* tw, void* tp, void* tu_store, void* tu_load, int nv);
-// TMA descriptors of P and T'' (at the start of the U array) as 64x64 bf16 boxes.
-int encode_tile_maps(const Problem& p, const Workspace& ws, void* tp, void* tt2);
 // Number of SMs of the current device (cached per device).
 int sm_count();
 cudaError_t launch_rmsnorm_gated(const void* y, const void* z, const void* weight, void* out, long long n_rows,

@@ -163,6 +163,38 @@ def _forward(q, k, v, g, beta, output_final_state, initial_state, path, l2norm=F
     return out, hT
 
 
+def _forward_packed(q, k, v, g, beta, cu, output_final_state, initial_state, l2norm, gate_act):
+    """One pass over a packed batch (checked by the caller): [1, T, ...] tensors, cu the list of boundaries."""
+    import ctypes
+    lib = _lib.load()
+    dev = q.device
+    for name, x in (("k", k), ("v", v), ("g", g), ("beta", beta)):
+        if x.device != dev:
+            raise ValueError(f"{name} is on {x.device}, q on {dev}")
+    q, k, v = (x.to(torch.bfloat16).contiguous() for x in (q, k, v))
+    if g.dtype == torch.bfloat16 and beta.dtype == torch.bfloat16:
+        g, beta = g.contiguous(), beta.contiguous()
+        gate = _lib.GATE_BF16
+    else:
+        g, beta = g.float().contiguous(), beta.float().contiguous()
+        gate = _lib.GATE_F32
+    Hk, Hv, T, n_seq = q.size(2), v.size(2), q.size(1), len(cu) - 1
+    h0 = None if initial_state is None else initial_state.to(device=dev, dtype=torch.float32).contiguous()
+    out = torch.empty((1, T, Hv, GDN_D), dtype=torch.bfloat16, device=dev)
+    hT = torch.empty((n_seq, Hv, GDN_D, GDN_D), dtype=torch.float32, device=dev) if output_final_state else None
+    bounds = (ctypes.c_int * (n_seq + 1))(*cu)
+    with torch.cuda.device(dev):
+        scratch = _scratch_for(dev, int(lib.gdn_chunk_varlen_scratch_bytes(bounds, n_seq, Hv)))
+        st = lib.gdn_chunk_fwd_varlen_sm100(
+            q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr(), beta.data_ptr(), None if h0 is None else h0.data_ptr(),
+            out.data_ptr(), None if hT is None else hT.data_ptr(), scratch.data_ptr(), scratch.numel(), bounds, n_seq,
+            Hk, Hv, gate, _flags(l2norm, gate_act), torch.cuda.current_stream(dev).cuda_stream)
+        _lib.check(st, "gdn_chunk_fwd_varlen_sm100")
+        if os.environ.get("GDN_CHUNK_CHECK_STATUS", "0") == "1":
+            check_device_status(dev)
+    return out, hT
+
+
 def check_device_status(device=None):
     """Synchronise every stream of `device` this module has launched on and raise if a kernel on any of them
     reported a bounded wait that ran out (its result is then undefined).  Callers that launch asynchronously and
@@ -293,11 +325,13 @@ def gdn_chunk_varlen(q, k, v, g, beta, cu_seqlens, output_final_state=True, init
     over `n_streams` streams that are ordered after, and joined back into, the current stream.  Neighbouring
     sequences of equal length form a regular batch and share one launch (a packed batch of single tokens is one
     launch of the decode kernel).
-    strategy: "views" as described; "padded" gathers all sequences into one regular batch [n_seq, L_max, ...] whose
+    strategy: "views" as described; "packed" runs all sequences in one pass of the kernels, which find each chunk's
+    sequence through small tables (no padding, no copies, C ABI: gdn_chunk_fwd_varlen_sm100; sequences of at most 8
+    tokens take the decode kernel); "padded" gathers all sequences into one regular batch [n_seq, L_max, ...] whose
     padding tokens carry g = 0 and beta = 0 (they leave the state untouched and their outputs are dropped, so the
-    result is exact), runs one forward pass and scatters the outputs back - two extra passes over the data, but one
-    launch however many sequences there are; "auto" pads when there are more than 8 launches to make and padding
-    at most doubles the token count.  The reference has no
+    result is exact), runs one forward pass and scatters the outputs back - two extra passes over the data; "auto" is
+    "packed", or with a forced path "padded" when
+    there are more than 8 launches to make and padding at most doubles the token count, else "views".  The reference has no
     variable-length entry; its recurrent torch definition (reference/gdn_chunk_ref.py:103-147) applied per sequence
     defines the result.  initial_state / returned final state: [n_seq, Hv, D, D]; `options` are gdn_chunk's keywords
     (path, use_qk_l2norm_in_kernel, gate_activations).
@@ -318,6 +352,13 @@ def gdn_chunk_varlen(q, k, v, g, beta, cu_seqlens, output_final_state=True, init
     if not q.is_cuda:
         raise RuntimeError("gdn_chunk_varlen needs CUDA tensors (sm_100a); there is no CPU path")
     dev = q.device
+    if strategy not in ("auto", "views", "packed", "padded"):
+        raise ValueError(f"unknown strategy {strategy!r}")
+    if strategy == "packed" or (strategy == "auto" and options.get("path", "auto") == "auto"):
+        out, states = _forward_packed(q, k, v, g, beta, cu, output_final_state, initial_state,
+                                      bool(options.get("use_qk_l2norm_in_kernel", False)),
+                                      bool(options.get("gate_activations", False)))
+        return (out[0] if squeeze else out), states
     q, k, v, g, beta = (x.contiguous() for x in (q, k, v, g, beta))
     out = torch.empty((1, T, Hv, GDN_D), dtype=torch.bfloat16, device=dev)
     states = torch.empty((n_seq, Hv, GDN_D, GDN_D), dtype=torch.float32, device=dev) if output_final_state else None
@@ -333,8 +374,6 @@ def gdn_chunk_varlen(q, k, v, g, beta, cu_seqlens, output_final_state=True, init
             runs[-1][1] += 1
         else:
             runs.append([i, 1, n])
-    if strategy not in ("auto", "views", "padded"):
-        raise ValueError(f"unknown strategy {strategy!r}")
     l_max = max(r[2] for r in runs)
     if strategy == "padded" or (strategy == "auto" and len(runs) > 8 and n_seq * l_max <= 2 * T):
         import numpy as np

@@ -31,7 +31,7 @@ extern "C" {
 #define GDN_GATE_F32 1
 
 /* execution path */
-#define GDN_PATH_AUTO 0          /* DECODE when S <= 8; COOP when S <= 1024 and 4*B*Hv <= #SMs; else TWOPASS_T     */
+#define GDN_PATH_AUTO 0          /* DECODE when S <= 8, else TWOPASS_T                                          */
 #define GDN_PATH_SIMT 1          /* token-by-token fp32 kernel on CUDA cores (exact; slow; for checks) */
                                  /* (values 2, 3 and 10 belonged to kernels that have been removed)    */
 #define GDN_PATH_TWOPASS_NV64 4  /* prepare kernel + chain kernel, 64 value columns per chain CTA    */
@@ -140,6 +140,20 @@ size_t gdn_chunk_host_arena_bytes(int B, int S, int Hq, int Hv, int gate_dtype, 
 int gdn_chunk_fwd_host_sm100(const void* q, const void* k, const void* v, const void* g, const void* beta,
                              const float* h0, void* out, float* hT, void* arena, size_t arena_bytes, int B, int S,
                              int Hq, int Hv, int gate_dtype, int seg_tokens, unsigned flags, void* stream);
+
+/*
+ * The forward pass over a packed batch: n_seq sequences of different lengths laid end to end, sequence i = tokens
+ * [cu_seqlens[i], cu_seqlens[i+1]) of q, k [1,T,Hq,128], v, out [1,T,Hv,128], g, beta [1,T,Hv]; h0, hT
+ * [n_seq,Hv,128,128].  cu_seqlens is a HOST array of n_seq + 1 strictly rising ints from 0 to T, read during the call.
+ * One pass whatever the lengths (no padding, no copies); sequences of at most 8 tokens take the decode kernel.
+ * Results are those of gdn_chunk_fwd_sm100_ex (GDN_PATH_AUTO) on each sequence.  scratch: 256-byte aligned device memory of
+ * gdn_chunk_varlen_scratch_bytes(...) bytes.  Launches on `stream`, does not wait.  The reference has no counterpart; its
+ * recurrent torch definition (gdn_qsa_sm80/reference/gdn_chunk_ref.py:103-147) per sequence defines the result.
+ */
+size_t gdn_chunk_varlen_scratch_bytes(const int* cu_seqlens, int n_seq, int Hv);
+int gdn_chunk_fwd_varlen_sm100(const void* q, const void* k, const void* v, const void* g, const void* beta, const float* h0,
+                               void* out, float* hT, void* scratch, size_t scratch_bytes, const int* cu_seqlens, int n_seq,
+                               int Hq, int Hv, int gate_dtype, unsigned flags, void* stream);
 
 /*
  * Gated RMS normalisation of rows of 128 bf16 values, the step after gdn_chunk in the layer:
