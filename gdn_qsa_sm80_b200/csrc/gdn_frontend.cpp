@@ -34,8 +34,7 @@ bool plain(const at::Tensor& t, at::ScalarType dtype, const at::Device& dev) {
            !t.is_conj();
 }
 
-// forward(q, k, v, g, beta, output_final_state, initial_state, path, flags, output_gate) -> (out, state) or None
-PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+PyObject* forward_plain(PyObject* const* a, Py_ssize_t n) {
     if (n != 10) {
         PyErr_SetString(PyExc_TypeError, "forward takes 10 arguments");
         return nullptr;
@@ -102,13 +101,8 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     void* scratch = it->second.data_ptr();
     const size_t scratch_bytes = static_cast<size_t>(it->second.numel());
 
-    at::Tensor out, hT;
-    try {
-        out = at::Tensor(at::detail::empty_cuda({B, S, Hv, GDN_D}, at::kBFloat16, dev, std::nullopt));
-        if (want_state) hT = at::Tensor(at::detail::empty_cuda({B, Hv, GDN_D, GDN_D}, at::kFloat, dev, std::nullopt));
-    } catch (...) {
-        Py_RETURN_NONE;   // the wrapper meets the same error and reports it
-    }
+    at::Tensor out(at::detail::empty_cuda({B, S, Hv, GDN_D}, at::kBFloat16, dev, std::nullopt)), hT;
+    if (want_state) hT = at::Tensor(at::detail::empty_cuda({B, Hv, GDN_D, GDN_D}, at::kFloat, dev, std::nullopt));
     float* state = want_state ? hT.mutable_data_ptr<float>() : nullptr;
     const int gate_code = gate == at::kFloat ? GDN_GATE_F32 : GDN_GATE_BF16;
     const int st = z ? gdn_chunk_fwd_gated_sm100(q.const_data_ptr(), k.const_data_ptr(), v.const_data_ptr(), g.const_data_ptr(), beta.const_data_ptr(), h0,
@@ -138,6 +132,18 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     PyTuple_SET_ITEM(r, 0, po);
     PyTuple_SET_ITEM(r, 1, ps);
     return r;
+}
+
+// forward(q, k, v, g, beta, output_final_state, initial_state, path, flags, output_gate) -> (out, state) or None
+PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    // tensors without storage (fake, batched, nested) throw when their size or address is asked for; no exception may
+    // leave a function the interpreter called, and the wrapper meets the same error and reports it
+    try {
+        return forward_plain(a, n);
+    } catch (...) {
+        if (PyErr_Occurred()) return nullptr;
+        Py_RETURN_NONE;
+    }
 }
 
 // note_scratch(device index, stream handle, tensor): the buffer calls on that stream use from now on
