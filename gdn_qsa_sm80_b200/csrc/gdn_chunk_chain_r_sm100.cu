@@ -554,9 +554,19 @@ int launch_chain_r(const Problem& p, const Workspace& ws, const TileMaps& maps, 
         if (allow_smem(reinterpret_cast<const void*>(kernel), kRDynamic)) return GDN_ERR_CUDA;
         // The value heads that share a qk head read the same K and Q tiles: as a cluster of two CTAs they start together
         // and run in step, so the second read of a tile finds it in L2 (nothing else of the cluster is used).
-        const cudaError_t e = launch_dependent(kernel, dim3(p.Hv, p.pk_chunk ? p.pk_n : p.B, gz), dim3(kRThreads), kRDynamic, stream,
-                                               (p.Hv / p.Hq) % 2 == 0, map(maps.q), map(maps.k), map(maps.v), map(maps.p), map(maps.t2), p, ws);
-        return e == cudaSuccess ? GDN_OK : GDN_ERR_CUDA;
+        // A grid's y ends at 65535: a packed batch of more sequences takes several launches.
+        Problem part = p;
+        for (int done = 0, all = p.pk_chunk ? p.pk_n : 1; done < all; done += 65535) {
+            unsigned gy = static_cast<unsigned>(p.B);
+            if (p.pk_chunk) {
+                part.pk_order = p.pk_order + done;
+                gy = static_cast<unsigned>(all - done < 65535 ? all - done : 65535);
+            }
+            if (launch_dependent(kernel, dim3(p.Hv, gy, gz), dim3(kRThreads), kRDynamic, stream, (p.Hv / p.Hq) % 2 == 0, map(maps.q), map(maps.k),
+                                 map(maps.v), map(maps.p), map(maps.t2), part, ws) != cudaSuccess)
+                return GDN_ERR_CUDA;
+        }
+        return GDN_OK;
     };
     const int G = ws.n_seg;
     if (G <= 1 || G > kMaxSegments || !ws.meta) return go(gdn_chain_r_kernel<false>, 1);

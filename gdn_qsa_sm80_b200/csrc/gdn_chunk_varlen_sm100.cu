@@ -10,7 +10,6 @@
 // Without this a packed batch was gathered into a padded one and scattered back (torch indexing: two passes over all
 // tensors, and the padding's share of the work), or ran sequence by sequence.
 #include <algorithm>
-#include <numeric>
 #include <vector>
 
 #include "../../include/gdn_chunk_sm100.h"
@@ -104,12 +103,18 @@ int gdn_chunk_fwd_varlen_sm100(const void* q, const void* k, const void* v, cons
     bool clear = true;                // whichever kernel comes first clears the status word
 
     if (l.longs > 0) {
-        std::vector<int> rank(n_seq), order;
-        order.reserve(l.longs);
+        std::vector<int> rank, order;
+        try {
+            rank.resize(n_seq);
+            order.reserve(l.longs);
+        } catch (...) {               // nothing may be thrown through a C entry
+            return GDN_ERR_SCRATCH;
+        }
         for (int i = 0; i < n_seq; ++i)
             if (cu_seqlens[i + 1] - cu_seqlens[i] > kDecodeMaxTokens) order.push_back(i);
-        std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
-            return cu_seqlens[a + 1] - cu_seqlens[a] > cu_seqlens[b + 1] - cu_seqlens[b];
+        std::sort(order.begin(), order.end(), [&](int a, int b) {
+            const int x = cu_seqlens[a + 1] - cu_seqlens[a], y = cu_seqlens[b + 1] - cu_seqlens[b];
+            return x != y ? x > y : a < b;
         });
         for (int r = 0; r < l.longs; ++r) rank[order[r]] = r;
         int* d_cu = reinterpret_cast<int*>(base + l.cu);

@@ -354,7 +354,10 @@ def gdn_chunk_varlen(q, k, v, g, beta, cu_seqlens, output_final_state=True, init
     dev = q.device
     if strategy not in ("auto", "views", "packed", "padded"):
         raise ValueError(f"unknown strategy {strategy!r}")
-    if strategy == "packed" or (strategy == "auto" and options.get("path", "auto") == "auto"):
+    # (the kernels want 16-byte aligned tensors; strided or converted ones are copied, a view at an odd offset is not and
+    # takes the routes below, which gather it or refuse it)
+    aligned = all(x is None or x.data_ptr() % 16 == 0 for x in (q, k, v, initial_state))
+    if strategy == "packed" or (strategy == "auto" and aligned and options.get("path", "auto") == "auto"):
         out, states = _forward_packed(q, k, v, g, beta, cu, output_final_state, initial_state,
                                       bool(options.get("use_qk_l2norm_in_kernel", False)),
                                       bool(options.get("gate_activations", False)))

@@ -59,3 +59,17 @@ def test_infinities_stay_in_their_sequence(layer):
     check_device_status()
     keep = list(range(70)) + list(range(110, 310))
     assert torch.equal(out[:, keep], clean_o[:, keep]) and torch.equal(st[[0, 2]], clean_s[[0, 2]])
+
+
+def test_views_at_odd_offsets_are_gathered():
+    """More than eight lengths and little padding: such a batch ran before the packed route existed, by gathering."""
+    lens = list(range(40, 50))
+    T, cu = sum(lens), np.concatenate([[0], np.cumsum(lens)]).tolist()
+    q, k, v, g, beta, _ = make_inputs("default", seed=3, B=1, S=T, Hq=1, Hv=2)
+    d = [t.cuda() for t in (q, k, v, g, beta)]
+    want = gdn_chunk_varlen(*d, cu)
+    odd = torch.empty(q.numel() + 1, dtype=q.dtype, device="cuda")[1:].view(q.shape).copy_(d[0])
+    assert odd.is_contiguous() and odd.data_ptr() % 16
+    got = gdn_chunk_varlen(odd, *d[1:], cu)
+    for a, b in zip(got, want):
+        assert ((a.float() - b.float()).norm() / b.float().norm()).item() <= 1e-2   # (padding changes where a chunk ends)
