@@ -223,15 +223,14 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
             ws.meta[2 * tile] = ps.gam[kChunk - 1] * (1.f / kLog2e);
             ws.meta[2 * tile + 1] = ps.gates_ok ? fmaxf(ps.bound[0], ps.bound[1]) : INFINITY;
         }
-        lean_invert_level2(At, ctx);
+        lean_finish_T2(At, ps.bet, t2tile, ctx);
         GDN_PHASE(4)
-        if (warp == 0 && more) {   // the next item's product, into the other accumulator (read last an item ago)
+        if (warp == 3 && more) {   // the next item's product, into the other accumulator (read last an item ago)
             ok = mbar_wait(&bar_tma, ph ^ 1, p.status, kDevTimeoutTma);
             if (ok && elect_one()) issue_product(tmem + (ph ^ 1) * 64);
             __syncwarp();
         }
         GDN_PHASE(5)
-        lean_store_T2(At, ps.bet, i, htid >> 6, t2tile, ctx);
         fence_proxy_async_smem();
         ctx.sync();
         if (hwarp == 0 && elect_one()) {

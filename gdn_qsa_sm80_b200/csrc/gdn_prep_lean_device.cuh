@@ -1,9 +1,8 @@
 // Device-side pieces of the "lean" prepare (gdn_chunk_prepare_lean_sm100.cu): the gate cumsum by one warp, the mask
 // epilogues that write straight to their shared-memory destination, and the 64x64 unit-lower-triangular inverse IN
 // PLACE.  Same mathematics as gdn_prep_device.cuh; what differs is what has to fit: three CTAs of two heads per SM
-// leave 73 KB of shared memory and 80 registers to each, so A, T and the merge temporaries share one 64 x 68 fp32 array:
-// T overwrites A block by block, and the temporaries live in the block above the two 32x32 diagonal blocks (rows
-// 0-31, columns 32-63), which neither matrix uses.
+// leave 73 KB of shared memory and 80 registers to each, so A and T share one 64 x 68 fp32 array: T overwrites A block by
+// block.
 #pragma once
 
 #include "gdn_common.cuh"
@@ -184,13 +183,67 @@ __device__ __forceinline__ float lean_bound_of_rows(const LeanScratch& ps, bool 
 }
 
 // In-place inverse of I + A (A strictly lower triangular, zeros on and above its diagonal inside the 32x32 diagonal
-// blocks) in `At`, row stride kSolveStride.  The merge temporaries use the block above the diagonal (rows 0-31, columns
-// 32-63), so neither function leaves anything defined there.
+// blocks) in `At`, row stride kSolveStride.  The block above the two 32x32 diagonal blocks (rows 0-31, columns 32-63) is not used.
+//
+// What bounds the prepare kernel is the shared-memory pipe: it delivers one word to every lane per cycle, so a broadcast
+// float4 costs as much as 512 bytes of data.  (With the 8 -> 16 level on CUDA cores, Y = A21 X11 passed through shared memory
+// at every level and T read back for its conversion, that pipe was busy 72 % of the kernel's time.)  Products are therefore
+// taken as (X22 A21) X11 with the accumulator of the first kept in registers as the A fragment of the second: an accumulator
+// holds columns (2t, 2t + 1) where an A fragment wants k = (t, t + 4), so the second product runs over k in that order and
+// its B fragments are rows 2t, 2t + 1 - which also lie in different banks.  Per call, before and after: 16 sequences of 2048
+// tokens 418 -> 389 us, one of 8192 tokens 121.6 -> 117.0 us, 64 of 4096 tokens 3127 -> 2967 us.
 
-// One warp: the 32x32 diagonal block p.  8x8 blocks by forward substitution in fp32 registers, 8 -> 16 in fp32,
-// 16 -> 32 with TF32 warp MMAs.  Needs the warp's own 32 rows only (a __syncwarp after they were written).
+__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
+    hi = f32_to_tf32(x) & 0xffffe000u;
+    lo = f32_to_tf32(x - __uint_as_float(hi));
+}
+// Two 8x8x8 products at once with about fp32 precision (every factor as the sum of two TF32 numbers, the product of the low
+// parts left out): d rows 0-7 = a rows 0-7 * B0, d rows 8-15 = a rows 8-15 * B1.  B fragments: words b[0] and b[step].
+__device__ __forceinline__ void mma_split(float (&d)[4], const float (&av)[4], const float* b0, const float* b1, int step) {
+    uint32_t ah[4], al[4], b0h[2], b0l[2], b1h[2], b1l[2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) split_tf32(av[i], ah[i], al[i]);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        split_tf32(b0[i * step], b0h[i], b0l[i]);
+        split_tf32(b1[i * step], b1h[i], b1l[i]);
+    }
+    float c[4] = {0.f, 0.f, 0.f, 0.f}, e[4] = {0.f, 0.f, 0.f, 0.f};
+    mma_tf32_16x8x8(c, ah, b0l);
+    mma_tf32_16x8x8(e, ah, b1l);
+    mma_tf32_16x8x8(c, al, b0h);
+    mma_tf32_16x8x8(e, al, b1h);
+    mma_tf32_16x8x8(c, ah, b0h);
+    mma_tf32_16x8x8(e, ah, b1h);
+    d[0] = c[0];
+    d[1] = c[1];
+    d[2] = e[2];
+    d[3] = e[3];
+}
+
+// x = columns [8 N0, 8 N0 + 16) of z X: z (16 x 8 NT) in accumulator fragments, X lower triangular (8 NT x 8 NT).
+template <int NT, int N0>
+__device__ __forceinline__ void mma_times_lower(float (&x)[2][4], const float (&z)[NT][4], const float* X, int lane) {
+    const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e >> 2][e & 3] = 0.f;
+#pragma unroll
+    for (int ks = N0; ks < NT; ++ks) {
+        const uint32_t a[4] = {f32_to_tf32(z[ks][0]), f32_to_tf32(z[ks][2]), f32_to_tf32(z[ks][1]), f32_to_tf32(z[ks][3])};
+#pragma unroll
+        for (int nt = N0; nt < N0 + 2; ++nt) {
+            if (nt > ks) continue;
+            const float* b = X + (8 * ks + 2 * t) * kSolveStride + 8 * nt + g;
+            const uint32_t bv[2] = {f32_to_tf32(b[0]), f32_to_tf32(b[kSolveStride])};
+            mma_tf32_16x8x8(x[nt - N0], a, bv);
+        }
+    }
+}
+
+// One warp: the 32x32 diagonal block p.  8x8 blocks by forward substitution in fp32 registers, 8 -> 16 in split TF32,
+// 16 -> 32 in TF32.  Needs the warp's own 32 rows only (a __syncwarp after they were written).
 __device__ __forceinline__ void lean_invert_diag32(float* At, int p, int lane) {
-    float* tmp = At + 16 * p * kSolveStride + 32;      // 16 rows of temporaries of this warp
+    asm volatile("" : "+r"(lane));   // (its addresses are computed here, not kept in registers across the items' loop)
     {   // four 8x8 diagonal blocks: lane = (block, column)
         const int blk = 4 * p + (lane >> 3), c = lane & 7;
         float* a = At + (8 * blk) * kSolveStride + 8 * blk;
@@ -220,61 +273,26 @@ __device__ __forceinline__ void lean_invert_diag32(float* At, int p, int lane) {
         for (int i = 0; i < 8; ++i) a[i * kSolveStride + c] = x[i];
     }
     __syncwarp();
-    {   // 8 -> 16 in fp32: X21 = -X22 (A21 X11); lane = (16-block, row r, four columns c0 ..)
-        const int b16 = 2 * p + (lane & 1), r = (lane >> 1) & 7, c0 = 4 * (lane >> 4);
-        float* a21 = At + (16 * b16 + 8 + r) * kSolveStride + 16 * b16;
-        const float* x11 = At + (16 * b16) * kSolveStride + 16 * b16 + c0;
-        const float* x22 = a21 + 8;
-        float* yb = tmp + 16 * (lane & 1);
-        {
-            const float4 a0 = *reinterpret_cast<const float4*>(a21), a1 = *reinterpret_cast<const float4*>(a21 + 4);
-            const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const float4 xv = *reinterpret_cast<const float4*>(x11 + k * kSolveStride);
-                acc.x = fmaf(av[k], xv.x, acc.x);
-                acc.y = fmaf(av[k], xv.y, acc.y);
-                acc.z = fmaf(av[k], xv.z, acc.z);
-                acc.w = fmaf(av[k], xv.w, acc.w);
-            }
-            *reinterpret_cast<float4*>(yb + r * kSolveStride + c0) = acc;
-        }
+    const int g = lane >> 2, t = lane & 3;
+    {   // 8 -> 16: X21 = -(X22 A21) X11 of the warp's two 16x16 blocks, rows 0-7 of the fragments block 0's, rows 8-15 block 1's
+        float* b0 = At + (32 * p) * kSolveStride + 32 * p;
+        float* b1 = b0 + 16 * kSolveStride + 16;
+        const float* a0 = b0 + (8 + g) * kSolveStride + 8 + t;
+        const float* a1 = b1 + (8 + g) * kSolveStride + 8 + t;
+        const float av[4] = {a0[0], a1[0], a0[4], a1[4]};
+        float z[4], x[4];
+        mma_split(z, av, b0 + (8 + t) * kSolveStride + g, b1 + (8 + t) * kSolveStride + g, 4 * kSolveStride);
+        const float zv[4] = {z[0], z[2], z[1], z[3]};   // the accumulator as an A fragment: its columns (2t, 2t + 1) are k
+        mma_split(x, zv, b0 + 2 * t * kSolveStride + g, b1 + 2 * t * kSolveStride + g, kSolveStride);
         __syncwarp();
-        {
-            const float4 b0 = *reinterpret_cast<const float4*>(x22), b1 = *reinterpret_cast<const float4*>(x22 + 4);
-            const float bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const float4 yv = *reinterpret_cast<const float4*>(yb + k * kSolveStride + c0);
-                acc.x = fmaf(-bv[k], yv.x, acc.x);
-                acc.y = fmaf(-bv[k], yv.y, acc.y);
-                acc.z = fmaf(-bv[k], yv.z, acc.z);
-                acc.w = fmaf(-bv[k], yv.w, acc.w);
-            }
-            *reinterpret_cast<float4*>(a21 + c0) = acc;
-        }
+        *reinterpret_cast<float2*>(b0 + (8 + g) * kSolveStride + 2 * t) = make_float2(-x[0], -x[1]);
+        *reinterpret_cast<float2*>(b1 + (8 + g) * kSolveStride + 2 * t) = make_float2(-x[2], -x[3]);
     }
     __syncwarp();
-    {   // 16 -> 32 with TF32 warp MMAs: Y = A21 X11, X21 = -X22 Y (16 x 16 each)
-        float* a21 = At + (32 * p + 16) * kSolveStride + 32 * p;
-        float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-#pragma unroll
-        for (int ks = 0; ks < 2; ++ks) {
-            uint32_t a[4];
-            load_a_frag(a, a21 + 8 * ks, kSolveStride, lane);
-#pragma unroll
-            for (int nt = 0; nt < 2; ++nt) {
-                uint32_t b[2];
-                load_b_frag(b, At + (32 * p + 8 * ks) * kSolveStride + 32 * p + 8 * nt, kSolveStride, lane);
-                mma_tf32_16x8x8(acc[nt], a, b);
-            }
-        }
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) store_c_frag(tmp + 8 * nt, kSolveStride, lane, acc[nt], 1.f);
-        __syncwarp();
-        float acc2[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+    {   // 16 -> 32 in TF32: X21 = -(X22 A21) X11 (16 x 16 each)
+        float* x11 = At + (32 * p) * kSolveStride + 32 * p;
+        float* a21 = x11 + 16 * kSolveStride;
+        float z[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks) {
             uint32_t a[4];
@@ -282,80 +300,81 @@ __device__ __forceinline__ void lean_invert_diag32(float* At, int p, int lane) {
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
                 uint32_t b[2];
-                load_b_frag(b, tmp + (8 * ks) * kSolveStride + 8 * nt, kSolveStride, lane);
-                mma_tf32_16x8x8(acc2[nt], a, b);
+                load_b_frag(b, a21 + (8 * ks) * kSolveStride + 8 * nt, kSolveStride, lane);
+                mma_tf32_16x8x8(z[nt], a, b);
             }
         }
+        float x[2][4];
+        mma_times_lower<2, 0>(x, z, x11, lane);
+        __syncwarp();
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt) store_c_frag(a21 + 8 * nt, kSolveStride, lane, acc2[nt], -1.f);
+        for (int nt = 0; nt < 2; ++nt) store_c_frag(a21 + 8 * nt, kSolveStride, lane, x[nt], -1.f);
     }
 }
 
-// 128 threads: the 32x32 lower-left block, X21 = -X22 (A21 X11); both diagonal blocks complete (one barrier before).
-// Ends with a group barrier.
-__device__ __forceinline__ void lean_invert_level2(float* At, PrepCtx ctx) {
-    const int warp = ctx.tid >> 5, lane = ctx.tid & 31;
-    const int rb = warp >> 1, cb = warp & 1;
-    float* y = At + 32;                                // 32 x 32, row stride kSolveStride
-    float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+// The last level, X21 = -(X22 A21) X11 on 32x32 blocks, and T'' = T diag(beta) as bf16, 128 threads; both diagonal blocks
+// are complete (one barrier before).  Warps 0 and 1 own 16 rows each of X21, which goes from the accumulators straight to
+// its bf16 place; warps 2 and 3 convert the diagonal blocks meanwhile.  The tile (128-byte swizzle) overwrites the start of
+// `At`, hence the barrier between reading and writing.
+__device__ __forceinline__ void lean_finish_T2(const float* At, const float* bet, uint8_t* tile, PrepCtx ctx) {
+    const int warp = ctx.tid >> 5;
+    int lane = ctx.tid & 31;
+    asm volatile("" : "+r"(lane));   // (see lean_invert_diag32)
+    const int g = lane >> 2, t = lane & 3;
+    if (warp < 2) {
+        const int row0 = 32 + 16 * warp;
+        float z[4][4] = {};
 #pragma unroll
-    for (int ks = 0; ks < 4; ++ks) {
-        uint32_t a[4];
-        load_a_frag(a, At + (32 + 16 * rb) * kSolveStride + 8 * ks, kSolveStride, lane);
+        for (int ks = 0; ks < 4; ++ks) {
+            if (ks >= 2 * warp + 2) continue;              // X22 is lower triangular
+            uint32_t a[4];
+            load_a_frag(a, At + row0 * kSolveStride + 32 + 8 * ks, kSolveStride, lane);
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-            if (ks < 2 * cb) continue;                 // X11 is lower triangular: rows above the column block are zero
-            uint32_t b[2];
-            load_b_frag(b, At + (8 * ks) * kSolveStride + 16 * cb + 8 * nt, kSolveStride, lane);
-            mma_tf32_16x8x8(acc[nt], a, b);
+            for (int nt = 0; nt < 4; ++nt) {
+                uint32_t b[2];
+                load_b_frag(b, At + (32 + 8 * ks) * kSolveStride + 8 * nt, kSolveStride, lane);
+                mma_tf32_16x8x8(z[nt], a, b);
+            }
         }
-    }
+        uint32_t pk[4][2];
+        auto pack_half = [&](const float (&x)[2][4], int nt0) {
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
-        store_c_frag(y + (16 * rb) * kSolveStride + 16 * cb + 8 * nt, kSolveStride, lane, acc[nt], 1.f);
-    ctx.sync();
-    float acc2[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+            for (int nt = 0; nt < 2; ++nt) {
+                const float2 b = *reinterpret_cast<const float2*>(bet + 8 * (nt0 + nt) + 2 * t);
+                pk[nt0 + nt][0] = pack_bf16x2(-x[nt][0] * b.x, -x[nt][1] * b.y);
+                pk[nt0 + nt][1] = pack_bf16x2(-x[nt][2] * b.x, -x[nt][3] * b.y);
+            }
+        };
+        float x[2][4];
+        mma_times_lower<4, 0>(x, z, At, lane);
+        pack_half(x, 0);
+        mma_times_lower<4, 2>(x, z, At, lane);
+        pack_half(x, 2);
+        ctx.sync();
+        uint8_t* dst = tile + (row0 + g) * 128 + 4 * t;    // row mod 8 = g
 #pragma unroll
-    for (int ks = 0; ks < 4; ++ks) {
-        if (ks >= 2 * rb + 2) continue;                // X22 is lower triangular
-        uint32_t a[4];
-        load_a_frag(a, At + (32 + 16 * rb) * kSolveStride + 32 + 8 * ks, kSolveStride, lane);
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-            uint32_t b[2];
-            load_b_frag(b, y + (8 * ks) * kSolveStride + 16 * cb + 8 * nt, kSolveStride, lane);
-            mma_tf32_16x8x8(acc2[nt], a, b);
+        for (int nt = 0; nt < 4; ++nt) {
+            *reinterpret_cast<uint32_t*>(dst + ((nt ^ g) << 4)) = pk[nt][0];
+            *reinterpret_cast<uint32_t*>(dst + 1024 + ((nt ^ g) << 4)) = pk[nt][1];
         }
-    }
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
-        store_c_frag(At + (32 + 16 * rb) * kSolveStride + 16 * cb + 8 * nt, kSolveStride, lane, acc2[nt], -1.f);
-    ctx.sync();
-}
-
-// T'' = T diag(beta) as bf16: 128 threads, thread = (row i, columns [32 hh, +32)); the tile (128-byte swizzle) overwrites
-// the start of `At`, hence the barrier between reading and writing.  hh and i < 32 are uniform over a warp.
-__device__ __forceinline__ void lean_store_T2(const float* At, const float* bet, int i, int hh, uint8_t* tile, PrepCtx ctx) {
-    uint4 pk[4];
-    if (hh == 1 && i < 32) {
-#pragma unroll
-        for (int c4 = 0; c4 < 4; ++c4) pk[c4] = make_uint4(0, 0, 0, 0);
     } else {
+        const int blk = warp - 2, r = lane >> 3, c = lane & 7;   // four rows at a time, four columns a lane
+        const float* src = At + (32 * blk + r) * kSolveStride + 32 * blk + 4 * c;
+        const float4 b = *reinterpret_cast<const float4*>(bet + 32 * blk + 4 * c);
+        uint2 pk[8];
 #pragma unroll
-        for (int c4 = 0; c4 < 4; ++c4) {
-            const int ch = 4 * hh + c4;
-            const float4 t0 = *reinterpret_cast<const float4*>(At + i * kSolveStride + ch * 8);
-            const float4 t1 = *reinterpret_cast<const float4*>(At + i * kSolveStride + ch * 8 + 4);
-            const float4 b0 = *reinterpret_cast<const float4*>(bet + ch * 8), b1 = *reinterpret_cast<const float4*>(bet + ch * 8 + 4);
-            pk[c4].x = pack_bf16x2(t0.x * b0.x, t0.y * b0.y);
-            pk[c4].y = pack_bf16x2(t0.z * b0.z, t0.w * b0.w);
-            pk[c4].z = pack_bf16x2(t1.x * b1.x, t1.y * b1.y);
-            pk[c4].w = pack_bf16x2(t1.z * b1.z, t1.w * b1.w);
+        for (int it = 0; it < 8; ++it) {
+            const float4 x = *reinterpret_cast<const float4*>(src + 4 * it * kSolveStride);
+            pk[it] = make_uint2(pack_bf16x2(x.x * b.x, x.y * b.y), pack_bf16x2(x.z * b.z, x.w * b.w));
+        }
+        ctx.sync();
+#pragma unroll
+        for (int it = 0; it < 8; ++it) {
+            const int row = 32 * blk + 4 * it + r;
+            *reinterpret_cast<uint2*>(tile + swz_chunk_offset<128>(row, 4 * blk + (c >> 1)) + (c & 1) * 8) = pk[it];
+            if (blk == 0 && c < 4) *reinterpret_cast<uint4*>(tile + swz_chunk_offset<128>(row, 4 + c)) = make_uint4(0, 0, 0, 0);
         }
     }
-    ctx.sync();
-#pragma unroll
-    for (int c4 = 0; c4 < 4; ++c4) *reinterpret_cast<uint4*>(tile + swz_chunk_offset<128>(i, 4 * hh + c4)) = pk[c4];
 }
 
 }  // namespace gdn
