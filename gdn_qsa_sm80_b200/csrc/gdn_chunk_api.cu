@@ -51,7 +51,8 @@ int encode_tma(void* tmap_out, const void* base, int elem_bytes, int rank, const
     const CUtensorMapDataType dt = elem_bytes == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
     const CUresult r = fn(static_cast<CUtensorMap*>(tmap_out), dt, rank,
                           const_cast<void*>(base), gdim, gstr, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
-                          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                          swizzle_bytes == 64 ? CU_TENSOR_MAP_L2_PROMOTION_L2_64B : CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? 0 : 1;
 }
 
@@ -100,8 +101,8 @@ int encode_tile_maps(const Problem& p, const Workspace& ws, TileMaps& maps) {
     const unsigned long long tiles = p.pk_chunk ? static_cast<unsigned long long>(p.pk_chunks) * p.Hv
                                                 : static_cast<unsigned long long>(p.B) * p.Hv * ((p.S + kChunk - 1) / kChunk);
     const unsigned long long d[2] = {64, tiles * kChunk}, s[1] = {128};
-    const unsigned box[2] = {64, 64};
-    return encode_tma(maps.p, ws.P, 2, 2, d, s, box, 128) || encode_tma(maps.t2, ws.U, 2, 2, d, s, box, 128);
+    const unsigned box[2] = {32, 32};
+    return encode_tma(maps.p, ws.P, 2, 2, d, s, box, 64) || encode_tma(maps.t2, ws.U, 2, 2, d, s, box, 64);
 }
 
 int sm_count() {

@@ -77,6 +77,14 @@ __device__ __forceinline__ uint64_t r_desc(uint32_t lo) {
     asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"((1024u >> 4) | (1u << 14) | (SWZ_128B << 29)));
     return d;
 }
+__device__ __forceinline__ uint64_t r_desc64(uint32_t lo) {   // triangular tiles: 64-byte rows and swizzle, 512 bytes per 8 rows
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"((512u >> 4) | (1u << 14) | (SWZ_64B << 29)));
+    return d;
+}
+// Where k step `ks` (16 columns) of a triangular tile starts: steps 0, 1 are columns of all 64 rows, 2, 3 of rows 32-63 only -
+// products with it are N = 64 and, for the later two, N = 32 into the second half of the accumulator.
+__device__ constexpr uint32_t tri_bytes(int ks) { return (ks >> 1) * 4096 + (ks & 1) * 32; }
 constexpr uint32_t kLoK = (16u >> 4) << 16, kLoMN = (8192u >> 4) << 16;
 
 // Bounded, abortable wait (see mbar_wait_abortable_a) that holds next to nothing in registers: what only its slow path
@@ -238,12 +246,17 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                     bulk_load_1d_a(sm_u32 + R_VEC + s * 1024, vec, 1024, fb);
                 }
             };
+            auto load_tri = [](uint32_t dst, const void* map, uint32_t bar, int row0) {
+                tma_load_2d_a(dst, map, bar, 0, row0);
+                tma_load_2d_a(dst + 2048, map, bar, 0, row0 + 32);
+                tma_load_2d_a(dst + 4096, map, bar, 32, row0 + 32);
+            };
             auto load_t2 = [&](int n) {
                 const uint32_t s = n & 1, fb = cb(R_TFULL + s);
                 const int row0 = static_cast<int>((work.tile0 + work.t0 + n) * kChunk);
                 if (elect_one()) {
-                    mbar_arrive_expect_tx_a(fb, 8192);
-                    tma_load_2d_a(sm_u32 + R_T2 + s * 8192, &tm_t2, fb, 0, row0);
+                    mbar_arrive_expect_tx_a(fb, kTriBytes);
+                    load_tri(sm_u32 + R_T2 + s * 8192, &tm_t2, fb, row0);
                 }
             };
             load_k(0);
@@ -271,15 +284,17 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 }
                 if (n > 0 && !wait(R_O, n - 1)) break;
                 if (elect_one()) {
-                    mbar_arrive_expect_tx_a(cb(R_PFULL), 8192);
-                    tma_load_2d_a(sm_u32 + R_P, &tm_p, cb(R_PFULL), 0, row0);
+                    mbar_arrive_expect_tx_a(cb(R_PFULL), kTriBytes);
+                    load_tri(sm_u32 + R_P, &tm_p, cb(R_PFULL), row0);
                 }
             }
         } else if (warp == 13) {
             // ------------------------------- UMMA issuer ------------------------------------------------------------
             constexpr uint32_t idesc_n64 = umma_idesc_bf16(128, 64, MAJOR_K, MAJOR_K);
-            constexpr uint32_t idesc_e0 = umma_idesc_bf16(128, 64, MAJOR_MN, MAJOR_K);
+            constexpr uint32_t idesc_n32 = umma_idesc_bf16(128, 32, MAJOR_K, MAJOR_K);
+            constexpr uint32_t idesc_e0 = umma_idesc_bf16(128, 64, MAJOR_MN, MAJOR_K), idesc_e0_n32 = umma_idesc_bf16(128, 32, MAJOR_MN, MAJOR_K);
             constexpr uint32_t idesc_neg = umma_idesc_bf16(128, 64, MAJOR_K, MAJOR_K, 1);   // negated A
+            constexpr uint32_t idesc_neg_n32 = umma_idesc_bf16(128, 32, MAJOR_K, MAJOR_K, 1);
             constexpr uint32_t idesc_e2 = umma_idesc_bf16(128, 128, MAJOR_K, MAJOR_MN);
             const uint32_t base = (sm_u32 & 0x3FFFFu) >> 4;   // (a cluster CTA's window address has bits above)
             for (int n = 0; n < steps; ++n) {
@@ -298,16 +313,16 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 if (elect_one()) {
 #pragma unroll
                     for (int ks = 0; ks < 4; ++ks)               // E0
-                        umma_bf16_ss(tmem + C_VN, r_desc(base + s * (16384 >> 4) + kLoMN + ((R_V + ks * 2048) >> 4)),
-                                     r_desc(base + s * (8192 >> 4) + kLoK + ((R_T2 + ks * 32) >> 4)), idesc_e0, ks > 0);
+                        umma_bf16_ss(tmem + C_VN + (ks >> 1) * 32, r_desc(base + s * (16384 >> 4) + kLoMN + ((R_V + ks * 2048) >> 4)),
+                                     r_desc64(base + s * (8192 >> 4) + kLoK + ((R_T2 + tri_bytes(ks)) >> 4)), ks < 2 ? idesc_e0 : idesc_e0_n32, ks > 0);
                 }
                 if (!wait(R_X, n)) break;
                 tc_fence_after_sync();
                 if (elect_one()) {
 #pragma unroll
                     for (int ks = 0; ks < 4; ++ks)               // ER
-                        umma_bf16_ts(tmem + C_VN, tmem + C_KS + (ks >> 1) * 32 + (ks & 1) * 8,
-                                     r_desc(base + s * (8192 >> 4) + kLoK + ((R_T2 + ks * 32) >> 4)), idesc_neg, 1);
+                        umma_bf16_ts(tmem + C_VN + (ks >> 1) * 32, tmem + C_KS + (ks >> 1) * 32 + (ks & 1) * 8,
+                                     r_desc64(base + s * (8192 >> 4) + kLoK + ((R_T2 + tri_bytes(ks)) >> 4)), ks < 2 ? idesc_neg : idesc_neg_n32, 1);
                     umma_commit_a(cb(R_VACC));
                 }
                 if (!wait(R_QFULL, n)) break;
@@ -333,7 +348,8 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 if (elect_one()) {
 #pragma unroll
                     for (int ks = 0; ks < 4; ++ks)               // E3
-                        umma_bf16_ts(tmem + C_O, tmem + C_VP + ks * 8, r_desc(base + kLoK + ((R_P + ks * 32) >> 4)), idesc_n64, 1);
+                        umma_bf16_ts(tmem + C_O + (ks >> 1) * 32, tmem + C_VP + ks * 8, r_desc64(base + kLoK + ((R_P + tri_bytes(ks)) >> 4)),
+                                     ks < 2 ? idesc_n64 : idesc_n32, 1);
                     umma_commit_a(cb(R_O));
                 }
             }

@@ -3,7 +3,7 @@
 //   P [64][64] bf16 (masked, scaled Q K^T),  T'' = T diag(beta) [64][64] bf16,  the per-token factors  and the two
 //   scalars of the decay bound (sum of g, max beta |k|^2)
 // - no W, no U: the chain applies T'' to the residual V - exp(gamma) K S, so nothing of size [64][128] is formed, staged
-// or written here (17 KB per chunk and head instead of 33 KB).
+// or written here, and P and T'' leave without the blocks above their diagonals (13 KB per chunk and head instead of 33 KB).
 //
 // HEADS = 2: one item = the chunk of the two value heads that share a qk head (the reference's head mapping,
 // csrc/gdn_chunk/gdn_kernel.cu:385-387): one K / Q load and one [K;Q] K^T product, then one half of the CTA per head.
@@ -119,6 +119,13 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         umma_commit(&bar_mma);
     };
 
+    auto store_tri = [&](const void* map, const uint8_t* src, size_t tile) {   // the three blocks of a triangular tile
+        const int row = static_cast<int>(tile * kChunk);
+        tma_store_2d(map, src, 0, row);
+        tma_store_2d(map, src + 2048, 0, row + 32);
+        tma_store_2d(map, src + 4096, 32, row + 32);
+    };
+
     const bool prof_on = GDN_DIAG(p.prof != nullptr && tid == 0 && blockIdx.x == 0);
     long long prof_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     long long prof_t = prof_on ? clock64() : 0, prof_n = 0;
@@ -204,7 +211,7 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                 fence_proxy_async_smem();
                 named_bar_sync(3 + h, 64);
                 if (hwarp == 2 && elect_one()) {
-                    tma_store_2d(&tm_p, ptile, 0, static_cast<int>(tile * kChunk));
+                    store_tri(&tm_p, ptile, tile);
                     tma_store_commit();
                     if (more) {
                         tma_store_wait_read();
@@ -234,7 +241,7 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         fence_proxy_async_smem();
         ctx.sync();
         if (hwarp == 0 && elect_one()) {
-            tma_store_2d(&tm_t2, t2tile, 0, static_cast<int>(tile * kChunk));
+            store_tri(&tm_t2, t2tile, tile);
             tma_store_commit();
         }
         GDN_PHASE(6)

@@ -135,7 +135,13 @@ __device__ __forceinline__ float lean_mask_row_A(const LeanScratch& ps, bool l2n
     return i < valid ? ksq : 0.f;
 }
 
-// Row i of P = tril(scale * decay * Q K^T) as bf16 into row i of a 128-byte-swizzled tile.
+// Byte offset of the 16-byte chunk `ch` (8 columns) of row `row` in a lower-triangular 64x64 bf16 tile without its upper
+// right block: 64-byte rows, 64-byte swizzle (see TileMaps).
+__device__ __forceinline__ uint32_t tri_offset(uint32_t row, uint32_t ch) {
+    return (ch < 4 ? 0u : 4096u - 2048u) + swz_chunk_offset<64>(row, ch & 3);
+}
+
+// Row i of P = tril(scale * decay * Q K^T) as bf16 into row i of a triangular tile.
 __device__ __forceinline__ void lean_mask_row_P(const LeanScratch& ps, bool l2norm, float scale0, uint32_t trow, int i,
                                                 bool low_rows, int valid, uint8_t* tile) {
     const float* gcol = l2norm ? ps.gcol : ps.gam;
@@ -143,11 +149,7 @@ __device__ __forceinline__ void lean_mask_row_P(const LeanScratch& ps, bool l2no
     const int lim = i < valid ? i : -1;
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
-        if (half == 1 && low_rows) {               // above the diagonal: zeros
-#pragma unroll
-            for (int ch = 4; ch < 8; ++ch) *reinterpret_cast<uint4*>(tile + swz_chunk_offset<128>(i, ch)) = make_uint4(0, 0, 0, 0);
-            break;
-        }
+        if (half == 1 && low_rows) break;          // above the diagonal
         uint32_t r[32];
         tmem_ld_x32(trow + half * 32, r);
         tmem_ld_wait();
@@ -168,7 +170,7 @@ __device__ __forceinline__ void lean_mask_row_P(const LeanScratch& ps, bool l2no
             pk.y = pack_bf16x2(x[2], x[3]);
             pk.z = pack_bf16x2(x[4], x[5]);
             pk.w = pack_bf16x2(x[6], x[7]);
-            *reinterpret_cast<uint4*>(tile + swz_chunk_offset<128>(i, 4 * half + ch)) = pk;
+            *reinterpret_cast<uint4*>(tile + tri_offset(i, 4 * half + ch)) = pk;
         }
     }
 }
@@ -314,8 +316,8 @@ __device__ __forceinline__ void lean_invert_diag32(float* At, int p, int lane) {
 
 // The last level, X21 = -(X22 A21) X11 on 32x32 blocks, and T'' = T diag(beta) as bf16, 128 threads; both diagonal blocks
 // are complete (one barrier before).  Warps 0 and 1 own 16 rows each of X21, which goes from the accumulators straight to
-// its bf16 place; warps 2 and 3 convert the diagonal blocks meanwhile.  The tile (128-byte swizzle) overwrites the start of
-// `At`, hence the barrier between reading and writing.
+// its bf16 place; warps 2 and 3 convert the diagonal blocks meanwhile.  The tile overwrites the start of `At`,
+// hence the barrier between reading and writing.
 __device__ __forceinline__ void lean_finish_T2(const float* At, const float* bet, uint8_t* tile, PrepCtx ctx) {
     const int warp = ctx.tid >> 5;
     int lane = ctx.tid & 31;
@@ -351,11 +353,10 @@ __device__ __forceinline__ void lean_finish_T2(const float* At, const float* bet
         mma_times_lower<4, 2>(x, z, At, lane);
         pack_half(x, 2);
         ctx.sync();
-        uint8_t* dst = tile + (row0 + g) * 128 + 4 * t;    // row mod 8 = g
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
-            *reinterpret_cast<uint32_t*>(dst + ((nt ^ g) << 4)) = pk[nt][0];
-            *reinterpret_cast<uint32_t*>(dst + 1024 + ((nt ^ g) << 4)) = pk[nt][1];
+            *reinterpret_cast<uint32_t*>(tile + tri_offset(row0 + g, nt) + 4 * t) = pk[nt][0];
+            *reinterpret_cast<uint32_t*>(tile + tri_offset(row0 + 8 + g, nt) + 4 * t) = pk[nt][1];
         }
     } else {
         const int blk = warp - 2, r = lane >> 3, c = lane & 7;   // four rows at a time, four columns a lane
@@ -370,9 +371,7 @@ __device__ __forceinline__ void lean_finish_T2(const float* At, const float* bet
         ctx.sync();
 #pragma unroll
         for (int it = 0; it < 8; ++it) {
-            const int row = 32 * blk + 4 * it + r;
-            *reinterpret_cast<uint2*>(tile + swz_chunk_offset<128>(row, 4 * blk + (c >> 1)) + (c & 1) * 8) = pk[it];
-            if (blk == 0 && c < 4) *reinterpret_cast<uint4*>(tile + swz_chunk_offset<128>(row, 4 + c)) = make_uint4(0, 0, 0, 0);
+            *reinterpret_cast<uint2*>(tile + tri_offset(32 * blk + 4 * it + r, 4 * blk + (c >> 1)) + (c & 1) * 8) = pk[it];
         }
     }
 }
