@@ -124,6 +124,9 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
         const int rg = lane & 7, ch = half * 4 + (lane >> 3); // rows rg, rg + 8, ...; 16-byte chunk of a 128-byte row
         const uint32_t off0 = rg * 128 + ((ch ^ rg) << 4);    // the same chunk in every row = rg mod 8
         const float scale = rsqrtf(static_cast<float>(kD));
+        // Slot of ssq: changes with every row of the CTA, across work items too.  Between a warp's reads of a slot and its next
+        // write to it lies the other slot's barrier, which every warp reaches only after those reads.
+        int slot = 0;
         int n = 0;
         for (int it = first; it < items; it += step, ++n) {
             const int s = n % kDecStages;
@@ -218,11 +221,12 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
                     ss = fmaf(a[1], a[1], ss); ss = fmaf(a[2], a[2], ss); ss = fmaf(a[3], a[3], ss);
                     ss += __shfl_xor_sync(0xffffffffu, ss, 8);
                     ss += __shfl_xor_sync(0xffffffffu, ss, 16);
-                    if (lane == 0) ssq[t & 1][warp] = ss;
-                    named_bar_sync(1, GROUPS * 64);       // (the next token writes the other slot)
+                    if (lane == 0) ssq[slot][warp] = ss;
+                    named_bar_sync(1, GROUPS * 64);
                     float tot = 0.f;
 #pragma unroll
-                    for (int w = 0; w < GROUPS * 2; ++w) tot += ssq[t & 1][w];
+                    for (int w = 0; w < GROUPS * 2; ++w) tot += ssq[slot][w];
+                    slot ^= 1;
                     const float rstd = rsqrtf(tot * (1.f / 128.f) + gate.eps);
                     const float z4[4] = {__uint_as_float(zr.x << 16), __uint_as_float(zr.x & 0xffff0000u),
                                          __uint_as_float(zr.y << 16), __uint_as_float(zr.y & 0xffff0000u)};

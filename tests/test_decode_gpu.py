@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 import torch
 
-from gdn_qsa_sm80 import gdn_chunk
+from gdn_qsa_sm80 import gdn_chunk, rmsnorm_gated
 from gdn_qsa_sm80_b200.gdn_chunk_interface import check_device_status
 from gdn_qsa_sm80_b200.synthetic import make_inputs
 from oracle import gdn_chunk_oracle as O
@@ -71,3 +71,33 @@ def test_decode_updates_the_state_in_place_through_the_c_abi():
     assert st == _lib.GDN_OK
     torch.cuda.synchronize()
     assert torch.equal(out, ref_o) and torch.equal(state, ref_s)
+
+
+@pytest.mark.parametrize("B,S,Hq,Hv", [(1, 1, 2, 4), (64, 1, 16, 32), (40, 3, 8, 16), (5, 4, 1, 4), (75, 5, 4, 8), (40, 8, 8, 16)])
+@pytest.mark.parametrize("gates", ["fp32", "bf16"])
+@pytest.mark.parametrize("stored", [True, False])
+def test_gated_decode(B, S, Hq, Hv, gates, stored):
+    """Normalisation fused into the decode kernel: fewer states than SMs and up to 14 per CTA (148 SMs), more tokens than travel
+    with the tile (4), with and without states.  The row that is normalised is the ungated call's; what may differ from the separate
+    normalisation is the order of its fp32 sums: one bf16 rounding, 2^-8 relative at most on either side."""
+    q, k, v, g, beta, _ = make_inputs("default", seed=B + S, B=B, S=S, Hq=Hq, Hv=Hv)
+    if gates == "bf16":
+        g, beta = g.bfloat16(), beta.bfloat16()
+    gen = torch.Generator().manual_seed(S)
+    z = (1.5 * torch.randn(B, S, Hv, 128, generator=gen)).bfloat16().cuda()
+    w = (1 + 0.1 * torch.randn(128, generator=gen)).bfloat16().cuda()
+    h0 = torch.randn(B, Hv, 128, 128, generator=gen).cuda() if stored else None
+    d = [t.cuda() for t in (q, k, v, g, beta)]
+    plain, st = gdn_chunk(*d, output_final_state=stored, initial_state=h0)
+    ref = rmsnorm_gated(plain, z, w).float()
+    for _ in range(20):   # the same bits every time: the partial sums of a row meet no other row's
+        out, st2 = gdn_chunk(*d, output_final_state=stored, initial_state=h0, output_gate=(z, w))
+        first = out if _ == 0 else first
+        assert torch.equal(out, first)
+    check_device_status()
+    assert (st is None and st2 is None) or torch.equal(st, st2)
+    assert ((first.float() - ref).abs() <= 2.0 ** -7 * ref.abs() + 1e-6).all()
+    if B * S * Hv <= 2048:
+        ro, _ = oracle_f32(q, k, v, g, beta, None if h0 is None else h0.cpu(), form="recurrent")
+        ro = O.rmsnorm_gated(ro, z.float().cpu().numpy(), w.float().cpu().numpy())
+        assert O.rel_l2(first.float().cpu().numpy(), ro) < 6e-3   # two bf16 roundings: the row, then the result
