@@ -189,7 +189,7 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     if (SPLIT) {
         __syncthreads();
         const int nt = work.steps;
-        plan_segments<kRThreads>(ws.meta + 2 * work.tile0, nt, ws.n_seg, reinterpret_cast<float*>(sm), plan, &plan_best);
+        plan_segments<kRThreads>(ws.meta + 2 * work.tile0, nt, ws.n_seg, reinterpret_cast<unsigned*>(sm), plan, &plan_best);
         if (tid == 0) {
             const int seg = static_cast<int>(blockIdx.z), g = plan.g;
             if (g > 1) {

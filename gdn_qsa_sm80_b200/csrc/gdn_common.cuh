@@ -78,9 +78,10 @@ inline WorkspaceLayout workspace_layout(size_t tiles, bool with_meta = false) {
 // the device, gdn_segment_plan.cuh): as many CTAs as the GPU holds at once, segments of at least four chunks on average.
 // `slots`: CTAs the GPU holds at once.  A function of the shape and of the SM count alone.
 constexpr int kMaxSegments = 15;
+constexpr int kPlanChunks = 24000;   // the prefix sums of a head have to fit the ring's shared memory
 inline int chain_segments(long long seqs, int S, int slots) {
     const int NT = (S + kChunk - 1) / kChunk;
-    if (seqs * 2 > slots || NT > 24000) return 1;    // (the prefix sums of a head have to fit the ring's shared memory)
+    if (seqs * 2 > slots || NT > kPlanChunks) return 1;
     int g = static_cast<int>(slots / seqs);
     if (g > kMaxSegments) g = kMaxSegments;
     if (g > NT / 4) g = NT / 4;

@@ -1,4 +1,4 @@
-// How a long sequence is cut into segments that run as independent CTAs of one launch (both transposed chains).
+// How a long sequence is cut into segments that run as independent CTAs of one launch of the chain.
 //
 // The second level of the reference's scan has the same purpose (csrc/gdn_chunk/gdn_ops.cu:1002-1012,
 // gdn_scan_stage1.cu:7-18); here it rests on an exact bound instead of a propagated transfer matrix.  A stretch of tokens
@@ -8,6 +8,13 @@
 // state.  So a segment s >= 1 starts from a ZERO state p chunks before its first chunk, p the shortest stretch ending at
 // the boundary whose sum of g is below -115 ("warm-up": its outputs are not stored), and from its first chunk on its state,
 // its outputs and its final state are those of the serial run.
+//
+// The sums are prefix sums, and a difference of two prefixes has to be the sum of what lies between them whatever lies in front: in
+// fp32 a gate of -1e9 (a reset, a mask's fill value) leaves prefixes with a spacing of 64 and more, and a rounding step behind it read
+// as "-128, forgotten" where the decay was -2 (errors up to 100 % behind such a boundary).  So they are integers:
+// -sum of g in units of 2^-10, rounded towards zero (a boundary counts as forgotten late, never early), and a chunk counts
+// 128 at most - one below -115 forgets on its own.  kPlanChunks of them stay below 2^32, and integer sums are exact and monotone,
+// which the binary search needs.
 //
 // Every CTA of a head makes the same plan from the per-chunk scalars the prepare kernel left: for each number of segments
 // g up to the launch's most (a warp each), equal segments first, then segment 0, which has no warm-up, longer by about the
@@ -26,14 +33,18 @@ struct SegmentPlan {          // segment 0 = chunks [0, L0), segment s >= 1 = L1
     int warm[kMaxSegments];    // chunks of warm-up before each segment s >= 1
 };
 
-// Smallest p <= t0 whose chunks [t0 - p, t0) sum to less than kForgetLn (pre: prefix sums, non-increasing); 0 = none.
-__device__ __forceinline__ int forget_stretch(const float* pre, int t0) {
-    const float at = pre[t0];
-    if (!(at - pre[0] < kForgetLn)) return 0;
+constexpr float kForgetScale = 1024.f, kForgetCap = 128.f;
+constexpr unsigned kForget = static_cast<unsigned>(-kForgetLn * kForgetScale);
+static_assert(kForgetCap > -kForgetLn && kForgetCap * kForgetScale * kPlanChunks < 4294967296.0, "prefix sums of a whole sequence fit 32 bits");
+
+// Smallest p <= t0 whose chunks [t0 - p, t0) forget (pre: prefix sums, non-decreasing); 0 = none.
+__device__ __forceinline__ int forget_stretch(const unsigned* pre, int t0) {
+    const unsigned at = pre[t0];
+    if (at - pre[0] <= kForget) return 0;
     int lo = 1, hi = t0;
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
-        if (at - pre[t0 - mid] < kForgetLn) hi = mid;
+        if (at - pre[t0 - mid] > kForget) hi = mid;
         else lo = mid + 1;
     }
     return lo;
@@ -41,7 +52,7 @@ __device__ __forceinline__ int forget_stretch(const float* pre, int t0) {
 
 // One warp: warm-ups of g segments, segment 0 = [0, L0), then L1 chunks each.  Lane s holds segment s's; returns the
 // largest, or -1 when a segment has none.
-__device__ __forceinline__ int warmups(const float* pre, int NT, int g, int L0, int L1, int lane, int& mine) {
+__device__ __forceinline__ int warmups(const unsigned* pre, int NT, int g, int L0, int L1, int lane, int& mine) {
     int w = 0, bad = 0;
     if (lane >= 1 && lane < g) {
         const int t0 = L0 + (lane - 1) * L1;
@@ -55,30 +66,30 @@ __device__ __forceinline__ int warmups(const float* pre, int NT, int g, int L0, 
     return __reduce_max_sync(0xffffffffu, w);
 }
 
-// All threads of the CTA: the split of this head (plan.g = 1: serial).  `pre`: NT + 1 floats of shared memory.
+// All threads of the CTA: the split of this head (plan.g = 1: serial).  `pre`: NT + 1 words of shared memory.
 template <int THREADS>
-__device__ __forceinline__ void plan_segments(const float* meta, int NT, int G, float* pre, SegmentPlan& plan, int* best) {
+__device__ __forceinline__ void plan_segments(const float* meta, int NT, int G, unsigned* pre, SegmentPlan& plan, int* best) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int bad = 0;
     for (int t = tid; t < NT; t += THREADS) {
         const float2 m = *reinterpret_cast<const float2*>(meta + 2 * t);
-        pre[t + 1] = m.x;
+        pre[t + 1] = __float2uint_rd(fminf(-m.x, kForgetCap) * kForgetScale);
         if (!(m.y <= 2.f) || !(m.x <= 0.f)) bad = 1;    // outside the premise (also NaN, and +inf for a gate out of range)
     }
     if (tid == 0) {
-        pre[0] = 0.f;
+        pre[0] = 0;
         plan.g = 1;
         *best = NT * 64;                                // score of the serial run
     }
     bad = __syncthreads_or(bad);
     if (bad) return;
     if (warp == 0) {
-        float carry = 0.f;
+        unsigned carry = 0;
         for (int base = 0; base < NT; base += 32) {
-            float x = base + lane < NT ? pre[base + lane + 1] : 0.f;
+            unsigned x = base + lane < NT ? pre[base + lane + 1] : 0;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
-                const float y = __shfl_up_sync(0xffffffffu, x, o);
+                const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
                 if (lane >= o) x += y;
             }
             x += carry;

@@ -77,3 +77,22 @@ def test_key_norms_outside_the_premise_run_serially():
     beta = beta.clone()
     beta[:, 1000:1003] = 0.9
     _check(q, k, v, g, beta, None, "large keys")
+
+
+@pytest.mark.parametrize("size,at", [(-1e9, [191, 319]), (-2e9, [191]), (-1e8, range(63, 12 * 192, 192))])
+def test_resets_do_not_hide_what_is_remembered(size, at):
+    """A very large finite |g| (a hard reset, a mask's fill value) on the last token of some chunks of slowly decaying heads: no
+    boundary behind it may count as forgotten because of it.  Held chunk by chunk: an error behind one boundary is a small part of
+    the whole output."""
+    S = 8192
+    q, k, v, g, beta, h0 = make_inputs("default", seed=11, S=S, Hq=2, Hv=4)
+    g = 0.1 * g                   # about -2.6 a chunk: 45 chunks forget
+    g[:, list(at)] = size
+    (o, s), _ = _both(q, k, v, g, beta, h0)
+    ro, rs = oracle_f32(q, k, v, g, beta, h0)
+    assert_close(s, rs, "state")
+    rest = np.ones(S, bool)
+    rest[list(at)] = False
+    o, ro = (x[0] * rest[:, None, None] for x in (o, ro))
+    err = np.linalg.norm((o - ro).reshape(S // 64, 64, 4, 128), axis=(1, 3)) / np.linalg.norm(ro.reshape(S // 64, 64, 4, 128), axis=(1, 3))
+    assert err.max() <= 1e-2, f"chunk {np.unravel_index(err.argmax(), err.shape)}: rel-L2 {err.max():.3e}"
