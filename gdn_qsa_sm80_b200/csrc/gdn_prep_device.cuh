@@ -71,6 +71,13 @@ __device__ __forceinline__ void prep_activate_gates(float& gv, float& bv) {
     bv = 1.f / (1.f + __expf(-bv));
 }
 
+// Decays below exp(-128) < 2^-149 are zero in fp32, and so is every product that contains one: a log gate below -128 counts as -128.
+// The chunk's cumulative sums then stay above -8192 (spacing 2^-10 in units of log2), where a gate of -1e9 left the tokens
+// behind it in the chunk without their own decay and the row scale that travels in P's exponent (the reset token's own output came
+// out 11 times too large), and -inf gave NaN.
+constexpr float kGateFloor = -128.f;
+__device__ __forceinline__ float prep_floor_gate(float gv) { return gv < kGateFloor ? kGateFloor : gv; }   // (NaN stays)
+
 // Gate cumsum over the chunk by warp shuffles (threads 0-63 hold one token each: gv, bv) and the decay tables.
 // Contains two barriers of the group; a third one is needed before the tables are read.
 // If vec_out != nullptr, also writes the per-token factors a later kernel needs:
@@ -82,7 +89,7 @@ __device__ __forceinline__ void prep_gates(PrepScratch& ps, float gv, float bv, 
     const int tid = ctx.tid, warp = tid >> 5, lane = tid & 31;
     float gsum = 0.f;
     if (tid < kChunk) {
-        gsum = gv;
+        gsum = prep_floor_gate(gv);
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const float y = __shfl_up_sync(0xffffffffu, gsum, o);

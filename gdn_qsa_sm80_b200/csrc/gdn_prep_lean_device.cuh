@@ -52,6 +52,8 @@ __device__ __forceinline__ void lean_gates(LeanScratch& ps, LaneGates x, bool ra
     }
     const bool in_range = __all_sync(0xffffffffu, x.g0 <= 0.f && x.g1 <= 0.f && x.b0 >= 0.f && x.b1 >= 0.f);
     if (lane == 0) ps.gates_ok = in_range;
+    x.g0 = prep_floor_gate(x.g0);
+    x.g1 = prep_floor_gate(x.g1);
     float s = x.g0 + x.g1;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {

@@ -5,6 +5,7 @@ Tolerance: the parity bar of the operator (rel-L2 <= 1e-2, max-abs <= 2e-2); bf1
 2^-9 = 2e-3 relative) enter four products in a row, so a correct result lies at 3-4e-3.
 """
 
+import numpy as np
 import pytest
 import torch
 
@@ -43,3 +44,24 @@ def test_matches_oracle(B, S, Hq, Hv, decay, h0, layer):
     ro, rs = oracle_f32(q, k, v, g, beta, state, l2norm=layer)
     assert_close(out.float().cpu().numpy(), ro, "out")
     assert_close(st.cpu().numpy(), rs, "state")
+
+
+@pytest.mark.parametrize("size", [-130.0, -1e4, -1e9, -3e38, float("-inf")])
+@pytest.mark.parametrize("path", ["twopass_t", "twopass_nv64", "coop"])
+@pytest.mark.parametrize("l2norm", [False, True])
+def test_resets(size, path, l2norm):
+    """Gates that end all memory, first, inside and last of a chunk: each token behind one keeps its own decay.  Held row by row;
+    a row is a bf16 product of one to 64 terms, so its error is that of its largest operands: 2^-8 each, three in a row, and the row's
+    own rounding."""
+    B, S, Hq, Hv, at = 1, 300, 2, 4, [0, 64, 90, 100, 127, 191, 200]
+    q, k, v, g, beta, h0 = make_inputs("default", seed=21, B=B, S=S, Hq=Hq, Hv=Hv)
+    g[:, at] = size
+    d = [t.cuda() for t in (q, k, v, g, beta)]
+    h0 = h0[:, :Hv]
+    out, st = gdn_chunk(*d, initial_state=h0.cuda(), path=path, use_qk_l2norm_in_kernel=l2norm)
+    check_device_status()
+    ro, rs = oracle_f32(q, k, v, g, beta, h0, form="recurrent", l2norm=l2norm)
+    assert_close(out.float().cpu().numpy(), ro, "out")
+    assert_close(st.cpu().numpy(), rs, "state")
+    rows = np.linalg.norm(out.float().cpu().numpy() - ro, axis=-1) / np.linalg.norm(ro, axis=-1)
+    assert rows[:, at].max() <= 2e-2 and np.median(rows) <= 1e-2
