@@ -177,10 +177,12 @@ __device__ __forceinline__ void lean_mask_row_P(const LeanScratch& ps, bool l2no
     }
 }
 
-// max over the warp's rows of beta_i |k_i|^2.
+// max over the warp's rows of beta_i |k_i|^2; +inf when one of them is not a number (fmaxf would drop it): what such a key leaves in
+// the state is bounded by nothing.
 __device__ __forceinline__ float lean_bound_of_rows(const LeanScratch& ps, bool l2norm, int i, float ksq) {
     const float rk = l2norm ? ps.rn[i] : 1.f;
     float bound = ps.bet[i] * ksq * rk * rk;
+    if (!(bound < INFINITY)) bound = INFINITY;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) bound = fmaxf(bound, __shfl_xor_sync(0xffffffffu, bound, o));
     return bound;

@@ -96,3 +96,18 @@ def test_resets_do_not_hide_what_is_remembered(size, at):
     o, ro = (x[0] * rest[:, None, None] for x in (o, ro))
     err = np.linalg.norm((o - ro).reshape(S // 64, 64, 4, 128), axis=(1, 3)) / np.linalg.norm(ro.reshape(S // 64, 64, 4, 128), axis=(1, 3))
     assert err.max() <= 1e-2, f"chunk {np.unravel_index(err.argmax(), err.shape)}: rel-L2 {err.max():.3e}"
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("l2norm", [False, True])
+def test_non_finite_keys_run_serially(value, l2norm):
+    """A key that is not finite stays in the state of a serial run for ever; nothing bounds what it leaves, so its head is not split."""
+    q, k, v, g, beta, _ = make_inputs("default", seed=12, S=1024, Hq=2, Hv=4)
+    g = 2.0 * g                   # about -52 a chunk: three chunks forget
+    k[:, 5, 0, 3] = value         # value heads 0 and 1
+    d = [t.cuda() for t in (q, k, v, g, beta)]
+    o, s = gdn_chunk(*d, use_qk_l2norm_in_kernel=l2norm)
+    o2, s2 = gdn_chunk(*d, use_qk_l2norm_in_kernel=l2norm, path="twopass_nv64")
+    check_device_status()
+    assert torch.equal(o[:, 64:].isfinite(), o2[:, 64:].isfinite()) and torch.equal(s.isfinite(), s2.isfinite())
+    assert not s[:, :2].isfinite().any() and s[:, 2:].isfinite().all()
