@@ -162,7 +162,7 @@ static bool path_uses_workspace(int path) {
 // the most segments the path cuts every sequence into (only the transposed chain splits sequences; 1 = not split)
 static int segments_of(int B, int S, int Hv, int path) {
     if (path != GDN_PATH_AUTO && !transposed_path(path)) return 1;
-    return chain_segments(static_cast<long long>(B) * Hv, S, 2 * sm_count());   // two CTAs per SM
+    return chain_segments(static_cast<long long>(tiles_of(B, S, Hv)), (S + kChunk - 1) / kChunk, 2 * sm_count());   // two CTAs per SM
 }
 
 size_t gdn_chunk_scratch_bytes(int B, int S, int Hq, int Hv, int path) {

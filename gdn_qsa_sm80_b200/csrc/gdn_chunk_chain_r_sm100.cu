@@ -63,6 +63,7 @@ __device__ constexpr uint32_t dk_bytes(int ks) { return ((ks >> 1) & 1) * 8192 +
 struct RWork {
     int t0, steps, store_from, len;        // len: tokens of the sequence
     int b, s_first;                        // TMA coordinates of the sequence's first token
+    int seg, segs;                         // which segment of the sequence this CTA runs, of how many at most
     size_t tok0, tile0;                    // first token and first workspace tile of the sequence and head
     const float* s_in;                     // state it starts from (null: zeros) and where the one it ends with goes
     float* s_out;
@@ -166,8 +167,10 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     if (tid == 0) {   // which sequence: its tokens, chunks and workspace tiles
         int seq;
         if (p.pk_chunk) {
-            const int2 o = p.pk_order[blockIdx.y];
+            const int4 o = p.pk_order[blockIdx.y];
             seq = o.x;
+            work.seg = o.z;
+            work.segs = o.w;
             work.b = 0;
             work.s_first = p.pk_cu[seq];
             work.len = p.pk_cu[seq + 1] - work.s_first;
@@ -175,6 +178,8 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             work.tile0 = static_cast<size_t>(o.y) * p.Hv + static_cast<size_t>(hv) * ((work.len + kChunk - 1) / kChunk);
         } else {
             seq = work.b = blockIdx.y;
+            work.seg = blockIdx.z;
+            work.segs = ws.n_seg;
             work.s_first = 0;
             work.len = p.S;
             work.tok0 = static_cast<size_t>(seq) * p.S;
@@ -189,9 +194,10 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     if (SPLIT) {
         __syncthreads();
         const int nt = work.steps;
-        plan_segments<kRThreads>(ws.meta + 2 * work.tile0, nt, ws.n_seg, reinterpret_cast<unsigned*>(sm), plan, &plan_best);
+        if (work.segs > 1) plan_segments<kRThreads>(ws.meta + 2 * work.tile0, nt, work.segs, reinterpret_cast<unsigned*>(sm), plan, &plan_best);
+        else if (tid == 0) plan.g = 1;      // (of a packed batch whose longer sequences are cut)
         if (tid == 0) {
-            const int seg = static_cast<int>(blockIdx.z), g = plan.g;
+            const int seg = work.seg, g = plan.g;
             if (g > 1) {
                 const int a = seg == 0 ? 0 : plan.L0 + (seg - 1) * plan.L1;
                 const int e = min(nt, seg == 0 ? plan.L0 : a + plan.L1);
@@ -256,8 +262,11 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 tma_prefetch_2d(map, 0, row0 + 32);
                 tma_prefetch_2d(map, 32, row0 + 32);
             };
-            // how many CTAs have work: those of a head's segments that its plan does not use have left already
-            const bool ahead = gridDim.x * gridDim.y * (SPLIT ? static_cast<unsigned>(plan.g) : 1u) <= sms;
+            // How many CTAs are at work: those of a head's segments that its plan does not use have left already, and so have
+            // most of a packed batch's shorter sequences while its longest one runs.
+            const unsigned g = SPLIT ? static_cast<unsigned>(plan.g) : 1u;
+            const bool ahead = p.pk_chunk ? static_cast<unsigned long long>(p.Hv) * p.pk_chunks * g <= static_cast<unsigned long long>(sms) * p.pk_longest
+                                          : gridDim.x * gridDim.y * g <= sms;
             auto load_t2 = [&](int n) {
                 const uint32_t s = n & 1, fb = cb(R_TFULL + s);
                 const int row0 = static_cast<int>((work.tile0 + work.t0 + n) * kChunk);
@@ -595,7 +604,7 @@ int launch_chain_r(const Problem& p, const Workspace& ws, const TileMaps& maps, 
         if (allow_smem(reinterpret_cast<const void*>(kernel), kRDynamic)) return GDN_ERR_CUDA;
         // The value heads that share a qk head read the same K and Q tiles: as a cluster of two CTAs they start together
         // and run in step, so the second read of a tile finds it in L2 (nothing else of the cluster is used).
-        // A grid's y ends at 65535: a packed batch of more sequences takes several launches.
+        // A grid's y ends at 65535: a packed batch of more entries takes several launches.
         Problem part = p;
         for (int done = 0, all = p.pk_chunk ? p.pk_n : 1; done < all; done += 65535) {
             unsigned gy = static_cast<unsigned>(p.B);
@@ -611,7 +620,7 @@ int launch_chain_r(const Problem& p, const Workspace& ws, const TileMaps& maps, 
     };
     const int G = ws.n_seg;
     if (G <= 1 || G > kMaxSegments || !ws.meta) return go(gdn_chain_r_kernel<false>, 1);
-    return go(gdn_chain_r_kernel<true>, static_cast<unsigned>(G));
+    return go(gdn_chain_r_kernel<true>, p.pk_chunk ? 1u : static_cast<unsigned>(G));
 }
 
 }  // namespace gdn

@@ -1,8 +1,7 @@
 // Packed batch: sequences of different lengths laid end to end in [1, T, H, .] tensors, in one pass of the two-kernel path.
 //
 // The kernels find a chunk's sequence through three small tables (first token of each sequence; (sequence, chunk) per 64-token
-// chunk; (sequence, first chunk) longest first, so that the last CTAs of the chain's grid are the short ones), written to the
-// scratch buffer by a kernel whose parameters carry the lengths: no copy from the host, and a captured graph keeps them.
+// chunk; (sequence, first chunk, segment) in the order the chain's CTAs take them), written to the scratch buffer by a kernel whose parameters carry the lengths: no copy from the host, and a captured graph keeps them.
 // The last tile of a sequence also holds the next one's first tokens; gates and beta count as zero there, and the kernels
 // mask those rows (prepare) or clear them in the tile (chain), so no sequence ever sees another's values.
 // Sequences of at most kDecodeMaxTokens tokens take the decode kernel, neighbours of equal length in one launch.
@@ -25,10 +24,11 @@ struct TablePiece {
     int first;                        // sequence of entry 0
     int start[kPiece], len[kPiece];
     int chunk0[kPiece];               // its first entry in the chunk table; -1: a short sequence, in no table but cu
-    int rank[kPiece];                 // its place in the longest-first order
+    int rank[kPiece], segs[kPiece];   // its entries in the chain's work list: layer[s] + rank for s < segs
+    int layer[kMaxSegments];
 };
 
-__global__ void __launch_bounds__(64) gdn_pack_tables_kernel(const __grid_constant__ TablePiece piece, int* cu, int2* chunk, int2* order,
+__global__ void __launch_bounds__(64) gdn_pack_tables_kernel(const __grid_constant__ TablePiece piece, int* cu, int2* chunk, int4* order,
                                                              int* status) {
     grid_dependency_wait();           // earlier kernels of the stream may still read the tables of their own call
     grid_launch_dependents();
@@ -36,11 +36,11 @@ __global__ void __launch_bounds__(64) gdn_pack_tables_kernel(const __grid_consta
     if (threadIdx.x == 0) {
         cu[seq] = piece.start[i];
         cu[seq + 1] = piece.start[i] + piece.len[i];   // (the next sequence's block writes the same value)
-        if (c0 >= 0) order[piece.rank[i]] = make_int2(seq, c0);
         if (seq == 0 && status) *status = 0;
     }
     if (c0 < 0) return;
-    const int nt = (piece.len[i] + kChunk - 1) / kChunk;
+    const int nt = (piece.len[i] + kChunk - 1) / kChunk, segs = piece.segs[i];
+    if (threadIdx.x < segs) order[piece.layer[threadIdx.x] + piece.rank[i]] = make_int4(seq, c0, threadIdx.x, segs);
     for (int t = threadIdx.x; t < nt; t += blockDim.x) chunk[c0 + t] = make_int2(seq, t);
 }
 
@@ -49,15 +49,15 @@ struct PackedLayout {
     size_t cu, chunk, order, total;
     size_t chunks;                    // 64-token chunks of the sequences that take the two-kernel path
     int longs;                        // how many those are
-    int max_len;
+    int longest;                      // chunks of the longest
 };
 PackedLayout packed_layout(const int* cu, int n_seq, int Hv) {
     PackedLayout l{};
     for (int i = 0; i < n_seq; ++i) {
-        const int n = cu[i + 1] - cu[i];
-        if (n > l.max_len) l.max_len = n;
+        const int n = cu[i + 1] - cu[i], nt = (n + kChunk - 1) / kChunk;
         if (n <= kDecodeMaxTokens) continue;
-        l.chunks += (n + kChunk - 1) / kChunk;
+        if (nt > l.longest) l.longest = nt;
+        l.chunks += nt;
         ++l.longs;
     }
     l.ws = workspace_layout(l.chunks * Hv, true);
@@ -65,7 +65,7 @@ PackedLayout packed_layout(const int* cu, int n_seq, int Hv) {
     l.cu = up(l.ws.total);
     l.chunk = up(l.cu + (static_cast<size_t>(n_seq) + 1) * 4);
     l.order = up(l.chunk + l.chunks * 8);
-    l.total = up(l.order + static_cast<size_t>(l.longs) * 8);
+    l.total = up(l.order + static_cast<size_t>(l.longs) * kMaxSegments * sizeof(int4));
     return l;
 }
 bool bounds_rise(const int* cu, int n_seq) {
@@ -103,33 +103,59 @@ int gdn_chunk_fwd_varlen_sm100(const void* q, const void* k, const void* v, cons
     bool clear = true;                // whichever kernel comes first clears the status word
 
     if (l.longs > 0) {
-        std::vector<int> rank, order;
+        std::vector<int> rank, order, segs;
         try {
             rank.resize(n_seq);
+            segs.resize(n_seq);
             order.reserve(l.longs);
         } catch (...) {               // nothing may be thrown through a C entry
             return GDN_ERR_SCRATCH;
         }
-        for (int i = 0; i < n_seq; ++i)
-            if (cu_seqlens[i + 1] - cu_seqlens[i] > kDecodeMaxTokens) order.push_back(i);
+        auto chunks_of = [&](int s) { return (cu_seqlens[s + 1] - cu_seqlens[s] + kChunk - 1) / kChunk; };
+        for (int i = 0; i < n_seq; ++i) {
+            if (cu_seqlens[i + 1] - cu_seqlens[i] <= kDecodeMaxTokens) continue;
+            order.push_back(i);
+            segs[i] = chain_segments(static_cast<long long>(l.chunks) * Hv, chunks_of(i), 2 * sm_count());   // two CTAs per SM
+        }
+        // Order of the chain's work list.  First what takes long, segment by segment: the first segments of all sequences that may be
+        // cut (and the long ones that may not), their second ones, ...: a head whose decay forbids the cut runs all of it in
+        // its first segment's CTA, and those then find SMs of their own (4 sequences of 4096 tokens of slow decay, 32 heads: 220 us,
+        // 278 us with the segments of a sequence side by side).  Last the short sequences, longest first: they fill what is left.
+        int entries = 0, most = 1, longest_run = 0, layer[kMaxSegments] = {};
+        auto run = [&](int s) { return chunks_of(s) / segs[s]; };
+        for (int s : order) longest_run = std::max(longest_run, run(s));
+        auto fills = [&](int s) { return segs[s] == 1 && 2 * run(s) < longest_run; };
         std::sort(order.begin(), order.end(), [&](int a, int b) {
-            const int x = cu_seqlens[a + 1] - cu_seqlens[a], y = cu_seqlens[b + 1] - cu_seqlens[b];
-            return x != y ? x > y : a < b;
+            if (fills(a) != fills(b)) return fills(b);
+            if (segs[a] != segs[b]) return segs[a] > segs[b];
+            return run(a) != run(b) ? run(a) > run(b) : a < b;
         });
-        for (int r = 0; r < l.longs; ++r) rank[order[r]] = r;
+        int firsts = 0;
+        for (int s : order) {
+            if (fills(s)) break;
+            rank[s] = firsts++;
+            most = std::max(most, segs[s]);
+        }
+        for (int seg = 0; seg < most; ++seg) {
+            layer[seg] = entries;
+            for (int r = 0; r < firsts && segs[order[r]] > seg; ++r) ++entries;
+        }
+        for (int r = firsts; r < l.longs; ++r) rank[order[r]] = entries++;
         int* d_cu = reinterpret_cast<int*>(base + l.cu);
         int2* d_chunk = reinterpret_cast<int2*>(base + l.chunk);
-        int2* d_order = reinterpret_cast<int2*>(base + l.order);
+        int4* d_order = reinterpret_cast<int4*>(base + l.order);
         int c = 0;
         for (int i0 = 0; i0 < n_seq; i0 += kPiece) {
             TablePiece piece;
             piece.first = i0;
+            std::copy(layer, layer + kMaxSegments, piece.layer);
             const int n = std::min(kPiece, n_seq - i0);
             for (int i = 0; i < n; ++i) {
                 const int s = i0 + i, len = cu_seqlens[s + 1] - cu_seqlens[s];
                 piece.start[i] = cu_seqlens[s];
                 piece.len[i] = len;
                 piece.rank[i] = rank[s];
+                piece.segs[i] = segs[s];
                 piece.chunk0[i] = len > kDecodeMaxTokens ? c : -1;
                 if (len > kDecodeMaxTokens) c += (len + kChunk - 1) / kChunk;
             }
@@ -158,13 +184,14 @@ int gdn_chunk_fwd_varlen_sm100(const void* q, const void* k, const void* v, cons
         p.pk_cu = d_cu;
         p.pk_chunk = d_chunk;
         p.pk_order = d_order;
-        p.pk_n = l.longs;
+        p.pk_n = entries;
         p.pk_chunks = static_cast<int>(l.chunks);
+        p.pk_longest = l.longest;
         Workspace ws = {};
         ws.P = reinterpret_cast<__nv_bfloat16*>(base + l.ws.P);
         ws.U = reinterpret_cast<__nv_bfloat16*>(base + l.ws.U);
         ws.vec = reinterpret_cast<float*>(base + l.ws.vec);
-        ws.n_seg = chain_segments(static_cast<long long>(l.longs) * Hv, l.max_len, 2 * sm_count());
+        ws.n_seg = most;
         ws.meta = ws.n_seg > 1 ? reinterpret_cast<float*>(base + l.ws.meta) : nullptr;
         TileMaps maps;
         if (encode_tile_maps(p, ws, maps)) return GDN_ERR_DRIVER;

@@ -73,3 +73,30 @@ def test_views_at_odd_offsets_are_gathered():
     got = gdn_chunk_varlen(odd, *d[1:], cu)
     for a, b in zip(got, want):
         assert ((a.float() - b.float()).norm() / b.float().norm()).item() <= 1e-2   # (padding changes where a chunk ends)
+
+
+def test_a_long_sequence_among_short_ones_is_split():
+    """Sequences are cut by what they hold of the batch's work: a long one costs about as much with short ones beside it as alone."""
+    lens = [50] * 10 + [30000] + [100] * 10
+    T, cu = sum(lens), np.concatenate([[0], np.cumsum(lens)]).tolist()
+    q, k, v, g, beta, _ = make_inputs("default", seed=6, B=1, S=T, Hq=16, Hv=32)
+    d = [t.cuda() for t in (q, k, v, g, beta)]
+    own = [x[:, cu[10]:cu[11]].contiguous() for x in d]
+    out, st = gdn_chunk_varlen(*d, cu)
+    o1, s1 = gdn_chunk(*own)
+    check_device_status()
+    assert torch.equal(o1, out[:, cu[10]:cu[11]]) and torch.equal(s1, st[10:11])
+
+    def best(call):
+        times = []
+        for _ in range(10):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            call()
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+
+    alone, packed = best(lambda: gdn_chunk(*own)), best(lambda: gdn_chunk_varlen(*d, cu))
+    assert packed < 2 * alone, f"{packed:.3f} ms, the long one alone {alone:.3f} ms"     # unsplit: more than three times
