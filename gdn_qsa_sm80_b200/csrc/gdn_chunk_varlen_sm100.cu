@@ -4,7 +4,9 @@
 // chunk; (sequence, first chunk, segment) in the order the chain's CTAs take them), written to the scratch buffer by a kernel whose parameters carry the lengths: no copy from the host, and a captured graph keeps them.
 // The last tile of a sequence also holds the next one's first tokens; gates and beta count as zero there, and the kernels
 // mask those rows (prepare) or clear them in the tile (chain), so no sequence ever sees another's values.
-// Sequences of at most kDecodeMaxTokens tokens take the decode kernel, neighbours of equal length in one launch.
+// Sequences of at most kDecodeMaxTokens tokens take the decode kernel, all of them in one launch through a table of their own (256
+// sequences of 1 to 8 tokens, 32 heads: 1491 us with a launch per run of equal lengths, 348 now; before the packed route a padded
+// batch, 957).
 //
 // Without this a packed batch was gathered into a padded one and scattered back (torch indexing: two passes over all
 // tensors, and the padding's share of the work), or ran sequence by sequence.
@@ -19,43 +21,52 @@
 namespace gdn {
 namespace {
 
-constexpr int kPiece = 1024;          // sequences per launch of the table kernel (kernel parameters: 32 KB at most)
+constexpr int kPiece = 1024;          // sequences per launch of the table kernel (kernel parameters: 12 KB)
 struct TablePiece {
     int first;                        // sequence of entry 0
-    int start[kPiece], len[kPiece];
-    int chunk0[kPiece];               // its first entry in the chunk table; -1: a short sequence, in no table but cu
-    int rank[kPiece], segs[kPiece];   // its entries in the chain's work list: layer[s] + rank for s < segs
+    int start[kPiece + 1];
+    int chunk0[kPiece];               // its first entry in the chunk table; -1: a short sequence, entry `rank` of their table
+    unsigned rank[kPiece];            // 16 rank + segs: its entries in the chain's work list are layer[s] + rank for s < segs
+    static_assert(kMaxSegments < 16, "segs in four bits");
     int layer[kMaxSegments];
 };
 
 __global__ void __launch_bounds__(64) gdn_pack_tables_kernel(const __grid_constant__ TablePiece piece, int* cu, int2* chunk, int4* order,
-                                                             int* status) {
+                                                             int4* shorts, int* status) {
     grid_dependency_wait();           // earlier kernels of the stream may still read the tables of their own call
     grid_launch_dependents();
-    const int i = blockIdx.x, seq = piece.first + i, c0 = piece.chunk0[i];
+    const int i = blockIdx.x, seq = piece.first + i, c0 = piece.chunk0[i], len = piece.start[i + 1] - piece.start[i];
+    const int rank = static_cast<int>(piece.rank[i] >> 4), segs = piece.rank[i] & 15;
     if (threadIdx.x == 0) {
         cu[seq] = piece.start[i];
-        cu[seq + 1] = piece.start[i] + piece.len[i];   // (the next sequence's block writes the same value)
+        cu[seq + 1] = piece.start[i + 1];   // (the next sequence's block writes the same value)
+        if (c0 < 0) shorts[rank] = make_int4(seq, piece.start[i], len, 0);
         if (seq == 0 && status) *status = 0;
     }
     if (c0 < 0) return;
-    const int nt = (piece.len[i] + kChunk - 1) / kChunk, segs = piece.segs[i];
-    if (threadIdx.x < segs) order[piece.layer[threadIdx.x] + piece.rank[i]] = make_int4(seq, c0, threadIdx.x, segs);
+    const int nt = (len + kChunk - 1) / kChunk;
+    if (threadIdx.x < segs) order[piece.layer[threadIdx.x] + rank] = make_int4(seq, c0, threadIdx.x, segs);
     for (int t = threadIdx.x; t < nt; t += blockDim.x) chunk[c0 + t] = make_int2(seq, t);
 }
 
 struct PackedLayout {
     WorkspaceLayout ws;
-    size_t cu, chunk, order, total;
+    size_t cu, chunk, order, shorts, total;
     size_t chunks;                    // 64-token chunks of the sequences that take the two-kernel path
     int longs;                        // how many those are
     int longest;                      // chunks of the longest
+    int n_short, short_runs, most;    // the other sequences, their runs of equal lengths, the most tokens one has
 };
 PackedLayout packed_layout(const int* cu, int n_seq, int Hv) {
     PackedLayout l{};
     for (int i = 0; i < n_seq; ++i) {
         const int n = cu[i + 1] - cu[i], nt = (n + kChunk - 1) / kChunk;
-        if (n <= kDecodeMaxTokens) continue;
+        if (n <= kDecodeMaxTokens) {
+            if (i == 0 || cu[i] - cu[i - 1] != n) ++l.short_runs;
+            if (n > l.most) l.most = n;
+            ++l.n_short;
+            continue;
+        }
         if (nt > l.longest) l.longest = nt;
         l.chunks += nt;
         ++l.longs;
@@ -65,7 +76,8 @@ PackedLayout packed_layout(const int* cu, int n_seq, int Hv) {
     l.cu = up(l.ws.total);
     l.chunk = up(l.cu + (static_cast<size_t>(n_seq) + 1) * 4);
     l.order = up(l.chunk + l.chunks * 8);
-    l.total = up(l.order + static_cast<size_t>(l.longs) * kMaxSegments * sizeof(int4));
+    l.shorts = up(l.order + static_cast<size_t>(l.longs) * kMaxSegments * sizeof(int4));
+    l.total = up(l.shorts + static_cast<size_t>(l.n_short) * sizeof(int4));
     return l;
 }
 bool bounds_rise(const int* cu, int n_seq) {
@@ -102,7 +114,24 @@ int gdn_chunk_fwd_varlen_sm100(const void* q, const void* k, const void* v, cons
     uint8_t* base = static_cast<uint8_t*>(scratch);
     bool clear = true;                // whichever kernel comes first clears the status word
 
-    if (l.longs > 0) {
+    Problem p = {};
+    p.q = static_cast<const __nv_bfloat16*>(q);
+    p.k = static_cast<const __nv_bfloat16*>(k);
+    p.v = static_cast<const __nv_bfloat16*>(v);
+    p.g = g;
+    p.beta = beta;
+    p.h0 = h0;
+    p.out = static_cast<__nv_bfloat16*>(out);
+    p.hT = hT;
+    p.status = static_cast<int*>(scratch);
+    p.Hq = Hq;
+    p.Hv = Hv;
+    p.gate_f32 = gate_dtype == GDN_GATE_F32;
+    p.l2norm = (flags & GDN_FLAG_QK_L2NORM) ? 1 : 0;
+    p.gate_act = (flags & GDN_FLAG_GATE_ACTIVATIONS) ? 1 : 0;
+    const bool listed = l.short_runs > 1;   // one run needs no table
+    int most_segments = 1;
+    if (l.longs > 0 || listed) {
         std::vector<int> rank, order, segs;
         try {
             rank.resize(n_seq);
@@ -111,9 +140,13 @@ int gdn_chunk_fwd_varlen_sm100(const void* q, const void* k, const void* v, cons
         } catch (...) {               // nothing may be thrown through a C entry
             return GDN_ERR_SCRATCH;
         }
+        int n_short = 0;
         auto chunks_of = [&](int s) { return (cu_seqlens[s + 1] - cu_seqlens[s] + kChunk - 1) / kChunk; };
         for (int i = 0; i < n_seq; ++i) {
-            if (cu_seqlens[i + 1] - cu_seqlens[i] <= kDecodeMaxTokens) continue;
+            if (cu_seqlens[i + 1] - cu_seqlens[i] <= kDecodeMaxTokens) {
+                rank[i] = n_short++;
+                continue;
+            }
             order.push_back(i);
             segs[i] = chain_segments(static_cast<long long>(l.chunks) * Hv, chunks_of(i), 2 * sm_count());   // two CTAs per SM
         }
@@ -144,6 +177,7 @@ int gdn_chunk_fwd_varlen_sm100(const void* q, const void* k, const void* v, cons
         int* d_cu = reinterpret_cast<int*>(base + l.cu);
         int2* d_chunk = reinterpret_cast<int2*>(base + l.chunk);
         int4* d_order = reinterpret_cast<int4*>(base + l.order);
+        int4* d_shorts = reinterpret_cast<int4*>(base + l.shorts);
         int c = 0;
         for (int i0 = 0; i0 < n_seq; i0 += kPiece) {
             TablePiece piece;
@@ -153,45 +187,34 @@ int gdn_chunk_fwd_varlen_sm100(const void* q, const void* k, const void* v, cons
             for (int i = 0; i < n; ++i) {
                 const int s = i0 + i, len = cu_seqlens[s + 1] - cu_seqlens[s];
                 piece.start[i] = cu_seqlens[s];
-                piece.len[i] = len;
-                piece.rank[i] = rank[s];
-                piece.segs[i] = segs[s];
+                piece.rank[i] = 16u * static_cast<unsigned>(rank[s]) + static_cast<unsigned>(segs[s]);
                 piece.chunk0[i] = len > kDecodeMaxTokens ? c : -1;
                 if (len > kDecodeMaxTokens) c += (len + kChunk - 1) / kChunk;
             }
-            const cudaError_t e = launch_dependent(gdn_pack_tables_kernel, dim3(n), dim3(64), 0, stream, false, piece, d_cu, d_chunk, d_order,
+            piece.start[n] = cu_seqlens[i0 + n];
+            const cudaError_t e = launch_dependent(gdn_pack_tables_kernel, dim3(n), dim3(64), 0, stream, false, piece, d_cu, d_chunk, d_order, d_shorts,
                                                    i0 == 0 ? static_cast<int*>(scratch) : static_cast<int*>(nullptr));
             if (e != cudaSuccess) return GDN_ERR_CUDA;
         }
         clear = false;
-        Problem p = {};
-        p.q = static_cast<const __nv_bfloat16*>(q);
-        p.k = static_cast<const __nv_bfloat16*>(k);
-        p.v = static_cast<const __nv_bfloat16*>(v);
-        p.g = g;
-        p.beta = beta;
-        p.h0 = h0;
-        p.out = static_cast<__nv_bfloat16*>(out);
-        p.hT = hT;
-        p.status = static_cast<int*>(scratch);
-        p.B = 1;
-        p.S = cu_seqlens[n_seq];
-        p.Hq = Hq;
-        p.Hv = Hv;
-        p.gate_f32 = gate_dtype == GDN_GATE_F32;
-        p.l2norm = (flags & GDN_FLAG_QK_L2NORM) ? 1 : 0;
-        p.gate_act = (flags & GDN_FLAG_GATE_ACTIVATIONS) ? 1 : 0;
         p.pk_cu = d_cu;
         p.pk_chunk = d_chunk;
         p.pk_order = d_order;
         p.pk_n = entries;
         p.pk_chunks = static_cast<int>(l.chunks);
         p.pk_longest = l.longest;
+        p.pk_short = d_shorts;
+        p.pk_shorts = l.n_short;
+        most_segments = most;
+    }
+    if (l.longs > 0) {
+        p.B = 1;
+        p.S = cu_seqlens[n_seq];
         Workspace ws = {};
         ws.P = reinterpret_cast<__nv_bfloat16*>(base + l.ws.P);
         ws.U = reinterpret_cast<__nv_bfloat16*>(base + l.ws.U);
         ws.vec = reinterpret_cast<float*>(base + l.ws.vec);
-        ws.n_seg = most;
+        ws.n_seg = most_segments;
         ws.meta = ws.n_seg > 1 ? reinterpret_cast<float*>(base + l.ws.meta) : nullptr;
         TileMaps maps;
         if (encode_tile_maps(p, ws, maps)) return GDN_ERR_DRIVER;
@@ -199,7 +222,12 @@ int gdn_chunk_fwd_varlen_sm100(const void* q, const void* k, const void* v, cons
         if (st == GDN_OK) st = launch_chain_r(p, ws, maps, stream);
         if (st != GDN_OK) return st;
     }
-    // short sequences: the decode kernel, neighbours of equal length in one launch
+    if (listed) {
+        p.B = n_seq;
+        p.S = l.most;
+        return launch_decode(p, nullptr, stream);
+    }
+    // one run of short sequences (or none): a regular batch of the decode kernel
     const size_t gate_bytes = gate_dtype == GDN_GATE_F32 ? 4 : 2;
     for (int i = 0; i < n_seq;) {
         const int n = cu_seqlens[i + 1] - cu_seqlens[i];

@@ -44,6 +44,8 @@ struct Problem {
     const int4* pk_order;  // [pk_n] what a row of the chain's grid runs: (sequence, its first entry in pk_chunk, segment, segments
                            // it may be cut into)
     int pk_n, pk_chunks, pk_longest;   // entries of the two tables; chunks of the longest sequence
+    const int4* pk_short;  // decode kernel: [pk_shorts] (sequence, first token, tokens); B = all sequences, S = the most tokens
+    int pk_shorts;
 };
 
 // Workspace of the two-kernel path (device pointers into the caller's scratch buffer).

@@ -10,6 +10,7 @@
 // The tile is 128-byte swizzled and lane l owns rows = l mod 8 and the four columns of chunk l / 8, so a 16-byte access
 // of eight lanes covers all banks, and the column sums a token needs (S^T k, S^T q) are three shuffles: no barrier.
 //   GROUPS = 1: a CTA of two compute warps and a producer warp, four per SM; 32 states give 128 CTAs.
+//   PACKED: the sequences of a packed batch that have at most kDecodeMaxTokens tokens, of any lengths, found through a table.
 //   GROUPS = 4: the four tiles of a state in one CTA, for the gated normalisation of the output rows (their sum of squares
 //   needs all 128 columns: one barrier a token), which then costs no launch and no pass over the rows of its own.
 #include <cuda.h>
@@ -47,7 +48,7 @@ __device__ __forceinline__ float sum_rows(float x) {   // over the eight lanes t
 // bytes of the token area of one stage: k, q rows, 32 columns of v, g and beta
 __host__ __device__ constexpr uint32_t dec_token_bytes(int nt) { return nt * (256 + 256 + 64) + 2 * kDecTokens * 4; }
 
-template <int GROUPS, bool GATE_F32>
+template <int GROUPS, bool GATE_F32, bool PACKED>
 __global__ void __launch_bounds__(GROUPS * 64 + 32, GROUPS == 1 ? 4 : 1)
 gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_out,
                   const __grid_constant__ Problem p, const __grid_constant__ DecodeGate gate, int items, int nt) {
@@ -55,6 +56,7 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     __shared__ __align__(8) uint64_t full[GROUPS][kDecStages], empty[GROUPS][kDecStages];
     __shared__ float ssq[2][GROUPS * 2];
+    __shared__ int4 seq_of[PACKED ? kDecStages : 1];   // (sequence, first token, tokens) of the stage's tile
     __shared__ int failed;
 
     const int tid = threadIdx.x, warp = static_cast<int>(warp_uniform(tid >> 5)), lane = tid & 31;
@@ -85,18 +87,25 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
         int n = 0;
         for (int it = first; it < items; it += step, ++n) {
             const int s = n % kDecStages;
-            const int state = GROUPS == 1 ? it >> 2 : it;
+            int state = GROUPS == 1 ? it >> 2 : it, tokens = nt;
             const int b = state / p.Hv, h = state - b * p.Hv, hq = h / rep;
-            const size_t tok0 = static_cast<size_t>(b) * p.S;
+            size_t tok0 = static_cast<size_t>(b) * p.S;
+            int4 seq = {};
+            if (PACKED) {
+                seq = p.pk_short[b];
+                state = seq.x * p.Hv + h;
+                tok0 = seq.y;
+                tokens = seq.z;
+            }
             bool ok = true;
             for (int g = 0; g < GROUPS && ok; ++g) {
                 if (n >= kDecStages) ok = mbar_wait(&empty[g][s], ((n / kDecStages) - 1) & 1, p.status, kDecTimeoutEmpty);
                 const int quarter = GROUPS == 1 ? it & 3 : g;
                 if (ok && elect_one()) {
                     uint8_t* tk = tok_of(g, s);
-                    mbar_arrive_expect_tx(&full[g][s], (p.h0 ? 16384 : 0) + nt * (256 + 256 + 64));
+                    mbar_arrive_expect_tx(&full[g][s], (p.h0 ? 16384 : 0) + tokens * (256 + 256 + 64));
                     if (p.h0) tma_load_2d(tile_of(g, s), &tm_in, &full[g][s], quarter * 32, state * kD);
-                    for (int t = 0; t < nt; ++t) {
+                    for (int t = 0; t < tokens; ++t) {
                         const size_t row = (tok0 + t) * p.Hq + hq;
                         bulk_load_1d(tk + t * 256, p.k + row * kD, 256, &full[g][s]);
                         bulk_load_1d(tk + (nt + t) * 256, p.q + row * kD, 256, &full[g][s]);
@@ -110,9 +119,10 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
                 break;
             }
             float x = 0.f;
-            if (lane < 2 * kDecTokens && (lane & 7) < nt)
+            if (lane < 2 * kDecTokens && (lane & 7) < tokens)
                 x = dec_gate<GATE_F32>(lane < kDecTokens ? p.g : p.beta, (tok0 + (lane & 7)) * p.Hv + h);
             for (int g = 0; g < GROUPS; ++g) {
+                if (PACKED && lane == 0) seq_of[s] = seq;
                 if (lane < 2 * kDecTokens) *reinterpret_cast<float*>(tok_of(g, s) + nt * (256 + 256 + 64) + lane * 4) = x;
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&full[g][s]);
@@ -130,13 +140,20 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
         int n = 0;
         for (int it = first; it < items; it += step, ++n) {
             const int s = n % kDecStages;
-            const int state = GROUPS == 1 ? it >> 2 : it, quarter = GROUPS == 1 ? it & 3 : g;
+            int state = GROUPS == 1 ? it >> 2 : it, tokens = p.S;
+            const int quarter = GROUPS == 1 ? it & 3 : g;
             const int b = state / p.Hv, h = state - b * p.Hv, hq = h / rep;
-            const size_t tok0 = static_cast<size_t>(b) * p.S;
+            size_t tok0 = static_cast<size_t>(b) * p.S;
             // after a wait that ran out nobody waits again, but every warp keeps to the loop: its barriers count all of them
             const bool ok = !*const_cast<volatile int*>(&failed) &&
                             mbar_wait(&full[g][s], (n / kDecStages) & 1, p.status, kDecTimeoutFull);
             if (!ok) *const_cast<volatile int*>(&failed) = 1;
+            if (PACKED) {
+                const int4 seq = seq_of[s];
+                state = seq.x * p.Hv + h;
+                tok0 = seq.y;
+                tokens = ok ? seq.z : 0;          // (nothing may have been written there)
+            }
             uint8_t* tile = tile_of(g, s) + off0;
             const uint8_t* tk = tok_of(g, s);
             float4 st[16];
@@ -144,7 +161,7 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
             for (int i = 0; i < 16; ++i)
                 st[i] = p.h0 ? *reinterpret_cast<const float4*>(tile + i * 1024) : make_float4(0.f, 0.f, 0.f, 0.f);
             const float* gates = reinterpret_cast<const float*>(tk + nt * (256 + 256 + 64));
-            for (int t = 0; t < p.S; ++t) {
+            for (int t = 0; t < tokens; ++t) {
                 const size_t tok = tok0 + t;
                 // this lane's rows of k and q (fp32), its four values, the gates
                 const unsigned short *kr, *qr;
@@ -267,7 +284,7 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
 
 // `og`: gated normalisation applied to the output rows by the same kernel (null: none).
 int launch_decode(const Problem& p, const OutputGate* og, cudaStream_t stream) {
-    const long long states = static_cast<long long>(p.B) * p.Hv;
+    const long long states = static_cast<long long>(p.B) * p.Hv;   // (of a packed batch: all sequences', the map's extent)
     if (states * kD >= (1ll << 31)) return GDN_ERR_BAD_ARGUMENT;
     alignas(64) CUtensorMap tin, tout;
     const unsigned long long d[2] = {kD, static_cast<unsigned long long>(states) * kD}, sb[1] = {kD * 4};
@@ -293,8 +310,12 @@ int launch_decode(const Problem& p, const OutputGate* og, cudaStream_t stream) {
                                                gate, static_cast<int>(items), nt);
         return e == cudaSuccess ? GDN_OK : GDN_ERR_CUDA;
     };
-    if (og) return p.gate_f32 ? go(gdn_decode_kernel<4, true>, 4, states) : go(gdn_decode_kernel<4, false>, 4, states);
-    return p.gate_f32 ? go(gdn_decode_kernel<1, true>, 1, states * 4) : go(gdn_decode_kernel<1, false>, 1, states * 4);
+    if (p.pk_short) {
+        const long long tiles = 4ll * p.pk_shorts * p.Hv;
+        return p.gate_f32 ? go(gdn_decode_kernel<1, true, true>, 1, tiles) : go(gdn_decode_kernel<1, false, true>, 1, tiles);
+    }
+    if (og) return p.gate_f32 ? go(gdn_decode_kernel<4, true, false>, 4, states) : go(gdn_decode_kernel<4, false, false>, 4, states);
+    return p.gate_f32 ? go(gdn_decode_kernel<1, true, false>, 1, states * 4) : go(gdn_decode_kernel<1, false, false>, 1, states * 4);
 }
 
 }  // namespace gdn

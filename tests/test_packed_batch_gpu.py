@@ -8,6 +8,7 @@ import pytest
 import torch
 
 from gdn_qsa_sm80 import gdn_chunk, gdn_chunk_varlen
+from gdn_qsa_sm80_b200 import _lib
 from gdn_qsa_sm80_b200.gdn_chunk_interface import check_device_status
 from gdn_qsa_sm80_b200.synthetic import make_inputs
 
@@ -100,3 +101,20 @@ def test_a_long_sequence_among_short_ones_is_split():
 
     alone, packed = best(lambda: gdn_chunk(*own)), best(lambda: gdn_chunk_varlen(*d, cu))
     assert packed < 2 * alone, f"{packed:.3f} ms, the long one alone {alone:.3f} ms"     # unsplit: more than three times
+
+
+def test_short_sequences_of_different_lengths_share_a_launch():
+    """A few new tokens per request, as many as each has: one launch besides the table's, not one per run of equal lengths."""
+    lens = [1 + (i * 5) % 8 for i in range(300)]
+    T, cu = sum(lens), np.concatenate([[0], np.cumsum(lens)]).tolist()
+    q, k, v, g, beta, _ = make_inputs("default", seed=4, B=1, S=T, Hq=2, Hv=4)
+    h0 = 0.1 * torch.randn(len(lens), 4, 128, 128, generator=torch.Generator().manual_seed(5)).cuda()
+    d = [t.cuda() for t in (q, k, v, g, beta)]
+    before = _lib.kernel_launches()
+    out, st = gdn_chunk_varlen(*d, cu, initial_state=h0)
+    assert _lib.kernel_launches() - before <= 2
+    check_device_status()
+    for i in list(range(20)) + [150, 298, 299]:
+        a, b = cu[i], cu[i + 1]
+        o1, s1 = gdn_chunk(*[x[:, a:b].contiguous() for x in d], initial_state=h0[i:i + 1])
+        assert torch.equal(o1, out[:, a:b]) and torch.equal(s1, st[i:i + 1]), i
