@@ -84,9 +84,9 @@ inline WorkspaceLayout workspace_layout(size_t tiles, bool with_meta = false) {
 // A function of the lengths and of the SM count alone.  One of 30000 tokens with twenty of 50-100 beside it, 32 heads: 1.18 ms
 // when the NUMBER of sequences decided, 0.36 now (the long one alone 0.31).
 constexpr int kMaxSegments = 15;
-constexpr int kPlanChunks = 24000;   // the prefix sums of a head have to fit the ring's shared memory
+constexpr int kPlanChunks = 24000;   // units of the plan: their prefix sums have to fit the ring's shared memory (longer sequences: several chunks a unit)
 inline int chain_segments(long long chunks, int NT, int slots) {
-    if (chunks <= 0 || NT > kPlanChunks) return 1;
+    if (chunks <= 0) return 1;
     const long long share = static_cast<long long>(NT) * slots / chunks;
     int g = share > kMaxSegments ? kMaxSegments : static_cast<int>(share);
     if (g > NT / 4) g = NT / 4;

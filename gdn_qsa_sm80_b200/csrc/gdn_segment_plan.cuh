@@ -14,7 +14,8 @@
 // as "-128, forgotten" where the decay was -2 (errors up to 100 % behind such a boundary).  So they are integers:
 // -sum of g in units of 2^-10, rounded towards zero (a boundary counts as forgotten late, never early), and a chunk counts
 // 128 at most - one below -115 forgets on its own.  kPlanChunks of them stay below 2^32, and integer sums are exact and monotone,
-// which the binary search needs.
+// which the binary search needs.  A sequence of more chunks is planned in units of several: the smallest number that leaves at most
+// kPlanChunks units, each counting 128 at most.
 //
 // Every CTA of a head makes the same plan from the per-chunk scalars the prepare kernel left: for each number of segments
 // g up to the launch's most (a warp each), equal segments first, then segment 0, which has no warm-up, longer by about the
@@ -28,7 +29,7 @@
 
 namespace gdn {
 
-struct SegmentPlan {          // segment 0 = chunks [0, L0), segment s >= 1 = L1 chunks from L0 + (s - 1) L1 on
+struct SegmentPlan {          // in chunks: segment 0 = chunks [0, L0), segment s >= 1 = L1 chunks from L0 + (s - 1) L1 on
     int g, L0, L1;
     int warm[kMaxSegments];    // chunks of warm-up before each segment s >= 1
 };
@@ -66,15 +67,21 @@ __device__ __forceinline__ int warmups(const unsigned* pre, int NT, int g, int L
     return __reduce_max_sync(0xffffffffu, w);
 }
 
-// All threads of the CTA: the split of this head (plan.g = 1: serial).  `pre`: NT + 1 words of shared memory.
+// All threads of the CTA: the split of this head (plan.g = 1: serial), `chunks` of them.  `pre`: kPlanChunks + 1 words of shared memory.
 template <int THREADS>
-__device__ __forceinline__ void plan_segments(const float* meta, int NT, int G, unsigned* pre, SegmentPlan& plan, int* best) {
+__device__ __forceinline__ void plan_segments(const float* meta, int chunks, int G, unsigned* pre, SegmentPlan& plan, int* best) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int unit = (chunks + kPlanChunks - 1) / kPlanChunks, NT = (chunks + unit - 1) / unit;   // chunks of a unit; units
+    constexpr unsigned cap = static_cast<unsigned>(kForgetCap * kForgetScale);
     int bad = 0;
     for (int t = tid; t < NT; t += THREADS) {
-        const float2 m = *reinterpret_cast<const float2*>(meta + 2 * t);
-        pre[t + 1] = __float2uint_rd(fminf(-m.x, kForgetCap) * kForgetScale);
-        if (!(m.y <= 2.f) || !(m.x <= 0.f)) bad = 1;    // outside the premise (also NaN, and +inf for a gate out of range)
+        unsigned sum = 0;
+        for (int c = t * unit; c < min(chunks, (t + 1) * unit); ++c) {
+            const float2 m = *reinterpret_cast<const float2*>(meta + 2 * c);
+            sum = min(cap, sum + __float2uint_rd(fminf(-m.x, kForgetCap) * kForgetScale));
+            if (!(m.y <= 2.f) || !(m.x <= 0.f)) bad = 1;    // outside the premise (also NaN, and +inf for a gate out of range)
+        }
+        pre[t + 1] = sum;
     }
     if (tid == 0) {
         pre[0] = 0;
@@ -126,10 +133,10 @@ __device__ __forceinline__ void plan_segments(const float* meta, int NT, int G, 
     if (g <= G && score == *best) {
         if (lane == 0) {
             plan.g = g;
-            plan.L0 = L0;
-            plan.L1 = L1;
+            plan.L0 = L0 * unit;
+            plan.L1 = L1 * unit;
         }
-        if (lane < g) plan.warm[lane] = mine;
+        if (lane < g) plan.warm[lane] = mine * unit;
     }
     __syncthreads();
 }

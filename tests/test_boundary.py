@@ -88,3 +88,12 @@ def test_missing_library_fails_loudly(monkeypatch):
     monkeypatch.setattr(_lib, "LIB_PATH", os.path.join(ROOT, "does", "not", "exist.so"))
     with pytest.raises(_lib.GdnLibraryError, match="no fallback"):
         _lib.load()
+
+
+def test_very_long_sequences_may_still_be_split():
+    """Room for the split's per-tile scalars is asked for beyond 24000 chunks (1,536,000 tokens) too."""
+    L = _lib.load()
+    for S in (1_536_000, 1_536_001, 4_000_000):
+        unsplit = (ctypes.c_size_t * 5)()
+        assert L.gdn_chunk_workspace_offsets(1, S, 1, 1, unsplit) == 0
+        assert L.gdn_chunk_scratch_bytes(1, S, 1, 1, _lib.PATH_AUTO) >= unsplit[4] + 8 * (S // 64)

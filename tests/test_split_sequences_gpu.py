@@ -111,3 +111,23 @@ def test_non_finite_keys_run_serially(value, l2norm):
     check_device_status()
     assert torch.equal(o[:, 64:].isfinite(), o2[:, 64:].isfinite()) and torch.equal(s.isfinite(), s2.isfinite())
     assert not s[:, :2].isfinite().any() and s[:, 2:].isfinite().all()
+
+
+def test_more_chunks_than_the_plan_has_room_for():
+    """Beyond 24000 chunks the plan works on groups of chunks."""
+    S, Hq, Hv = 64 * 24000 + 64 * 1001 + 5, 1, 1
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    rand = lambda *shape: torch.randn(*shape, generator=gen, device="cuda")
+    q, k = (torch.nn.functional.normalize(rand(1, S, Hq, 128), dim=-1).bfloat16() for _ in range(2))
+    v, g, beta = rand(1, S, Hv, 128).bfloat16(), -0.1 * torch.nn.functional.softplus(rand(1, S, Hv)), torch.sigmoid(rand(1, S, Hv))
+    g[:, 1000:200000] *= 1e-3     # one stretch that forgets nothing
+    h0 = rand(1, Hv, 128, 128)
+    o1, s1 = gdn_chunk(q, k, v, g, beta, initial_state=h0)
+    check_device_status()
+    o2, s2 = gdn_chunk(q, k, v, g, beta, initial_state=h0, path="twopass_nv64")
+    check_device_status()
+    n = S // 64 * 64
+    # block by block: the two kernels differ by bf16 operand rounding only (as above)
+    a, b = (x[0, :n, 0].float().reshape(-1, 64 * 128) for x in (o1, o2))
+    assert ((a - b).norm(dim=1) <= 1e-2 * b.norm(dim=1)).all()
+    assert ((s1 - s2).norm() <= 6e-3 * s2.norm()).item() and ((o1[0, n:].float() - o2[0, n:].float()).norm() <= 1e-2 * o2[0, n:].float().norm()).item()
