@@ -80,12 +80,6 @@ def load() -> ctypes.CDLL:
             f"{LIB_PATH} is missing: build it with `python -m gdn_qsa_sm80_b200.build` "
             "(sm_100a only; there is no fallback implementation)")
     lib = ctypes.CDLL(LIB_PATH)
-    # These enqueue several kernels that hand data over in the scratch buffer of their stream (a packed batch: tables the
-    # kernels index with), so two threads' calls on one stream must not interleave: they keep the interpreter lock, as the
-    # native front end does.
-    held = ctypes.PyDLL(LIB_PATH)
-    for name in ("gdn_chunk_fwd_sm100_ex", "gdn_chunk_fwd_gated_sm100", "gdn_chunk_fwd_varlen_sm100"):
-        setattr(lib, name, getattr(held, name))
     vp, ci, sz = ctypes.c_void_p, ctypes.c_int, ctypes.c_size_t
     lib.gdn_chunk_scratch_bytes.argtypes = [ci, ci, ci, ci, ci]
     lib.gdn_chunk_scratch_bytes.restype = sz

@@ -5,6 +5,7 @@
 #include <stdlib.h>
 
 #include <atomic>
+#include <condition_variable>
 #include <mutex>
 
 #include "../../include/gdn_chunk_sm100.h"
@@ -139,6 +140,32 @@ int allow_smem(const void* kernel, size_t bytes) {
     return 0;
 }
 
+// the calls that enqueue at the moment, one entry per buffer (the entries live on the callers' stacks)
+static std::mutex g_enqueue_mutex;
+static std::condition_variable g_enqueue_done;
+static EnqueueLock* g_enqueueing = nullptr;
+
+EnqueueLock::EnqueueLock(const void* scratch) : scratch_(scratch) {
+    std::unique_lock<std::mutex> lock(g_enqueue_mutex);
+    g_enqueue_done.wait(lock, [&] {
+        for (const EnqueueLock* e = g_enqueueing; e; e = e->next_)
+            if (e->scratch_ == scratch) return false;
+        return true;
+    });
+    next_ = g_enqueueing;
+    g_enqueueing = this;
+}
+
+EnqueueLock::~EnqueueLock() {
+    {
+        std::lock_guard<std::mutex> lock(g_enqueue_mutex);
+        EnqueueLock** e = &g_enqueueing;
+        while (*e != this) e = &(*e)->next_;
+        *e = next_;
+    }
+    g_enqueue_done.notify_all();
+}
+
 static long long* g_phase_profile = nullptr;
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -195,6 +222,7 @@ int gdn_chunk_fwd_sm100(const void* q, const void* k, const void* v, const void*
 int gdn_chunk_fwd_sm100_ex(const void* q, const void* k, const void* v, const void* g, const void* beta,
                            const float* h0, void* out, float* hT, void* scratch, size_t scratch_bytes,
                            int B, int S, int Hq, int Hv, int gate_dtype, int path, unsigned flags, void* stream_) {
+    const EnqueueLock lock(scratch);
     return forward_device(q, k, v, g, beta, h0, out, hT, scratch, scratch_bytes, B, S, Hq, Hv, gate_dtype, path,
                           flags, static_cast<cudaStream_t>(stream_), true);
 }
@@ -206,6 +234,7 @@ int gdn_chunk_fwd_gated_sm100(const void* q, const void* k, const void* v, const
     if (!z || !weight || !aligned16(z) || !aligned16(weight)) return GDN_ERR_BAD_ARGUMENT;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     const OutputGate gate{z, weight, eps};
+    const EnqueueLock lock(scratch);
     return forward_device(q, k, v, g, beta, h0, out, hT, scratch, scratch_bytes, B, S, Hq, Hv, gate_dtype, path, flags,
                           stream, true, &gate);
 }

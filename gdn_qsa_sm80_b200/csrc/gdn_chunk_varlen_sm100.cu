@@ -111,6 +111,7 @@ int gdn_chunk_fwd_varlen_sm100(const void* q, const void* k, const void* v, cons
     if (bits & 15u) return GDN_ERR_BAD_ARGUMENT;
     const PackedLayout l = packed_layout(cu_seqlens, n_seq, Hv);
     if (!scratch || (reinterpret_cast<uintptr_t>(scratch) & 255u) || scratch_bytes < l.total) return GDN_ERR_SCRATCH;
+    const EnqueueLock lock(scratch);
     uint8_t* base = static_cast<uint8_t*>(scratch);
     bool clear = true;                // whichever kernel comes first clears the status word
 

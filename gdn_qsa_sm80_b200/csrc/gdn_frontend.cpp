@@ -22,12 +22,25 @@
 namespace {
 
 // Scratch buffers by (device, stream), handed over by the Python wrapper, which owns the policy (one per device and stream,
-// grown when too small).  Guarded by the interpreter lock.
+// grown when too small).  Guarded by the interpreter lock; a call keeps its own reference, since the lock is released while
+// it enqueues and another thread may put a larger buffer in place meanwhile.
 std::map<std::pair<int, void*>, at::Tensor>& scratch_buffers() {
     static auto* m = new std::map<std::pair<int, void*>, at::Tensor>;   // lives as long as the process: no CUDA calls at exit
     return *m;
 }
 PyObject* g_grow_scratch = nullptr;   // _scratch_for(device index, bytes), which calls note_scratch
+
+// Releases the interpreter lock: a launch may block on a full queue behind work that needs it, an allocation may synchronise.
+class Unlocked {
+public:
+    Unlocked() : state_(PyEval_SaveThread()) {}
+    ~Unlocked() { PyEval_RestoreThread(state_); }
+    Unlocked(const Unlocked&) = delete;
+    Unlocked& operator=(const Unlocked&) = delete;
+
+private:
+    PyThreadState* state_;
+};
 
 bool plain(const at::Tensor& t, at::ScalarType dtype, const at::Device& dev) {
     return t.defined() && t.scalar_type() == dtype && t.device() == dev && t.layout() == at::kStrided && t.is_contiguous() && !t.is_neg() &&
@@ -98,21 +111,26 @@ PyObject* forward_plain(PyObject* const* a, Py_ssize_t n) {
         it = buffers.find({dev.index(), stream});
         if (it == buffers.end() || static_cast<size_t>(it->second.numel()) < need) Py_RETURN_NONE;
     }
-    void* scratch = it->second.data_ptr();
-    const size_t scratch_bytes = static_cast<size_t>(it->second.numel());
+    const at::Tensor buffer = it->second;
+    void* scratch = buffer.data_ptr();
+    const size_t scratch_bytes = static_cast<size_t>(buffer.numel());
 
-    at::Tensor out(at::detail::empty_cuda({B, S, Hv, GDN_D}, at::kBFloat16, dev, std::nullopt)), hT;
-    if (want_state) hT = at::Tensor(at::detail::empty_cuda({B, Hv, GDN_D, GDN_D}, at::kFloat, dev, std::nullopt));
-    float* state = want_state ? hT.mutable_data_ptr<float>() : nullptr;
+    const void *qp = q.const_data_ptr(), *kp = k.const_data_ptr(), *vp = v.const_data_ptr(), *gp = g.const_data_ptr(), *bp = beta.const_data_ptr();
     const int gate_code = gate == at::kFloat ? GDN_GATE_F32 : GDN_GATE_BF16;
-    const int st = z ? gdn_chunk_fwd_gated_sm100(q.const_data_ptr(), k.const_data_ptr(), v.const_data_ptr(), g.const_data_ptr(), beta.const_data_ptr(), h0,
-                                                 z, w, static_cast<float>(eps), out.mutable_data_ptr(), state, scratch, scratch_bytes,
-                                                 static_cast<int>(B), static_cast<int>(S), static_cast<int>(Hk), static_cast<int>(Hv), gate_code,
-                                                 static_cast<int>(path), static_cast<unsigned>(flags), stream)
-                     : gdn_chunk_fwd_sm100_ex(q.const_data_ptr(), k.const_data_ptr(), v.const_data_ptr(), g.const_data_ptr(), beta.const_data_ptr(), h0,
-                                              out.mutable_data_ptr(), state, scratch, scratch_bytes, static_cast<int>(B), static_cast<int>(S),
-                                              static_cast<int>(Hk), static_cast<int>(Hv), gate_code, static_cast<int>(path),
-                                              static_cast<unsigned>(flags), stream);
+    at::Tensor out, hT;
+    int st;
+    {
+        const Unlocked unlocked;   // (its destructor runs before an exception reaches the handler)
+        out = at::Tensor(at::detail::empty_cuda({B, S, Hv, GDN_D}, at::kBFloat16, dev, std::nullopt));
+        if (want_state) hT = at::Tensor(at::detail::empty_cuda({B, Hv, GDN_D, GDN_D}, at::kFloat, dev, std::nullopt));
+        float* state = want_state ? hT.mutable_data_ptr<float>() : nullptr;
+        st = z ? gdn_chunk_fwd_gated_sm100(qp, kp, vp, gp, bp, h0, z, w, static_cast<float>(eps), out.mutable_data_ptr(), state, scratch,
+                                           scratch_bytes, static_cast<int>(B), static_cast<int>(S), static_cast<int>(Hk), static_cast<int>(Hv),
+                                           gate_code, static_cast<int>(path), static_cast<unsigned>(flags), stream)
+               : gdn_chunk_fwd_sm100_ex(qp, kp, vp, gp, bp, h0, out.mutable_data_ptr(), state, scratch, scratch_bytes, static_cast<int>(B),
+                                        static_cast<int>(S), static_cast<int>(Hk), static_cast<int>(Hv), gate_code, static_cast<int>(path),
+                                        static_cast<unsigned>(flags), stream);
+    }
     if (st != GDN_OK) Py_RETURN_NONE;   // the wrapper makes the call again and raises its status
     PyObject* po = THPVariable_Wrap(std::move(out));
     if (!po) return nullptr;

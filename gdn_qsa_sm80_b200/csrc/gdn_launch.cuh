@@ -9,6 +9,21 @@
 
 namespace gdn {
 
+// Held by an entry point while it enqueues: calls that use the same scratch buffer hand data from kernel to kernel through it (a
+// packed batch: tables the kernels index with), so two threads' calls must not interleave.  Calls on different buffers
+// do not wait for each other; nothing is allocated and nothing kept behind the call.
+class EnqueueLock {
+public:
+    explicit EnqueueLock(const void* scratch);
+    ~EnqueueLock();
+    EnqueueLock(const EnqueueLock&) = delete;
+    EnqueueLock& operator=(const EnqueueLock&) = delete;
+
+private:
+    const void* scratch_;
+    EnqueueLock* next_;
+};
+
 // Lets `kernel` use `bytes` of dynamic shared memory on the current device; 0 on success.
 int allow_smem(const void* kernel, size_t bytes);
 

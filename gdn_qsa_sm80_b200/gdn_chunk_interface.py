@@ -16,6 +16,7 @@ CUDA library behind the C ABI.  There is no CPU or eager fallback.
 from __future__ import annotations
 
 import os
+import threading
 
 import torch
 
@@ -27,6 +28,7 @@ GDN_D = 128      # head dim (compile-time constant in the kernels)
 GDN_CHUNK = 64   # intra-chunk size (compile-time constant)
 
 _scratch = {}
+_scratch_lock = threading.Lock()   # growing one: this dictionary and the front end hold the same buffer
 
 
 def _check_inputs(q, k, v, g, beta):
@@ -85,11 +87,12 @@ def rmsnorm_gated(y, z, weight, eps=1e-6, out=None):
 def _scratch_for(device, nbytes):
     # one buffer per (device, stream): calls on different streams may overlap on the GPU and must not share scratch
     key = (device.index, torch.cuda.current_stream(device).cuda_stream)
-    buf = _scratch.get(key)
-    if buf is None or buf.numel() < nbytes:
-        buf = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
-        _scratch[key] = buf
-        _lib.frontend().note_scratch(*key, buf)
+    with _scratch_lock:
+        buf = _scratch.get(key)
+        if buf is None or buf.numel() < nbytes:
+            buf = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
+            _scratch[key] = buf
+            _lib.frontend().note_scratch(*key, buf)
     return buf
 
 

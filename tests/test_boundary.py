@@ -97,3 +97,12 @@ def test_very_long_sequences_may_still_be_split():
         unsplit = (ctypes.c_size_t * 5)()
         assert L.gdn_chunk_workspace_offsets(1, S, 1, 1, unsplit) == 0
         assert L.gdn_chunk_scratch_bytes(1, S, 1, 1, _lib.PATH_AUTO) >= unsplit[4] + 8 * (S // 64)
+
+
+def test_calls_leave_the_interpreter_lock():
+    """A launch may block on a full queue behind work that needs the interpreter: no entry point is called with its lock held."""
+    L = _lib.load()
+    python_api = ctypes.PyDLL(_lib.LIB_PATH).gdn_chunk_read_status._flags_ & ~ctypes.CDLL(_lib.LIB_PATH).gdn_chunk_read_status._flags_
+    assert python_api
+    for name in _lib.EXPORTS:
+        assert not getattr(L, name)._flags_ & python_api, name

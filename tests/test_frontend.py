@@ -1,12 +1,15 @@
 """Tensors that have no memory behind them reach the native front end as errors, not as a C++ exception through the
 interpreter (which would end the process)."""
+import sys
 import threading
+import time
 
 import pytest
 import torch
 from torch._subclasses.fake_tensor import FakeTensorMode
 
-from gdn_qsa_sm80 import gdn_chunk
+from gdn_qsa_sm80 import gdn_chunk, gdn_chunk_varlen
+from gdn_qsa_sm80_b200 import gdn_chunk_interface as interface
 
 
 def _call(dev):
@@ -56,3 +59,78 @@ def test_a_threads_first_cuda_call(S):
     assert len(got) == 2
     assert torch.equal(got[0][0], want[0]) and torch.equal(got[0][1], want[1])
     assert torch.equal(got[1][0], gdn_chunk(*x, initial_state=h0)[0])
+
+
+@pytest.mark.gpu
+def test_other_threads_run_during_launches():
+    """The forward call lets go of the interpreter while it launches.  With a switch interval of a minute another thread only
+    runs when it does: enough calls to fill the launch queue give it hundreds of turns, or none."""
+    x = _inputs(1, 1, 16, 32, 0)
+    gdn_chunk(*x)                          # scratch buffer and kernels in place
+    torch.cuda.synchronize()
+    turns, stop, started = [0], threading.Event(), threading.Event()
+
+    def count():
+        started.set()
+        while not stop.is_set():
+            turns[0] += 1
+            time.sleep(0)
+
+    t = threading.Thread(target=count)
+    t.start()
+    started.wait()
+    old = sys.getswitchinterval()
+    sys.setswitchinterval(60.0)
+    try:
+        before = turns[0]
+        for _ in range(5000):
+            gdn_chunk(*x)
+        during = turns[0] - before
+    finally:
+        sys.setswitchinterval(old)
+        stop.set()
+        t.join()
+    torch.cuda.synchronize()
+    assert during > 100     # (7 with the lock held: what the call does before it launches)
+
+
+@pytest.mark.gpu
+def test_threads_on_one_stream():
+    """Calls of several threads on one stream share its scratch buffer, which grows meanwhile: each gives the bits it gives alone."""
+    def plain(seed, B, S):
+        x = _inputs(B, S, 2, 4, seed)
+        return lambda: gdn_chunk(*x)
+
+    def converted(seed, S):                # through the Python wrapper
+        q, k, v, g, beta = _inputs(1, S, 2, 4, seed)
+        return lambda: gdn_chunk(q.float(), k, v, g, beta)
+
+    def packed(seed, lens):
+        x = _inputs(1, sum(lens), 2, 4, seed)
+        cu = [sum(lens[:i]) for i in range(len(lens) + 1)]
+        return lambda: gdn_chunk_varlen(*x, cu)
+
+    jobs = [[plain(1, 1, 700), packed(2, [3, 100, 9, 64]), converted(3, 200)], [packed(4, [500, 20, 1, 1, 1500]), plain(5, 3, 130)],
+            [converted(6, 2000), plain(7, 64, 1), packed(8, [5, 6, 7])], [plain(9, 8, 4), packed(10, [40] * 30), plain(11, 2, 3000)]]
+    want = [[job() for job in mine] for mine in jobs]
+    torch.cuda.synchronize()
+    interface._scratch.clear()             # (the Python wrapper's buffers start small again)
+    wrong = []
+
+    def work(i):
+        try:
+            for _ in range(40):
+                for job, (o, s) in zip(jobs[i], want[i]):
+                    a, b = job()
+                    if not (torch.equal(a, o) and torch.equal(b, s)):
+                        wrong.append(i)
+        except Exception as e:
+            wrong.append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(jobs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    interface.check_device_status()
+    assert not wrong
