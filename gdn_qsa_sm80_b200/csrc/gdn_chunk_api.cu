@@ -123,19 +123,36 @@ int sm_count() {
     return cached[dev];
 }
 
+// Id of the current context (never used twice in a process), 0 if there is none.
+static unsigned long long context_id() {
+    typedef CUresult (*GetIdFn)(CUcontext, unsigned long long*);
+    static GetIdFn fn = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* sym = nullptr;
+        cudaDriverEntryPointQueryResult qres;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &sym, cudaEnableDefault, &qres) == cudaSuccess && qres == cudaDriverEntryPointSuccess)
+            fn = reinterpret_cast<GetIdFn>(sym);
+    });
+    unsigned long long id = 0;
+    return fn && fn(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+
+// The limit belongs to the kernel as the current context has loaded it: a program may have several contexts on a device, one after
+// another or side by side (one that owns a part of the SMs, for instance).
 int allow_smem(const void* kernel, size_t bytes) {
-    struct Set { const void* kernel; int dev; size_t bytes; };
+    struct Set { const void* kernel; unsigned long long context; size_t bytes; };
     static Set set[64];
     static int n = 0;
     static std::mutex mutex;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 1;
+    const unsigned long long context = context_id();
     std::lock_guard<std::mutex> lock(mutex);
     int i = 0;
-    while (i < n && (set[i].kernel != kernel || set[i].dev != dev)) ++i;
-    if (i < n && set[i].bytes >= bytes) return 0;
+    while (i < n && (set[i].kernel != kernel || set[i].context != context)) ++i;
+    if (context && i < n && set[i].bytes >= bytes) return 0;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)) != cudaSuccess) return 1;
-    if (i == n && n < 64) set[n++] = Set{kernel, dev, 0};
+    if (!context) return 0;
+    if (i == n && n < 64) set[n++] = Set{kernel, context, 0};
     if (i < n) set[i].bytes = bytes;
     return 0;
 }

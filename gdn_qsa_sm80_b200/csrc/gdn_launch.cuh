@@ -1,4 +1,4 @@
-// Host side of a kernel launch: the dynamic shared-memory limit (set once per kernel and device, not on every call) and
+// Host side of a kernel launch: the dynamic shared-memory limit (set once per kernel and context, not on every call) and
 // the launch as a programmatic dependent of the kernel before it in the stream.
 #pragma once
 
@@ -24,7 +24,7 @@ private:
     EnqueueLock* next_;
 };
 
-// Lets `kernel` use `bytes` of dynamic shared memory on the current device; 0 on success.
+// Lets `kernel` use `bytes` of dynamic shared memory in the current context; 0 on success.
 int allow_smem(const void* kernel, size_t bytes);
 
 // Launches with the programmatic-stream-serialization attribute: the CTAs may set up while the kernel before this one in the
