@@ -285,7 +285,8 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
 // `og`: gated normalisation applied to the output rows by the same kernel (null: none).
 int launch_decode(const Problem& p, const OutputGate* og, cudaStream_t stream) {
     const long long states = static_cast<long long>(p.B) * p.Hv;   // (of a packed batch: all sequences', the map's extent)
-    if (states * kD >= (1ll << 31)) return GDN_ERR_BAD_ARGUMENT;
+    // a state's row is a map coordinate (2^31 rows of states: 1 TB); without states only the number of tiles is an int
+    if (states * ((p.h0 || p.hT) ? kD : 4) >= (1ll << 31)) return GDN_ERR_BAD_ARGUMENT;
     alignas(64) CUtensorMap tin, tout;
     const unsigned long long d[2] = {kD, static_cast<unsigned long long>(states) * kD}, sb[1] = {kD * 4};
     const unsigned box[2] = {32, kD};

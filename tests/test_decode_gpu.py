@@ -101,3 +101,17 @@ def test_gated_decode(B, S, Hq, Hv, gates, stored):
         ro, _ = oracle_f32(q, k, v, g, beta, None if h0 is None else h0.cpu(), form="recurrent")
         ro = O.rmsnorm_gated(ro, z.float().cpu().numpy(), w.float().cpu().numpy())
         assert O.rel_l2(first.float().cpu().numpy(), ro) < 6e-3   # two bf16 roundings: the row, then the result
+
+
+def test_more_rows_than_a_state_map_could_address():
+    """Without states the decode kernel's range is that of its inputs: more than 2^24 (sequence, head) pairs."""
+    B, Hv, tail = (1 << 21) + 3, 8, 1000
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    q, k = (torch.randn(B, 1, 1, 128, generator=gen, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    v = torch.randn(B, 1, Hv, 128, generator=gen, device="cuda", dtype=torch.bfloat16)
+    g, beta = -torch.rand(B, 1, Hv, generator=gen, device="cuda"), torch.rand(B, 1, Hv, generator=gen, device="cuda")
+    out, _ = gdn_chunk(q, k, v, g, beta, output_final_state=False, path="decode")
+    check_device_status()
+    for part in (slice(0, tail), slice(B - tail, B)):
+        ref, _ = gdn_chunk(*[x[part].contiguous() for x in (q, k, v, g, beta)], output_final_state=False)
+        assert torch.equal(out[part], ref)
