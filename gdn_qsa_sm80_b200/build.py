@@ -23,6 +23,7 @@ LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libgdn_chunk_sm100.so")
 FRONTEND_PATH = os.path.join(LIB_DIR, "_gdn_frontend.so")
 OBJ_DIR = os.path.join(HERE, "build")
+TORCH_STAMP = os.path.join(OBJ_DIR, "frontend_torch_version")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -50,8 +51,19 @@ def _deps_mtime() -> float:
     return max(os.path.getmtime(f) for f in files)
 
 
+def _torch_version() -> str:
+    import importlib.metadata
+    return importlib.metadata.version("torch")
+
+
 def needs_build() -> bool:
-    return any(not os.path.exists(p) or os.path.getmtime(p) < _deps_mtime() for p in (LIB_PATH, FRONTEND_PATH))
+    if any(not os.path.exists(p) or os.path.getmtime(p) < _deps_mtime() for p in (LIB_PATH, FRONTEND_PATH)):
+        return True
+    try:    # the front end links torch's libraries
+        with open(TORCH_STAMP) as f:
+            return f.read() != _torch_version()
+    except OSError:
+        return True
 
 
 def _build_frontend() -> None:
@@ -69,6 +81,8 @@ def _build_frontend() -> None:
     if r.returncode != 0:
         sys.stderr.write(r.stdout + r.stderr)
         raise RuntimeError("g++ failed on gdn_frontend.cpp")
+    with open(TORCH_STAMP, "w") as f:
+        f.write(_torch_version())
 
 
 def build(force: bool = False, verbose: bool = False, diagnostics: bool | None = None) -> str:

@@ -11,6 +11,7 @@
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/version.h>
 
 #include <cstdlib>
 #include <cstring>
@@ -193,4 +194,11 @@ PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_gdn_frontend", nullptr, -1, m
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__gdn_frontend(void) { return PyModule_Create(&module_def); }
+PyMODINIT_FUNC PyInit__gdn_frontend(void) {
+    PyObject* m = PyModule_Create(&module_def);
+    if (m && PyModule_AddStringConstant(m, "torch_version", TORCH_VERSION) < 0) {   // what it was built against
+        Py_DECREF(m);
+        return nullptr;
+    }
+    return m;
+}

@@ -92,7 +92,9 @@ def _scratch_for(device, nbytes):
         if buf is None or buf.numel() < nbytes:
             buf = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
             _scratch[key] = buf
-            _lib.frontend().note_scratch(*key, buf)
+            front = _lib.frontend()
+            if front is not None:
+                front.note_scratch(*key, buf)
     return buf
 
 
@@ -105,6 +107,9 @@ def _native():
     global _native_forward
     if _native_forward is None:
         front = _lib.frontend()
+        if front is None:
+            _native_forward = lambda *args: None
+            return _native_forward
         front.set_grow_scratch(lambda index, nbytes: _scratch_for(torch.device("cuda", index), nbytes))
         _native_forward = front.forward
     return _native_forward

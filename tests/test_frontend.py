@@ -9,7 +9,10 @@ import torch
 from torch._subclasses.fake_tensor import FakeTensorMode
 
 from gdn_qsa_sm80 import gdn_chunk, gdn_chunk_varlen
+from gdn_qsa_sm80_b200 import _lib
 from gdn_qsa_sm80_b200 import gdn_chunk_interface as interface
+
+FRONTEND_PATH = _lib.FRONTEND_PATH
 
 
 def _call(dev):
@@ -134,3 +137,32 @@ def test_threads_on_one_stream():
         t.join()
     interface.check_device_status()
     assert not wrong
+
+
+@pytest.fixture
+def without_front_end(monkeypatch, tmp_path):
+    """A front end that cannot be loaded here: built against another torch, or not at all."""
+    monkeypatch.setattr(_lib, "FRONTEND_PATH", str(tmp_path / "_gdn_frontend.so"))
+    monkeypatch.setattr(_lib, "_frontend", False)
+    monkeypatch.setattr(interface, "_native_forward", None)
+
+
+def test_the_wrapper_runs_without_the_front_end(without_front_end):
+    with pytest.warns(RuntimeWarning, match="front end"), pytest.raises(RuntimeError, match="needs CUDA tensors"):
+        _call("cpu")
+    with pytest.raises(RuntimeError, match="needs CUDA tensors"):
+        _call("cpu")
+
+
+@pytest.mark.gpu
+@pytest.mark.filterwarnings("ignore:gdn_chunk runs without")
+def test_results_without_the_front_end(without_front_end):
+    x = _inputs(2, 130, 2, 4, 1)
+    wrapped, packed = gdn_chunk(*x), gdn_chunk_varlen(*[t.reshape(1, 260, *t.shape[2:]) for t in x], [0, 130, 260])
+    assert _lib._frontend is None
+    _lib._frontend = False
+    _lib.FRONTEND_PATH, interface._native_forward = FRONTEND_PATH, None
+    native = gdn_chunk(*x)
+    assert _lib._frontend
+    for a, b, c in zip(wrapped, native, packed):
+        assert torch.equal(a, b) and torch.equal(c.reshape(a.shape), a)
