@@ -220,7 +220,20 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = warp_uniform(tmem_slot);
-    const bool prof_cta = GDN_DIAG(p.prof != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0);
+#ifdef GDN_DIAGNOSTICS   // cycles of one thread of the critical warps (in shared memory: the roles have no registers to spare)
+    __shared__ long long prof_acc[7];   // phases 0-5 and the last time stamp
+    const bool prof_on = p.prof != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && tid == 0;
+    if (prof_on)
+        for (int n = 0; n < 7; ++n) prof_acc[n] = n == 6 ? clock64() : 0;
+#define GDN_PHASE(n)                              \
+    if (prof_on) {                                \
+        const long long now_ = clock64();         \
+        prof_acc[n] += now_ - prof_acc[6];        \
+        prof_acc[6] = now_;                       \
+    }
+#else
+#define GDN_PHASE(n)
+#endif
     const int steps = work.steps;
     auto wait = [&](uint32_t bar, uint32_t parity) {
         return r_wait(cb(bar), parity & 1, kRTimeout + static_cast<int>(bar), work);
@@ -508,6 +521,7 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             ok = wait(R_VFULL + s, n >> 1) && wait(R_KS, n);
             if (!ok) break;
             tc_fence_after_sync();
+            GDN_PHASE(0)
             const float* vec = reinterpret_cast<const float*>(sm + R_VEC + s * 1024);
             const float dC = vec[2 * kChunk];                 // exp(gamma_C); read now, the slot is released below
 #pragma unroll
@@ -527,9 +541,11 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive_a(cb(R_X));
+            GDN_PHASE(1)
             ok = wait(R_VACC, n);
             if (!ok) break;
             tc_fence_after_sync();
+            GDN_PHASE(2)
 #pragma unroll
             for (int u = 0; u < 4; ++u) {                     // v_new and v~ of tokens [32 hf + 8 u, +8)
                 uint32_t x[8], pk[4];
@@ -553,9 +569,11 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 mbar_arrive_a(cb(R_VN));
                 mbar_arrive_a(cb(R_VEMPTY + s));
             }
+            GDN_PHASE(3)
             ok = wait(R_S, n);
             if (!ok) break;
             tc_fence_after_sync();
+            GDN_PHASE(4)
             const bool more = n + 1 < steps;
 #pragma unroll
             for (int u = 0; u < 4; ++u) {                     // S^T <- exp(gamma_C) S^T + v~^T K, 16 columns at a time
@@ -577,7 +595,14 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 __syncwarp();
                 if (lane == 0) mbar_arrive_a(cb(R_STATE));
             }
+            GDN_PHASE(5)
         }
+#ifdef GDN_DIAGNOSTICS   // behind the prepare kernel's: waits for KS, v_new, the state's product and the epilogues behind them
+        if (prof_on) {
+            for (int n = 0; n < 6; ++n) p.prof[8 + n] = prof_acc[n];
+            p.prof[14] = steps;
+        }
+#endif
         if (ok && work.s_out) {
             float* s_out = work.s_out + 32 * hf * kD + dv;
 #pragma unroll
@@ -593,7 +618,7 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         __syncthreads();
     }
     if (warp == 0) tmem_dealloc(tmem, kRTmemCols);
-    (void)prof_cta;
+#undef GDN_PHASE
 }
 
 }  // namespace
