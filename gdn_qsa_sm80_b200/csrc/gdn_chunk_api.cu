@@ -197,7 +197,7 @@ static size_t tiles_of(int B, int S, int Hv) {
     return static_cast<size_t>(B) * Hv * ((S + kChunk - 1) / kChunk);
 }
 
-// the residual-form chain, or the prepare kernels that write what it reads
+// the residual-form chain, or the prepare kernel in front of it
 static bool transposed_path(int path) {
     return path == GDN_PATH_TWOPASS_T || path == GDN_PATH_PREPARE_ONLY_T || path == GDN_PATH_CHAIN_ONLY_T || path == GDN_PATH_PREPARE_ONLY_R;
 }
@@ -332,7 +332,6 @@ int forward_device(const void* q, const void* k, const void* v, const void* g, c
     else nv = 64;
     // the transposed chain splits sequences when the scratch buffer has room for the per-tile scalars its decision
     // reads (a caller that sized it for an unsplit run, like the fixed-array entry point, gets the unsplit run)
-    const bool transposed = transposed_path(path);
     int n_seg = segments_of(B, S, Hv, path);
     if (n_seg > 1 && scratch_bytes < workspace_layout(tiles_of(B, S, Hv), true).total) n_seg = 1;
     const WorkspaceLayout l = workspace_layout(tiles_of(B, S, Hv), n_seg > 1);
@@ -344,21 +343,21 @@ int forward_device(const void* q, const void* k, const void* v, const void* g, c
     ws.vec = reinterpret_cast<float*>(base + l.vec);
     ws.meta = n_seg > 1 ? reinterpret_cast<float*>(base + l.meta) : nullptr;
     ws.n_seg = n_seg;
-    if (path != GDN_PATH_TWOPASS_T && path != GDN_PATH_PREPARE_ONLY_R && !clear()) return GDN_ERR_CUDA;
+    const bool prepare_only = path == GDN_PATH_PREPARE_ONLY_T || path == GDN_PATH_PREPARE_ONLY_R;
+    if (path != GDN_PATH_TWOPASS_T && !prepare_only && !clear()) return GDN_ERR_CUDA;
     if (path == GDN_PATH_COOP_CHAIN_ONLY)
         return then_gate(launch_coop(p, ws, reinterpret_cast<int*>(base + l.flags), l.flag_bytes, stream, true));
     if (path == GDN_PATH_COOP) return then_gate(launch_coop(p, ws, reinterpret_cast<int*>(base + l.flags), l.flag_bytes, stream));
-    if (path == GDN_PATH_TWOPASS_T || path == GDN_PATH_PREPARE_ONLY_R || path == GDN_PATH_CHAIN_ONLY_T) {
+    if (transposed_path(path)) {
         TileMaps maps;
         if (encode_tile_maps(p, ws, maps)) return GDN_ERR_DRIVER;
         int st = path == GDN_PATH_CHAIN_ONLY_T ? GDN_OK : launch_prepare_lean(p, ws, maps, stream);
-        if (st != GDN_OK || path == GDN_PATH_PREPARE_ONLY_R) return st;
+        if (st != GDN_OK || prepare_only) return st;
         return then_gate(launch_chain_r(p, ws, maps, stream));
     }
     if (path == GDN_PATH_CHAIN_ONLY) return then_gate(launch_chain(p, ws, nv, stream));   // workspace left by an earlier call
-    const bool pairs = transposed && (Hv / Hq) % 2 == 0 && p.dbg != 3;
-    const int st = pairs ? launch_prepare_pair(p, ws, stream) : launch_prepare(p, ws, stream, !transposed);
-    if (st != GDN_OK || path == GDN_PATH_PREPARE_ONLY || path == GDN_PATH_PREPARE_ONLY_T) return st;
+    const int st = launch_prepare(p, ws, stream);
+    if (st != GDN_OK || path == GDN_PATH_PREPARE_ONLY) return st;
     return then_gate(launch_chain(p, ws, nv, stream));
 }
 }  // namespace gdn

@@ -42,16 +42,11 @@ struct PSmem {
 constexpr uint32_t kPrepTmemCols = 128;
 constexpr int kPrepCtasPerSm = 3;
 
-// WITH_U = false: for the transposed chain, which forms U^T = V^T T''^T itself from the raw V tile: no V load, no
-// second product, no U tile; T'' = T diag(beta) (bf16, 64 x 64, row-major) goes to the workspace instead (tm_u then
-// describes T''), and both T'' and P leave through swizzled tiles and TMA stores: T'' from the operand's rows 64-127,
-// P from a tile in Q's place (rows stored one per thread straight to global memory cost a wavefront per lane).
-template <bool GATE_F32, bool WITH_U>
+template <bool GATE_F32>
 __global__ void __launch_bounds__(128, kPrepCtasPerSm)
 gdn_prepare_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_w,
-                   const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ CUtensorMap tm_p, Problem p,
-                   Workspace ws, int NT, long long num_tiles) {
+                   const __grid_constant__ CUtensorMap tm_u, Problem p, Workspace ws, int NT, long long num_tiles) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const uint32_t sm_u32 = smem_u32(sm);
@@ -163,7 +158,7 @@ gdn_prepare_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         // TMA wait and the first UMMAs have hidden most of that latency.  Q is dead now: V takes its place.
         if (tid == 0) {
             tma_store_wait_read();
-            if (WITH_U) issue_v(cur);
+            issue_v(cur);
         }
         ok = __syncthreads_and(ok);
         if (!ok) break;
@@ -171,37 +166,17 @@ gdn_prepare_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         prep_zero_upper_blocks(Tm);   // the T buffer held the previous tile's W staging tile until the wait above
 
         tc_fence_after_sync();
-        {   // mask epilogue (one exponential per element, shared with gdn_prepare_pair_kernel, so that both kernels
-            // produce the same bits): thread = row i = TMEM lane
+        {   // mask epilogue (one exponential per element): thread = row i = TMEM lane
             const bool low_rows = (warp & 1) == 0;           // rows 0-31: columns 32-63 lie above the diagonal
             if (warp < 2) {   // A = tril(beta_i * decay * K K^T, -1), fp32, for the inverse
-                const float ksq = prep_mask_row_A(ps, p.l2norm != 0, tmem_addr(tmem, lane_base, 0), i, low_rows, As, ws.meta != nullptr);
-                if (ws.meta) {
-                    const float bound = prep_bound_of_rows(ps, p.l2norm != 0, i, ksq);
-                    if ((tid & 31) == 0) ps.wsum[warp] = bound;   // the cumsum's slots are free again by now
-                }
-            } else if (WITH_U) {   // P = tril(scale * decay * Q K^T), bf16, straight to the workspace (V is taking Q's place)
+                prep_mask_row_A(ps, p.l2norm != 0, tmem_addr(tmem, lane_base, 0), i, low_rows, As);
+            } else {               // P = tril(scale * decay * Q K^T), bf16, straight to the workspace (V is taking Q's place)
                 prep_mask_row_P(ps, p.l2norm != 0, scale0, tmem_addr(tmem, lane_base, 0), i, low_rows,
                                 ws.P + tile * (kChunk * kChunk) + static_cast<size_t>(i) * kChunk);
-            } else {               // ... into a staging tile in the place of Q's first k-half (Q is dead, no V comes)
-                uint4 pk[8];
-                prep_mask_row_P_packed(ps, p.l2norm != 0, scale0, tmem_addr(tmem, lane_base, 0), i, low_rows, pk);
-#pragma unroll
-                for (int ch = 0; ch < 8; ++ch)
-                    *reinterpret_cast<uint4*>(sm + PSmem::KQ + 8192 + swz_chunk_offset<128>(i, ch)) = pk[ch];
-                fence_proxy_async_smem();
             }
         }
         tc_fence_before_sync();
         __syncthreads();
-        if (!WITH_U && tid == 0) {
-            tma_store_2d(&tm_p, sm + PSmem::KQ + 8192, 0, static_cast<int>(tile * kChunk));
-            tma_store_commit();
-        }
-        if (ws.meta && tid == 0) {
-            ws.meta[2 * tile] = ps.gam[kChunk - 1] * (1.f / kLog2e);
-            ws.meta[2 * tile + 1] = fmaxf(ps.wsum[0], ps.wsum[1]);
-        }
         GDN_PHASE(3)
 
         prep_invert_unit_lower(As, Tm, Yt);
@@ -209,21 +184,14 @@ gdn_prepare_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 
         {   // [T diag(beta e^gamma) ; T diag(beta)] as one 128-row K-major operand
             const int which = tid >> 6;
-            // without U, rows 64-127 are only the staging tile of T'' (their product rows are never read)
             prep_store_scaled_T_row(Tm, which == 0 ? ps.eg : ps.bet, i, sm + PSmem::AS, which * 64 + i);   // A is dead
         }
         fence_proxy_async_smem();
         __syncthreads();
-        if (!WITH_U && tid == 0) {
-            tma_store_2d(&tm_u, sm + PSmem::AS + 8192, 0, static_cast<int>(tile * kChunk));
-            tma_store_commit();
-        }
-        if (WITH_U) {
-            ok = mbar_wait(&bar_tma, ph_tma, p.status, kDevTimeoutTma);   // V has landed
-            ph_tma ^= 1;
-            ok = __syncthreads_and(ok);
-            if (!ok) break;
-        }
+        ok = mbar_wait(&bar_tma, ph_tma, p.status, kDevTimeoutTma);   // V has landed
+        ph_tma ^= 1;
+        ok = __syncthreads_and(ok);
+        if (!ok) break;
         GDN_PHASE(5)
 
         // W = T' K and U = T'' V go through the same 128 TMEM columns one after the other.  Both products use the
@@ -262,7 +230,6 @@ gdn_prepare_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 }
             }
         }
-        if (WITH_U) {
         tc_fence_before_sync();
         __syncthreads();          // W has left the accumulator
         if (tid == 0) {
@@ -279,7 +246,6 @@ gdn_prepare_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         ph_mma ^= 1;
         ok = __syncthreads_and(ok);
         if (!ok) break;
-        }
         GDN_PHASE(6)
 
         // K, V and the [T';T''] operand are dead: start the next tile's loads and gate reads before the epilogue
@@ -287,15 +253,12 @@ gdn_prepare_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         Tile nxt = cur;
         if (Ln < num_tiles) {
             nxt = decode(Ln);
-            if (tid == 0) {
-                if (!WITH_U) tma_store_wait_read();   // the P tile in Q's place has been read
-                issue_loads(nxt);
-            }
+            if (tid == 0) issue_loads(nxt);
             prep_load_gates<GATE_F32>(p.g, p.beta, static_cast<size_t>(nxt.b) * p.S + nxt.s0, nxt.hv, p.Hv,
                                       min(kChunk, p.S - nxt.s0), gv, bv, PrepCtx::whole_cta(), p.gate_act != 0);
         }
         tc_fence_after_sync();
-        if (WITH_U && warp >= 2) {   // U rows (lanes 64-127) -> staging tile in the A buffer (the operand there is dead)
+        if (warp >= 2) {   // U rows (lanes 64-127) -> staging tile in the A buffer (the operand there is dead)
             uint32_t r[32];
 #pragma unroll
             for (int q4 = 0; q4 < 4; ++q4) {
@@ -320,10 +283,8 @@ gdn_prepare_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             const int row0 = static_cast<int>(tile * kChunk);
             tma_store_2d(&tm_w, sm + PSmem::TM, 0, row0);
             tma_store_2d(&tm_w, sm + PSmem::TM + 8192, 64, row0);
-            if (WITH_U) {
 #pragma unroll
-                for (int h2 = 0; h2 < 2; ++h2) tma_store_2d(&tm_u, sm + PSmem::AS + h2 * 8192, h2 * 64, row0);
-            }
+            for (int h2 = 0; h2 < 2; ++h2) tma_store_2d(&tm_u, sm + PSmem::AS + h2 * 8192, h2 * 64, row0);
             tma_store_commit();
         }
         GDN_PHASE(7)
@@ -343,29 +304,22 @@ gdn_prepare_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 
 }  // namespace
 
-int launch_prepare(const Problem& p, const Workspace& ws, cudaStream_t stream, bool with_u) {
+int launch_prepare(const Problem& p, const Workspace& ws, cudaStream_t stream) {
     alignas(64) CUtensorMap tq, tk, tv, tw, tp, tu;
     if (encode_qkv_maps(p, &tq, &tk, &tv, 64)) return GDN_ERR_DRIVER;
     if (encode_workspace_maps(p, ws, &tw, &tp, &tu, nullptr, 64)) return GDN_ERR_DRIVER;
     const int NT = (p.S + kChunk - 1) / kChunk;
-    if (!with_u) {   // T'' = T diag(beta): [tiles * 64][64] bf16 at the start of the U array
-        const unsigned long long rows = static_cast<unsigned long long>(p.B) * p.Hv * NT * kChunk;
-        const unsigned long long d[2] = {64, rows}, sb[1] = {128};
-        const unsigned box[2] = {64, 64};
-        if (encode_tma(&tu, ws.U, 2, 2, d, sb, box, 128)) return GDN_ERR_DRIVER;
-    }
     const long long tiles = static_cast<long long>(p.B) * p.Hv * NT;
     const long long max_ctas = static_cast<long long>(kPrepCtasPerSm) * sm_count();
     const unsigned grid = static_cast<unsigned>(tiles < max_ctas ? tiles : max_ctas);
     auto go = [&](auto kernel) -> int {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PSmem::kDynamic) != cudaSuccess)
             return GDN_ERR_CUDA;
-        kernel<<<grid, 128, PSmem::kDynamic, stream>>>(tq, tk, tv, tw, tu, tp, p, ws, NT, tiles);
+        kernel<<<grid, 128, PSmem::kDynamic, stream>>>(tq, tk, tv, tw, tu, p, ws, NT, tiles);
         count_launch();
         return cudaGetLastError() == cudaSuccess ? GDN_OK : GDN_ERR_CUDA;
     };
-    if (with_u) return p.gate_f32 ? go(gdn_prepare_kernel<true, true>) : go(gdn_prepare_kernel<false, true>);
-    return p.gate_f32 ? go(gdn_prepare_kernel<true, false>) : go(gdn_prepare_kernel<false, false>);
+    return p.gate_f32 ? go(gdn_prepare_kernel<true>) : go(gdn_prepare_kernel<false>);
 }
 
 }  // namespace gdn

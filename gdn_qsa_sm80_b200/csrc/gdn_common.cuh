@@ -106,12 +106,7 @@ cudaError_t launch_simt(const Problem& p, cudaStream_t stream);
 
 // "prepare" (state-independent per-chunk quantities into the workspace) and "chain" (the serial
 // state recurrence plus outputs, reading the workspace).  Both return a GDN_* status.
-// with_u = false (for the transposed chain): no U tile; T'' = T diag(beta), bf16 [tiles][64][64], is written at the
-// start of the U array instead.
-int launch_prepare(const Problem& p, const Workspace& ws, cudaStream_t stream, bool with_u = true);
-// The same as launch_prepare(with_u = false), two value heads of a qk head per CTA (shared K / Q load and raw
-// products, one product for both W); needs an even number of value heads per qk head.
-int launch_prepare_pair(const Problem& p, const Workspace& ws, cudaStream_t stream);
+int launch_prepare(const Problem& p, const Workspace& ws, cudaStream_t stream);
 int launch_chain(const Problem& p, const Workspace& ws, int nv, cudaStream_t stream);
 // The two kernels of the automatic path: "lean" prepare (P, T'', factors; no W) and the transposed chain that applies T'' to
 // the residual V - exp(gamma) K S, one CTA per (sequence, value head[, segment]); with ws.n_seg > 1 sequences may be cut

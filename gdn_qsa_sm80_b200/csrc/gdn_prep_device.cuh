@@ -81,8 +81,7 @@ __device__ __forceinline__ float prep_floor_gate(float gv) { return gv < kGateFl
 // Gate cumsum over the chunk by warp shuffles (threads 0-63 hold one token each: gv, bv) and the decay tables.
 // Contains two barriers of the group; a third one is needed before the tables are read.
 // If vec_out != nullptr, also writes the per-token factors a later kernel needs:
-//   vec_out[i] = exp(gamma_C - gamma_i), vec_out[64+i] = scale * exp(gamma_i), vec_out[128] = exp(gamma_C),
-//   vec_out[192+i] = exp(gamma_i).
+//   vec_out[i] = exp(gamma_C - gamma_i), vec_out[64+i] = scale * exp(gamma_i), vec_out[128] = exp(gamma_C).
 // tables = false skips the block decay tables (ctab) for callers whose mask epilogue does not use them.
 __device__ __forceinline__ void prep_gates(PrepScratch& ps, float gv, float bv, float scale, float* vec_out,
                                            PrepCtx ctx = PrepCtx::whole_cta(), bool tables = true) {
@@ -111,7 +110,6 @@ __device__ __forceinline__ void prep_gates(PrepScratch& ps, float gv, float bv, 
         if (vec_out) {
             vec_out[tid] = exp2f(gC - gi);
             vec_out[kChunk + tid] = scale * e;
-            vec_out[3 * kChunk + tid] = e;
             if (tid == 0) vec_out[2 * kChunk] = exp2f(gC);
         }
     }
@@ -181,7 +179,6 @@ __device__ __forceinline__ void prep_l2norm_fold(PrepScratch& ps, const uint8_t*
         if (vec_out) {
             vec_out[tid] *= ps.rn[tid];
             vec_out[kChunk + tid] *= ps.rn[kChunk + tid];
-            vec_out[3 * kChunk + tid] *= ps.rn[tid];
         }
     }
     if (tid < 96) {
@@ -260,24 +257,18 @@ __device__ __forceinline__ float fast_exp2(float x) {
 // the warp's rows are 0-31, whose columns 32-63 lie above the diagonal.
 
 // Raw K K^T row -> row i of A = tril(beta_i * decay * K K^T, -1), fp32, into `As` (columns 32-63 of rows 0-31 are
-// not written: the inverse never reads them).  Returns |k_i|^2 (the diagonal entry) when want_ksq.
-__device__ __forceinline__ float prep_mask_row_A(const PrepScratch& ps, bool l2norm, uint32_t trow, int i, bool low_rows,
-                                                 float* As, bool want_ksq) {
+// not written: the inverse never reads them).
+__device__ __forceinline__ void prep_mask_row_A(const PrepScratch& ps, bool l2norm, uint32_t trow, int i, bool low_rows,
+                                                float* As) {
     const float* gcol = l2norm ? ps.ctab[0] : ps.gam;
     const float gi = ps.gam[i];
     const float bi = l2norm ? ps.bet[i] * ps.rn[i] : ps.bet[i];
-    float ksq = 0.f;
     uint32_t r[32];
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
         if (half == 1 && low_rows) break;
         tmem_ld_x32(trow + half * 32, r);
         tmem_ld_wait();
-        if (want_ksq && (i >> 5) == half) {
-#pragma unroll
-            for (int c = 0; c < 32; ++c)
-                if (c == (i & 31)) ksq = __uint_as_float(r[c]);
-        }
 #pragma unroll
         for (int c = 0; c < 32; c += 4) {
             const float4 gj = *reinterpret_cast<const float4*>(gcol + half * 32 + c);
@@ -289,18 +280,6 @@ __device__ __forceinline__ float prep_mask_row_A(const PrepScratch& ps, bool l2n
             *reinterpret_cast<float4*>(As + i * kSolveStride + half * 32 + c) = o;
         }
     }
-    return ksq;
-}
-
-// max over the warp's rows of beta_i |k_i|^2 (the premise of the decay bound for split sequences), +inf when a gate
-// of the row is outside beta >= 0, g <= 0.  ksq: the raw diagonal entry of K K^T.
-__device__ __forceinline__ float prep_bound_of_rows(const PrepScratch& ps, bool l2norm, int i, float ksq) {
-    const float rk = l2norm ? ps.rn[i] : 1.f;
-    const bool in_range = ps.bet[i] >= 0.f && ps.gam[i] <= (i > 0 ? ps.gam[i - 1] : 0.f);
-    float bound = in_range ? ps.bet[i] * ksq * rk * rk : INFINITY;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) bound = fmaxf(bound, __shfl_xor_sync(0xffffffffu, bound, o));
-    return bound;
 }
 
 // Raw Q K^T row -> row i of P = tril(scale * decay * Q K^T) as 64 bf16 values in registers (eight 16-byte chunks).

@@ -54,10 +54,10 @@ extern "C" {
 #define GDN_PATH_TWOPASS_T 12    /* prepare kernel + transposed chain kernel: one CTA per (batch, value head[, segment])
                                     carries all 128 value columns, state-dependent operands in tensor memory */
 
-#define GDN_PATH_PREPARE_ONLY_T 13 /* stage-level check: prepare with W as well as what TWOPASS_T's chain reads */
+#define GDN_PATH_PREPARE_ONLY_T 13 /* measurement aid: only the prepare kernel as TWOPASS_T runs it          */
 #define GDN_PATH_CHAIN_ONLY_T 14   /* measurement aid: only the transposed chain, on the workspace an earlier TWOPASS_T /
                                       PREPARE_ONLY_* call with the same arguments and scratch left             */
-#define GDN_PATH_PREPARE_ONLY_R 15 /* measurement aid: only the prepare kernel as TWOPASS_T runs it          */
+#define GDN_PATH_PREPARE_ONLY_R 15 /* the same as PREPARE_ONLY_T                                             */
 
 #define GDN_D 128                /* head dimension of keys and values (compile-time in the kernels) */
 #define GDN_CHUNK 64             /* tokens per chunk                                                */
