@@ -16,14 +16,14 @@ from gdn_qsa_sm80_b200.synthetic import make_inputs
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("S", [4096, 1024])      # 4096: prepare + transposed chain; 1024: the cooperative single launch
-def test_two_streams_fifty_rounds(S):
+@pytest.mark.parametrize("S,path", [(4096, "auto"), (1024, "auto"), (1024, "coop")])   # prepare + chain; the cooperative single launch
+def test_two_streams_fifty_rounds(S, path):
     dev = torch.device("cuda", 0)
     probs = []
     for seed in (1, 2):
         q, k, v, g, beta, h0 = make_inputs("default", seed=seed, S=S, Hq=16, Hv=32)
         d = [t.to(dev) for t in (q, k, v, g, beta, h0)]
-        ref = gdn_chunk(*d[:5], initial_state=d[5])
+        ref = gdn_chunk(*d[:5], initial_state=d[5], path=path)
         check_device_status(dev)
         probs.append((d, ref))
     streams = [torch.cuda.Stream(dev), torch.cuda.Stream(dev)]
@@ -32,7 +32,7 @@ def test_two_streams_fifty_rounds(S):
         outs = []
         for (d, _), s in zip(probs, streams):
             with torch.cuda.stream(s):
-                outs.append(gdn_chunk(*d[:5], initial_state=d[5]))
+                outs.append(gdn_chunk(*d[:5], initial_state=d[5], path=path))
         for s in streams:
             s.synchronize()
         for s in streams:
