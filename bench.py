@@ -768,10 +768,9 @@ def main():
 
     # ---- the two kernels of a step timed on their own (CUDA events on the launching stream, L2 flushed) ----
     per_kernel = None
-    n_sm = torch.cuda.get_device_properties(dev).multi_processor_count
-    single_launch = args.path == "coop" or (args.path == "auto" and w.S <= 2048 and 4 * B_local * w.Hv <= n_sm)
-    transposed = args.path == "twopass_t" or (args.path == "auto" and not single_launch)
-    kernels = ("gdn_coop_kernel (one launch)" if single_launch else
+    decode = args.path == "decode" or (args.path == "auto" and w.S <= 8)
+    transposed = args.path == "twopass_t" or (args.path == "auto" and not decode)
+    kernels = ("gdn_coop_kernel (one launch)" if args.path == "coop" else "gdn_decode_kernel" if decode else
                "gdn_prepare_lean_kernel + gdn_chain_r_kernel (few long sequences are split into warmed-up segments on the device)"
                if transposed else
                "gdn_prepare_kernel + gdn_chain_kernel" if args.path in ("twopass_nv32", "twopass_nv64") else args.path)
@@ -839,7 +838,7 @@ def main():
         if traffic:   # the same launch against the HBM roofline, at the DRAM bytes it really moves
             roofline["traffic_hbm"] = {"achieved": traffic / k_s / 1e9, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                                        "frac": traffic / k_s / 1e9 / peaks["hbm_gbs"]}
-    elif single_launch:
+    elif args.path == "coop":
         # one kernel per step: its duration is the step's (CUDA events around the launch)
         traffic = DRAM_TRAFFIC.get((args.workload, "gdn_coop_kernel")) if world == 1 else None
         roofline = {"kernel": "gdn_coop_kernel", "bound": "tensor", "achieved": whole["achieved"], "peak": peaks["bf16_tflops"],
