@@ -333,6 +333,7 @@ int forward_device(const void* q, const void* k, const void* v, const void* g, c
     // the transposed chain splits sequences when the scratch buffer has room for the per-tile scalars its decision
     // reads (a caller that sized it for an unsplit run, like the fixed-array entry point, gets the unsplit run)
     int n_seg = segments_of(B, S, Hv, path);
+    if (h0 && h0 == hT) n_seg = 1;   // in place: the CTA that reads a state must be the one that writes it
     if (n_seg > 1 && scratch_bytes < workspace_layout(tiles_of(B, S, Hv), true).total) n_seg = 1;
     const WorkspaceLayout l = workspace_layout(tiles_of(B, S, Hv), n_seg > 1);
     uint8_t* base = static_cast<uint8_t*>(scratch);

@@ -149,7 +149,8 @@ int gdn_chunk_fwd_varlen_sm100(const void* q, const void* k, const void* v, cons
                 continue;
             }
             order.push_back(i);
-            segs[i] = chain_segments(static_cast<long long>(l.chunks) * Hv, chunks_of(i), 2 * sm_count());   // two CTAs per SM
+            // two CTAs per SM; states in place: the CTA that reads a state must be the one that writes it
+            segs[i] = h0 && h0 == hT ? 1 : chain_segments(static_cast<long long>(l.chunks) * Hv, chunks_of(i), 2 * sm_count());
         }
         // Order of the chain's work list.  First what takes long, segment by segment: the first segments of all sequences that may be
         // cut (and the long ones that may not), their second ones, ...: a head whose decay forbids the cut runs all of it in

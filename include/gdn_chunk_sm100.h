@@ -83,7 +83,8 @@ int gdn_chunk_workspace_offsets(int B, int S, int Hq, int Hv, size_t* offsets);
  * Forward pass of the chunked gated delta rule.
  *
  *   q, k   [B,S,Hq,128] bf16        v   [B,S,Hv,128] bf16        g, beta [B,S,Hv] bf16 or fp32
- *   h0     [B,Hv,128,128] fp32 (Dk rows, Dv columns) or NULL for a zero initial state
+ *   h0     [B,Hv,128,128] fp32 (Dk rows, Dv columns) or NULL for a zero initial state; hT may be the same buffer (in
+ *          place; a long sequence is then not split), but must not overlap it otherwise
  *   out    [B,S,Hv,128] bf16        hT  [B,Hv,128,128] fp32 or NULL when the final state is not wanted
  *
  * g is the log decay (<= 0), beta the update gate; q is scaled by 128^-0.5 inside; v-head h reads

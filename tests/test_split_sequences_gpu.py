@@ -6,11 +6,14 @@ with the CPU oracle at the benchmark's tolerance (rel-L2 <= 1e-2, max-abs <= 2e-
 two-kernel path on the same device.
 """
 
+import ctypes
+
 import numpy as np
 import pytest
 import torch
 
 from gdn_qsa_sm80 import gdn_chunk
+from gdn_qsa_sm80_b200 import _lib
 from gdn_qsa_sm80_b200.gdn_chunk_interface import check_device_status
 from gdn_qsa_sm80_b200.synthetic import make_inputs, make_reference_test_inputs
 
@@ -131,3 +134,29 @@ def test_more_chunks_than_the_plan_has_room_for():
     a, b = (x[0, :n, 0].float().reshape(-1, 64 * 128) for x in (o1, o2))
     assert ((a - b).norm(dim=1) <= 1e-2 * b.norm(dim=1)).all()
     assert ((s1 - s2).norm() <= 6e-3 * s2.norm()).item() and ((o1[0, n:].float() - o2[0, n:].float()).norm() <= 1e-2 * o2[0, n:].float().norm()).item()
+
+
+@pytest.mark.parametrize("S", [4, 1000, 4096])
+@pytest.mark.parametrize("packed", [False, True])
+def test_states_in_place(S, packed):
+    """h0 and hT in one buffer (C entry points): a sequence is not split then, since another segment's CTA would write what the first
+    one reads."""
+    lib, Hq, Hv = _lib.load(), 2, 4
+    q, k, v, g, beta, h0 = make_inputs("default", seed=S, S=S, Hq=Hq, Hv=Hv)
+    d = [t.cuda() for t in (q, k, v, g, beta)]
+    want_o, want_s = gdn_chunk(*d, initial_state=h0.cuda(), path="decode" if S <= 8 else "twopass_nv64")
+    state, out = h0.cuda(), torch.empty_like(want_o)
+    cu = (ctypes.c_int * 2)(0, S)
+    n = max(lib.gdn_chunk_scratch_bytes(1, S, Hq, Hv, 0), lib.gdn_chunk_varlen_scratch_bytes(cu, 1, Hv))
+    scratch = torch.empty(n, dtype=torch.uint8, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    p = [t.data_ptr() for t in d] + [state.data_ptr(), out.data_ptr(), state.data_ptr(), scratch.data_ptr(), n]
+    if packed:
+        st = lib.gdn_chunk_fwd_varlen_sm100(*p, cu, 1, Hq, Hv, _lib.GATE_F32, 0, stream)
+    else:
+        st = lib.gdn_chunk_fwd_sm100(*p, 1, S, Hq, Hv, _lib.GATE_F32, 0, stream)
+    word = ctypes.c_int(0)
+    assert st == 0 and lib.gdn_chunk_read_status(scratch.data_ptr(), stream, ctypes.byref(word)) == 0
+    tol = {"rel": 0.0, "mabs": 0.0} if S <= 8 else {"rel": 6e-3, "mabs": 1e-2}   # (the two chains differ by bf16 operand rounding)
+    assert_close(out.float().cpu().numpy(), want_o.float().cpu().numpy(), "out", **tol)
+    assert_close(state.cpu().numpy(), want_s.cpu().numpy(), "state", **tol)
