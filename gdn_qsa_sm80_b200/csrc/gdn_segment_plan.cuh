@@ -71,17 +71,23 @@ __device__ __forceinline__ int warmups(const unsigned* pre, int NT, int g, int L
 template <int THREADS>
 __device__ __forceinline__ void plan_segments(const float* meta, int chunks, int G, unsigned* pre, SegmentPlan& plan, int* best) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int unit = (chunks + kPlanChunks - 1) / kPlanChunks, NT = (chunks + unit - 1) / unit;   // chunks of a unit; units
-    constexpr unsigned cap = static_cast<unsigned>(kForgetCap * kForgetScale);
-    int bad = 0;
-    for (int t = tid; t < NT; t += THREADS) {
-        unsigned sum = 0;
-        for (int c = t * unit; c < min(chunks, (t + 1) * unit); ++c) {
-            const float2 m = *reinterpret_cast<const float2*>(meta + 2 * c);
-            sum = min(cap, sum + __float2uint_rd(fminf(-m.x, kForgetCap) * kForgetScale));
-            if (!(m.y <= 2.f) || !(m.x <= 0.f)) bad = 1;    // outside the premise (also NaN, and +inf for a gate out of range)
+    int unit = 1, NT = chunks, bad = 0;   // chunks of a unit; units
+    auto chunk = [&](int c) -> unsigned {
+        const float2 m = *reinterpret_cast<const float2*>(meta + 2 * c);
+        if (!(m.y <= 2.f) || !(m.x <= 0.f)) bad = 1;    // outside the premise (also NaN, and +inf for a gate out of range)
+        return __float2uint_rd(fminf(-m.x, kForgetCap) * kForgetScale);
+    };
+    if (chunks <= kPlanChunks) {
+        for (int t = tid; t < NT; t += THREADS) pre[t + 1] = chunk(t);
+    } else {
+        unit = (chunks + kPlanChunks - 1) / kPlanChunks;
+        NT = (chunks + unit - 1) / unit;
+        for (int t = tid; t < NT; t += THREADS) {
+            unsigned sum = 0;
+            for (int c = t * unit; c < min(chunks, (t + 1) * unit); ++c)
+                sum = min(static_cast<unsigned>(kForgetCap * kForgetScale), sum + chunk(c));
+            pre[t + 1] = sum;
         }
-        pre[t + 1] = sum;
     }
     if (tid == 0) {
         pre[0] = 0;
