@@ -317,8 +317,9 @@ int forward_device(const void* q, const void* k, const void* v, const void* g, c
                                                                                                           : GDN_ERR_CUDA;
     };
 
-    // a few new tokens: the state read and write is all there is, and the decode kernel streams it (measured on
-    // 2048 states: 55 us at one token = 4.8 TB/s, against 238 us through the chunk kernels; the two meet near 16 tokens)
+    // A few new tokens: the state read and write is all there is, and the decode kernel streams it, in exact fp32 (2048
+    // states: 47.8 us at one token = 5.6 TB/s, 74.7 at four, 121.5 at eight; the chunk kernels 93-94 whatever the number.  Fewer states
+    // favour it longer: the line lies where an eight-token chunk would be one eighth full).
     if (decode) return launch_decode(p, gate, stream);
     if (path == GDN_PATH_SIMT && !clear()) return GDN_ERR_CUDA;
     if (path == GDN_PATH_SIMT) return then_gate(launch_simt(p, stream) == cudaSuccess ? GDN_OK : GDN_ERR_CUDA);
@@ -331,7 +332,7 @@ int forward_device(const void* q, const void* k, const void* v, const void* g, c
     if (path == GDN_PATH_TWOPASS_NV32) nv = 32;
     else nv = 64;
     // the transposed chain splits sequences when the scratch buffer has room for the per-tile scalars its decision
-    // reads (a caller that sized it for an unsplit run, like the fixed-array entry point, gets the unsplit run)
+    // reads (a caller that sized it for an unsplit run gets the unsplit run)
     int n_seg = segments_of(B, S, Hv, path);
     if (h0 && h0 == hT) n_seg = 1;   // in place: the CTA that reads a state must be the one that writes it
     if (n_seg > 1 && scratch_bytes < workspace_layout(tiles_of(B, S, Hv), true).total) n_seg = 1;

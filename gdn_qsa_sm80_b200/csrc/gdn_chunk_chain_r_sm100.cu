@@ -12,7 +12,7 @@
 //        S^T   <- e^gamma_C S^T + ACC_S                                                                    (ref :94)
 //   E3   O     += v_new^T P^T                                                                           (ref :92-93)
 // Against the form with W (this library's chain before) a chunk has one hand-off more on its critical path, but reads 16 KB
-// less and needs 256 tensor-memory columns, 100 KB of shared memory and 32 K registers, so TWO CTAs share an SM and
+// less and needs 256 tensor-memory columns, 110 KB of shared memory and 32 K registers, so TWO CTAs share an SM and
 // each fills the other's waits: what counts here is the time of a chunk step per SM, not its latency.
 //
 // Tensor memory of a CTA (columns; each operand is written over an accumulator that is dead by then - UMMAs of one thread

@@ -9,7 +9,8 @@
 // leaves by TMA store, which the load-compute-store phases of one CTA per state could not do (75 % of the copy bandwidth).
 // The tile is 128-byte swizzled and lane l owns rows = l mod 8 and the four columns of chunk l / 8, so a 16-byte access
 // of eight lanes covers all banks, and the column sums a token needs (S^T k, S^T q) are three shuffles: no barrier.
-//   GROUPS = 1: a CTA of two compute warps and a producer warp, four per SM; 32 states give 128 CTAs.
+//   GROUPS = 1: a CTA of two compute warps and a producer warp, four per SM (three from four tokens on, whose vectors take
+//   room in every stage); 32 states give 128 CTAs.
 //   PACKED: the sequences of a packed batch that have at most kDecodeMaxTokens tokens, of any lengths, found through a table.
 //   GROUPS = 4: the four tiles of a state in one CTA, for the gated normalisation of the output rows (their sum of squares
 //   needs all 128 columns: one barrier a token), which then costs no launch and no pass over the rows of its own.

@@ -328,18 +328,19 @@ def gdn_chunk_varlen(q, k, v, g, beta, cu_seqlens, output_final_state=True, init
 
     q, k: [1, T, Hk, D] (or [T, Hk, D]); v: [1, T, Hv, D]; g, beta: [1, T, Hv]; cu_seqlens: the n_seq + 1 cumulative
     sequence boundaries 0 = c_0 < c_1 < ... < c_n = T as a list or CPU tensor (a CUDA tensor is read back, which
-    synchronises).  Sequence i is tokens [c_i, c_{i+1}); its slice of every packed tensor is contiguous, so each
-    sequence runs as an ordinary forward pass on a view - no padding, no copies - with the launches spread round-robin
-    over `n_streams` streams that are ordered after, and joined back into, the current stream.  Neighbouring
-    sequences of equal length form a regular batch and share one launch (a packed batch of single tokens is one
-    launch of the decode kernel).
-    strategy: "views" as described; "packed" runs all sequences in one pass of the kernels, which find each chunk's
-    sequence through small tables (no padding, no copies, C ABI: gdn_chunk_fwd_varlen_sm100; sequences of at most 8
-    tokens take the decode kernel); "padded" gathers all sequences into one regular batch [n_seq, L_max, ...] whose
-    padding tokens carry g = 0 and beta = 0 (they leave the state untouched and their outputs are dropped, so the
-    result is exact), runs one forward pass and scatters the outputs back - two extra passes over the data; "auto" is
-    "packed", or with a forced path "padded" when
-    there are more than 8 launches to make and padding at most doubles the token count, else "views".  The reference has no
+    synchronises).  Sequence i is tokens [c_i, c_{i+1}).
+    strategy:
+      "packed"  all sequences in one pass of the kernels, which find each chunk's sequence through small tables (no
+                padding, no copies; C ABI: gdn_chunk_fwd_varlen_sm100); sequences of at most 8 tokens share a launch of the
+                decode kernel.  What "auto" does.
+      "views"   every sequence as an ordinary forward pass on its slice, neighbours of equal length as one regular batch, the
+                launches spread round-robin over `n_streams` streams that are ordered after, and joined back into, the
+                current one.
+      "padded"  all sequences gathered into one regular batch [n_seq, L_max, ...] whose padding tokens carry g = 0 and
+                beta = 0 (they leave the state untouched and their outputs are dropped, so the result is exact), one forward
+                pass, the outputs scattered back: two extra passes over the data.
+    With a forced path, or contiguous tensors at an address that is no multiple of 16 bytes, "auto" is "padded" when there
+    are more than 8 launches to make and padding at most doubles the token count, else "views".  The reference has no
     variable-length entry; its recurrent torch definition (reference/gdn_chunk_ref.py:103-147) applied per sequence
     defines the result.  initial_state / returned final state: [n_seq, Hv, D, D]; `options` are gdn_chunk's keywords
     (path, use_qk_l2norm_in_kernel, gate_activations).
