@@ -67,8 +67,8 @@ def test_a_threads_first_cuda_call(S):
 @pytest.mark.gpu
 def test_other_threads_run_during_launches():
     """The forward call lets go of the interpreter while it launches.  With a switch interval of a minute another thread only
-    runs when it does: enough calls to fill the launch queue give it hundreds of turns, or none."""
-    x = _inputs(1, 1, 16, 32, 0)
+    runs when it does: enough calls of 50 us to fill the launch queue give it thousands of turns, or a few."""
+    x = _inputs(64, 1, 16, 32, 0)
     gdn_chunk(*x)                          # scratch buffer and kernels in place
     torch.cuda.synchronize()
     turns, stop, started = [0], threading.Event(), threading.Event()
@@ -86,7 +86,7 @@ def test_other_threads_run_during_launches():
     sys.setswitchinterval(60.0)
     try:
         before = turns[0]
-        for _ in range(5000):
+        for _ in range(3000):
             gdn_chunk(*x)
         during = turns[0] - before
     finally:
@@ -94,7 +94,7 @@ def test_other_threads_run_during_launches():
         stop.set()
         t.join()
     torch.cuda.synchronize()
-    assert during > 100     # (7 with the lock held: what the call does before it launches)
+    assert during > 100, during
 
 
 @pytest.mark.gpu
