@@ -7,7 +7,9 @@
 // (exp(-115) < 2^-149) the incoming state no longer shows in fp32: the state after the stretch is the same from a zero
 // state.  So a segment s >= 1 starts from a ZERO state p chunks before its first chunk, p the shortest stretch ending at
 // the boundary whose sum of g is below -115 ("warm-up": its outputs are not stored), and from its first chunk on its state,
-// its outputs and its final state are those of the serial run.
+// its outputs and its final state are those of the serial run - bit for bit where the decay is strong (a sum of -10 a chunk);
+// where the warm-up is a hundred chunks long the two states end a last bit apart and their bf16 copies round differently now and
+// then (up to 5e-3 of a chunk's outputs, 120000 random calls, as far as either is from the exact result).
 //
 // The sums are prefix sums, and a difference of two prefixes has to be the sum of what lies between them whatever lies in front: in
 // fp32 a gate of -1e9 (a reset, a mask's fill value) leaves prefixes with a spacing of 64 and more, and a rounding step behind it read
