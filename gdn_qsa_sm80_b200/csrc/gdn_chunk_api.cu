@@ -318,7 +318,7 @@ int forward_device(const void* q, const void* k, const void* v, const void* g, c
     };
 
     // A few new tokens: the state read and write is all there is, and the decode kernel streams it, in exact fp32 (2048
-    // states: 47.8 us at one token = 5.6 TB/s, 74.7 at four, 121.5 at eight; the chunk kernels 93-94 whatever the number.  Fewer states
+    // states: 47.8 us at one token = 5.6 TB/s, 65 at four, 112 at eight; the chunk kernels 93-94 whatever the number.  Fewer states
     // favour it longer: the line lies where an eight-token chunk would be one eighth full).
     if (decode) return launch_decode(p, gate, stream);
     if (path == GDN_PATH_SIMT && !clear()) return GDN_ERR_CUDA;

@@ -7,13 +7,18 @@
 // [128 rows][32 columns] (16 KB): two warps own one, 64 values per thread, and a persistent CTA streams tiles through a
 // ring of three TMA stages - the loads of the next tiles are in flight while this one is computed and the one before
 // leaves by TMA store, which the load-compute-store phases of one CTA per state could not do (75 % of the copy bandwidth).
-// The tile is 128-byte swizzled and lane l owns rows = l mod 8 and the four columns of chunk l / 8, so a 16-byte access
-// of eight lanes covers all banks, and the column sums a token needs (S^T k, S^T q) are three shuffles: no barrier.
+// The tile is 128-byte swizzled; a lane owns eight pairs of rows and the four columns of a chunk, so that a 16-byte access of eight
+// lanes covers all banks, a pair's two values of k arrive in one word, and the column sums a token needs (S^T k, S^T q) are three
+// shuffles: no barrier.  With several tokens a tile what bounds it is the two warps' instructions, not HBM: two multiply-adds in one
+// (f32x2), and their vectors fetched as one box a tensor instead of a copy a row.  32 heads, before and after: 8 sequences of 4 tokens
+// 14.5 -> 12.7 us, 256 of 4 277 -> 241, 64 of 8 121 -> 111; one token each as before (64 sequences 47 us, 86 % of the copy bandwidth).
 //   GROUPS = 1: a CTA of two compute warps and a producer warp, four per SM (three from four tokens on, whose vectors take
 //   room in every stage); 32 states give 128 CTAs.
 //   PACKED: the sequences of a packed batch that have at most kDecodeMaxTokens tokens, of any lengths, found through a table.
 //   GROUPS = 4: the four tiles of a state in one CTA, for the gated normalisation of the output rows (their sum of squares
-//   needs all 128 columns: one barrier a token), which then costs no launch and no pass over the rows of its own.
+//   needs all 128 columns: one barrier a token), which then costs no launch and no pass over the rows of its own.  One token: a ring of
+//   three, one CTA per SM (HBM-bound).  Several: its barriers and instructions bound it, and two CTAs per SM with one stage each fill
+//   each other's waits (8 sequences of 4 tokens 19.1 -> 15.7 us, 64 of 4 111 -> 94, 8 of 8 38.8 -> 26.9).
 #include <cuda.h>
 
 #include "../../include/gdn_chunk_sm100.h"
@@ -24,7 +29,7 @@
 namespace gdn {
 namespace {
 
-constexpr int kDecStages = 3, kDecTokens = 8;      // tokens whose vectors travel through the ring (later ones: global loads)
+constexpr int kDecTokens = 8;                      // tokens whose vectors travel through the ring (later ones: global loads)
 constexpr int kDecTimeoutFull = 0x601, kDecTimeoutEmpty = 0x602;
 
 struct DecodeGate {                                // gated normalisation of the output rows (z null: none)
@@ -38,7 +43,6 @@ __device__ __forceinline__ float dec_gate(const void* p, size_t idx) {
     if (GATE_F32) return static_cast<const float*>(p)[idx];
     return __bfloat162float(static_cast<const __nv_bfloat16*>(p)[idx]);
 }
-__device__ __forceinline__ float bf16_bits(unsigned short x) { return __uint_as_float(static_cast<uint32_t>(x) << 16); }
 __device__ __forceinline__ float sum_rows(float x) {   // over the eight lanes that share a column
     x += __shfl_xor_sync(0xffffffffu, x, 1);
     x += __shfl_xor_sync(0xffffffffu, x, 2);
@@ -47,29 +51,40 @@ __device__ __forceinline__ float sum_rows(float x) {   // over the eight lanes t
 }
 
 // bytes of the token area of one stage: k, q rows, 32 columns of v, g and beta
-__host__ __device__ constexpr uint32_t dec_token_bytes(int nt) { return nt * (256 + 256 + 64) + 2 * kDecTokens * 4; }
+__host__ __device__ constexpr uint32_t dec_token_bytes(int nt) { return (nt * (256 + 256 + 64) + 2 * kDecTokens * 4 + 127) & ~127u; }
 
-template <int GROUPS, bool GATE_F32, bool PACKED>
-__global__ void __launch_bounds__(GROUPS * 64 + 32, GROUPS == 1 ? 4 : 1)
+// Where the vectors of several tokens come from: a box of nt rows each, three copies a tile instead of three a token (256 sequences of 4
+// tokens 250 -> 241 us).  A single token's need no map, whose encoding would cost the smallest calls host time.
+template <bool SEVERAL>
+struct TokenMaps {
+    CUtensorMap q, k, v;
+};
+template <>
+struct TokenMaps<false> {};
+
+__host__ __device__ constexpr int dec_ctas_per_sm(int groups, int stages) { return groups == 1 ? 4 : (stages == 3 ? 1 : 2); }
+
+template <int GROUPS, bool GATE_F32, bool PACKED, int STAGES, bool SEVERAL>
+__global__ void __launch_bounds__(GROUPS * 64 + 32, dec_ctas_per_sm(GROUPS, STAGES))
 gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_out,
-                  const __grid_constant__ Problem p, const __grid_constant__ DecodeGate gate, int items, int nt) {
+                  const __grid_constant__ TokenMaps<SEVERAL> maps, const __grid_constant__ Problem p, const __grid_constant__ DecodeGate gate, int items, int nt) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    __shared__ __align__(8) uint64_t full[GROUPS][kDecStages], empty[GROUPS][kDecStages];
+    __shared__ __align__(8) uint64_t full[GROUPS][STAGES], empty[GROUPS][STAGES];
     __shared__ float ssq[2][GROUPS * 2];
-    __shared__ int4 seq_of[PACKED ? kDecStages : 1];   // (sequence, first token, tokens) of the stage's tile
+    __shared__ int4 seq_of[PACKED ? STAGES : 1];   // (sequence, first token, tokens) of the stage's tile
     __shared__ int failed;
 
     const int tid = threadIdx.x, warp = static_cast<int>(warp_uniform(tid >> 5)), lane = tid & 31;
     const uint32_t tok_bytes = dec_token_bytes(nt);
-    // stage s of group g: the tile at (g * kDecStages + s) * 16 KB; the token areas behind all tiles
-    auto tile_of = [&](int g, int s) { return sm + (g * kDecStages + s) * 16384; };
-    auto tok_of = [&](int g, int s) { return sm + GROUPS * kDecStages * 16384 + (g * kDecStages + s) * tok_bytes; };
+    // stage s of group g: the tile at (g * STAGES + s) * 16 KB; the token areas behind all tiles
+    auto tile_of = [&](int g, int s) { return sm + (g * STAGES + s) * 16384; };
+    auto tok_of = [&](int g, int s) { return sm + GROUPS * STAGES * 16384 + (g * STAGES + s) * tok_bytes; };
     const int rep = p.Hv / p.Hq;
 
     if (tid == 0) {
         for (int g = 0; g < GROUPS; ++g)
-            for (int s = 0; s < kDecStages; ++s) {
+            for (int s = 0; s < STAGES; ++s) {
                 mbar_init(&full[g][s], 2);       // the copies (bytes) and the gates (written by the producer warp)
                 mbar_init(&empty[g][s], 1);
             }
@@ -87,7 +102,7 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
         // ------------------------------- producer ---------------------------------------------------------------------
         int n = 0;
         for (int it = first; it < items; it += step, ++n) {
-            const int s = n % kDecStages;
+            const int s = n % STAGES;
             int state = GROUPS == 1 ? it >> 2 : it, tokens = nt;
             const int b = state / p.Hv, h = state - b * p.Hv, hq = h / rep;
             size_t tok0 = static_cast<size_t>(b) * p.S;
@@ -100,17 +115,22 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
             }
             bool ok = true;
             for (int g = 0; g < GROUPS && ok; ++g) {
-                if (n >= kDecStages) ok = mbar_wait(&empty[g][s], ((n / kDecStages) - 1) & 1, p.status, kDecTimeoutEmpty);
+                if (n >= STAGES) ok = mbar_wait(&empty[g][s], ((n / STAGES) - 1) & 1, p.status, kDecTimeoutEmpty);
                 const int quarter = GROUPS == 1 ? it & 3 : g;
                 if (ok && elect_one()) {
                     uint8_t* tk = tok_of(g, s);
-                    mbar_arrive_expect_tx(&full[g][s], (p.h0 ? 16384 : 0) + tokens * (256 + 256 + 64));
+                    mbar_arrive_expect_tx(&full[g][s], (p.h0 ? 16384 : 0) + nt * (256 + 256 + 64));
                     if (p.h0) tma_load_2d(tile_of(g, s), &tm_in, &full[g][s], quarter * 32, state * kD);
-                    for (int t = 0; t < tokens; ++t) {
-                        const size_t row = (tok0 + t) * p.Hq + hq;
-                        bulk_load_1d(tk + t * 256, p.k + row * kD, 256, &full[g][s]);
-                        bulk_load_1d(tk + (nt + t) * 256, p.q + row * kD, 256, &full[g][s]);
-                        bulk_load_1d(tk + nt * 512 + t * 64, p.v + ((tok0 + t) * p.Hv + h) * kD + quarter * 32, 64, &full[g][s]);
+                    if constexpr (SEVERAL) {   // (rows past the sequence's own are read by nobody)
+                        const int row = PACKED ? seq.y : 0, batch = PACKED ? 0 : b;
+                        tma_load_4d(tk, &maps.k, &full[g][s], 0, hq, row, batch);
+                        tma_load_4d(tk + nt * 256, &maps.q, &full[g][s], 0, hq, row, batch);
+                        tma_load_4d(tk + nt * 512, &maps.v, &full[g][s], quarter * 32, h, row, batch);
+                    } else {
+                        const size_t row = tok0 * p.Hq + hq;
+                        bulk_load_1d(tk, p.k + row * kD, 256, &full[g][s]);
+                        bulk_load_1d(tk + 256, p.q + row * kD, 256, &full[g][s]);
+                        bulk_load_1d(tk + 512, p.v + (tok0 * p.Hv + h) * kD + quarter * 32, 64, &full[g][s]);
                     }
                 }
                 __syncwarp();
@@ -132,22 +152,26 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
     } else {
         // ------------------------------- compute: two warps per tile ------------------------------------------------------
         const int g = warp >> 1, half = warp & 1;             // half: which 16 of the tile's 32 columns
-        const int rg = lane & 7, ch = half * 4 + (lane >> 3); // rows rg, rg + 8, ...; 16-byte chunk of a 128-byte row
-        const uint32_t off0 = rg * 128 + ((ch ^ rg) << 4);    // the same chunk in every row = rg mod 8
+        // Lane l owns the row pairs 16 m + 2 rg, + 1 (one word of k and one of q each) of 16-byte chunk ch of the 128-byte rows.  In the
+        // swizzled tile rows eight apart share their banks, so lanes 4-7 of a column group take a pair's rows in the other order.
+        const int rg = lane & 7, ch = half * 4 + (lane >> 3), odd = rg >> 2;
+        const int row0 = 2 * rg + odd, row1 = 2 * rg + 1 - odd;
+        const uint32_t off0 = row0 * 128 + ((ch ^ (row0 & 7)) << 4), off1 = row1 * 128 + ((ch ^ (row1 & 7)) << 4);
+        const uint32_t first_half = odd ? 0x3244u : 0x1044u, second_half = odd ? 0x1044u : 0x3244u;   // byte selectors: a pair's rows as fp32
         const float scale = rsqrtf(static_cast<float>(kD));
         // Slot of ssq: changes with every row of the CTA, across work items too.  Between a warp's reads of a slot and its next
         // write to it lies the other slot's barrier, which every warp reaches only after those reads.
         int slot = 0;
         int n = 0;
         for (int it = first; it < items; it += step, ++n) {
-            const int s = n % kDecStages;
+            const int s = n % STAGES;
             int state = GROUPS == 1 ? it >> 2 : it, tokens = p.S;
             const int quarter = GROUPS == 1 ? it & 3 : g;
             const int b = state / p.Hv, h = state - b * p.Hv, hq = h / rep;
             size_t tok0 = static_cast<size_t>(b) * p.S;
             // after a wait that ran out nobody waits again, but every warp keeps to the loop: its barriers count all of them
             const bool ok = !*const_cast<volatile int*>(&failed) &&
-                            mbar_wait(&full[g][s], (n / kDecStages) & 1, p.status, kDecTimeoutFull);
+                            mbar_wait(&full[g][s], (n / STAGES) & 1, p.status, kDecTimeoutFull);
             if (!ok) *const_cast<volatile int*>(&failed) = 1;
             if (PACKED) {
                 const int4 seq = seq_of[s];
@@ -155,28 +179,31 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
                 tok0 = seq.y;
                 tokens = ok ? seq.z : 0;          // (nothing may have been written there)
             }
-            uint8_t* tile = tile_of(g, s) + off0;
+            uint8_t* tile = tile_of(g, s);
             const uint8_t* tk = tok_of(g, s);
-            float4 st[16];
+            float2 st[16][2];
 #pragma unroll
-            for (int i = 0; i < 16; ++i)
-                st[i] = p.h0 ? *reinterpret_cast<const float4*>(tile + i * 1024) : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int i = 0; i < 16; ++i) {
+                const float4 x = p.h0 ? *reinterpret_cast<const float4*>(tile + (i >> 1) * 2048 + (i & 1 ? off1 : off0)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                st[i][0] = make_float2(x.x, x.y);
+                st[i][1] = make_float2(x.z, x.w);
+            }
             const float* gates = reinterpret_cast<const float*>(tk + nt * (256 + 256 + 64));
             for (int t = 0; t < tokens; ++t) {
                 const size_t tok = tok0 + t;
-                // this lane's rows of k and q (fp32), its four values, the gates
-                const unsigned short *kr, *qr;
+                // this lane's rows of k and q, its four values, the gates
+                const uint32_t *kr, *qr;
                 uint2 vraw;
                 float gt, bt;
                 if (t < nt) {
-                    kr = reinterpret_cast<const unsigned short*>(tk + t * 256);
-                    qr = reinterpret_cast<const unsigned short*>(tk + (nt + t) * 256);
+                    kr = reinterpret_cast<const uint32_t*>(tk + t * 256);
+                    qr = reinterpret_cast<const uint32_t*>(tk + (nt + t) * 256);
                     vraw = *reinterpret_cast<const uint2*>(tk + nt * 512 + t * 64 + ch * 8);
                     gt = gates[t];
                     bt = gates[kDecTokens + t];
                 } else {
-                    kr = reinterpret_cast<const unsigned short*>(p.k + (tok * p.Hq + hq) * kD);
-                    qr = reinterpret_cast<const unsigned short*>(p.q + (tok * p.Hq + hq) * kD);
+                    kr = reinterpret_cast<const uint32_t*>(p.k + (tok * p.Hq + hq) * kD);
+                    qr = reinterpret_cast<const uint32_t*>(p.q + (tok * p.Hq + hq) * kD);
                     vraw = *reinterpret_cast<const uint2*>(p.v + (tok * p.Hv + h) * kD + quarter * 32 + ch * 4);
                     gt = dec_gate<GATE_F32>(p.g, tok * p.Hv + h);
                     bt = dec_gate<GATE_F32>(p.beta, tok * p.Hv + h);
@@ -186,49 +213,56 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
                     bt = 1.f / (1.f + __expf(-bt));
                 }
                 const float dec = __expf(gt);
-                float kf[16], qf[16];
+                uint32_t kw[8], qw[8];
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    kf[i] = bf16_bits(kr[rg + 8 * i]);
-                    qf[i] = bf16_bits(qr[rg + 8 * i]) * scale;
+                for (int m = 0; m < 8; ++m) {
+                    kw[m] = kr[rg + 8 * m];
+                    qw[m] = qr[rg + 8 * m];
                 }
+                auto both = [&](const uint32_t (&w)[8], int i) {   // row i of the lane's sixteen, twice
+                    const float x = __uint_as_float(__byte_perm(w[i >> 1], 0, i & 1 ? second_half : first_half));
+                    return make_float2(x, x);
+                };
                 float rk = 1.f, rq = 1.f;
                 if (p.l2norm) {
                     float kk = 0.f, qq = 0.f;
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
-                        kk = fmaf(kf[i], kf[i], kk);
-                        qq = fmaf(qf[i], qf[i], qq);
+                        const float x = both(kw, i).x, y = both(qw, i).x;
+                        kk = fmaf(x, x, kk);
+                        qq = fmaf(y, y, qq);
                     }
                     rk = rsqrtf(sum_rows(kk) + 1e-6f);
-                    rq = rsqrtf(sum_rows(qq) / (scale * scale) + 1e-6f);   // qf holds q * scale
+                    rq = rsqrtf(sum_rows(qq) + 1e-6f);
                 }
-                float4 kv = make_float4(0.f, 0.f, 0.f, 0.f);              // S^T k
+                float2 kv[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};   // S^T k
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                    kv.x = fmaf(st[i].x, kf[i], kv.x); kv.y = fmaf(st[i].y, kf[i], kv.y);
-                    kv.z = fmaf(st[i].z, kf[i], kv.z); kv.w = fmaf(st[i].w, kf[i], kv.w);
+                    const float2 x = both(kw, i);
+                    kv[0] = fma2(st[i][0], x, kv[0]);
+                    kv[1] = fma2(st[i][1], x, kv[1]);
                 }
-                kv.x = sum_rows(kv.x); kv.y = sum_rows(kv.y); kv.z = sum_rows(kv.z); kv.w = sum_rows(kv.w);
                 const float f = dec * rk, bk = bt * rk;
-                float4 dl;   // delta = beta (v - (decayed S)^T k), with the key's norm folded in
-                dl.x = (__uint_as_float(vraw.x << 16) - kv.x * f) * bk;
-                dl.y = (__uint_as_float(vraw.x & 0xffff0000u) - kv.y * f) * bk;
-                dl.z = (__uint_as_float(vraw.y << 16) - kv.z * f) * bk;
-                dl.w = (__uint_as_float(vraw.y & 0xffff0000u) - kv.w * f) * bk;
-                float4 oa = make_float4(0.f, 0.f, 0.f, 0.f);
+                float2 dl[2];   // delta = beta (v - (decayed S)^T k), with the key's norm folded in
+                dl[0].x = (__uint_as_float(vraw.x << 16) - sum_rows(kv[0].x) * f) * bk;
+                dl[0].y = (__uint_as_float(vraw.x & 0xffff0000u) - sum_rows(kv[0].y) * f) * bk;
+                dl[1].x = (__uint_as_float(vraw.y << 16) - sum_rows(kv[1].x) * f) * bk;
+                dl[1].y = (__uint_as_float(vraw.y & 0xffff0000u) - sum_rows(kv[1].y) * f) * bk;
+                const float2 dec2 = make_float2(dec, dec);
+                float2 oa[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                    st[i].x = fmaf(kf[i], dl.x, dec * st[i].x); st[i].y = fmaf(kf[i], dl.y, dec * st[i].y);
-                    st[i].z = fmaf(kf[i], dl.z, dec * st[i].z); st[i].w = fmaf(kf[i], dl.w, dec * st[i].w);
-                    oa.x = fmaf(st[i].x, qf[i], oa.x); oa.y = fmaf(st[i].y, qf[i], oa.y);
-                    oa.z = fmaf(st[i].z, qf[i], oa.z); oa.w = fmaf(st[i].w, qf[i], oa.w);
+                    const float2 x = both(kw, i), y = both(qw, i);
+                    st[i][0] = fma2(x, dl[0], mul2(dec2, st[i][0]));
+                    st[i][1] = fma2(x, dl[1], mul2(dec2, st[i][1]));
+                    oa[0] = fma2(st[i][0], y, oa[0]);
+                    oa[1] = fma2(st[i][1], y, oa[1]);
                 }
-                oa.x = sum_rows(oa.x) * rq; oa.y = sum_rows(oa.y) * rq; oa.z = sum_rows(oa.z) * rq; oa.w = sum_rows(oa.w) * rq;
-                const size_t o_at = (tok * p.Hv + h) * kD + quarter * 32 + ch * 4;
+                rq *= scale;
                 uint2 pk;
-                pk.x = pack_bf16x2(oa.x, oa.y);
-                pk.y = pack_bf16x2(oa.z, oa.w);
+                pk.x = pack_bf16x2(sum_rows(oa[0].x) * rq, sum_rows(oa[0].y) * rq);
+                pk.y = pack_bf16x2(sum_rows(oa[1].x) * rq, sum_rows(oa[1].y) * rq);
+                const size_t o_at = (tok * p.Hv + h) * kD + quarter * 32 + ch * 4;
                 if (GROUPS == 4 && gate.z) {
                     // the row as bf16, normalised and gated (the arithmetic of gdn_output_gate_sm100.cu on the rounded row)
                     const float a[4] = {__uint_as_float(pk.x << 16), __uint_as_float(pk.x & 0xffff0000u),
@@ -261,16 +295,22 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
             // the tile goes back into its stage and leaves by TMA; the stage before it is free once its store has been read
             if (p.hT) {
 #pragma unroll
-                for (int i = 0; i < 16; ++i) *reinterpret_cast<float4*>(tile + i * 1024) = st[i];
+                for (int i = 0; i < 16; ++i)
+                    *reinterpret_cast<float4*>(tile + (i >> 1) * 2048 + (i & 1 ? off1 : off0)) = make_float4(st[i][0].x, st[i][0].y, st[i][1].x, st[i][1].y);
                 fence_proxy_async_smem();
             }
             named_bar_sync(2 + g, 64);
             if (half == 0 && elect_one()) {
-                if (p.hT) {
+                if (p.hT && STAGES == 3) {
                     tma_store_wait_read();                // tile n - 1's store has read its stage
-                    if (n > 0) mbar_arrive(&empty[g][(n - 1) % kDecStages]);
+                    if (n > 0) mbar_arrive(&empty[g][(n - 1) % STAGES]);
                     if (ok) tma_store_2d(&tm_out, tile_of(g, s), quarter * 32, state * kD);
                     tma_store_commit();
+                } else if (p.hT) {                        // too few stages to wait a tile: the CTAs beside this one fill the time
+                    if (ok) tma_store_2d(&tm_out, tile_of(g, s), quarter * 32, state * kD);
+                    tma_store_commit();
+                    tma_store_wait_read();
+                    mbar_arrive(&empty[g][s]);
                 } else {
                     mbar_arrive(&empty[g][s]);
                 }
@@ -300,24 +340,37 @@ int launch_decode(const Problem& p, const OutputGate* og, cudaStream_t stream) {
     }
     DecodeGate gate{};
     if (og) gate = DecodeGate{static_cast<const __nv_bfloat16*>(og->z), static_cast<const __nv_bfloat16*>(og->weight), og->eps};
-    auto go = [&](auto kernel, int groups, long long items) -> int {
-        const int most = groups == 4 ? 4 : kDecTokens;            // tokens whose vectors fit the ring of four groups
-        const int nt = p.S < most ? p.S : most;
-        const uint32_t smem = groups * kDecStages * (16384 + dec_token_bytes(nt)) + 1024;
+    const bool gated = og && !p.pk_short;
+    const int groups = gated ? 4 : 1, stages = gated && p.S > 1 ? 1 : 3, most = gated ? 4 : kDecTokens;   // (most: tokens whose vectors fit the ring)
+    const int nt = p.S < most ? p.S : most;
+    const long long items = p.pk_short ? 4ll * p.pk_shorts * p.Hv : gated ? states : states * 4;
+    auto go = [&](auto kernel, const auto& maps) -> int {
+        const uint32_t smem = groups * stages * (16384 + dec_token_bytes(nt)) + 1024;
         if (allow_smem(reinterpret_cast<const void*>(kernel), smem)) return GDN_ERR_CUDA;
-        const int fit = static_cast<int>(228 * 1024 / (smem + 1536)), per_sm = fit > 4 ? 4 : fit;
+        const int fit = static_cast<int>(228 * 1024 / (smem + 1536)), most_ctas = dec_ctas_per_sm(groups, stages), per_sm = fit > most_ctas ? most_ctas : fit;
         const long long cap = static_cast<long long>(sm_count()) * per_sm;
         const unsigned grid = static_cast<unsigned>(items < cap ? items : cap);
-        const cudaError_t e = launch_dependent(kernel, dim3(grid), dim3(groups * 64 + 32), smem, stream, false, tin, tout, p,
+        const cudaError_t e = launch_dependent(kernel, dim3(grid), dim3(groups * 64 + 32), smem, stream, false, tin, tout, maps, p,
                                                gate, static_cast<int>(items), nt);
         return e == cudaSuccess ? GDN_OK : GDN_ERR_CUDA;
     };
-    if (p.pk_short) {
-        const long long tiles = 4ll * p.pk_shorts * p.Hv;
-        return p.gate_f32 ? go(gdn_decode_kernel<1, true, true>, 1, tiles) : go(gdn_decode_kernel<1, false, true>, 1, tiles);
+    if (p.S == 1 && !p.pk_short) {
+        const TokenMaps<false> none;
+        if (gated) return p.gate_f32 ? go(gdn_decode_kernel<4, true, false, 3, false>, none) : go(gdn_decode_kernel<4, false, false, 3, false>, none);
+        return p.gate_f32 ? go(gdn_decode_kernel<1, true, false, 3, false>, none) : go(gdn_decode_kernel<1, false, false, 3, false>, none);
     }
-    if (og) return p.gate_f32 ? go(gdn_decode_kernel<4, true, false>, 4, states) : go(gdn_decode_kernel<4, false, false>, 4, states);
-    return p.gate_f32 ? go(gdn_decode_kernel<1, true, false>, 1, states * 4) : go(gdn_decode_kernel<1, false, false>, 1, states * 4);
+    alignas(64) TokenMaps<true> maps;
+    {
+        const unsigned long long tokens = p.pk_short ? p.pk_tokens : p.S, batch = p.pk_short ? 1 : p.B, Hq = p.Hq, Hv = p.Hv;
+        const unsigned long long dq[4] = {kD, Hq, tokens, batch}, sq[3] = {kD * 2, Hq * kD * 2, tokens * Hq * kD * 2};
+        const unsigned long long dv[4] = {kD, Hv, tokens, batch}, sv[3] = {kD * 2, Hv * kD * 2, tokens * Hv * kD * 2};
+        const unsigned row[4] = {kD, 1, static_cast<unsigned>(nt), 1}, quarter[4] = {32, 1, static_cast<unsigned>(nt), 1};
+        if (encode_tma(&maps.q, p.q, 2, 4, dq, sq, row, 0) || encode_tma(&maps.k, p.k, 2, 4, dq, sq, row, 0) || encode_tma(&maps.v, p.v, 2, 4, dv, sv, quarter, 0))
+            return GDN_ERR_DRIVER;
+    }
+    if (p.pk_short) return p.gate_f32 ? go(gdn_decode_kernel<1, true, true, 3, true>, maps) : go(gdn_decode_kernel<1, false, true, 3, true>, maps);
+    if (gated) return p.gate_f32 ? go(gdn_decode_kernel<4, true, false, 1, true>, maps) : go(gdn_decode_kernel<4, false, false, 1, true>, maps);
+    return p.gate_f32 ? go(gdn_decode_kernel<1, true, false, 3, true>, maps) : go(gdn_decode_kernel<1, false, false, 3, true>, maps);
 }
 
 }  // namespace gdn

@@ -115,3 +115,18 @@ def test_more_rows_than_a_state_map_could_address():
     for part in (slice(0, tail), slice(B - tail, B)):
         ref, _ = gdn_chunk(*[x[part].contiguous() for x in (q, k, v, g, beta)], output_final_state=False)
         assert torch.equal(out[part], ref)
+
+
+@pytest.mark.parametrize("S", [2, 7, 8, 9])
+@pytest.mark.parametrize("Hq,Hv", [(1, 2), (3, 3)])
+def test_several_tokens_over_a_ring_that_wraps(S, Hq, Hv):
+    """Vectors of several tokens come as boxes of up to eight rows of a sequence; with more than 444 x 3 tiles every stage of every
+    CTA's ring is used again.  fp32 throughout: bounds as above."""
+    B = 600 // Hv
+    q, k, v, g, beta, _ = make_inputs("default", seed=S, B=B, S=S, Hq=Hq, Hv=Hv)
+    h0 = torch.randn(B, Hv, 128, 128, generator=torch.Generator().manual_seed(S))
+    out, st = gdn_chunk(*[t.cuda() for t in (q, k, v, g, beta)], initial_state=h0.cuda(), path="decode")
+    check_device_status()
+    ro, rs = oracle_f32(q, k, v, g, beta, h0, form="recurrent")
+    assert O.rel_l2(st.cpu().numpy(), rs) < 1e-5
+    assert np.all(np.abs(out.float().cpu().numpy() - ro) <= 2.0 ** -7 * np.abs(ro) + 1e-6)
