@@ -103,6 +103,15 @@ __device__ __forceinline__ void lean_l2norm_fold(LeanScratch& ps, const uint8_t*
     ctx.sync();
 }
 
+// The bits of the columns below `lim` (of 32).
+__device__ __forceinline__ uint32_t columns_below(int lim) { return lim <= 0 ? 0u : lim >= 32 ? 0xffffffffu : (1u << lim) - 1u; }
+// 2^(g - g_j) of two columns: the mask epilogues take two elements an instruction where they can, and their predicates from the bits of
+// one word several at a time (prepare of 16 sequences of 2048 tokens, 32 heads: 128.3 -> 123.4 us; the same results).
+__device__ __forceinline__ float2 decay2(float g, float gj0, float gj1) {
+    const float2 d = fma2(make_float2(gj0, gj1), make_float2(-1.f, -1.f), make_float2(g, g));
+    return make_float2(fast_exp2(d.x), fast_exp2(d.y));
+}
+
 // Row i of A = tril(beta_i * decay * K K^T, -1), fp32, into At (columns 32-63 of rows 0-31 are not written); rows of
 // padding tokens (i >= valid) are zeros whatever the tile holds there.  Returns |k_i|^2.
 __device__ __forceinline__ float lean_mask_row_A(const LeanScratch& ps, bool l2norm, uint32_t trow, int i, bool low_rows,
@@ -111,10 +120,12 @@ __device__ __forceinline__ float lean_mask_row_A(const LeanScratch& ps, bool l2n
     const float gi = ps.gam[i];
     const float bi = l2norm ? ps.bet[i] * ps.rn[i] : ps.bet[i];
     const int lim = i < valid ? i : 0;
+    const float2 b2 = make_float2(bi, bi);
     float ksq = 0.f;
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
         if (half == 1 && low_rows) break;
+        const uint32_t keep = columns_below(lim - 32 * half);
         uint32_t r[32];
         tmem_ld_x32(trow + half * 32, r);
         tmem_ld_wait();
@@ -126,12 +137,10 @@ __device__ __forceinline__ float lean_mask_row_A(const LeanScratch& ps, bool l2n
 #pragma unroll
         for (int c = 0; c < 32; c += 4) {
             const float4 gj = *reinterpret_cast<const float4*>(gcol + half * 32 + c);
-            float4 o;
-            o.x = (half * 32 + c + 0 < lim) ? bi * fast_exp2(gi - gj.x) * __uint_as_float(r[c + 0]) : 0.f;
-            o.y = (half * 32 + c + 1 < lim) ? bi * fast_exp2(gi - gj.y) * __uint_as_float(r[c + 1]) : 0.f;
-            o.z = (half * 32 + c + 2 < lim) ? bi * fast_exp2(gi - gj.z) * __uint_as_float(r[c + 2]) : 0.f;
-            o.w = (half * 32 + c + 3 < lim) ? bi * fast_exp2(gi - gj.w) * __uint_as_float(r[c + 3]) : 0.f;
-            *reinterpret_cast<float4*>(At + i * kSolveStride + half * 32 + c) = o;
+            const float2 x = mul2(mul2(decay2(gi, gj.x, gj.y), b2), make_float2(__uint_as_float(r[c]), __uint_as_float(r[c + 1])));
+            const float2 y = mul2(mul2(decay2(gi, gj.z, gj.w), b2), make_float2(__uint_as_float(r[c + 2]), __uint_as_float(r[c + 3])));
+            *reinterpret_cast<float4*>(At + i * kSolveStride + half * 32 + c) =
+                make_float4(keep & (1u << c) ? x.x : 0.f, keep & (2u << c) ? x.y : 0.f, keep & (4u << c) ? y.x : 0.f, keep & (8u << c) ? y.y : 0.f);
         }
     }
     return i < valid ? ksq : 0.f;
@@ -152,6 +161,7 @@ __device__ __forceinline__ void lean_mask_row_P(const LeanScratch& ps, bool l2no
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
         if (half == 1 && low_rows) break;          // above the diagonal
+        const uint32_t keep = columns_below(lim + 1 - 32 * half);
         uint32_t r[32];
         tmem_ld_x32(trow + half * 32, r);
         tmem_ld_wait();
@@ -162,10 +172,12 @@ __device__ __forceinline__ void lean_mask_row_P(const LeanScratch& ps, bool l2no
             for (int c = 0; c < 8; c += 4) {
                 const int col = half * 32 + 8 * ch + c;
                 const float4 gj = *reinterpret_cast<const float4*>(gcol + col);
-                x[c + 0] = (col + 0 <= lim) ? fast_exp2(gis - gj.x) * __uint_as_float(r[8 * ch + c + 0]) : 0.f;
-                x[c + 1] = (col + 1 <= lim) ? fast_exp2(gis - gj.y) * __uint_as_float(r[8 * ch + c + 1]) : 0.f;
-                x[c + 2] = (col + 2 <= lim) ? fast_exp2(gis - gj.z) * __uint_as_float(r[8 * ch + c + 2]) : 0.f;
-                x[c + 3] = (col + 3 <= lim) ? fast_exp2(gis - gj.w) * __uint_as_float(r[8 * ch + c + 3]) : 0.f;
+                const float2 y = mul2(decay2(gis, gj.x, gj.y), make_float2(__uint_as_float(r[8 * ch + c]), __uint_as_float(r[8 * ch + c + 1])));
+                const float2 z = mul2(decay2(gis, gj.z, gj.w), make_float2(__uint_as_float(r[8 * ch + c + 2]), __uint_as_float(r[8 * ch + c + 3])));
+                x[c + 0] = keep & (1u << (8 * ch + c)) ? y.x : 0.f;
+                x[c + 1] = keep & (2u << (8 * ch + c)) ? y.y : 0.f;
+                x[c + 2] = keep & (4u << (8 * ch + c)) ? z.x : 0.f;
+                x[c + 3] = keep & (8u << (8 * ch + c)) ? z.y : 0.f;
             }
             uint4 pk;
             pk.x = pack_bf16x2(x[0], x[1]);
