@@ -52,6 +52,7 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     __shared__ __align__(8) uint64_t bar_mma;
     __shared__ uint32_t tmem_slot;
     __shared__ __align__(16) LeanScratch ps2[HEADS];
+    __shared__ float squares[HEADS][128];         // with L2 normalisation: of the rows of [K;Q], per k-half
 
     const int tid = threadIdx.x, warp = static_cast<int>(warp_uniform(tid >> 5)), lane = tid & 31;
     const int h = HEADS == 2 ? tid >> 7 : 0;      // which head of the pair this half of the CTA prepares
@@ -177,18 +178,20 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         // the gate cumsum and the decay tables need nothing from the tiles: they run while the product does
         if (hwarp == 0) {
             if (elect_one()) tma_store_wait_read();   // (the lane that issued it) the previous item's T'' has left the array A goes into
-            lean_gates(ps, gates, p.gate_act != 0, scale0, vec, lane);
+            lean_gates(ps, gates, p.gate_act != 0, scale0, p.l2norm ? ps.vec : vec, lane);
         }
         ctx.sync();
         if (p.l2norm) {
             ok = mbar_wait(&bar_tma, ph, p.status, kDevTimeoutTma);
-            lean_l2norm_fold(ps, kq, vec, cur.valid, ctx);
+            squares[h][htid] = lean_row_squares(kq + h * 16384, htid);
+            if (HEADS == 1) squares[h][htid] += lean_row_squares(kq + 16384, htid);
         }
         GDN_PHASE(0)
         ok = mbar_wait(&bar_mma, ph, p.status, kDevTimeoutMma) && ok;
         ok = __syncthreads_and(ok);
         if (!ok) break;
         tc_fence_after_sync();
+        if (p.l2norm) lean_l2norm_fold(ps, HEADS == 1 ? squares[0][htid] : squares[0][htid] + squares[HEADS - 1][htid], vec, cur.valid, ctx);
         GDN_PHASE(1)
         Item nxt = cur;
         if (more) {

@@ -16,6 +16,7 @@ struct alignas(16) LeanScratch {
     float bet[kChunk];      // beta_j (0 for padding tokens)
     float gcol[kChunk];     // with L2 normalisation: gamma_j - log2(1/|k_j|), the mask epilogue's column table
     float rn[2 * kChunk];   // with L2 normalisation: 1/|k_j| (0..63) and 1/|q_i| (64..127)
+    float vec[4 * kChunk];  // with L2 normalisation: the chain's factors before the norms are known
     float bound[2];         // per warp: max over its rows of beta_i |k_i|^2
     int gates_ok;           // every gate of the chunk is inside beta >= 0, g <= 0 (tested on the gates themselves: the
                             // cumsum's rounding can make two of its neighbours change places)
@@ -72,33 +73,37 @@ __device__ __forceinline__ void lean_gates(LeanScratch& ps, LaneGates x, bool ra
     if (lane == 0) vec_out[2 * kChunk] = exp2f(cC);
 }
 
-// L2 normalisation of q and k, folded into factors that exist anyway (see prep_l2norm_fold): 128 threads, thread r sums
-// row r of the [K;Q] stack; ends with a group barrier.  Rows of padding tokens count as zeros.
-__device__ __forceinline__ void lean_l2norm_fold(LeanScratch& ps, const uint8_t* kq, float* vec_out, int valid, PrepCtx ctx) {
-    const int tid = ctx.tid;
-    float ss = 0.f;
+// L2 normalisation of q and k, folded into factors that exist anyway (see prep_l2norm_fold).  Sum of the squares of the 64 values that
+// row `row` of the [K;Q] stack has in k-half `tile`; where two heads share the stack, each half of the CTA sums one k-half.
+__device__ __forceinline__ float lean_row_squares(const uint8_t* tile, int row) {
+    float2 ss = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int half = 0; half < 2; ++half)
+    for (int ch = 0; ch < 8; ++ch) {
+        const uint4 v = *reinterpret_cast<const uint4*>(tile + row * 128 + ((ch + row) & 7) * 16);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int ch = 0; ch < 8; ++ch) {
-            const uint4 v = *reinterpret_cast<const uint4*>(kq + half * 16384 + tid * 128 + ((ch + tid) & 7) * 16);
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float lo = __uint_as_float(w[e] << 16), hi = __uint_as_float(w[e] & 0xffff0000u);
-                ss = fmaf(lo, lo, ss);
-                ss = fmaf(hi, hi, ss);
-            }
+        for (int e = 0; e < 4; ++e) {
+            const float2 x = make_float2(__uint_as_float(w[e] << 16), __uint_as_float(w[e] & 0xffff0000u));
+            ss = fma2(x, x, ss);
         }
+    }
+    return ss.x + ss.y;
+}
+// 128 threads, thread r holds row r's sum; ends with a group barrier.  Rows of padding tokens count as zeros.  The chain's factors go
+// from the tables (lean_gates wrote them to ps.vec) to vec_out: multiplied there in place, their way through L2 and back was most of
+// what normalisation cost, and both heads summed all rows (four sequences of 1999 tokens with all a layer adds: 152.5 -> 146.6 us a
+// call, 144-170 instead of 180-190 in prepare of 16 of 2048, 125 without normalisation).
+__device__ __forceinline__ void lean_l2norm_fold(LeanScratch& ps, float ss, float* vec_out, int valid, PrepCtx ctx) {
+    const int tid = ctx.tid;
     if ((tid & 63) >= valid) ss = 0.f;
     const float r = rsqrtf(ss + 1e-6f);
     ps.rn[tid] = r;
+    vec_out[tid] = ps.vec[tid] * r;
     if (tid < kChunk) {
         ps.gcol[tid] = ps.gam[tid] - __log2f(r);
-        vec_out[tid] *= r;
-        vec_out[3 * kChunk + tid] *= r;
-    } else {
-        vec_out[tid] *= r;           // scale exp(gamma_i) of token tid - 64
+        vec_out[3 * kChunk + tid] = ps.vec[3 * kChunk + tid] * r;
+    } else if (tid == kChunk) {
+        vec_out[2 * kChunk] = ps.vec[2 * kChunk];
     }
     ctx.sync();
 }
