@@ -207,7 +207,6 @@ int gdn_chunk_fwd_varlen_sm100(const void* q, const void* k, const void* v, cons
         p.pk_longest = l.longest;
         p.pk_short = d_shorts;
         p.pk_shorts = l.n_short;
-        p.pk_tokens = cu_seqlens[n_seq];
         most_segments = most;
     }
     if (l.longs > 0) {

@@ -45,7 +45,7 @@ struct Problem {
                            // it may be cut into)
     int pk_n, pk_chunks, pk_longest;   // entries of the two tables; chunks of the longest sequence
     const int4* pk_short;  // decode kernel: [pk_shorts] (sequence, first token, tokens); B = all sequences, S = the most tokens
-    int pk_shorts, pk_tokens;   // pk_tokens: of the whole batch, short sequences and long
+    int pk_shorts;
 };
 
 // Workspace of the two-kernel path (device pointers into the caller's scratch buffer).

@@ -53,9 +53,10 @@ __device__ __forceinline__ float sum_rows(float x) {   // over the eight lanes t
 // bytes of the token area of one stage: k, q rows, 32 columns of v, g and beta
 __host__ __device__ constexpr uint32_t dec_token_bytes(int nt) { return (nt * (256 + 256 + 64) + 2 * kDecTokens * 4 + 127) & ~127u; }
 
-// Where the vectors of several tokens come from: a box of nt rows each, three copies a tile instead of three a token (256 sequences of 4
-// tokens 250 -> 241 us).  A single token's need no map, whose encoding would cost the smallest calls host time.
-template <bool SEVERAL>
+// Where the vectors of several tokens come from: a box of nt rows each, three copies a tile instead of three a token.  A single token's
+// need no map, whose encoding would cost the smallest calls host time; a packed batch's sequences have tokens of their own number each, and
+// a box of the longest one's rows for all of them is slower (256 sequences of one token but one of 8: 174 us, by rows 164; of 1 to 8: 278, 271).
+template <bool BOXES>
 struct TokenMaps {
     CUtensorMap q, k, v;
 };
@@ -64,10 +65,10 @@ struct TokenMaps<false> {};
 
 __host__ __device__ constexpr int dec_ctas_per_sm(int groups, int stages) { return groups == 1 ? 4 : (stages == 3 ? 1 : 2); }
 
-template <int GROUPS, bool GATE_F32, bool PACKED, int STAGES, bool SEVERAL>
+template <int GROUPS, bool GATE_F32, bool PACKED, int STAGES, bool BOXES>
 __global__ void __launch_bounds__(GROUPS * 64 + 32, dec_ctas_per_sm(GROUPS, STAGES))
 gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_out,
-                  const __grid_constant__ TokenMaps<SEVERAL> maps, const __grid_constant__ Problem p, const __grid_constant__ DecodeGate gate, int items, int nt) {
+                  const __grid_constant__ TokenMaps<BOXES> maps, const __grid_constant__ Problem p, const __grid_constant__ DecodeGate gate, int items, int nt) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     __shared__ __align__(8) uint64_t full[GROUPS][STAGES], empty[GROUPS][STAGES];
@@ -119,18 +120,19 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
                 const int quarter = GROUPS == 1 ? it & 3 : g;
                 if (ok && elect_one()) {
                     uint8_t* tk = tok_of(g, s);
-                    mbar_arrive_expect_tx(&full[g][s], (p.h0 ? 16384 : 0) + nt * (256 + 256 + 64));
+                    mbar_arrive_expect_tx(&full[g][s], (p.h0 ? 16384 : 0) + tokens * (256 + 256 + 64));
                     if (p.h0) tma_load_2d(tile_of(g, s), &tm_in, &full[g][s], quarter * 32, state * kD);
-                    if constexpr (SEVERAL) {   // (rows past the sequence's own are read by nobody)
-                        const int row = PACKED ? seq.y : 0, batch = PACKED ? 0 : b;
-                        tma_load_4d(tk, &maps.k, &full[g][s], 0, hq, row, batch);
-                        tma_load_4d(tk + nt * 256, &maps.q, &full[g][s], 0, hq, row, batch);
-                        tma_load_4d(tk + nt * 512, &maps.v, &full[g][s], quarter * 32, h, row, batch);
+                    if constexpr (BOXES) {
+                        tma_load_4d(tk, &maps.k, &full[g][s], 0, hq, 0, b);
+                        tma_load_4d(tk + nt * 256, &maps.q, &full[g][s], 0, hq, 0, b);
+                        tma_load_4d(tk + nt * 512, &maps.v, &full[g][s], quarter * 32, h, 0, b);
                     } else {
-                        const size_t row = tok0 * p.Hq + hq;
-                        bulk_load_1d(tk, p.k + row * kD, 256, &full[g][s]);
-                        bulk_load_1d(tk + 256, p.q + row * kD, 256, &full[g][s]);
-                        bulk_load_1d(tk + 512, p.v + (tok0 * p.Hv + h) * kD + quarter * 32, 64, &full[g][s]);
+                        for (int t = 0; t < tokens; ++t) {
+                            const size_t row = (tok0 + t) * p.Hq + hq;
+                            bulk_load_1d(tk + t * 256, p.k + row * kD, 256, &full[g][s]);
+                            bulk_load_1d(tk + (nt + t) * 256, p.q + row * kD, 256, &full[g][s]);
+                            bulk_load_1d(tk + nt * 512 + t * 64, p.v + ((tok0 + t) * p.Hv + h) * kD + quarter * 32, 64, &full[g][s]);
+                        }
                     }
                 }
                 __syncwarp();
@@ -354,21 +356,21 @@ int launch_decode(const Problem& p, const OutputGate* og, cudaStream_t stream) {
                                                gate, static_cast<int>(items), nt);
         return e == cudaSuccess ? GDN_OK : GDN_ERR_CUDA;
     };
-    if (p.S == 1 && !p.pk_short) {
-        const TokenMaps<false> none;
+    const TokenMaps<false> none;
+    if (p.pk_short) return p.gate_f32 ? go(gdn_decode_kernel<1, true, true, 3, false>, none) : go(gdn_decode_kernel<1, false, true, 3, false>, none);
+    if (p.S == 1) {
         if (gated) return p.gate_f32 ? go(gdn_decode_kernel<4, true, false, 3, false>, none) : go(gdn_decode_kernel<4, false, false, 3, false>, none);
         return p.gate_f32 ? go(gdn_decode_kernel<1, true, false, 3, false>, none) : go(gdn_decode_kernel<1, false, false, 3, false>, none);
     }
     alignas(64) TokenMaps<true> maps;
     {
-        const unsigned long long tokens = p.pk_short ? p.pk_tokens : p.S, batch = p.pk_short ? 1 : p.B, Hq = p.Hq, Hv = p.Hv;
+        const unsigned long long tokens = p.S, batch = p.B, Hq = p.Hq, Hv = p.Hv;
         const unsigned long long dq[4] = {kD, Hq, tokens, batch}, sq[3] = {kD * 2, Hq * kD * 2, tokens * Hq * kD * 2};
         const unsigned long long dv[4] = {kD, Hv, tokens, batch}, sv[3] = {kD * 2, Hv * kD * 2, tokens * Hv * kD * 2};
         const unsigned row[4] = {kD, 1, static_cast<unsigned>(nt), 1}, quarter[4] = {32, 1, static_cast<unsigned>(nt), 1};
         if (encode_tma(&maps.q, p.q, 2, 4, dq, sq, row, 0) || encode_tma(&maps.k, p.k, 2, 4, dq, sq, row, 0) || encode_tma(&maps.v, p.v, 2, 4, dv, sv, quarter, 0))
             return GDN_ERR_DRIVER;
     }
-    if (p.pk_short) return p.gate_f32 ? go(gdn_decode_kernel<1, true, true, 3, true>, maps) : go(gdn_decode_kernel<1, false, true, 3, true>, maps);
     if (gated) return p.gate_f32 ? go(gdn_decode_kernel<4, true, false, 1, true>, maps) : go(gdn_decode_kernel<4, false, false, 1, true>, maps);
     return p.gate_f32 ? go(gdn_decode_kernel<1, true, false, 3, true>, maps) : go(gdn_decode_kernel<1, false, false, 3, true>, maps);
 }

@@ -118,3 +118,20 @@ def test_short_sequences_of_different_lengths_share_a_launch():
         a, b = cu[i], cu[i + 1]
         o1, s1 = gdn_chunk(*[x[:, a:b].contiguous() for x in d], initial_state=h0[i:i + 1])
         assert torch.equal(o1, out[:, a:b]) and torch.equal(s1, st[i:i + 1]), i
+
+
+@pytest.mark.parametrize("lens", [[1] * 20 + [8] + [1] * 19, [8, 1], [3, 8, 2], [1, 70, 1], [5] * 7 + [4]])
+@pytest.mark.parametrize("layer", [False, True])
+def test_short_sequences_beside_a_longer_one(lens, layer):
+    """Every sequence's own tokens are fetched and no more: among others of fewer tokens than the longest, and at the batch's end, where
+    behind a sequence there is no further token."""
+    T, cu = sum(lens), np.concatenate([[0], np.cumsum(lens)]).tolist()
+    q, k, v, g, beta, _ = make_inputs("default", seed=T, B=1, S=T, Hq=2, Hv=4)
+    h0 = 0.1 * torch.randn(len(lens), 4, 128, 128, generator=torch.Generator().manual_seed(T)).cuda()
+    opts = {"use_qk_l2norm_in_kernel": True, "gate_activations": True} if layer else {}
+    d = [t.cuda() for t in (q, k, v, g, beta)]
+    out, st = gdn_chunk_varlen(*d, cu, initial_state=h0, **opts)
+    check_device_status()
+    for i, (a, b) in enumerate(zip(cu, cu[1:])):
+        o1, s1 = gdn_chunk(*[x[:, a:b].contiguous() for x in d], initial_state=h0[i:i + 1], **opts)
+        assert torch.equal(o1, out[:, a:b]) and torch.equal(s1, st[i:i + 1]), i
