@@ -53,9 +53,12 @@ __device__ __forceinline__ float sum_rows(float x) {   // over the eight lanes t
 // bytes of the token area of one stage: k, q rows, 32 columns of v, g and beta
 __host__ __device__ constexpr uint32_t dec_token_bytes(int nt) { return (nt * (256 + 256 + 64) + 2 * kDecTokens * 4 + 127) & ~127u; }
 
-// Where the vectors of several tokens come from: a box of nt rows each, three copies a tile instead of three a token.  A single token's
-// need no map, whose encoding would cost the smallest calls host time; a packed batch's sequences have tokens of their own number each, and
-// a box of the longest one's rows for all of them is slower (256 sequences of one token but one of 8: 174 us, by rows 164; of 1 to 8: 278, 271).
+// Where the vectors of several tokens come from: a box of nt rows each, three copies a tile instead of three a token, where a CTA has
+// more than one tile (32 heads, 18 sequences of 2 tokens 12.5 us, by rows 13.7; 32 of 2 22.0, 23.3; of 3 and more tokens the same within
+// 2 %).  Smaller calls are as long as the host takes to encode the maps and launch (one sequence of 2 to 4 tokens 5.7 us, by rows
+// 5.1), up to four tokens; beyond, up to a tile per SM (one sequence of 5 tokens 5.7, 5.4; two 6.2, 6.3).  A packed batch's sequences
+// have tokens of their own number each, and a box of the longest one's rows for all of them is slower (256 sequences of one token but
+// one of 8: 174 us, by rows 164; of 1 to 8: 278, 271).
 template <bool BOXES>
 struct TokenMaps {
     CUtensorMap q, k, v;
@@ -346,11 +349,11 @@ int launch_decode(const Problem& p, const OutputGate* og, cudaStream_t stream) {
     const int groups = gated ? 4 : 1, stages = gated && p.S > 1 ? 1 : 3, most = gated ? 4 : kDecTokens;   // (most: tokens whose vectors fit the ring)
     const int nt = p.S < most ? p.S : most;
     const long long items = p.pk_short ? 4ll * p.pk_shorts * p.Hv : gated ? states : states * 4;
+    const uint32_t smem = groups * stages * (16384 + dec_token_bytes(nt)) + 1024;
+    const int fit = static_cast<int>(228 * 1024 / (smem + 1536)), most_ctas = dec_ctas_per_sm(groups, stages), per_sm = fit > most_ctas ? most_ctas : fit;
+    const long long cap = static_cast<long long>(sm_count()) * per_sm;
     auto go = [&](auto kernel, const auto& maps) -> int {
-        const uint32_t smem = groups * stages * (16384 + dec_token_bytes(nt)) + 1024;
         if (allow_smem(reinterpret_cast<const void*>(kernel), smem)) return GDN_ERR_CUDA;
-        const int fit = static_cast<int>(228 * 1024 / (smem + 1536)), most_ctas = dec_ctas_per_sm(groups, stages), per_sm = fit > most_ctas ? most_ctas : fit;
-        const long long cap = static_cast<long long>(sm_count()) * per_sm;
         const unsigned grid = static_cast<unsigned>(items < cap ? items : cap);
         const cudaError_t e = launch_dependent(kernel, dim3(grid), dim3(groups * 64 + 32), smem, stream, false, tin, tout, maps, p,
                                                gate, static_cast<int>(items), nt);
@@ -358,10 +361,10 @@ int launch_decode(const Problem& p, const OutputGate* og, cudaStream_t stream) {
     };
     const TokenMaps<false> none;
     if (p.pk_short) return p.gate_f32 ? go(gdn_decode_kernel<1, true, true, 3, false>, none) : go(gdn_decode_kernel<1, false, true, 3, false>, none);
-    if (p.S == 1) {
-        if (gated) return p.gate_f32 ? go(gdn_decode_kernel<4, true, false, 3, false>, none) : go(gdn_decode_kernel<4, false, false, 3, false>, none);
+    if (p.S == 1 && gated) return p.gate_f32 ? go(gdn_decode_kernel<4, true, false, 3, false>, none) : go(gdn_decode_kernel<4, false, false, 3, false>, none);
+    // one tile a CTA (from five tokens on: an SM): the host's time for three more maps is not hidden behind the kernel
+    if (!gated && (p.S == 1 || items <= (p.S > 4 ? sm_count() : cap)))
         return p.gate_f32 ? go(gdn_decode_kernel<1, true, false, 3, false>, none) : go(gdn_decode_kernel<1, false, false, 3, false>, none);
-    }
     alignas(64) TokenMaps<true> maps;
     {
         const unsigned long long tokens = p.S, batch = p.B, Hq = p.Hq, Hv = p.Hv;

@@ -130,3 +130,23 @@ def test_several_tokens_over_a_ring_that_wraps(S, Hq, Hv):
     ro, rs = oracle_f32(q, k, v, g, beta, h0, form="recurrent")
     assert O.rel_l2(st.cpu().numpy(), rs) < 1e-5
     assert np.all(np.abs(out.float().cpu().numpy() - ro) <= 2.0 ** -7 * np.abs(ro) + 1e-6)
+
+
+@pytest.mark.parametrize("S", [2, 4, 5, 8, 9])
+@pytest.mark.parametrize("Hq,Hv", [(1, 4), (4, 4)])
+@pytest.mark.parametrize("stored", [True, False])
+def test_vectors_by_rows_and_by_boxes(S, Hq, Hv, stored):
+    """Calls of few tiles (four a state) fetch several tokens' vectors row by row, larger ones as boxes: the same bits on either side
+    of the line, which lies at a tile per CTA (four per SM, at four tokens three) or, from five tokens on, per SM."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    line = sms * (4 if S < 4 else 3 if S == 4 else 1) // (4 * Hv)
+    B = line + 1
+    q, k, v, g, beta, _ = make_inputs("default", seed=S, B=B, S=S, Hq=Hq, Hv=Hv)
+    h0 = torch.randn(B, Hv, 128, 128, generator=torch.Generator().manual_seed(S)).cuda() if stored else None
+    d = [t.cuda() for t in (q, k, v, g, beta)]
+    out, st = gdn_chunk(*d, initial_state=h0, output_final_state=stored, path="decode")
+    for n in (1, line):
+        o1, s1 = gdn_chunk(*[t[:n].contiguous() for t in d], initial_state=None if h0 is None else h0[:n].contiguous(),
+                           output_final_state=stored, path="decode")
+        assert torch.equal(o1, out[:n]) and (st is None or torch.equal(s1, st[:n])), n
+    check_device_status()
