@@ -18,7 +18,8 @@
 //   GROUPS = 4: the four tiles of a state in one CTA, for the gated normalisation of the output rows (their sum of squares
 //   needs all 128 columns: one barrier a token), which then costs no launch and no pass over the rows of its own.  One token: a ring of
 //   three, one CTA per SM (HBM-bound).  Several: its barriers and instructions bound it, and two CTAs per SM with one stage each fill
-//   each other's waits (8 sequences of 4 tokens 19.1 -> 15.7 us, 64 of 4 111 -> 94, 8 of 8 38.8 -> 26.9).
+//   each other's waits where there are states for both (8 sequences of 4 tokens 19.1 -> 15.7 us, 64 of 4 111 -> 94, 8 of 8 38.8 -> 26.9;
+//   at 96 registers a thread, for which the compiler keeps 88 bytes of it in local memory).
 #include <cuda.h>
 
 #include "../../include/gdn_chunk_sm100.h"
@@ -326,6 +327,26 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
     }
 }
 
+// Gated rows: two CTAs per SM of one stage each, or one of three stages?  Two fill each other's barriers and instructions; one overlaps
+// the next state's load and this one's store.  Of an odd number of states per SM the last runs alone, beside a CTA that has no more.
+// 32 heads, fp32 states in and out, all a layer adds, us per call (two / one):
+//   (states an SM) 1 (<= 1)     9 (2)         13 (3)        23 (5)        32 (7)        37 (8)        64 (14)
+//   2 tokens       7.1 / 6.4    11.8 / 12.4   19.9 / 16.4   31.6 / 26.3   41.4 / 35.9   42.6 / 40.3   67.7 / 66.2
+//   3 tokens       8.6 / 7.7    13.9 / 15.3   23.9 / 20.7   37.3 / 33.3   48.8 / 45.7   49.9 / 51.6   80.3 / 85.8
+//   4 tokens       10.0 / 8.8   16.1 / 18.0   27.9 / 24.7   43.1 / 40.1   56.4 / 55.2   57.5 / 62.7   94.2 / 105
+//   6 tokens       13.4 / 11.7  21.5 / 27.0   38.7 / 38.0   59.8 / 62.4   78.7 / 86.3   -             134 / 168
+// A state that is not written weighs little beside the instructions: one CTA only at two and a half to three states per SM (13 sequences
+// of 2 tokens, state in 15.5 / 14.2, none 12.2 / 10.7; 64 of 2, 46.8 / 52.4 and 38.9 / 43.0).  Out only, 2 tokens: 32 sequences
+// 32.2 / 28.9, 37 33.8 / 34.0, 64 57.6 / 57.9.
+bool two_gated_ctas(const Problem& p, long long states) {
+    const long long sms = sm_count(), rounds = (states + sms - 1) / sms, pairs = (states + 2 * sms - 1) / (2 * sms);
+    if (p.S == 1 || rounds == 1) return false;
+    if (p.S > 4 || rounds == 2) return true;
+    if (!p.hT) return rounds != 3 || 2 * states <= 5 * sms;
+    if (p.S == 2 && p.h0) return false;
+    return 10 * rounds >= (p.S == 2 ? 19 : p.S == 3 ? 18 : 17) * pairs;
+}
+
 }  // namespace
 
 // `og`: gated normalisation applied to the output rows by the same kernel (null: none).
@@ -346,7 +367,8 @@ int launch_decode(const Problem& p, const OutputGate* og, cudaStream_t stream) {
     DecodeGate gate{};
     if (og) gate = DecodeGate{static_cast<const __nv_bfloat16*>(og->z), static_cast<const __nv_bfloat16*>(og->weight), og->eps};
     const bool gated = og && !p.pk_short;
-    const int groups = gated ? 4 : 1, stages = gated && p.S > 1 ? 1 : 3, most = gated ? 4 : kDecTokens;   // (most: tokens whose vectors fit the ring)
+    const int groups = gated ? 4 : 1, stages = gated && two_gated_ctas(p, states) ? 1 : 3;
+    const int most = gated ? 4 : kDecTokens;                       // tokens whose vectors fit three stages of four groups
     const int nt = p.S < most ? p.S : most;
     const long long items = p.pk_short ? 4ll * p.pk_shorts * p.Hv : gated ? states : states * 4;
     const uint32_t smem = groups * stages * (16384 + dec_token_bytes(nt)) + 1024;
@@ -374,6 +396,7 @@ int launch_decode(const Problem& p, const OutputGate* og, cudaStream_t stream) {
         if (encode_tma(&maps.q, p.q, 2, 4, dq, sq, row, 0) || encode_tma(&maps.k, p.k, 2, 4, dq, sq, row, 0) || encode_tma(&maps.v, p.v, 2, 4, dv, sv, quarter, 0))
             return GDN_ERR_DRIVER;
     }
+    if (gated && stages == 3) return p.gate_f32 ? go(gdn_decode_kernel<4, true, false, 3, true>, maps) : go(gdn_decode_kernel<4, false, false, 3, true>, maps);
     if (gated) return p.gate_f32 ? go(gdn_decode_kernel<4, true, false, 1, true>, maps) : go(gdn_decode_kernel<4, false, false, 1, true>, maps);
     return p.gate_f32 ? go(gdn_decode_kernel<1, true, false, 3, true>, maps) : go(gdn_decode_kernel<1, false, false, 3, true>, maps);
 }

@@ -150,3 +150,71 @@ def test_vectors_by_rows_and_by_boxes(S, Hq, Hv, stored):
                            output_final_state=stored, path="decode")
         assert torch.equal(o1, out[:n]) and (st is None or torch.equal(s1, st[:n])), n
     check_device_status()
+
+
+def layer_inputs(seed, B, S, Hq, Hv):
+    """Raw projections as a layer hands them over: q and k of any length, gates before their activations; z and the norm's weight."""
+    gen = torch.Generator().manual_seed(seed)
+    q, k = (3 * torch.randn(B, S, Hq, 128, generator=gen)).bfloat16(), (3 * torch.randn(B, S, Hq, 128, generator=gen)).bfloat16()
+    v = torch.randn(B, S, Hv, 128, generator=gen).bfloat16()
+    g, beta = 1.5 * torch.randn(B, S, Hv, generator=gen), 1.5 * torch.randn(B, S, Hv, generator=gen)
+    z, w = (1.5 * torch.randn(B, S, Hv, 128, generator=gen)).bfloat16(), (1 + 0.1 * torch.randn(128, generator=gen)).bfloat16()
+    return (q, k, v, g, beta), z, w
+
+
+@pytest.mark.parametrize("S", [2, 3, 4, 5, 9])
+@pytest.mark.parametrize("rounds", [1, 2, 3, 4])
+@pytest.mark.parametrize("h_in,h_out", [(True, True), (True, False), (False, False)])
+def test_gated_decode_of_a_layer(S, rounds, h_in, h_out):
+    """Both gated forms of several tokens with all that a layer adds, one to four states per SM: a stage used once and again, either
+    side of the lines between the forms.  The row that is normalised is the ungated call's (bounds as in test_gated_decode); the first
+    and last sequences against the oracle."""
+    Hq, Hv = 2, 4
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    B = rounds * sms // Hv
+    x, z, w = layer_inputs(10 * S + rounds, B, S, Hq, Hv)
+    h0 = 0.1 * torch.randn(B, Hv, 128, 128, generator=torch.Generator().manual_seed(S)).cuda() if h_in else None
+    d, opts = [t.cuda() for t in x], {"use_qk_l2norm_in_kernel": True, "gate_activations": True, "path": "decode"}
+    plain, st = gdn_chunk(*d, initial_state=h0, output_final_state=h_out, **opts)
+    out, st2 = gdn_chunk(*d, initial_state=h0, output_final_state=h_out, output_gate=(z.cuda(), w.cuda()), **opts)
+    check_device_status()
+    assert (st is None and st2 is None) or torch.equal(st, st2)
+    ref = rmsnorm_gated(plain, z.cuda(), w.cuda()).float()
+    assert ((out.float() - ref).abs() <= 2.0 ** -7 * ref.abs() + 1e-6).all()
+    for part in (slice(0, 2), slice(B - 2, B)):
+        q, k, v, g, beta = (t[part] for t in x)
+        ro, rs = oracle_f32(q, k, v, -torch.nn.functional.softplus(g), torch.sigmoid(beta), None if h0 is None else h0[part].cpu(),
+                            form="recurrent", l2norm=True)
+        ro = O.rmsnorm_gated(ro, z[part].float().numpy(), w.float().numpy())
+        assert O.rel_l2(out[part].float().cpu().numpy(), ro) < 6e-3
+        assert st is None or O.rel_l2(st[part].cpu().numpy(), rs) < 1e-5
+
+
+@pytest.mark.parametrize("S", [2, 3])
+def test_gated_decode_of_three_states_per_sm(S):
+    """Three states per SM take about half as long again as two, and not as long as four: times of graphs of 20 calls."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    times = []
+    for rounds in (2, 3):
+        B = rounds * sms // 4
+        x, z, w = layer_inputs(S, B, S, 2, 4)
+        d, gate = [t.cuda() for t in x], (z.cuda(), w.cuda())
+        h0 = torch.zeros(B, 4, 128, 128, device="cuda")
+        def call():
+            gdn_chunk(*d, initial_state=h0, use_qk_l2norm_in_kernel=True, gate_activations=True, output_gate=gate)
+        call()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for _ in range(20):
+                call()
+        best = float("inf")
+        for _ in range(20):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            graph.replay()
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        times.append(best)
+    assert times[1] < 1.56 * times[0], times
