@@ -202,7 +202,7 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         {   // mask epilogue: thread = row i = TMEM lane
             const bool low_rows = (hwarp & 1) == 0;          // rows 0-31: columns 32-63 lie above the diagonal
             if (hwarp < 2) {   // A = tril(beta_i * decay * K K^T, -1), fp32, and at once the inverse of the warp's 32x32 block
-                const float ksq = lean_mask_row_A(ps, p.l2norm != 0, tmem_addr(acc, lane_base, 0), i, low_rows, cur.valid, At);
+                const float ksq = lean_mask_row_A<HEADS == 2>(ps, p.l2norm != 0, tmem_addr(acc, lane_base, 0), i, low_rows, cur.valid, At);
                 if (ws.meta) {
                     const float bound = lean_bound_of_rows(ps, p.l2norm != 0, i, ksq);
                     if (lane == 0) ps.bound[hwarp] = bound;

@@ -119,6 +119,9 @@ __device__ __forceinline__ float2 decay2(float g, float gj0, float gj1) {
 
 // Row i of A = tril(beta_i * decay * K K^T, -1), fp32, into At (columns 32-63 of rows 0-31 are not written); rows of
 // padding tokens (i >= valid) are zeros whatever the tile holds there.  Returns |k_i|^2.
+// PAIRED: two elements an instruction.  With one head per CTA, 128 registers a thread, that gives nothing on many chunks (16 sequences of
+// 2048 tokens, 16 / 16 heads: 217 us a call either way) and takes 0.2 us longer on a few (100 tokens, 16 / 16 heads: 13.58 -> 13.79).
+template <bool PAIRED>
 __device__ __forceinline__ float lean_mask_row_A(const LeanScratch& ps, bool l2norm, uint32_t trow, int i, bool low_rows,
                                                  int valid, float* At) {
     const float* gcol = l2norm ? ps.gcol : ps.gam;
@@ -142,10 +145,19 @@ __device__ __forceinline__ float lean_mask_row_A(const LeanScratch& ps, bool l2n
 #pragma unroll
         for (int c = 0; c < 32; c += 4) {
             const float4 gj = *reinterpret_cast<const float4*>(gcol + half * 32 + c);
-            const float2 x = mul2(mul2(decay2(gi, gj.x, gj.y), b2), make_float2(__uint_as_float(r[c]), __uint_as_float(r[c + 1])));
-            const float2 y = mul2(mul2(decay2(gi, gj.z, gj.w), b2), make_float2(__uint_as_float(r[c + 2]), __uint_as_float(r[c + 3])));
-            *reinterpret_cast<float4*>(At + i * kSolveStride + half * 32 + c) =
-                make_float4(keep & (1u << c) ? x.x : 0.f, keep & (2u << c) ? x.y : 0.f, keep & (4u << c) ? y.x : 0.f, keep & (8u << c) ? y.y : 0.f);
+            float4 o;
+            if constexpr (PAIRED) {
+                const float2 x = mul2(mul2(decay2(gi, gj.x, gj.y), b2), make_float2(__uint_as_float(r[c]), __uint_as_float(r[c + 1])));
+                const float2 y = mul2(mul2(decay2(gi, gj.z, gj.w), b2), make_float2(__uint_as_float(r[c + 2]), __uint_as_float(r[c + 3])));
+                o = make_float4(keep & (1u << c) ? x.x : 0.f, keep & (2u << c) ? x.y : 0.f, keep & (4u << c) ? y.x : 0.f, keep & (8u << c) ? y.y : 0.f);
+            } else {
+                const int col = half * 32 + c;
+                o.x = col + 0 < lim ? bi * fast_exp2(gi - gj.x) * __uint_as_float(r[c + 0]) : 0.f;
+                o.y = col + 1 < lim ? bi * fast_exp2(gi - gj.y) * __uint_as_float(r[c + 1]) : 0.f;
+                o.z = col + 2 < lim ? bi * fast_exp2(gi - gj.z) * __uint_as_float(r[c + 2]) : 0.f;
+                o.w = col + 3 < lim ? bi * fast_exp2(gi - gj.w) * __uint_as_float(r[c + 3]) : 0.f;
+            }
+            *reinterpret_cast<float4*>(At + i * kSolveStride + half * 32 + c) = o;
         }
     }
     return i < valid ? ksq : 0.f;
