@@ -120,9 +120,10 @@ def test_more_rows_than_a_state_map_could_address():
 @pytest.mark.parametrize("S", [2, 7, 8, 9])
 @pytest.mark.parametrize("Hq,Hv", [(1, 2), (3, 3)])
 def test_several_tokens_over_a_ring_that_wraps(S, Hq, Hv):
-    """Vectors of several tokens come as boxes of up to eight rows of a sequence; with more than 444 x 3 tiles every stage of every
-    CTA's ring is used again.  fp32 throughout: bounds as above."""
-    B = 600 // Hv
+    """Vectors of several tokens come as boxes of up to eight rows of a sequence.  Of four tiles a state, a CTA (at most four per SM)
+    gets at least seven: each of its three stages is used twice and the first a third time.  fp32 throughout: bounds as above."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    B = -(-7 * sms // Hv)
     q, k, v, g, beta, _ = make_inputs("default", seed=S, B=B, S=S, Hq=Hq, Hv=Hv)
     h0 = torch.randn(B, Hv, 128, 128, generator=torch.Generator().manual_seed(S))
     out, st = gdn_chunk(*[t.cuda() for t in (q, k, v, g, beta)], initial_state=h0.cuda(), path="decode")
