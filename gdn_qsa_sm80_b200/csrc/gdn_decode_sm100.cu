@@ -60,19 +60,21 @@ __host__ __device__ constexpr uint32_t dec_token_bytes(int nt) { return (nt * (2
 // 5.1), up to four tokens; beyond, up to a tile per SM (one sequence of 5 tokens 5.7, 5.4; two 6.2, 6.3).  A packed batch's sequences
 // have tokens of their own number each, and a box of the longest one's rows for all of them is slower (256 sequences of one token but
 // one of 8: 174 us, by rows 164; of 1 to 8: 278, 271).
-template <bool BOXES>
-struct TokenMaps {
+// ONE_ROW is ROWS for a single token: without the loop over tokens 8 sequences of one token take 7.0 us, with it 7.4.
+enum class Fetch { ONE_ROW, ROWS, BOXES };
+template <Fetch FETCH>
+struct TokenMaps {};
+template <>
+struct TokenMaps<Fetch::BOXES> {
     CUtensorMap q, k, v;
 };
-template <>
-struct TokenMaps<false> {};
 
 __host__ __device__ constexpr int dec_ctas_per_sm(int groups, int stages) { return groups == 1 ? 4 : (stages == 3 ? 1 : 2); }
 
-template <int GROUPS, bool GATE_F32, bool PACKED, int STAGES, bool BOXES>
+template <int GROUPS, bool GATE_F32, bool PACKED, int STAGES, Fetch FETCH>
 __global__ void __launch_bounds__(GROUPS * 64 + 32, dec_ctas_per_sm(GROUPS, STAGES))
 gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_out,
-                  const __grid_constant__ TokenMaps<BOXES> maps, const __grid_constant__ Problem p, const __grid_constant__ DecodeGate gate, int items, int nt) {
+                  const __grid_constant__ TokenMaps<FETCH> maps, const __grid_constant__ Problem p, const __grid_constant__ DecodeGate gate, int items, int nt) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     __shared__ __align__(8) uint64_t full[GROUPS][STAGES], empty[GROUPS][STAGES];
@@ -126,12 +128,12 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
                     uint8_t* tk = tok_of(g, s);
                     mbar_arrive_expect_tx(&full[g][s], (p.h0 ? 16384 : 0) + tokens * (256 + 256 + 64));
                     if (p.h0) tma_load_2d(tile_of(g, s), &tm_in, &full[g][s], quarter * 32, state * kD);
-                    if constexpr (BOXES) {
+                    if constexpr (FETCH == Fetch::BOXES) {
                         tma_load_4d(tk, &maps.k, &full[g][s], 0, hq, 0, b);
                         tma_load_4d(tk + nt * 256, &maps.q, &full[g][s], 0, hq, 0, b);
                         tma_load_4d(tk + nt * 512, &maps.v, &full[g][s], quarter * 32, h, 0, b);
                     } else {
-                        for (int t = 0; t < tokens; ++t) {
+                        for (int t = 0; t < (FETCH == Fetch::ONE_ROW ? 1 : tokens); ++t) {
                             const size_t row = (tok0 + t) * p.Hq + hq;
                             bulk_load_1d(tk + t * 256, p.k + row * kD, 256, &full[g][s]);
                             bulk_load_1d(tk + (nt + t) * 256, p.q + row * kD, 256, &full[g][s]);
@@ -381,13 +383,15 @@ int launch_decode(const Problem& p, const OutputGate* og, cudaStream_t stream) {
                                                gate, static_cast<int>(items), nt);
         return e == cudaSuccess ? GDN_OK : GDN_ERR_CUDA;
     };
-    const TokenMaps<false> none;
-    if (p.pk_short) return p.gate_f32 ? go(gdn_decode_kernel<1, true, true, 3, false>, none) : go(gdn_decode_kernel<1, false, true, 3, false>, none);
-    if (p.S == 1 && gated) return p.gate_f32 ? go(gdn_decode_kernel<4, true, false, 3, false>, none) : go(gdn_decode_kernel<4, false, false, 3, false>, none);
+    const TokenMaps<Fetch::ONE_ROW> one;
+    const TokenMaps<Fetch::ROWS> rows;
+    if (p.pk_short) return p.gate_f32 ? go(gdn_decode_kernel<1, true, true, 3, Fetch::ROWS>, rows) : go(gdn_decode_kernel<1, false, true, 3, Fetch::ROWS>, rows);
+    if (p.S == 1 && gated) return p.gate_f32 ? go(gdn_decode_kernel<4, true, false, 3, Fetch::ONE_ROW>, one) : go(gdn_decode_kernel<4, false, false, 3, Fetch::ONE_ROW>, one);
+    if (p.S == 1) return p.gate_f32 ? go(gdn_decode_kernel<1, true, false, 3, Fetch::ONE_ROW>, one) : go(gdn_decode_kernel<1, false, false, 3, Fetch::ONE_ROW>, one);
     // one tile a CTA (from five tokens on: an SM): the host's time for three more maps is not hidden behind the kernel
-    if (!gated && (p.S == 1 || items <= (p.S > 4 ? sm_count() : cap)))
-        return p.gate_f32 ? go(gdn_decode_kernel<1, true, false, 3, false>, none) : go(gdn_decode_kernel<1, false, false, 3, false>, none);
-    alignas(64) TokenMaps<true> maps;
+    if (!gated && items <= (p.S > 4 ? sm_count() : cap))
+        return p.gate_f32 ? go(gdn_decode_kernel<1, true, false, 3, Fetch::ROWS>, rows) : go(gdn_decode_kernel<1, false, false, 3, Fetch::ROWS>, rows);
+    alignas(64) TokenMaps<Fetch::BOXES> maps;
     {
         const unsigned long long tokens = p.S, batch = p.B, Hq = p.Hq, Hv = p.Hv;
         const unsigned long long dq[4] = {kD, Hq, tokens, batch}, sq[3] = {kD * 2, Hq * kD * 2, tokens * Hq * kD * 2};
@@ -396,9 +400,9 @@ int launch_decode(const Problem& p, const OutputGate* og, cudaStream_t stream) {
         if (encode_tma(&maps.q, p.q, 2, 4, dq, sq, row, 0) || encode_tma(&maps.k, p.k, 2, 4, dq, sq, row, 0) || encode_tma(&maps.v, p.v, 2, 4, dv, sv, quarter, 0))
             return GDN_ERR_DRIVER;
     }
-    if (gated && stages == 3) return p.gate_f32 ? go(gdn_decode_kernel<4, true, false, 3, true>, maps) : go(gdn_decode_kernel<4, false, false, 3, true>, maps);
-    if (gated) return p.gate_f32 ? go(gdn_decode_kernel<4, true, false, 1, true>, maps) : go(gdn_decode_kernel<4, false, false, 1, true>, maps);
-    return p.gate_f32 ? go(gdn_decode_kernel<1, true, false, 3, true>, maps) : go(gdn_decode_kernel<1, false, false, 3, true>, maps);
+    if (gated && stages == 3) return p.gate_f32 ? go(gdn_decode_kernel<4, true, false, 3, Fetch::BOXES>, maps) : go(gdn_decode_kernel<4, false, false, 3, Fetch::BOXES>, maps);
+    if (gated) return p.gate_f32 ? go(gdn_decode_kernel<4, true, false, 1, Fetch::BOXES>, maps) : go(gdn_decode_kernel<4, false, false, 1, Fetch::BOXES>, maps);
+    return p.gate_f32 ? go(gdn_decode_kernel<1, true, false, 3, Fetch::BOXES>, maps) : go(gdn_decode_kernel<1, false, false, 3, Fetch::BOXES>, maps);
 }
 
 }  // namespace gdn
