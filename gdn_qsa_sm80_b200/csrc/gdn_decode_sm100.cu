@@ -9,9 +9,9 @@
 // leaves by TMA store, which the load-compute-store phases of one CTA per state could not do (75 % of the copy bandwidth).
 // The tile is 128-byte swizzled; a lane owns eight pairs of rows and the four columns of a chunk, so that a 16-byte access of eight
 // lanes covers all banks, a pair's two values of k arrive in one word, and the column sums a token needs (S^T k, S^T q) are three
-// shuffles: no barrier.  With several tokens a tile what bounds it is the two warps' instructions, not HBM: two multiply-adds in one
-// (f32x2), and their vectors fetched as one box a tensor instead of a copy a row.  32 heads, before and after: 8 sequences of 4 tokens
-// 14.5 -> 12.7 us, 256 of 4 277 -> 241, 64 of 8 121 -> 111; one token each as before (64 sequences 47 us, 86 % of the copy bandwidth).
+// shuffles: no barrier.  With several tokens a tile what bounds it is the two warps' serial run through the tokens, not HBM (64 sequences
+// of 4: DRAM 40 % busy, issue slots 37 % with six compute warps an SM): two multiply-adds in one instruction (f32x2).  32 heads, before
+// and after: 8 sequences of 4 tokens 14.5 -> 12.7 us, 256 of 4 277 -> 241, 64 of 8 121 -> 111; 64 of one 47 us, 86 % of the copy bandwidth.
 //   GROUPS = 1: a CTA of two compute warps and a producer warp, four per SM (three from four tokens on, whose vectors take
 //   room in every stage); 32 states give 128 CTAs.
 //   PACKED: the sequences of a packed batch that have at most kDecodeMaxTokens tokens, of any lengths, found through a table.
@@ -56,10 +56,10 @@ __host__ __device__ constexpr uint32_t dec_token_bytes(int nt) { return (nt * (2
 
 // Where the vectors of several tokens come from: a box of nt rows each, three copies a tile instead of three a token, where a CTA has
 // more than one tile (32 heads, 18 sequences of 2 tokens 12.5 us, by rows 13.7; 32 of 2 22.0, 23.3; of 3 and more tokens the same within
-// 2 %).  Smaller calls are as long as the host takes to encode the maps and launch (one sequence of 2 to 4 tokens 5.7 us, by rows
-// 5.1), up to four tokens; beyond, up to a tile per SM (one sequence of 5 tokens 5.7, 5.4; two 6.2, 6.3).  A packed batch's sequences
-// have tokens of their own number each, and a box of the longest one's rows for all of them is slower (256 sequences of one token but
-// one of 8: 174 us, by rows 164; of 1 to 8: 278, 271).
+// 2 %).  Smaller calls of up to four tokens are as long as the host takes to encode the maps and launch (one sequence of 2 to 4 tokens
+// 5.7 us, by rows 5.1; of 6, whose kernel is as long as that, 5.8 and 6.5).  A packed batch's sequences have tokens of their own number
+// each, and a box of the longest one's rows for all of them is slower (256 sequences of one token but one of 8: 174 us, by rows 164; of
+// 1 to 8: 278, 271).
 // ONE_ROW is ROWS for a single token: without the loop over tokens 8 sequences of one token take 7.0 us, with it 7.4.
 enum class Fetch { ONE_ROW, ROWS, BOXES };
 template <Fetch FETCH>
@@ -339,13 +339,13 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
 //   6 tokens       13.4 / 11.7  21.5 / 27.0   38.7 / 38.0   59.8 / 62.4   78.7 / 86.3   -             134 / 168
 // A state that is not written weighs little beside the instructions: one CTA only at two and a half to three states per SM (13 sequences
 // of 2 tokens, state in 15.5 / 14.2, none 12.2 / 10.7; 64 of 2, 46.8 / 52.4 and 38.9 / 43.0).  Out only, 2 tokens: 32 sequences
-// 32.2 / 28.9, 37 33.8 / 34.0, 64 57.6 / 57.9.
+// 32.2 / 28.9, 37 33.8 / 34.0, 64 57.6 / 57.9.  Two tokens, in and out, on many states: 128 sequences (28) 125.9 / 125.8, 256 (56) 242 / 246.
 bool two_gated_ctas(const Problem& p, long long states) {
     const long long sms = sm_count(), rounds = (states + sms - 1) / sms, pairs = (states + 2 * sms - 1) / (2 * sms);
     if (p.S == 1 || rounds == 1) return false;
     if (p.S > 4 || rounds == 2) return true;
     if (!p.hT) return rounds != 3 || 2 * states <= 5 * sms;
-    if (p.S == 2 && p.h0) return false;
+    if (p.S == 2 && p.h0) return rounds >= 40;
     return 10 * rounds >= (p.S == 2 ? 19 : p.S == 3 ? 18 : 17) * pairs;
 }
 
@@ -388,8 +388,8 @@ int launch_decode(const Problem& p, const OutputGate* og, cudaStream_t stream) {
     if (p.pk_short) return p.gate_f32 ? go(gdn_decode_kernel<1, true, true, 3, Fetch::ROWS>, rows) : go(gdn_decode_kernel<1, false, true, 3, Fetch::ROWS>, rows);
     if (p.S == 1 && gated) return p.gate_f32 ? go(gdn_decode_kernel<4, true, false, 3, Fetch::ONE_ROW>, one) : go(gdn_decode_kernel<4, false, false, 3, Fetch::ONE_ROW>, one);
     if (p.S == 1) return p.gate_f32 ? go(gdn_decode_kernel<1, true, false, 3, Fetch::ONE_ROW>, one) : go(gdn_decode_kernel<1, false, false, 3, Fetch::ONE_ROW>, one);
-    // one tile a CTA (from five tokens on: an SM): the host's time for three more maps is not hidden behind the kernel
-    if (!gated && items <= (p.S > 4 ? sm_count() : cap))
+    // one tile a CTA: the host's time for three more maps is not hidden behind the kernel
+    if (!gated && p.S <= 4 && items <= cap)
         return p.gate_f32 ? go(gdn_decode_kernel<1, true, false, 3, Fetch::ROWS>, rows) : go(gdn_decode_kernel<1, false, false, 3, Fetch::ROWS>, rows);
     alignas(64) TokenMaps<Fetch::BOXES> maps;
     {

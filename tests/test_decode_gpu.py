@@ -133,14 +133,14 @@ def test_several_tokens_over_a_ring_that_wraps(S, Hq, Hv):
     assert np.all(np.abs(out.float().cpu().numpy() - ro) <= 2.0 ** -7 * np.abs(ro) + 1e-6)
 
 
-@pytest.mark.parametrize("S", [2, 4, 5, 8, 9])
+@pytest.mark.parametrize("S", [2, 3, 4])
 @pytest.mark.parametrize("Hq,Hv", [(1, 4), (4, 4)])
 @pytest.mark.parametrize("stored", [True, False])
 def test_vectors_by_rows_and_by_boxes(S, Hq, Hv, stored):
     """Calls of few tiles (four a state) fetch several tokens' vectors row by row, larger ones as boxes: the same bits on either side
-    of the line, which lies at a tile per CTA (four per SM, at four tokens three) or, from five tokens on, per SM."""
+    of the line, which lies at a tile per CTA (four per SM, at four tokens three)."""
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    line = sms * (4 if S < 4 else 3 if S == 4 else 1) // (4 * Hv)
+    line = sms * (4 if S < 4 else 3) // (4 * Hv)
     B = line + 1
     q, k, v, g, beta, _ = make_inputs("default", seed=S, B=B, S=S, Hq=Hq, Hv=Hv)
     h0 = torch.randn(B, Hv, 128, 128, generator=torch.Generator().manual_seed(S)).cuda() if stored else None
@@ -164,11 +164,11 @@ def layer_inputs(seed, B, S, Hq, Hv):
 
 
 @pytest.mark.parametrize("S", [2, 3, 4, 5, 9])
-@pytest.mark.parametrize("rounds", [1, 2, 3, 4])
+@pytest.mark.parametrize("rounds", [1, 2, 3, 4, 40])
 @pytest.mark.parametrize("h_in,h_out", [(True, True), (True, False), (False, False)])
 def test_gated_decode_of_a_layer(S, rounds, h_in, h_out):
-    """Both gated forms of several tokens with all that a layer adds, one to four states per SM: a stage used once and again, either
-    side of the lines between the forms.  The row that is normalised is the ungated call's (bounds as in test_gated_decode); the first
+    """Both gated forms of several tokens with all that a layer adds, one to four states per SM and many: a stage used once and again,
+    either side of the lines between the forms.  The row that is normalised is the ungated call's (bounds as in test_gated_decode); the first
     and last sequences against the oracle."""
     Hq, Hv = 2, 4
     sms = torch.cuda.get_device_properties(0).multi_processor_count
