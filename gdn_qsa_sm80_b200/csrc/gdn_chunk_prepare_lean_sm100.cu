@@ -11,7 +11,7 @@
 //
 // What bounds it is latency: an item is a chain of dependent phases (product, mask, triangular inverse, T''), so what
 // counts is how many items an SM has in flight.  A and T share one fp32 array (gdn_prep_lean_device.cuh) and K / Q are
-// dead after the product, so a CTA needs 67 KB and 80 registers and three of them (24 warps) fit an SM; the next item's
+// dead after the product, so a CTA needs 73 KB and 80 registers and three of them (24 warps) fit an SM; the next item's
 // K is loaded as soon as this item's product is done, its Q as soon as P's staging tiles (in Q's place) have been read
 // by their TMA store, and its product is issued, into a second accumulator, before this item's T'' is written.
 // Stands in for the reference's gdn_prepare_kernel (csrc/gdn_chunk/gdn_kernel.cu:343-710).
@@ -182,6 +182,8 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         }
         ctx.sync();
         if (p.l2norm) {
+            // The other half reads this half's sums of the item before in lean_l2norm_fold, and no barrier of the CTA lies behind that: this
+            // wait does.  It needs the bytes of both halves of Q, which each half requests behind its own fold.
             ok = mbar_wait(&bar_tma, ph, p.status, kDevTimeoutTma);
             squares[h][htid] = lean_row_squares(kq + h * 16384, htid);
             if (HEADS == 1) squares[h][htid] += lean_row_squares(kq + 16384, htid);

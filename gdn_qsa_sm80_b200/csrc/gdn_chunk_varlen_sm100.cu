@@ -5,7 +5,7 @@
 // The last tile of a sequence also holds the next one's first tokens; gates and beta count as zero there, and the kernels
 // mask those rows (prepare) or clear them in the tile (chain), so no sequence ever sees another's values.
 // Sequences of at most kDecodeMaxTokens tokens take the decode kernel, all of them in one launch through a table of their own (256
-// sequences of 1 to 8 tokens, 32 heads: 1491 us with a launch per run of equal lengths, 348 now; before the packed route a padded
+// sequences of 1 to 8 tokens, 32 heads: 1491 us with a launch per run of equal lengths, 271 now; before the packed route a padded
 // batch, 957).
 //
 // Without this a packed batch was gathered into a padded one and scattered back (torch indexing: two passes over all

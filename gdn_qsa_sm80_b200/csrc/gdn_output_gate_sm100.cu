@@ -6,9 +6,9 @@
 //
 // The work is pure streaming (three 256-byte rows per output row), so the kernel is laid out for HBM: 16 threads
 // own one row (one 16-byte load per thread and tensor), a thread keeps kRowsPerThread rows in flight before it
-// touches any of them, the grid is a multiple of the SM count and strides over the rows.  Run directly after the
-// forward pass and in place (out == y), y is still in the 126 MB L2 for outputs up to that size, so only z is
-// read from and only the result written to HBM.  The launch is a programmatic dependent of the kernel before it: a prompt
+// touches any of them, the grid is a multiple of the SM count and strides over the rows.  Behind the forward pass, in
+// place (out == y), y comes from HBM again unless the call is small: the chain's inputs and workspace pass through the 126 MB
+// L2 beside it (39.5 us chained on 262144 rows, 41 alone).  The launch is a programmatic dependent of the kernel before it: a prompt
 // of 333 tokens with everything a layer adds takes 25.4 us instead of 26.7.
 #include "../../include/gdn_chunk_sm100.h"
 #include "gdn_common.cuh"

@@ -1,7 +1,7 @@
 // Device-side pieces of the "lean" prepare (gdn_chunk_prepare_lean_sm100.cu): the gate cumsum by one warp, the mask
 // epilogues that write straight to their shared-memory destination, and the 64x64 unit-lower-triangular inverse IN
 // PLACE.  Same mathematics as gdn_prep_device.cuh; what differs is what has to fit: three CTAs of two heads per SM
-// leave 73 KB of shared memory and 80 registers to each, so A and T share one 64 x 68 fp32 array: T overwrites A block by
+// leave 74 KB of shared memory and 80 registers to each, so A and T share one 64 x 68 fp32 array: T overwrites A block by
 // block.
 #pragma once
 
@@ -89,10 +89,11 @@ __device__ __forceinline__ float lean_row_squares(const uint8_t* tile, int row) 
     }
     return ss.x + ss.y;
 }
-// 128 threads, thread r holds row r's sum; ends with a group barrier.  Rows of padding tokens count as zeros.  The chain's factors go
-// from the tables (lean_gates wrote them to ps.vec) to vec_out: multiplied there in place, their way through L2 and back was most of
-// what normalisation cost, and both heads summed all rows (four sequences of 1999 tokens with all a layer adds: 152.5 -> 146.6 us a
-// call, 144-170 instead of 180-190 in prepare of 16 of 2048, 125 without normalisation).
+// 128 threads, thread r holds row r's sum (of two partial sums a k-half: against one running sum the norm's last bit differs here and
+// there, and with it single bf16 roundings behind it; error against 64 bits the same).  Ends with a group barrier.  Rows of padding tokens
+// count as zeros.  The chain's factors go from the tables (lean_gates wrote them to ps.vec) to vec_out: multiplied there in place, their
+// way through L2 and back was most of what normalisation cost, and both heads summed all rows (four sequences of 1999 tokens with all
+// a layer adds: 152.5 -> 146.6 us a call; prepare of 16 sequences of 2048 162.6 -> 143.4 us, 124.7 without normalisation).
 __device__ __forceinline__ void lean_l2norm_fold(LeanScratch& ps, float ss, float* vec_out, int valid, PrepCtx ctx) {
     const int tid = ctx.tid;
     if ((tid & 63) >= valid) ss = 0.f;
@@ -111,7 +112,7 @@ __device__ __forceinline__ void lean_l2norm_fold(LeanScratch& ps, float ss, floa
 // The bits of the columns below `lim` (of 32).
 __device__ __forceinline__ uint32_t columns_below(int lim) { return lim <= 0 ? 0u : lim >= 32 ? 0xffffffffu : (1u << lim) - 1u; }
 // 2^(g - g_j) of two columns: the mask epilogues take two elements an instruction where they can, and their predicates from the bits of
-// one word several at a time (prepare of 16 sequences of 2048 tokens, 32 heads: 128.3 -> 123.4 us; the same results).
+// one word several at a time (prepare of 16 sequences of 2048 tokens, 32 heads: 128.3 -> 124.7 us; the same results).
 __device__ __forceinline__ float2 decay2(float g, float gj0, float gj1) {
     const float2 d = fma2(make_float2(gj0, gj1), make_float2(-1.f, -1.f), make_float2(g, g));
     return make_float2(fast_exp2(d.x), fast_exp2(d.y));
