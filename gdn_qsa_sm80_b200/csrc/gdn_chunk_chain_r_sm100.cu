@@ -68,7 +68,7 @@ struct RWork {
     const float* s_in;                     // state it starts from (null: zeros) and where the one it ends with goes
     float* s_out;
     int* status;
-    int abort;
+    int late;                              // code of a wait that ran out
 };
 
 // Shared-memory descriptor of this file's operands: 1024 bytes between 8-row groups and the 128-byte swizzle throughout, so
@@ -88,28 +88,13 @@ __device__ __forceinline__ uint64_t r_desc64(uint32_t lo) {   // triangular tile
 __device__ constexpr uint32_t tri_bytes(int ks) { return (ks >> 1) * 4096 + (ks & 1) * 32; }
 constexpr uint32_t kLoK = (16u >> 4) << 16, kLoMN = (8192u >> 4) << 16;
 
-// Bounded, abortable wait (see mbar_wait_abortable_a) that holds next to nothing in registers: what only its slow path
-// needs (the status word's address, the CTA's abort flag) is read from shared memory there.
+// Bounded wait; a role whose wait ran out leaves, the others' waits run out behind it, and the CTA reports at its end.  With the inline
+// slow path of mbar_wait at 25 places (before / after, us a call): 2 x 1500 tokens, 8 / 8 heads 29.8 / 28.6, 333 tokens 21.5 / 20.9,
+// 4 x 1999 104.0 / 102.2, 8192 100.1 / 98.7; nothing where HBM bounds it.
 __device__ __forceinline__ bool r_wait(uint32_t bar, uint32_t parity, int code, RWork& work) {
-#pragma unroll 1
-    for (int i = 0; i < 128; ++i)
-        if (mbar_try_wait_a(bar, parity)) return true;
-    uint32_t t0;
-    asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(t0));
-#pragma unroll 1
-    while (true) {
-#pragma unroll 1
-        for (int i = 0; i < 256; ++i)
-            if (mbar_try_wait_a(bar, parity)) return true;
-        if (*const_cast<volatile int*>(&work.abort)) return false;
-        uint32_t now;
-        asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(now));
-        if (now - t0 > static_cast<uint32_t>(WAIT_LIMIT_NS)) {
-            atomicCAS(*const_cast<int* volatile*>(&work.status), 0, code);
-            *const_cast<volatile int*>(&work.abort) = 1;
-            return false;
-        }
-    }
+    if (mbar_wait_compact(bar, parity)) return true;
+    work.late = code;
+    return false;
 }
 
 // Row stores of the output warps; opaque to the compiler, which would otherwise keep dozens of precomputed addresses.
@@ -154,7 +139,7 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                                    : i == R_X || i == R_VN || i == R_STATE ? 8 : i == R_QSC || i == R_ODONE ? 4 : 1;
             mbar_init(&bars[i], count);
         }
-        work.abort = 0;
+        work.late = 0;
         work.status = p.status;
         fence_mbar_init();
     }
@@ -612,7 +597,8 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 
     tc_fence_before_sync();
     __syncthreads();
-    if (work.abort) {   // let copies that may still be in flight land before the CTA's memory is released
+    if (work.late) {   // let copies that may still be in flight land before the CTA's memory is released
+        if (tid == 0) atomicCAS(work.status, 0, work.late);
         const unsigned long long w0 = globaltimer_ns();
         while (globaltimer_ns() - w0 < 100000ull) {}
         __syncthreads();

@@ -69,6 +69,12 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     // Persistent CTA: items blockIdx.x, blockIdx.x + gridDim.x, ...; the head group index is the fastest, so the groups
     // that share a qk head are prepared at about the same time.
     struct Item { int b, hv, hq, s0, valid; size_t tok0, tile; };
+    int late = 0;                                 // code of a wait that ran out
+    auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
+        if (mbar_wait_compact(smem_u32(bar), parity)) return true;
+        late = code;
+        return false;
+    };
     auto decode = [&](unsigned n) {
         Item x;
         const unsigned c = n / groups, grp = n - c * groups;
@@ -165,7 +171,7 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     uint32_t ph = 0;            // parity of both barriers: one load and one product per item
     bool ok = true;
     if (warp == 0) {
-        ok = mbar_wait(&bar_tma, 0, p.status, kDevTimeoutTma);
+        ok = wait(&bar_tma, 0, kDevTimeoutTma);
         if (ok && elect_one()) issue_product(tmem);
     }
 
@@ -184,12 +190,12 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         if (p.l2norm) {
             // The other half reads this half's sums of the item before in lean_l2norm_fold, and no barrier of the CTA lies behind that: this
             // wait does.  It needs the bytes of both halves of Q, which each half requests behind its own fold.
-            ok = mbar_wait(&bar_tma, ph, p.status, kDevTimeoutTma);
+            ok = wait(&bar_tma, ph, kDevTimeoutTma);
             squares[h][htid] = lean_row_squares(kq + h * 16384, htid);
             if (HEADS == 1) squares[h][htid] += lean_row_squares(kq + 16384, htid);
         }
         GDN_PHASE(0)
-        ok = mbar_wait(&bar_mma, ph, p.status, kDevTimeoutMma) && ok;
+        ok = wait(&bar_mma, ph, kDevTimeoutMma) && ok;
         ok = __syncthreads_and(ok);
         if (!ok) break;
         tc_fence_after_sync();
@@ -238,7 +244,7 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         lean_finish_T2(At, ps.bet, t2tile, ctx);
         GDN_PHASE(4)
         if (warp == 3 && more) {   // the next item's product, into the other accumulator (read last an item ago)
-            ok = mbar_wait(&bar_tma, ph ^ 1, p.status, kDevTimeoutTma);
+            ok = wait(&bar_tma, ph ^ 1, kDevTimeoutTma);
             if (ok && elect_one()) issue_product(tmem + (ph ^ 1) * 64);
             __syncwarp();
         }
@@ -259,6 +265,7 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         for (int k = 0; k < 8; ++k) p.prof[k] = prof_acc[k];
         p.prof[15] = prof_n;
     }
+    if (late && lane == 0) atomicCAS(p.status, 0, late);
     // Only now may the chain kernel's CTAs start (and set up while the last CTAs of this grid finish): let in earlier, they
     // pile up two to an SM on the SMs that this grid leaves first while others stay empty.
     grid_launch_dependents();

@@ -2,8 +2,8 @@
 // mbarrier, TMA tile loads, tcgen05 (TMEM allocation, UMMA issue/commit, TMEM loads),
 // plus the shared-memory operand layouts and descriptors that go with them.
 //
-// Every spin-wait here is bounded: a wait that does not complete within WAIT_LIMIT_NS
-// records a code in a global status word and returns false, so a protocol bug ends
+// Every spin-wait here is bounded: a wait that does not complete within WAIT_LIMIT_NS (or a number of tries)
+// returns false and a code is recorded in a global status word, so a protocol bug ends
 // the kernel with an error instead of hanging the GPU.
 #pragma once
 
@@ -160,6 +160,32 @@ __device__ __forceinline__ bool mbar_wait_abortable_a(uint32_t bar, uint32_t par
             return false;
         }
     }
+}
+
+// The same wait where several roles of a kernel run at once: five instructions in a loop and no slow path, which at some twenty places
+// of a kernel took a quarter of its code (53 -> 44 KB in the residual-form chain, 1878 -> 518 requests of an SM to the second
+// instruction cache over 33 chunk steps).  16 million tries end it, each of which suspends for a while: between a fifth of a second
+// and a few.  The caller reports the code.
+__device__ __forceinline__ bool mbar_wait_compact(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        ".reg .u32 n;\n\t"
+        "mov.u32 n, 16000000;\n"
+        "WAIT:\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "@p bra DONE;\n\t"
+        "sub.u32 n, n, 1;\n\t"
+        "setp.ne.u32 q, n, 0;\n\t"
+        "@q bra WAIT;\n"
+        "DONE:\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
 }
 
 // Named barrier among `count` threads (count a multiple of 32); id 0 is __syncthreads().
