@@ -6,7 +6,7 @@
 // |I - beta k k^T|_2 <= 1 whenever 0 <= beta |k|^2 <= 2, so |A|_2 <= exp(sum of g).  Once that sum is below -115
 // (exp(-115) < 2^-149) the incoming state no longer shows in fp32: the state after the stretch is the same from a zero
 // state.  So a segment s >= 1 starts from a ZERO state p chunks before its first chunk, p the shortest stretch ending at
-// the boundary whose sum of g is below -115 ("warm-up": its outputs are not stored), and from its first chunk on its state,
+// the boundary whose sum of g is below -115 ("warm-up": its outputs are not formed), and from its first chunk on its state,
 // its outputs and its final state are those of the serial run - bit for bit where the decay is strong (a sum of -10 a chunk);
 // where the warm-up is a hundred chunks long the two states end a last bit apart and their bf16 copies round differently now and
 // then (up to 5e-3 of a chunk's outputs, 120000 random calls, as far as either is from the exact result).
