@@ -106,6 +106,11 @@ int encode_tile_maps(const Problem& p, const Workspace& ws, TileMaps& maps) {
     if (encode_qkv_maps(p, maps.q, maps.k, maps.v, 64)) return 1;
     const unsigned long long tiles = p.pk_chunk ? static_cast<unsigned long long>(p.pk_chunks) * p.Hv
                                                 : static_cast<unsigned long long>(p.B) * p.Hv * ((p.S + kChunk - 1) / kChunk);
+    const unsigned long long dims[4] = {static_cast<unsigned long long>(kD), static_cast<unsigned long long>(p.Hv), static_cast<unsigned long long>(p.S),
+                                        static_cast<unsigned long long>(p.B)};
+    const unsigned long long strides[3] = {kD * 2ull, kD * 2ull * dims[1], kD * 2ull * dims[1] * dims[2]};
+    const unsigned rows[4] = {64, 1, 64, 1};
+    if (encode_tma(maps.out, p.out, 2, 4, dims, strides, rows, 128)) return 1;
     const unsigned long long d[2] = {64, tiles * kChunk}, s[1] = {128};
     const unsigned box[2] = {32, 32};
     return encode_tma(maps.p, ws.P, 2, 2, d, s, box, 64) || encode_tma(maps.t2, ws.U, 2, 2, d, s, box, 64);

@@ -25,11 +25,16 @@
 // Order of issue: E1, E0, ER, E1', E2, E3 - E0 runs during the X epilogue and E1' during the v_new epilogue, so of the two
 // products nothing on the critical path waits for, neither delays one that is on it.
 // Shared memory: K, V and T'' in two slots, Q and P in one: every tile is used once (K twice, a few thousand cycles
-// apart), and its slot is reloaded as soon as the UMMA that read it has completed.
+// apart), and its slot is reloaded as soon as the UMMA that read it has completed.  V's slot is used again first: a chunk's outputs
+// are staged where its V was and leave by TMA.  Two-byte stores by the lanes cost the output warps 190 instructions a chunk, two thirds
+// of what they issue, and these share the issue slots of the critical warps (24.0 -> 20.0 million instructions on 4 x 2048 tokens, 32
+// heads, with the paired arithmetic of the other epilogues).  us a call, before / after: 8192 tokens 97.2 / 91.8, 4 x 1999 101.7 / 95.0,
+// 16 x 2048 322 / 310, 64 x 4096 2700 / 2580, 131072 tokens 1460 / 1380.  (Staged in Q's place, whose next tile is wanted a step earlier
+// than V's, 8192 tokens took 104.)
 //
 // Roles (16 warps): 0-7 critical (warp w: TMEM lane quadrant w % 4, column half w / 4): X, v_new and state epilogues,
 // fp32 state in registers; 8-11 output; 12 TMA producer; 13 issues every UMMA.  Registers are moved from the last two
-// groups of four warps to the first two (64 each at launch -> 88, 88, 48, 24).
+// groups of four warps to the first two (64 each at launch -> 88, 88, 56, 24).
 //
 // Sequences are split into segments when there are too few of them (gdn_segment_plan.cuh).
 // Stands in for the reference's gdn_recurrence_kernel (csrc/gdn_chunk/gdn_kernel.cu:1027-1271).
@@ -52,7 +57,7 @@ constexpr int kRTimeout = 0x500;   // + the barrier's index
 
 // barriers
 enum : uint32_t { R_KFULL = 0, R_VFULL = 2, R_VEMPTY = 4, R_TFULL = 6, R_QFULL = 8, R_PFULL, R_KS, R_QS, R_X, R_VACC, R_VN, R_S, R_STATE,
-                  R_QSC, R_O, R_ODONE, kRBars };
+                  R_QSC, R_O, R_ODONE, R_OUT, kRBars };
 
 // Byte offset, in a [64 tokens][128 dk] tile of two 64-column halves, of the 16 dk that k step `ks` of A_S holds (half ks / 4
 // of the warps packed the column blocks 32 h .. and 64 + 32 h ..).
@@ -97,15 +102,10 @@ __device__ __forceinline__ bool r_wait(uint32_t bar, uint32_t parity, int code, 
     return false;
 }
 
-// Row stores of the output warps; opaque to the compiler, which would otherwise keep dozens of precomputed addresses.
-__device__ __forceinline__ void next_row(unsigned long long& a, unsigned long long stride) {
-    asm volatile("add.u64 %0, %0, %1;" : "+l"(a) : "l"(stride));
-}
-__device__ __forceinline__ void store_lo(unsigned long long a, uint32_t x) {
-    asm volatile("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %1;\n\tst.global.b16 [%0], lo;\n\t}" ::"l"(a), "r"(x) : "memory");
-}
-__device__ __forceinline__ void store_hi(unsigned long long a, uint32_t x) {
-    asm volatile("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %1;\n\tst.global.b16 [%0], hi;\n\t}" ::"l"(a), "r"(x) : "memory");
+__device__ __forceinline__ float2 as_float2(uint32_t a, uint32_t b) { return make_float2(__uint_as_float(a), __uint_as_float(b)); }
+__device__ __forceinline__ uint32_t mul_bf16x2(float2 a, float2 b) {
+    const float2 x = mul2(a, b);
+    return pack_bf16x2(x.x, x.y);
 }
 
 template <int N>
@@ -117,7 +117,7 @@ template <bool SPLIT>
 __global__ void __launch_bounds__(kRThreads, 2)
 gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_p,
-                   const __grid_constant__ CUtensorMap tm_t2, const __grid_constant__ Problem p,
+                   const __grid_constant__ CUtensorMap tm_t2, const __grid_constant__ CUtensorMap tm_out, const __grid_constant__ Problem p,
                    const __grid_constant__ Workspace ws, const unsigned sms) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -302,27 +302,29 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                         prefetch_tri(&tm_t2, r1 + kChunk);
                     }
                 }
-                if (n + 1 < steps) {
-                    if (n > 0 && !wait(R_VEMPTY + ((n + 1) & 1), ((n + 1) >> 1) - 1)) break;
-                    load_v(n + 1);
-                }
                 if (n > 0 && !wait(R_S, n - 1)) break;          // E2, hence also ER and E1', of chunk n - 1
                 if (n + 1 < steps) {
                     load_k(n + 1);
                     load_t2(n + 1);
                 }
-                if (n < from) continue;
-                const int s0 = work.s_first + (work.t0 + n) * kChunk, b = work.b;
-                const int row0 = static_cast<int>((work.tile0 + work.t0 + n) * kChunk);
-                if (elect_one()) {
-                    mbar_arrive_expect_tx_a(cb(R_QFULL), 16384);
-                    tma_load_4d_a(sm_u32 + R_Q, &tm_q, cb(R_QFULL), 0, hq, s0, b);
-                    tma_load_4d_a(sm_u32 + R_Q + 8192, &tm_q, cb(R_QFULL), 64, hq, s0, b);
+                if (n >= from) {
+                    const int s0 = work.s_first + (work.t0 + n) * kChunk, b = work.b;
+                    const int row0 = static_cast<int>((work.tile0 + work.t0 + n) * kChunk);
+                    if (elect_one()) {
+                        mbar_arrive_expect_tx_a(cb(R_QFULL), 16384);
+                        tma_load_4d_a(sm_u32 + R_Q, &tm_q, cb(R_QFULL), 0, hq, s0, b);
+                        tma_load_4d_a(sm_u32 + R_Q + 8192, &tm_q, cb(R_QFULL), 64, hq, s0, b);
+                    }
+                    if (n > from && !wait(R_O, n - from - 1)) break;
+                    if (elect_one()) {
+                        mbar_arrive_expect_tx_a(cb(R_PFULL), kTriBytes);
+                        load_tri(sm_u32 + R_P, &tm_p, cb(R_PFULL), row0);
+                    }
                 }
-                if (n > from && !wait(R_O, n - from - 1)) break;
-                if (elect_one()) {
-                    mbar_arrive_expect_tx_a(cb(R_PFULL), kTriBytes);
-                    load_tri(sm_u32 + R_P, &tm_p, cb(R_PFULL), row0);
+                if (n + 1 < steps) {
+                    if (n > 0 && !wait(R_VEMPTY + ((n + 1) & 1), ((n + 1) >> 1) - 1)) break;
+                    if (n > from && !wait(R_OUT, n - from - 1)) break;   // the outputs of chunk n - 1, staged in its V's place, have left
+                    load_v(n + 1);
                 }
             }
         } else if (warp == 13) {
@@ -396,12 +398,14 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         }
     } else if (warp >= 8) {
         // ------------------------------- output warps ----------------------------------------------------------------
-        set_max_registers_down<48>();
+        set_max_registers_down<56>();
         const uint32_t lane_base = static_cast<uint32_t>(warp & 3) * 32u;
-        const int dv = (warp & 3) * 32 + lane;                // the value column (= TMEM lane) this thread owns
         const uint32_t o_addr = tmem_addr(tmem, lane_base, C_O);
-        const unsigned long long row_bytes = static_cast<unsigned long long>(p.Hv) * kD * 2;
-        unsigned long long dst = reinterpret_cast<unsigned long long>(p.out) + ((work.tok0 + static_cast<size_t>(work.t0 + from) * kChunk) * p.Hv + hv) * (kD * 2) + dv * 2;
+        const bool leader = warp == 8;
+        // Row (token) whose address this lane gives to stmatrix, and its 16-byte chunk (8 value columns) before the swizzle; the warp's 32
+        // value columns lie in one of the two halves of 64 columns.
+        const uint32_t srow = 8 * (lane >> 4) + (lane & 7), sch = 4 * (warp & 1) + ((lane >> 3) & 1);
+        const uint32_t stage = sm_u32 + R_V + ((warp >> 1) & 1) * 8192 + srow * 128;
         for (int n = 0; n < steps; ++n) {
             const uint32_t s = n & 1;
             if (!wait(R_VFULL + s, n >> 1)) break;            // the factors
@@ -421,10 +425,11 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 #pragma unroll
                 for (int j = 0; j < 8; j += 4) {
                     const float4 f = *reinterpret_cast<const float4*>(qf + 8 * u + j);
-                    x[j] = __float_as_uint(__uint_as_float(x[j]) * f.x);
-                    x[j + 1] = __float_as_uint(__uint_as_float(x[j + 1]) * f.y);
-                    x[j + 2] = __float_as_uint(__uint_as_float(x[j + 2]) * f.z);
-                    x[j + 3] = __float_as_uint(__uint_as_float(x[j + 3]) * f.w);
+                    const float2 y = mul2(as_float2(x[j], x[j + 1]), make_float2(f.x, f.y)), z = mul2(as_float2(x[j + 2], x[j + 3]), make_float2(f.z, f.w));
+                    x[j] = __float_as_uint(y.x);
+                    x[j + 1] = __float_as_uint(y.y);
+                    x[j + 2] = __float_as_uint(z.x);
+                    x[j + 3] = __float_as_uint(z.y);
                 }
                 tmem_st_x8(o_addr + 8 * u, x);
             }
@@ -437,43 +442,45 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             }
             if (!wait(R_O, n - from)) break;
             tc_fence_after_sync();
-            // O^T[dv][j]: a warp stores 64 contiguous bytes of row j
-            const int valid = min(kChunk, work.len - (work.t0 + n) * kChunk);
+            // O^T[dv][j] in fragments of 16 value columns by 32 tokens, transposed on their way into the place of V (E0 has read it)
 #pragma unroll
-            for (int h2 = 0; h2 < 2; ++h2) {                  // 32 tokens at a time through packed registers
-                uint32_t pk[16];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    uint32_t x[8];
-                    tmem_ld_x8(o_addr + 32 * h2 + 8 * u, x);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) pk[4 * u + c] = pack_bf16x2(__uint_as_float(x[2 * c]), __uint_as_float(x[2 * c + 1]));
-                }
-                if (h2 == 1) {                                // the accumulator has been read
+            for (int u = 0; u < 4; ++u) {                     // value columns 16 (u & 1), tokens 32 (u >> 1)
+                uint32_t x[16], pk[8];
+                tmem_ld_16x256b_x4(o_addr + (static_cast<uint32_t>(16 * (u & 1)) << 16) + 32 * (u >> 1), x);
+                tmem_ld_wait();
+                if (u == 3) {                                 // the accumulator has been read
                     tc_fence_before_sync();
                     __syncwarp();
                     if (lane == 0) mbar_arrive_a(cb(R_ODONE));
                 }
-                if (valid == kChunk) {
 #pragma unroll
-                    for (int c = 0; c < 16; ++c) {
-                        store_lo(dst, pk[c]);
-                        next_row(dst, row_bytes);
-                        store_hi(dst, pk[c]);
-                        next_row(dst, row_bytes);
-                    }
-                } else {
+                for (int c = 0; c < 8; ++c) pk[c] = pack_bf16x2(__uint_as_float(x[2 * c]), __uint_as_float(x[2 * c + 1]));
 #pragma unroll
-                    for (int c = 0; c < 16; ++c) {
-                        if (32 * h2 + 2 * c < valid) store_lo(dst, pk[c]);
-                        next_row(dst, row_bytes);
-                        if (32 * h2 + 2 * c + 1 < valid) store_hi(dst, pk[c]);
-                        next_row(dst, row_bytes);
-                    }
+                for (int t = 0; t < 2; ++t)
+                    stmatrix_x4_trans(stage + s * 16384 + (32 * (u >> 1) + 16 * t) * 128 + (((sch + 2 * (u & 1)) ^ (srow & 7)) << 4), pk[4 * t], pk[4 * t + 1], pk[4 * t + 2], pk[4 * t + 3]);
+            }
+            const int t0 = (work.t0 + n) * kChunk, valid = work.len - t0;
+            if (p.pk_chunk && valid < kChunk) {               // the rows below are the next sequence's: only this one's are copied
+                named_bar_sync(1, 128);
+                for (int e = tid & 127; e < valid * 16; e += 128) {
+                    const int row = e >> 4, ch = e & 15;
+                    const uint4 x = *reinterpret_cast<const uint4*>(sm + R_V + s * 16384 + (ch >> 3) * 8192 + row * 128 + (((ch & 7) ^ (row & 7)) << 4));
+                    *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.out) + ((work.tok0 + t0 + row) * p.Hv + hv) * (kD * 2) + ch * 16) = x;
                 }
+            } else {                                          // (rows behind a regular sequence's end are outside the map)
+                fence_proxy_async_smem();
+                named_bar_sync(1, 128);
+                if (leader && elect_one()) {
+                    tma_store_4d(&tm_out, sm + R_V + s * 16384, 0, hv, work.s_first + t0, work.b);
+                    tma_store_4d(&tm_out, sm + R_V + s * 16384 + 8192, 64, hv, work.s_first + t0, work.b);
+                    tma_store_commit();
+                    tma_store_wait_read();
+                    mbar_arrive_a(cb(R_OUT));
+                }
+                __syncwarp();
             }
         }
+        if (leader && elect_one()) tma_store_wait_all();
     } else {
         // ------------------------------- critical warps ----------------------------------------------------------------
         set_max_registers_up<88>();
@@ -530,8 +537,8 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 #pragma unroll
                 for (int j = 0; j < 8; j += 4) {
                     const float4 f = *reinterpret_cast<const float4*>(vec + 3 * kChunk + 32 * hf + 8 * u + j);
-                    pk[j / 2] = pack_bf16x2(__uint_as_float(x[j]) * f.x, __uint_as_float(x[j + 1]) * f.y);
-                    pk[j / 2 + 1] = pack_bf16x2(__uint_as_float(x[j + 2]) * f.z, __uint_as_float(x[j + 3]) * f.w);
+                    pk[j / 2] = mul_bf16x2(as_float2(x[j], x[j + 1]), make_float2(f.x, f.y));
+                    pk[j / 2 + 1] = mul_bf16x2(as_float2(x[j + 2], x[j + 3]), make_float2(f.z, f.w));
                 }
                 tmem_st_x4(a_ks + 4 * u, pk);
             }
@@ -557,8 +564,8 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 #pragma unroll
                 for (int c = 0; c < 4; c += 2) {
                     const float4 f = *reinterpret_cast<const float4*>(vec + 32 * hf + 8 * u + 2 * c);   // exp(gamma_C - gamma_j)
-                    pk[c] = pack_bf16x2(__uint_as_float(x[2 * c]) * f.x, __uint_as_float(x[2 * c + 1]) * f.y);
-                    pk[c + 1] = pack_bf16x2(__uint_as_float(x[2 * c + 2]) * f.z, __uint_as_float(x[2 * c + 3]) * f.w);
+                    pk[c] = mul_bf16x2(as_float2(x[2 * c], x[2 * c + 1]), make_float2(f.x, f.y));
+                    pk[c + 1] = mul_bf16x2(as_float2(x[2 * c + 2], x[2 * c + 3]), make_float2(f.z, f.w));
                 }
                 tmem_st_x4(tmem_addr(tmem, lane_base, C_VS + 16 * hf + 4 * u), pk);
             }
@@ -581,7 +588,11 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 tmem_ld_x16(a_s + (u >> 1) * 64 + (u & 1) * 16, x);
                 tmem_ld_wait();
 #pragma unroll
-                for (int c = 0; c < 16; ++c) st[16 * u + c] = fmaf(dC, st[16 * u + c], __uint_as_float(x[c]));
+                for (int c = 0; c < 16; c += 2) {
+                    const float2 y = fma2(make_float2(dC, dC), make_float2(st[16 * u + c], st[16 * u + c + 1]), as_float2(x[c], x[c + 1]));
+                    st[16 * u + c] = y.x;
+                    st[16 * u + c + 1] = y.y;
+                }
                 if (more) {
 #pragma unroll
                     for (int c = 0; c < 8; ++c) x[c] = pack_bf16x2(st[16 * u + 2 * c], st[16 * u + 2 * c + 1]);
@@ -639,7 +650,7 @@ int launch_chain_r(const Problem& p, const Workspace& ws, const TileMaps& maps, 
                 gy = static_cast<unsigned>(all - done < 65535 ? all - done : 65535);
             }
             if (launch_dependent(kernel, dim3(p.Hv, gy, gz), dim3(kRThreads), kRDynamic, stream, (p.Hv / p.Hq) % 2 == 0, map(maps.q), map(maps.k),
-                                 map(maps.v), map(maps.p), map(maps.t2), part, ws, static_cast<unsigned>(sm_count())) != cudaSuccess)
+                                 map(maps.v), map(maps.p), map(maps.t2), map(maps.out), part, ws, static_cast<unsigned>(sm_count())) != cudaSuccess)
                 return GDN_ERR_CUDA;
         }
         return GDN_OK;

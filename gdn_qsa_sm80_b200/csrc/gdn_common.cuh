@@ -111,14 +111,14 @@ int launch_chain(const Problem& p, const Workspace& ws, int nv, cudaStream_t str
 // The two kernels of the automatic path: "lean" prepare (P, T'', factors; no W) and the transposed chain that applies T'' to
 // the residual V - exp(gamma) K S, one CTA per (sequence, value head[, segment]); with ws.n_seg > 1 sequences may be cut
 // into up to that many segments (gdn_segment_plan.cuh).
-// TMA descriptors both of them read (128 bytes each, CUtensorMap): q, k, v as 64 x 64 boxes, P and T'' (at the start of the
+// TMA descriptors of both (128 bytes each, CUtensorMap): q, k, v and the outputs as 64 x 64 boxes, P and T'' (at the start of the
 // U array) as 32 x 32 boxes (64-byte swizzle): both are lower triangular, so a tile travels as its three blocks on and below
 // the diagonal and the fourth is neither written nor read (16 sequences of 2048 tokens: 391 -> 376 us per call, 64 of 4096
 // 2958 -> 2870 us).  Encoded once per call: each encoding costs the host 0.1-0.2
 // microseconds.
 constexpr uint32_t kTriBytes = 6144;   // a triangular tile in shared memory: rows 0-63 of columns 0-31, then rows 32-63 of columns 32-63
 struct alignas(64) TileMaps {
-    unsigned char q[128], k[128], v[128], p[128], t2[128];
+    unsigned char q[128], k[128], v[128], p[128], t2[128], out[128];
 };
 int encode_tile_maps(const Problem& p, const Workspace& ws, TileMaps& maps);
 int launch_prepare_lean(const Problem& p, const Workspace& ws, const TileMaps& maps, cudaStream_t stream);
