@@ -42,7 +42,7 @@ FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0}
 # dram__bytes_read.sum + dram__bytes_write.sum per step of the dominant kernel, from the ncu captures summarised under
 # profiles/ (workload, kernel) -> bytes; anything not listed is reported as null
 DRAM_TRAFFIC = {
-    ("default", "gdn_chain_r_kernel"): 293.9e6,
+    ("default", "gdn_chain_r_kernel"): 273.3e6,
     ("default", "gdn_chain_kernel"): 361.8e6,
     ("default", "gdn_coop_kernel"): 328.7e6,
 }
