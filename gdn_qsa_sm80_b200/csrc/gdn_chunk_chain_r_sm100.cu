@@ -57,7 +57,7 @@ constexpr int kRTimeout = 0x500;   // + the barrier's index
 
 // barriers
 enum : uint32_t { R_KFULL = 0, R_VFULL = 2, R_VEMPTY = 4, R_TFULL = 6, R_QFULL = 8, R_PFULL, R_KS, R_QS, R_X, R_VACC, R_VN, R_S, R_STATE,
-                  R_QSC, R_O, R_ODONE, R_OUT, kRBars };
+                  R_QSC, R_O, R_ODONE, R_OUT, R_STATE1, kRBars };
 
 // Byte offset, in a [64 tokens][128 dk] tile of two 64-column halves, of the 16 dk that k step `ks` of A_S holds (half ks / 4
 // of the warps packed the column blocks 32 h .. and 64 + 32 h ..).
@@ -136,7 +136,7 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     if (tid == 0) {
         for (uint32_t i = 0; i < kRBars; ++i) {
             const uint32_t count = i == R_VEMPTY || i == R_VEMPTY + 1 ? 12
-                                   : i == R_X || i == R_VN || i == R_STATE ? 8 : i == R_QSC || i == R_ODONE ? 4 : 1;
+                                   : i == R_X || i == R_VN || i == R_STATE || i == R_STATE1 ? 8 : i == R_QSC || i == R_ODONE ? 4 : 1;
             mbar_init(&bars[i], count);
         }
         work.late = 0;
@@ -339,12 +339,36 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             for (int n = 0; n < steps; ++n) {
                 const uint32_t s = n & 1;
                 if (!wait(R_KFULL + s, n >> 1)) break;
+                // E1.  Where sequences are split there are few of them and a step's length counts: the first four k steps begin when half of
+                // the state's copy is there, while the epilogue works on the rest.  us a call, before / after: 700 tokens 28.5 / 27.9; 2 x 1500,
+                // 8 / 8 heads 28.5 / 28.1; 2 x 2500, 8 / 16 heads 56.0 / 55.4; 4 x 1999 94.9 / 94.6; with many sequences nothing.
+                auto e1 = [&](int ks) {
+                    umma_bf16_ts(tmem + C_KS, tmem + C_S + ks * 8, r_desc(base + s * (16384 >> 4) + kLoK + ((R_K + dk_bytes(ks)) >> 4)), idesc_n64, ks > 0);
+                };
+                if (SPLIT) {
+                    if (!wait(R_STATE1, n)) break;
+                    tc_fence_after_sync();
+                    if (elect_one()) {
+                        e1(0);
+                        e1(1);
+                        e1(4);
+                        e1(5);
+                    }
+                    __syncwarp();
+                }
                 if (!wait(R_STATE, n)) break;
                 tc_fence_after_sync();
                 if (elect_one()) {
-#pragma unroll
-                    for (int ks = 0; ks < 8; ++ks)               // E1
-                        umma_bf16_ts(tmem + C_KS, tmem + C_S + ks * 8, r_desc(base + s * (16384 >> 4) + kLoK + ((R_K + dk_bytes(ks)) >> 4)), idesc_n64, ks > 0);
+                    if (!SPLIT) {
+                        e1(0);
+                        e1(1);
+                        e1(4);
+                        e1(5);
+                    }
+                    e1(2);
+                    e1(3);
+                    e1(6);
+                    e1(7);
                     umma_commit_a(cb(R_KS));
                 }
                 if (!wait(R_TFULL + s, n >> 1)) break;
@@ -519,7 +543,10 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         tmem_st_wait();
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive_a(cb(R_STATE));
+        if (lane == 0) {
+            if (SPLIT) mbar_arrive_a(cb(R_STATE1));
+            mbar_arrive_a(cb(R_STATE));
+        }
         bool ok = true;
         for (int n = 0; n < steps; ++n) {
             const uint32_t s = n & 1;
@@ -582,11 +609,18 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             tc_fence_after_sync();
             GDN_PHASE(4)
             const bool more = n + 1 < steps;
+            if (SPLIT && n + 2 == steps) clear_tail(n + 1);   // (before E1 reads the tile)
 #pragma unroll
             for (int u = 0; u < 4; ++u) {                     // S^T <- exp(gamma_C) S^T + v~^T K, 16 columns at a time
                 uint32_t x[16];
                 tmem_ld_x16(a_s + (u >> 1) * 64 + (u & 1) * 16, x);
                 tmem_ld_wait();
+                if (SPLIT && u == 2 && more) {                // the first two blocks' copies
+                    tmem_st_wait();
+                    tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_a(cb(R_STATE1));
+                }
 #pragma unroll
                 for (int c = 0; c < 16; c += 2) {
                     const float2 y = fma2(make_float2(dC, dC), make_float2(st[16 * u + c], st[16 * u + c + 1]), as_float2(x[c], x[c + 1]));
@@ -600,7 +634,7 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 }
             }
             if (more) {
-                if (n + 2 == steps) clear_tail(n + 1);
+                if (!SPLIT && n + 2 == steps) clear_tail(n + 1);
                 tmem_st_wait();
                 tc_fence_before_sync();
                 __syncwarp();
