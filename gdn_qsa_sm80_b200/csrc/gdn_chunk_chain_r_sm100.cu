@@ -56,7 +56,7 @@ constexpr uint32_t C_S = 0, C_VN = 64, C_KS = 128, C_VS = 128, C_VP = 160, C_O =
 constexpr int kRTimeout = 0x500;   // + the barrier's index
 
 // barriers
-enum : uint32_t { R_KFULL = 0, R_VFULL = 2, R_VEMPTY = 4, R_TFULL = 6, R_QFULL = 8, R_PFULL, R_KS, R_QS, R_X, R_VACC, R_VN, R_S, R_STATE,
+enum : uint32_t { R_KFULL = 0, R_VFULL = 2, R_VEMPTY = 4, R_TFULL = 6, R_QFULL = 8, R_PFULL, R_KS, R_QS, R_X, R_VACC, R_VN, R_S, R_STATE = R_S + 2,
                   R_QSC, R_O, R_ODONE, R_OUT, R_STATE1, kRBars };
 
 // Byte offset, in a [64 tokens][128 dk] tile of two 64-column halves, of the 16 dk that k step `ks` of A_S holds (half ks / 4
@@ -275,12 +275,20 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                     load_tri(sm_u32 + R_T2 + s * 8192, &tm_t2, fb, row0);
                 }
             };
+            auto dawdle = [&]() {                              // test hook: every barrier this role waits for is far ahead
+                if (p.dbg != kDbgLateProducer) return;
+                const unsigned long long t0 = globaltimer_ns();
+                while (globaltimer_ns() - t0 < 20000ull) {}
+            };
             load_k(0);
             load_t2(0);
             load_v(0);
-            // A slot's reload waits for the UMMA (or the epilogue) that read it.  The waits of one iteration are in the
-            // order in which those complete, and none of them can be overtaken by the next completion of the same
-            // barrier: that one needs a tile loaded later in the iteration.
+            // A slot's reload waits for the UMMA (or the epilogue) that read it, in the order in which those complete.  A wait names a parity,
+            // so the next completion of its barrier has to need a tile that is loaded behind it.  In iteration n:
+            //   R_S + slot of n - 1    next: E2 of n + 1, which needs K(n + 1), two lines below.  (One barrier for both slots would complete
+            //                          next with E2 of n, and a warm-up chunk n needs nothing of this iteration: it has no Q.)
+            //   R_O of n - 1           next: E3 of n, which needs P(n)
+            //   R_VEMPTY + slot        next: the epilogues of n + 1, which need V(n + 1)
             for (int n = 0; n < steps; ++n) {
                 // Alone on its SM, a CTA waits for tiles whose load a slot holds up (Q and P have one; a step is shorter than
                 // two HBM latencies under load), so what the next loads will read is brought into L2 first: 4 sequences of
@@ -302,7 +310,8 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                         prefetch_tri(&tm_t2, r1 + kChunk);
                     }
                 }
-                if (n > 0 && !wait(R_S, n - 1)) break;          // E2, hence also ER and E1', of chunk n - 1
+                dawdle();
+                if (n > 0 && !wait(R_S + ((n - 1) & 1), (n - 1) >> 1)) break;   // E2, hence also ER and E1', of chunk n - 1
                 if (n + 1 < steps) {
                     load_k(n + 1);
                     load_t2(n + 1);
@@ -405,7 +414,7 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 #pragma unroll
                     for (int ks = 0; ks < 4; ++ks)               // E2
                         umma_bf16_ts(tmem + C_S, tmem + C_VS + ks * 8, r_desc(base + s * (16384 >> 4) + kLoMN + ((R_K + ks * 2048) >> 4)), idesc_e2, ks > 0);
-                    umma_commit_a(cb(R_S));
+                    umma_commit_a(cb(R_S + s));
                 }
                 if (n < from) continue;
                 if (!wait(R_PFULL, n - from)) break;
@@ -604,7 +613,7 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 mbar_arrive_a(cb(R_VEMPTY + s));
             }
             GDN_PHASE(3)
-            ok = wait(R_S, n);
+            ok = wait(R_S + s, n >> 1);
             if (!ok) break;
             tc_fence_after_sync();
             GDN_PHASE(4)

@@ -21,6 +21,9 @@ constexpr int kD = 128;      // head dimension (keys and values)
 constexpr int kChunk = 64;   // tokens per chunk
 constexpr float kLog2e = 1.4426950408889634f;
 
+// Test hooks of Problem::dbg (7: gdn_chunk_coop_sm100.cu)
+constexpr int kDbgLateProducer = 8;    // residual-form chain: the TMA producer sleeps 20 us before it looks at a barrier
+
 struct Problem {
     const __nv_bfloat16* q;
     const __nv_bfloat16* k;
@@ -37,7 +40,7 @@ struct Problem {
     int gate_act;          // 1: g and beta hold raw values; the kernels apply g = -softplus(.), beta = sigmoid(.)
     int l2norm;            // 1: q and k are L2-normalised per head vector inside the kernels
     int clear_status;      // 1: the launch's first kernel clears the status word
-    int dbg;               // experiment switch (environment variable GDN_CHUNK_DBG); 0 in production
+    int dbg;               // test hook (environment variable GDN_CHUNK_DBG); 0 in production
     // Packed batch (residual-form kernels only; null / 0 otherwise): B = 1, S = all tokens, sequences laid end to end
     const int* pk_cu;      // [pk_n + 1] first token of each sequence
     const int2* pk_chunk;  // [pk_chunks] (sequence, chunk within it), sequences in order

@@ -1,0 +1,29 @@
+"""Waits of the chunked kernels under conditions that timing alone does not produce (test hooks, environment variable GDN_CHUNK_DBG)."""
+
+import pytest
+import torch
+
+from gdn_qsa_sm80 import gdn_chunk
+from gdn_qsa_sm80_b200.gdn_chunk_interface import check_device_status
+from gdn_qsa_sm80_b200.synthetic import make_inputs
+
+pytestmark = pytest.mark.gpu
+
+LATE_PRODUCER = "8"
+
+
+def inputs(workload, **sizes):
+    return [t.cuda() for t in make_inputs(workload, seed=3, **sizes)[:5]]
+
+
+@pytest.mark.parametrize("workload,S", [("default", 2000), ("default", 1984), ("long_context", 8000)])   # warm-ups of about 5 and 23 chunks
+def test_a_late_producer_is_not_overtaken_in_warm_up_chunks(workload, S, monkeypatch):
+    """A wait names the parity of a barrier's phase: a role that comes to it after two of them waits for a third.  Chunks without
+    outputs need nothing that the producer loads behind its wait for the chunk before."""
+    d = inputs(workload, S=S, Hq=1, Hv=2)
+    out, st = gdn_chunk(*d)
+    check_device_status()
+    monkeypatch.setenv("GDN_CHUNK_DBG", LATE_PRODUCER)
+    late, st_late = gdn_chunk(*d)
+    check_device_status()
+    assert torch.equal(out, late) and torch.equal(st, st_late)
