@@ -57,7 +57,7 @@ constexpr int kRTimeout = 0x500;   // + the barrier's index
 
 // barriers
 enum : uint32_t { R_KFULL = 0, R_VFULL = 2, R_VEMPTY = 4, R_TFULL = 6, R_QFULL = 8, R_PFULL, R_KS, R_QS, R_X, R_VACC, R_VN, R_S, R_STATE = R_S + 2,
-                  R_QSC, R_O, R_ODONE, R_OUT, R_STATE1, kRBars };
+                  R_QSC, R_O, R_ODONE, R_OUT, R_STATE1 = R_OUT + 2, kRBars };
 
 // Byte offset, in a [64 tokens][128 dk] tile of two 64-column halves, of the 16 dk that k step `ks` of A_S holds (half ks / 4
 // of the warps packed the column blocks 32 h .. and 64 + 32 h ..).
@@ -288,7 +288,8 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             //   R_S + slot of n - 1    next: E2 of n + 1, which needs K(n + 1), two lines below.  (One barrier for both slots would complete
             //                          next with E2 of n, and a warm-up chunk n needs nothing of this iteration: it has no Q.)
             //   R_O of n - 1           next: E3 of n, which needs P(n)
-            //   R_VEMPTY + slot        next: the epilogues of n + 1, which need V(n + 1)
+            //   R_VEMPTY, R_OUT + slot of n - 1    next: the epilogues and the outputs of n + 1, which need V(n + 1).  (All that chunk n's outputs
+            //                          need has been loaded by then.)
             for (int n = 0; n < steps; ++n) {
                 // Alone on its SM, a CTA waits for tiles whose load a slot holds up (Q and P have one; a step is shorter than
                 // two HBM latencies under load), so what the next loads will read is brought into L2 first: 4 sequences of
@@ -324,6 +325,7 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                         tma_load_4d_a(sm_u32 + R_Q, &tm_q, cb(R_QFULL), 0, hq, s0, b);
                         tma_load_4d_a(sm_u32 + R_Q + 8192, &tm_q, cb(R_QFULL), 64, hq, s0, b);
                     }
+                    dawdle();
                     if (n > from && !wait(R_O, n - from - 1)) break;
                     if (elect_one()) {
                         mbar_arrive_expect_tx_a(cb(R_PFULL), kTriBytes);
@@ -331,8 +333,9 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                     }
                 }
                 if (n + 1 < steps) {
+                    dawdle();
                     if (n > 0 && !wait(R_VEMPTY + ((n + 1) & 1), ((n + 1) >> 1) - 1)) break;
-                    if (n > from && !wait(R_OUT, n - from - 1)) break;   // the outputs of chunk n - 1, staged in its V's place, have left
+                    if (n > from && !wait(R_OUT + ((n - 1) & 1), (n - from - 1) >> 1)) break;   // the outputs of chunk n - 1, staged in its V's place, have left
                     load_v(n + 1);
                 }
             }
@@ -508,7 +511,7 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                     tma_store_4d(&tm_out, sm + R_V + s * 16384 + 8192, 64, hv, work.s_first + t0, work.b);
                     tma_store_commit();
                     tma_store_wait_read();
-                    mbar_arrive_a(cb(R_OUT));
+                    mbar_arrive_a(cb(R_OUT + s));
                 }
                 __syncwarp();
             }

@@ -27,3 +27,15 @@ def test_a_late_producer_is_not_overtaken_in_warm_up_chunks(workload, S, monkeyp
     late, st_late = gdn_chunk(*d)
     check_device_status()
     assert torch.equal(out, late) and torch.equal(st, st_late)
+
+
+@pytest.mark.parametrize("B,S", [(1, 64 * 9), (2, 150), (1, 65), (200, 200)])
+def test_a_late_producer_is_not_overtaken_by_the_outputs(B, S, monkeypatch):
+    """All that a chunk's outputs need has been loaded when the producer waits for those of the chunk before to leave."""
+    d = inputs("default", B=B, S=S, Hq=1, Hv=2)
+    out, st = gdn_chunk(*d)
+    check_device_status()
+    monkeypatch.setenv("GDN_CHUNK_DBG", LATE_PRODUCER)
+    late, st_late = gdn_chunk(*d)
+    check_device_status()
+    assert torch.equal(out, late) and torch.equal(st, st_late)
