@@ -282,7 +282,7 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             };
             load_k(0);
             load_t2(0);
-            load_v(0);
+            if (p.dbg != kDbgNoTile) load_v(0);
             // A slot's reload waits for the UMMA (or the epilogue) that read it, in the order in which those complete.  A wait names a parity,
             // so the next completion of its barrier has to need a tile that is loaded behind it.  In iteration n:
             //   R_S + slot of n - 1    next: E2 of n + 1, which needs K(n + 1), two lines below.  (One barrier for both slots would complete

@@ -172,7 +172,7 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     bool ok = true;
     if (warp == 0) {
         ok = wait(&bar_tma, 0, kDevTimeoutTma);
-        if (ok && elect_one()) issue_product(tmem);
+        if (ok && p.dbg != kDbgNoProduct && elect_one()) issue_product(tmem);
     }
 
     for (; n < num_items; n += gridDim.x) {

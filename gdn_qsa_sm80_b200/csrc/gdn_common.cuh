@@ -23,6 +23,8 @@ constexpr float kLog2e = 1.4426950408889634f;
 
 // Test hooks of Problem::dbg (7: gdn_chunk_coop_sm100.cu)
 constexpr int kDbgLateProducer = 8;    // residual-form chain: the TMA producer sleeps 20 us before it looks at a barrier
+constexpr int kDbgNoTile = 10;         // residual-form chain: the first tile of V is never announced
+constexpr int kDbgNoProduct = 11;      // lean prepare: no CTA's first product is issued
 
 struct Problem {
     const __nv_bfloat16* q;

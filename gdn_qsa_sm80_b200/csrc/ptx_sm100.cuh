@@ -162,17 +162,18 @@ __device__ __forceinline__ bool mbar_wait_abortable_a(uint32_t bar, uint32_t par
     }
 }
 
-// The same wait where several roles of a kernel run at once: five instructions in a loop and no slow path, which at some twenty places
-// of a kernel took a quarter of its code (53 -> 44 KB in the residual-form chain, 1878 -> 518 requests of an SM to the second
-// instruction cache over 33 chunk steps).  16 million tries end it, each of which suspends for a while: between a fifth of a second
-// and a few.  The caller reports the code.
+// Wait of the lean prepare kernel and the residual-form chain: five instructions in a loop, no status word, no abort flag.  An inline slow
+// path at some twenty places of a kernel took a quarter of its code (53 -> 44 KB in the chain, 1878 -> 518 requests of an SM to the second
+// instruction cache over 33 chunk steps).  The limit is a number of tries: one on a barrier that does not complete suspends its warp for
+// 3.96 us, whatever else runs (1 to 592 CTAs, 1 to 16 warps in each: 3.96-3.98), so half a million are the two seconds of WAIT_LIMIT_NS.
+// The caller reports the code.
 __device__ __forceinline__ bool mbar_wait_compact(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
         "{\n\t"
         ".reg .pred p, q;\n\t"
         ".reg .u32 n;\n\t"
-        "mov.u32 n, 16000000;\n"
+        "mov.u32 n, 500000;\n"
         "WAIT:\n\t"
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "@p bra DONE;\n\t"

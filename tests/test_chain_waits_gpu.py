@@ -1,15 +1,18 @@
 """Waits of the chunked kernels under conditions that timing alone does not produce (test hooks, environment variable GDN_CHUNK_DBG)."""
 
+import time
+
 import pytest
 import torch
 
 from gdn_qsa_sm80 import gdn_chunk
+from gdn_qsa_sm80_b200 import _lib
 from gdn_qsa_sm80_b200.gdn_chunk_interface import check_device_status
 from gdn_qsa_sm80_b200.synthetic import make_inputs
 
 pytestmark = pytest.mark.gpu
 
-LATE_PRODUCER = "8"
+LATE_PRODUCER, NO_TILE, NO_PRODUCT = "8", "10", "11"
 
 
 def inputs(workload, **sizes):
@@ -39,3 +42,22 @@ def test_a_late_producer_is_not_overtaken_by_the_outputs(B, S, monkeypatch):
     late, st_late = gdn_chunk(*d)
     check_device_status()
     assert torch.equal(out, late) and torch.equal(st, st_late)
+
+
+@pytest.mark.parametrize("hook,path,code", [(NO_TILE, "auto", "0x502"), (NO_PRODUCT, "prepare_only_t", "0x102")])
+@pytest.mark.parametrize("Hq,Hv", [(1, 2), (3, 3)])
+def test_a_wait_that_runs_out_is_reported_and_the_next_call_succeeds(hook, path, code, Hq, Hv, monkeypatch):
+    """Two seconds, as everywhere: the first tile of V (or the first product) never comes and whoever needs it gives up."""
+    d = inputs("default", S=40, Hq=Hq, Hv=Hv)
+    out, st = gdn_chunk(*d)
+    check_device_status()
+    monkeypatch.setenv("GDN_CHUNK_DBG", hook)
+    t0 = time.time()
+    gdn_chunk(*d, path=path)
+    with pytest.raises(_lib.GdnLibraryError, match=code):
+        check_device_status()
+    assert 1.5 < time.time() - t0 < 5.0      # all roles wait at the same time
+    monkeypatch.delenv("GDN_CHUNK_DBG")
+    again, st_again = gdn_chunk(*d)
+    check_device_status()
+    assert torch.equal(out, again) and torch.equal(st, st_again)
