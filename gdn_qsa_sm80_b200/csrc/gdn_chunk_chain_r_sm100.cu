@@ -57,7 +57,7 @@ constexpr int kRTimeout = 0x500;   // + the barrier's index
 
 // barriers
 enum : uint32_t { R_KFULL = 0, R_VFULL = 2, R_VEMPTY = 4, R_TFULL = 6, R_QFULL = 8, R_PFULL, R_KS, R_QS, R_X, R_VACC, R_VN, R_S, R_STATE = R_S + 2,
-                  R_QSC, R_O, R_ODONE, R_OUT, R_STATE1 = R_OUT + 2, kRBars };
+                  R_QSC, R_O, R_ODONE, R_OUT, R_STATE1 = R_OUT + 2, R_NEVER /* test hook */, kRBars };
 
 // Byte offset, in a [64 tokens][128 dk] tile of two 64-column halves, of the 16 dk that k step `ks` of A_S holds (half ks / 4
 // of the warps packed the column blocks 32 h .. and 64 + 32 h ..).
@@ -113,7 +113,7 @@ __device__ __forceinline__ void set_max_registers_up() { asm volatile("setmaxnre
 template <int N>
 __device__ __forceinline__ void set_max_registers_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
-template <bool SPLIT>
+template <bool SPLIT, bool HOOKS>
 __global__ void __launch_bounds__(kRThreads, 2)
 gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_p,
@@ -276,13 +276,13 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 }
             };
             auto dawdle = [&]() {                              // test hook: every barrier this role waits for is far ahead
-                if (p.dbg != kDbgLateProducer) return;
+                if (!HOOKS || p.dbg != kDbgLateProducer) return;
                 const unsigned long long t0 = globaltimer_ns();
                 while (globaltimer_ns() - t0 < 20000ull) {}
             };
             load_k(0);
             load_t2(0);
-            if (p.dbg != kDbgNoTile) load_v(0);
+            if (!HOOKS || p.dbg != kDbgNoTile) load_v(0);
             // A slot's reload waits for the UMMA (or the epilogue) that read it, in the order in which those complete.  A wait names a parity,
             // so the next completion of its barrier has to need a tile that is loaded behind it.  In iteration n:
             //   R_S + slot of n - 1    next: E2 of n + 1, which needs K(n + 1), two lines below.  (One barrier for both slots would complete
@@ -438,6 +438,7 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         const uint32_t lane_base = static_cast<uint32_t>(warp & 3) * 32u;
         const uint32_t o_addr = tmem_addr(tmem, lane_base, C_O);
         const bool leader = warp == 8;
+        const uint32_t o_bar = HOOKS && p.dbg == kDbgWarpGivesUp && warp == 9 ? R_NEVER : R_O;
         // Row (token) whose address this lane gives to stmatrix, and its 16-byte chunk (8 value columns) before the swizzle; the warp's 32
         // value columns lie in one of the two halves of 64 columns.
         const uint32_t srow = 8 * (lane >> 4) + (lane & 7), sch = 4 * (warp & 1) + ((lane >> 3) & 1);
@@ -476,7 +477,13 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 mbar_arrive_a(cb(R_QSC));
                 mbar_arrive_a(cb(R_VEMPTY + s));
             }
-            if (!wait(R_O, n - from)) break;
+            // The barrier below has no limit, so a warp whose tries run out here still takes part in it.  Whoever gets there has seen E3, hence
+            // the arrivals of all four warps on R_QSC: none of them can have left earlier, and none gets to the next chunk's without the R_ODONE of
+            // all.  (An mbarrier waited for with a limit: 700 tokens 26.3 -> 27.2 us a call.)
+            if (!wait(o_bar, n - from)) {
+                named_bar_arrive(1, 128);
+                break;
+            }
             tc_fence_after_sync();
             // O^T[dv][j] in fragments of 16 value columns by 32 tokens, transposed on their way into the place of V (E0 has read it)
 #pragma unroll
@@ -702,8 +709,9 @@ int launch_chain_r(const Problem& p, const Workspace& ws, const TileMaps& maps, 
         return GDN_OK;
     };
     const int G = ws.n_seg;
-    if (G <= 1 || G > kMaxSegments || !ws.meta) return go(gdn_chain_r_kernel<false>, 1);
-    return go(gdn_chain_r_kernel<true>, p.pk_chunk ? 1u : static_cast<unsigned>(G));
+    if (G <= 1 || G > kMaxSegments || !ws.meta) return p.dbg ? go(gdn_chain_r_kernel<false, true>, 1) : go(gdn_chain_r_kernel<false, false>, 1);
+    const unsigned gz = p.pk_chunk ? 1u : static_cast<unsigned>(G);
+    return p.dbg ? go(gdn_chain_r_kernel<true, true>, gz) : go(gdn_chain_r_kernel<true, false>, gz);
 }
 
 }  // namespace gdn

@@ -193,6 +193,10 @@ __device__ __forceinline__ bool mbar_wait_compact(uint32_t bar, uint32_t parity)
 __device__ __forceinline__ void named_bar_sync(uint32_t id, uint32_t count) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
+// Takes part in one without waiting for the others.
+__device__ __forceinline__ void named_bar_arrive(uint32_t id, uint32_t count) {
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
 
 // 1-D bulk copy global -> shared (16-byte aligned addresses, size a multiple of 16), completing on an mbarrier.
 __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {

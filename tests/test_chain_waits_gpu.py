@@ -12,7 +12,7 @@ from gdn_qsa_sm80_b200.synthetic import make_inputs
 
 pytestmark = pytest.mark.gpu
 
-LATE_PRODUCER, NO_TILE, NO_PRODUCT = "8", "10", "11"
+LATE_PRODUCER, WARP_GIVES_UP, NO_TILE, NO_PRODUCT = "8", "9", "10", "11"
 
 
 def inputs(workload, **sizes):
@@ -57,6 +57,25 @@ def test_a_wait_that_runs_out_is_reported_and_the_next_call_succeeds(hook, path,
     with pytest.raises(_lib.GdnLibraryError, match=code):
         check_device_status()
     assert 1.5 < time.time() - t0 < 5.0      # all roles wait at the same time
+    monkeypatch.delenv("GDN_CHUNK_DBG")
+    again, st_again = gdn_chunk(*d)
+    check_device_status()
+    assert torch.equal(out, again) and torch.equal(st, st_again)
+
+
+@pytest.mark.parametrize("S", [40, 64, 300])
+def test_an_output_warp_that_gives_up_holds_up_the_others_for_a_limited_time(S, monkeypatch):
+    """Each output warp counts its own tries, so one may leave while the others still see the barrier complete; they meet at a barrier
+    without a limit when a chunk's outputs are staged."""
+    d = inputs("default", S=S, Hq=1, Hv=2)
+    out, st = gdn_chunk(*d)
+    check_device_status()
+    monkeypatch.setenv("GDN_CHUNK_DBG", WARP_GIVES_UP)
+    t0 = time.time()
+    gdn_chunk(*d)
+    with pytest.raises(_lib.GdnLibraryError, match="0x5"):
+        check_device_status()
+    assert 1.5 < time.time() - t0 < 9.0      # its wait, then those of the others for the next chunk
     monkeypatch.delenv("GDN_CHUNK_DBG")
     again, st_again = gdn_chunk(*d)
     check_device_status()
