@@ -73,7 +73,7 @@ struct RWork {
     const float* s_in;                     // state it starts from (null: zeros) and where the one it ends with goes
     float* s_out;
     int* status;
-    int late;                              // code of a wait that ran out
+    int late;                              // code of the first wait that ran out
 };
 
 // Shared-memory descriptor of this file's operands: 1024 bytes between 8-row groups and the 128-byte swizzle throughout, so
@@ -98,7 +98,7 @@ constexpr uint32_t kLoK = (16u >> 4) << 16, kLoMN = (8192u >> 4) << 16;
 // 4 x 1999 104.0 / 102.2, 8192 100.1 / 98.7; nothing where HBM bounds it.
 __device__ __forceinline__ bool r_wait(uint32_t bar, uint32_t parity, int code, RWork& work) {
     if (mbar_wait_compact(bar, parity)) return true;
-    work.late = code;
+    atomicCAS(&work.late, 0, code);
     return false;
 }
 

@@ -66,14 +66,15 @@ def test_a_wait_that_runs_out_is_reported_and_the_next_call_succeeds(hook, path,
 @pytest.mark.parametrize("S", [40, 64, 300])
 def test_an_output_warp_that_gives_up_holds_up_the_others_for_a_limited_time(S, monkeypatch):
     """Each output warp counts its own tries, so one may leave while the others still see the barrier complete; they meet at a barrier
-    without a limit when a chunk's outputs are staged."""
+    without a limit when a chunk's outputs are staged.  What is reported is a wait that ran out first, not one behind it (0x50b: of the
+    others, for the next chunk)."""
     d = inputs("default", S=S, Hq=1, Hv=2)
     out, st = gdn_chunk(*d)
     check_device_status()
     monkeypatch.setenv("GDN_CHUNK_DBG", WARP_GIVES_UP)
     t0 = time.time()
     gdn_chunk(*d)
-    with pytest.raises(_lib.GdnLibraryError, match="0x5"):
+    with pytest.raises(_lib.GdnLibraryError, match="0x5(?!0b)"):
         check_device_status()
     assert 1.5 < time.time() - t0 < 9.0      # its wait, then those of the others for the next chunk
     monkeypatch.delenv("GDN_CHUNK_DBG")
