@@ -69,10 +69,10 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     // Persistent CTA: items blockIdx.x, blockIdx.x + gridDim.x, ...; the head group index is the fastest, so the groups
     // that share a qk head are prepared at about the same time.
     struct Item { int b, hv, hq, s0, valid; size_t tok0, tile; };
-    int late = 0;                                 // code of a wait that ran out
+    int late = 0;                                 // code of this thread's first wait that ran out
     auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
         if (mbar_wait_compact(smem_u32(bar), parity)) return true;
-        late = code;
+        if (late == 0) late = code;
         return false;
     };
     auto decode = [&](unsigned n) {
@@ -170,6 +170,7 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     const uint32_t lane_base = static_cast<uint32_t>(hwarp) * 32u;   // (warp % 4) * 32: the warp's TMEM lane quadrant
     uint32_t ph = 0;            // parity of both barriers: one load and one product per item
     bool ok = true;
+    if (p.dbg == kDbgLaneGivesUp && tid == 5) late = kDevTimeoutTma;
     if (warp == 0) {
         ok = wait(&bar_tma, 0, kDevTimeoutTma);
         if (ok && p.dbg != kDbgNoProduct && elect_one()) issue_product(tmem);
@@ -265,7 +266,7 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         for (int k = 0; k < 8; ++k) p.prof[k] = prof_acc[k];
         p.prof[15] = prof_n;
     }
-    if (late && lane == 0) atomicCAS(p.status, 0, late);
+    if (late) atomicCAS(p.status, 0, late);       // (each lane counts its own tries)
     // Only now may the chain kernel's CTAs start (and set up while the last CTAs of this grid finish): let in earlier, they
     // pile up two to an SM on the SMs that this grid leaves first while others stay empty.
     grid_launch_dependents();

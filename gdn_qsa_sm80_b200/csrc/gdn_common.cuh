@@ -27,6 +27,7 @@ constexpr int kDbgLateProducer = 8;    // residual-form chain: the TMA producer 
 constexpr int kDbgWarpGivesUp = 9;     // residual-form chain: one of the output warps waits for a barrier that nothing completes instead of the first outputs
 constexpr int kDbgNoTile = 10;         // residual-form chain: the first tile of V is never announced
 constexpr int kDbgNoProduct = 11;      // lean prepare: no CTA's first product is issued
+constexpr int kDbgLaneGivesUp = 12;    // lean prepare: one lane of each CTA that is not its warp's first has given up
 
 struct Problem {
     const __nv_bfloat16* q;

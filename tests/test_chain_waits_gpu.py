@@ -12,7 +12,7 @@ from gdn_qsa_sm80_b200.synthetic import make_inputs
 
 pytestmark = pytest.mark.gpu
 
-LATE_PRODUCER, WARP_GIVES_UP, NO_TILE, NO_PRODUCT = "8", "9", "10", "11"
+LATE_PRODUCER, WARP_GIVES_UP, NO_TILE, NO_PRODUCT, LANE_GIVES_UP = "8", "9", "10", "11", "12"
 
 
 def inputs(workload, **sizes):
@@ -81,3 +81,16 @@ def test_an_output_warp_that_gives_up_holds_up_the_others_for_a_limited_time(S, 
     again, st_again = gdn_chunk(*d)
     check_device_status()
     assert torch.equal(out, again) and torch.equal(st, st_again)
+
+
+@pytest.mark.parametrize("Hq,Hv", [(1, 2), (3, 3)])
+def test_a_single_lane_that_gave_up_is_reported(Hq, Hv, monkeypatch):
+    """Each lane counts its own tries; the prepare kernel's CTA leaves when any of them has run out."""
+    d = inputs("default", S=40, Hq=Hq, Hv=Hv)
+    monkeypatch.setenv("GDN_CHUNK_DBG", LANE_GIVES_UP)
+    gdn_chunk(*d, path="prepare_only_t")
+    with pytest.raises(_lib.GdnLibraryError, match="0x101"):
+        check_device_status()
+    monkeypatch.delenv("GDN_CHUNK_DBG")
+    gdn_chunk(*d)
+    check_device_status()
