@@ -125,42 +125,6 @@ __device__ __forceinline__ void mbar_arrive_a(uint32_t bar) {
 __device__ __forceinline__ void mbar_arrive_expect_tx_a(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait_a(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t"
-        "}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait_abortable_a(uint32_t bar, uint32_t parity, int* status, int code,
-                                                      volatile int* abort_flag) {
-    // the barrier first: the abort flag costs a shared-memory round trip, which a wait on the critical path of a
-    // recurrence pays every time; a thread that runs one step past an abort only computes on stale data, and the
-    // status word already says so
-#pragma unroll 1
-    for (int i = 0; i < 128; ++i)
-        if (mbar_try_wait_a(bar, parity)) return true;
-    if (*abort_flag) return false;
-    const unsigned long long t0 = globaltimer_ns();
-#pragma unroll 1
-    while (true) {
-#pragma unroll 1
-        for (int i = 0; i < 256; ++i)
-            if (mbar_try_wait_a(bar, parity)) return true;
-        if (*abort_flag) return false;
-        if (globaltimer_ns() - t0 > WAIT_LIMIT_NS) {
-            atomicCAS(status, 0, code);
-            *abort_flag = 1;
-            return false;
-        }
-    }
-}
 
 // Wait of the lean prepare kernel and the residual-form chain: five instructions in a loop, no status word, no abort flag.  An inline slow
 // path at some twenty places of a kernel took a quarter of its code (53 -> 44 KB in the chain, 1878 -> 518 requests of an SM to the second
