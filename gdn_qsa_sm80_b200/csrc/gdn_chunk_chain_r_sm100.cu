@@ -29,7 +29,7 @@
 // are staged where its V was and leave by TMA.  Two-byte stores by the lanes cost the output warps 190 instructions a chunk, two thirds
 // of what they issue, and these share the issue slots of the critical warps (24.0 -> 20.0 million instructions on 4 x 2048 tokens, 32
 // heads, with the paired arithmetic of the other epilogues).  us a call, before / after: 8192 tokens 97.2 / 91.8, 4 x 1999 101.7 / 95.0,
-// 16 x 2048 322 / 310, 64 x 4096 2700 / 2580, 131072 tokens 1460 / 1380.  (Staged in Q's place, whose next tile is wanted a step earlier
+// 16 x 2048 322 / 310, 64 x 4096 2700 / 2580, 131072 tokens 1460 / 1380; the paired arithmetic alone is 0 to 1 % of it.  (Staged in Q's place, whose next tile is wanted a step earlier
 // than V's, 8192 tokens took 104.)
 //
 // Roles (16 warps): 0-7 critical (warp w: TMEM lane quadrant w % 4, column half w / 4): X, v_new and state epilogues,
@@ -93,7 +93,7 @@ __device__ __forceinline__ uint64_t r_desc64(uint32_t lo) {   // triangular tile
 __device__ constexpr uint32_t tri_bytes(int ks) { return (ks >> 1) * 4096 + (ks & 1) * 32; }
 constexpr uint32_t kLoK = (16u >> 4) << 16, kLoMN = (8192u >> 4) << 16;
 
-// Bounded wait; a role whose wait ran out leaves, the others' waits run out behind it, and the CTA reports at its end.  With the inline
+// Bounded wait; a role whose wait ran out leaves, the others' waits run out behind it, and the CTA reports the first at its end.  With the inline
 // slow path of mbar_wait at 25 places (before / after, us a call): 2 x 1500 tokens, 8 / 8 heads 29.8 / 28.6, 333 tokens 21.5 / 20.9,
 // 4 x 1999 104.0 / 102.2, 8192 100.1 / 98.7; nothing where HBM bounds it.
 __device__ __forceinline__ bool r_wait(uint32_t bar, uint32_t parity, int code, RWork& work) {
@@ -352,8 +352,8 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 const uint32_t s = n & 1;
                 if (!wait(R_KFULL + s, n >> 1)) break;
                 // E1.  Where sequences are split there are few of them and a step's length counts: the first four k steps begin when half of
-                // the state's copy is there, while the epilogue works on the rest.  us a call, before / after: 700 tokens 28.5 / 27.9; 2 x 1500,
-                // 8 / 8 heads 28.5 / 28.1; 2 x 2500, 8 / 16 heads 56.0 / 55.4; 4 x 1999 94.9 / 94.6; with many sequences nothing.
+                // the state's copy is there, while the epilogue works on the rest.  us a call, before / after: 700 tokens 27.0 / 26.4; 2 x 1500,
+                // 8 / 8 heads 27.5 / 27.1; 2 x 2500, 8 / 16 heads 42.1 / 41.6; 4 x 1999 98.1 / 97.6, within the noise; with many sequences nothing.
                 auto e1 = [&](int ks) {
                     umma_bf16_ts(tmem + C_KS, tmem + C_S + ks * 8, r_desc(base + s * (16384 >> 4) + kLoK + ((R_K + dk_bytes(ks)) >> 4)), idesc_n64, ks > 0);
                 };

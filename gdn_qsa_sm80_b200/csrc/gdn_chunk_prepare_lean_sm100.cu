@@ -70,7 +70,7 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     // that share a qk head are prepared at about the same time.
     struct Item { int b, hv, hq, s0, valid; size_t tok0, tile; };
     int late = 0;                                 // code of this thread's first wait that ran out
-    auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
+    auto wait = [&](uint64_t* bar, uint32_t parity, int code) {   // (mbar_wait: 16 x 2048 tokens 125.8 us against 123.7, 8192 36.8 / 36.1)
         if (mbar_wait_compact(smem_u32(bar), parity)) return true;
         if (late == 0) late = code;
         return false;

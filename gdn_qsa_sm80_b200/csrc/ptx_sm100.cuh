@@ -2,7 +2,7 @@
 // mbarrier, TMA tile loads, tcgen05 (TMEM allocation, UMMA issue/commit, TMEM loads),
 // plus the shared-memory operand layouts and descriptors that go with them.
 //
-// Every spin-wait here is bounded: a wait that does not complete within WAIT_LIMIT_NS (or a number of tries)
+// Every spin-wait here is bounded: a wait that does not complete within WAIT_LIMIT_NS (or as many tries)
 // returns false and a code is recorded in a global status word, so a protocol bug ends
 // the kernel with an error instead of hanging the GPU.
 #pragma once

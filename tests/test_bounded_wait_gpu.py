@@ -1,6 +1,7 @@
 """A device-side wait that nothing satisfies must end by itself and be reported, and the GPU must stay usable.
 
-Every wait inside the kernels (mbarrier phases, tile flags written by other CTAs) is bounded (2 s).  Here the
+Every wait inside the kernels (mbarrier phases, tile flags written by other CTAs) is bounded (2 s).  (Those of the two-kernel path have a form of their
+own: test_chain_waits_gpu.py.)  Here the
 single-launch kernel runs with its prepare roles switched off and no tile flag raised (a test hook), so each chain
 CTA's first wait runs out: the kernel sets the status word, drains and returns; the host sees GDN_ERR_DEVICE through
 the status read; the next ordinary call works and gives the right result.  No fault, no trap, no endless loop.
