@@ -9,11 +9,16 @@
 // csrc/gdn_chunk/gdn_kernel.cu:385-387): one K / Q load and one [K;Q] K^T product, then one half of the CTA per head.
 // HEADS = 1 (odd number of value heads per qk head): one head per CTA of 128 threads.
 //
-// What bounds it is latency: an item is a chain of dependent phases (product, mask, triangular inverse, T''), so what
-// counts is how many items an SM has in flight.  A and T share one fp32 array (gdn_prep_lean_device.cuh) and K / Q are
-// dead after the product, so a CTA needs 73 KB and 80 registers and three of them (24 warps) fit an SM; the next item's
-// K is loaded as soon as this item's product is done, its Q as soon as P's staging tiles (in Q's place) have been read
-// by their TMA store, and its product is issued, into a second accumulator, before this item's T'' is written.
+// The four warps of a head are roles that run several items apart, each with its own part of a chain of dependent phases (product, masks, triangular inverse,
+// T''): a phase is some hundred instructions that wait for one another, and what an SM gets done is decided by how many of its 24 warps have one to issue.
+//   role 0, 1   the two 32x32 diagonal blocks of T (lean_diagonal), item i; role 1 also the mask of A below them
+//   role 2      tiles and product of item i + 1; P, rows 0-31, of item i; T'' below the diagonal blocks, left half, of item i - 1
+//   role 3      gates and tables of item i + 1; P, rows 32-63, of item i; T'' below the diagonal blocks, right half, of item i - 1
+// All four at the same item, with barriers of the head between the phases, left a quarter of the warps' time at them.
+//
+// What bounds it: the shared-memory pipe (16 sequences of 2048 tokens: 56 % of the cycles for loads and stores, about 25 % for operands and copies), then HBM (29 KB
+// per chunk and head).  us alone, against the form that passed A and T through shared memory row by row and ran its phases in step: 16 x 2048 124 / 96, 8192 tokens
+// 36.3 / 29.8, 4 x 1999 36.3 / 29.6 (with L2 normalisation 41.8 / 38.9), 64 x 4096 941 / 744; 16 x 2048 with 16 / 16 heads 81.5 / 65.4.
 // Stands in for the reference's gdn_prepare_kernel (csrc/gdn_chunk/gdn_kernel.cu:343-710).
 #include <cuda.h>
 
@@ -29,15 +34,31 @@ namespace {
 template <int HEADS>
 struct LeanSmem {
     static constexpr uint32_t KQ = 0;                    // [K;Q]: 2 k-halves x 128 rows x 128 B (K rows 0-63, Q rows 64-127);
-                                                         //   P staging of head h in Q's rows of k-half h once the product is done
-    static constexpr uint32_t AT = 32768;                // A, then T, fp32 64 x 68, of head h at AT + h * 17408; then its T'' staging
-    static constexpr uint32_t kBytes = AT + HEADS * 17408;
+                                                         //   P of head h on its way out in Q's rows of k-half h once the product is done
+    static constexpr uint32_t T2 = 32768;                // T'' of head h on its way out at T2 + h * kTriBytes
+    static constexpr uint32_t EX = T2 + HEADS * kTriBytes;
+    static constexpr uint32_t kBytes = EX + HEADS * sizeof(LeanExchange);
     static constexpr uint32_t kDynamic = kBytes + 1024;
-    static_assert(AT % 1024 == 0 && 17408 % 1024 == 0, "UMMA / TMA tiles must be 1024-byte aligned");
+    static_assert(T2 % 512 == 0 && kTriBytes % 512 == 0, "the 64-byte swizzle repeats every 512 bytes");
 };
 constexpr uint32_t kLeanTmemCols = 128;                  // two accumulators of 64 columns
 template <int HEADS>
 constexpr int kLeanCtasPerSm = HEADS == 2 ? 3 : 4;
+
+// Barriers; those with + head are one per head.  Each completes once an item.
+enum : uint32_t {
+    B_K = 0,         // K is there
+    B_Q,             // Q is there
+    B_MMA,           // the product is done
+    B_ENT,           // every warp has seen the product (and the tables), and has read the accumulator of the item before
+    B_SQ,            // with L2 normalisation: the rows' squares are there
+    B_TAB,           // + head: the tables
+    B_PAIR = B_TAB + 2,  // + head: both parts of P have left shared memory
+    B_EXF = B_PAIR + 2,  // + head: the exchange is full
+    B_EXE = B_EXF + 2,   // + head: and has been read
+    B_LOW = B_EXE + 2,   // + head: role 3's half of T'' below the diagonal blocks is there
+    B_BARS = B_LOW + 2
+};
 
 template <int HEADS, bool GATE_F32>
 __global__ void __launch_bounds__(128 * HEADS, kLeanCtasPerSm<HEADS>)
@@ -46,37 +67,36 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                         Workspace ws, unsigned NT, unsigned num_items) {
     using L = LeanSmem<HEADS>;
     extern __shared__ uint8_t smem_raw[];
-    uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* sm = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);   // (an offset, so that the compiler knows the address space)
     const uint32_t sm_u32 = warp_uniform(smem_u32(sm));
-    __shared__ __align__(8) uint64_t bar_tma;
-    __shared__ __align__(8) uint64_t bar_mma;
+    __shared__ __align__(8) uint64_t bars[B_BARS];
     __shared__ uint32_t tmem_slot;
     __shared__ __align__(16) LeanScratch ps2[HEADS];
-    __shared__ float squares[HEADS][128];         // with L2 normalisation: of the rows of [K;Q], per k-half
+    __shared__ float squares[2][HEADS][128];      // with L2 normalisation: of the rows of [K;Q], per k-half
 
     const int tid = threadIdx.x, warp = static_cast<int>(warp_uniform(tid >> 5)), lane = tid & 31;
-    const int h = HEADS == 2 ? tid >> 7 : 0;      // which head of the pair this half of the CTA prepares
-    const int htid = tid & 127, hwarp = warp & 3, i = htid & 63;
-    const PrepCtx ctx{htid, 1 + h};               // the half's own thread numbering and named barrier
+    const int h = HEADS == 2 ? warp >> 2 : 0;     // which head of the pair this half of the CTA prepares
+    const int role = warp & 3;                    // and the warp's quadrant of the accumulator's lanes
     LeanScratch& ps = ps2[h];
     const float scale0 = rsqrtf(static_cast<float>(kD));
     const unsigned rep = p.Hv / p.Hq, groups = p.Hv / HEADS;
-    float* At = reinterpret_cast<float*>(sm + L::AT + h * 17408);
-    uint8_t* t2tile = sm + L::AT + h * 17408;
+    uint8_t* t2tile = sm + L::T2 + h * kTriBytes;
     uint8_t* ptile = sm + L::KQ + 8192 + h * 16384;
+    LeanExchange& ex = *reinterpret_cast<LeanExchange*>(sm + L::EX + h * sizeof(LeanExchange));
     uint8_t* kq = sm + L::KQ;
+    const uint32_t bar0 = smem_u32(bars);
+    auto cb = [&](uint32_t i) { return bar0 + 8u * i; };
 
     // Persistent CTA: items blockIdx.x, blockIdx.x + gridDim.x, ...; the head group index is the fastest, so the groups
     // that share a qk head are prepared at about the same time.
-    struct Item { int b, hv, hq, s0, valid; size_t tok0, tile; };
     int late = 0;                                 // code of this thread's first wait that ran out
-    auto wait = [&](uint64_t* bar, uint32_t parity, int code) {   // (mbar_wait: 16 x 2048 tokens 125.8 us against 123.7, 8192 36.8 / 36.1)
-        if (mbar_wait_compact(smem_u32(bar), parity)) return true;
-        if (late == 0) late = code;
+    auto wait = [&](uint32_t bar, uint32_t item) {
+        if (mbar_wait_compact(cb(bar), item & 1)) return true;
+        if (late == 0) late = bar <= B_Q ? kDevTimeoutTma : kDevTimeoutMma;
         return false;
     };
     auto decode = [&](unsigned n) {
-        Item x;
+        LeanItem x{};
         const unsigned c = n / groups, grp = n - c * groups;
         unsigned seq, t, len, nt;
         size_t tile0;
@@ -107,13 +127,14 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         x.tile = tile0 + static_cast<size_t>(x.hv) * nt + t;
         return x;
     };
-    auto load_k = [&](const Item& x) {   // one thread; announces the bytes of Q as well
-        mbar_arrive_expect_tx(&bar_tma, 4 * 8192);
-        tma_load_4d(kq + 0, &tm_k, &bar_tma, 0, x.hq, x.s0, x.b);
-        tma_load_4d(kq + 16384, &tm_k, &bar_tma, 64, x.hq, x.s0, x.b);
+    auto load_k = [&](const LeanItem& x) {   // one thread; announces the bytes of Q as well
+        mbar_arrive_expect_tx_a(cb(B_K), 2 * 8192);
+        mbar_arrive_expect_tx_a(cb(B_Q), 2 * 8192);
+        tma_load_4d_a(sm_u32 + L::KQ, &tm_k, cb(B_K), 0, x.hq, x.s0, x.b);
+        tma_load_4d_a(sm_u32 + L::KQ + 16384, &tm_k, cb(B_K), 64, x.hq, x.s0, x.b);
     };
-    auto load_q_half = [&](const Item& x, int half) {
-        tma_load_4d(kq + 8192 + half * 16384, &tm_q, &bar_tma, 64 * half, x.hq, x.s0, x.b);
+    auto load_q_half = [&](const LeanItem& x, int half) {
+        tma_load_4d_a(sm_u32 + L::KQ + 8192 + half * 16384, &tm_q, cb(B_Q), 64 * half, x.hq, x.s0, x.b);
     };
     auto issue_product = [&](uint32_t d) {   // raw K K^T (lanes 0-63) and Q K^T (lanes 64-127), shared by the heads
         tc_fence_after_sync();
@@ -123,14 +144,7 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
             const uint64_t ad = umma_smem_desc(sm_u32 + L::KQ + (ks >> 2) * 16384 + (ks & 3) * 32, 16, 1024, SWZ_128B);
             umma_bf16_ss(d, ad, ad, idesc, ks > 0);
         }
-        umma_commit(&bar_mma);
-    };
-
-    auto store_tri = [&](const void* map, const uint8_t* src, size_t tile) {   // the three blocks of a triangular tile
-        const int row = static_cast<int>(tile * kChunk);
-        tma_store_2d(map, src, 0, row);
-        tma_store_2d(map, src + 2048, 0, row + 32);
-        tma_store_2d(map, src + 4096, 32, row + 32);
+        umma_commit_a(cb(B_MMA));
     };
 
     const bool prof_on = GDN_DIAG(p.prof != nullptr && tid == 0 && blockIdx.x == 0);
@@ -143,9 +157,12 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         prof_t = now_;                                 \
     }
 
-    if (tid == 0) {
-        mbar_init(&bar_tma, 1);
-        mbar_init(&bar_mma, 1);
+    if (warp == 2 && elect_one()) {
+        for (uint32_t i = 0; i < B_BARS; ++i) {
+            const uint32_t count = i == B_ENT ? 4 * HEADS : i == B_SQ ? 3 * HEADS : i == B_TAB || i == B_TAB + 1 ? (p.l2norm ? 2 : 1)
+                                   : i >= B_PAIR && i < B_LOW ? 2 : 1;
+            mbar_init(&bars[i], count);
+        }
         fence_mbar_init();
     }
     if (warp == 0) {
@@ -153,113 +170,182 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         tmem_relinquish();
     }
     grid_dependency_wait();   // launched ahead of the end of the kernel before: no memory is touched above
-    unsigned n = blockIdx.x;
-    Item cur = decode(n);
-    if (tid == 0) {
-        if (p.clear_status && n == 0) *p.status = 0;
-        load_k(cur);
-        load_q_half(cur, 0);
-        load_q_half(cur, 1);
-    }
-    LaneGates gates{0.f, 0.f, 0.f, 0.f};
-    if (hwarp == 0) gates = lean_load_gates<GATE_F32>(p, cur.tok0, cur.hv, cur.valid, lane);
+    if (tid == 0 && p.clear_status && blockIdx.x == 0) *p.status = 0;
+    // Role 2 looks ahead, two items.
+    auto look = [&](unsigned item) {
+        const LeanItem x = decode(blockIdx.x + item * gridDim.x);
+        if (lane == 0) ps.item[item & 3] = x;
+        __syncwarp();
+    };
+    if (role == 3) look(0);
+    if (role == 2 && blockIdx.x + gridDim.x < num_items) look(1);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = warp_uniform(tmem_slot);
-    const uint32_t lane_base = static_cast<uint32_t>(hwarp) * 32u;   // (warp % 4) * 32: the warp's TMEM lane quadrant
-    uint32_t ph = 0;            // parity of both barriers: one load and one product per item
-    bool ok = true;
     if (p.dbg == kDbgLaneGivesUp && tid == 5) late = kDevTimeoutTma;
-    if (warp == 0) {
-        ok = wait(&bar_tma, 0, kDevTimeoutTma);
-        if (ok && p.dbg != kDbgNoProduct && elect_one()) issue_product(tmem);
-    }
 
-    for (; n < num_items; n += gridDim.x) {
-        const size_t tile = cur.tile;
-        float* vec = ws.vec + tile * 256;
-        const uint32_t acc = tmem + ph * 64;
-        const unsigned nn = n + gridDim.x;
-        const bool more = nn < num_items;
-        // the gate cumsum and the decay tables need nothing from the tiles: they run while the product does
-        if (hwarp == 0) {
-            if (elect_one()) tma_store_wait_read();   // (the lane that issued it) the previous item's T'' has left the array A goes into
-            lean_gates(ps, gates, p.gate_act != 0, scale0, p.l2norm ? ps.vec : vec, lane);
-        }
-        ctx.sync();
-        if (p.l2norm) {
-            // The other half reads this half's sums of the item before in lean_l2norm_fold, and no barrier of the CTA lies behind that: this
-            // wait does.  It needs the bytes of both halves of Q, which each half requests behind its own fold.
-            ok = wait(&bar_tma, ph, kDevTimeoutTma);
-            squares[h][htid] = lean_row_squares(kq + h * 16384, htid);
-            if (HEADS == 1) squares[h][htid] += lean_row_squares(kq + 16384, htid);
-        }
-        GDN_PHASE(0)
-        ok = wait(&bar_mma, ph, kDevTimeoutMma) && ok;
-        ok = __syncthreads_and(ok);
-        if (!ok) break;
+    // Items of a CTA are counted from 0; `item & 1` names the buffer of its tables, its accumulator and the parity of its barriers.  A wait names a
+    // parity, so the next completion of its barrier has to need something behind the wait: that of K, Q, MMA and TAB an arrival on ENT by each
+    // warp that waits for them, the others an arrival by the one that waits.
+    auto enter = [&](unsigned item) {
+        if (!wait(B_TAB + h, item) || !wait(B_MMA, item)) return false;
         tc_fence_after_sync();
-        if (p.l2norm) lean_l2norm_fold(ps, HEADS == 1 ? squares[0][htid] : squares[0][htid] + squares[HEADS - 1][htid], vec, cur.valid, ctx);
-        GDN_PHASE(1)
-        Item nxt = cur;
-        if (more) {
-            nxt = decode(nn);
-            if (warp == 0 && elect_one()) load_k(nxt);
-            if (hwarp == 0) gates = lean_load_gates<GATE_F32>(p, nxt.tok0, nxt.hv, nxt.valid, lane);
+        if (lane == 0) mbar_arrive_a(cb(B_ENT));
+        return true;
+    };
+    auto tables = [&](unsigned item) {
+        const uint32_t buf = item & 1;
+        return MaskTables{ps.gam[buf], p.l2norm ? ps.gcol[buf] : ps.gam[buf], p.l2norm ? ps.brow[buf] : ps.bet[item & 3], ps.t16[buf], ps.t32[buf]};
+    };
+    // L2 normalisation.  Squares of the next item's rows, of one k-half (of both where there is one head), by the warps of its head's diagonal blocks: role 0
+    // K's, role 1 Q's.
+    auto row_squares = [&](unsigned item) {
+        if (!wait(role == 0 ? B_K : B_Q, item)) return false;
+#pragma unroll 1
+        for (int e = 0; e < 2; ++e) {
+            const int row = 64 * role + 32 * e + lane;
+            float ss = lean_row_squares(kq + h * 16384, row);
+            if (HEADS == 1) ss += lean_row_squares(kq + 16384, row);
+            squares[item & 1][h][row] = ss;
         }
-        {   // mask epilogue: thread = row i = TMEM lane
-            const bool low_rows = (hwarp & 1) == 0;          // rows 0-31: columns 32-63 lie above the diagonal
-            if (hwarp < 2) {   // A = tril(beta_i * decay * K K^T, -1), fp32, and at once the inverse of the warp's 32x32 block
-                const float ksq = lean_mask_row_A<HEADS == 2>(ps, p.l2norm != 0, tmem_addr(acc, lane_base, 0), i, low_rows, cur.valid, At);
-                if (ws.meta) {
-                    const float bound = lean_bound_of_rows(ps, p.l2norm != 0, i, ksq);
-                    if (lane == 0) ps.bound[hwarp] = bound;
+        __syncwarp();
+        if (lane == 0) mbar_arrive_a(cb(B_SQ));
+        return true;
+    };
+    // What is made of them behind role 3's gates: role 3 the keys' share of the tables, role 2 the queries'.
+    auto norms = [&](unsigned item) {
+        const uint32_t buf = item & 1;
+        if (!wait(B_SQ, item)) return false;
+        const LeanItem& x = ps.item[item & 3];
+        float* vec = ws.vec + x.tile * 256;
+#pragma unroll 1
+        for (int e = 0; e < 2; ++e) {
+            const int tok = 32 * e + lane, row = 64 * (3 - role) + tok;
+            lean_l2norm_fold(ps, item, role == 2, tok, HEADS == 1 ? squares[buf][0][row] : squares[buf][0][row] + squares[buf][HEADS - 1][row], scale0, vec, x.valid);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive_a(cb(B_TAB + h));
+        return true;
+    };
+
+    const unsigned count = (num_items - 1 - blockIdx.x) / gridDim.x + 1;
+    if (role < 2) {
+        // ------------------------------- diagonal blocks of the inverse --------------------------------------------------
+        bool go = !p.l2norm || row_squares(0);
+#pragma unroll 1
+        for (unsigned item = 0; go && item < count; ++item) {
+            if (!enter(item)) break;
+            GDN_PHASE(0)
+            const uint32_t buf = item & 1;
+            const LeanItem& x = ps.item[item & 3];
+            auto ready = [&]() {                           // (the next item's squares while the exchange is still read)
+                return (!p.l2norm || item + 1 == count || row_squares(item + 1)) && (item == 0 || wait(B_EXE + h, item - 1));
+            };
+            go = lean_diagonal(tables(item), ps.bet[item & 3], p.l2norm != 0, ws.meta ? &ps.bound[buf][role] : nullptr, tmem + buf * 64, role, lane, x.valid, ex,
+                               t2tile + 4096 * role, &tm_t2, static_cast<int>(x.tile * kChunk), cb(B_EXF + h), ready);
+            tc_fence_before_sync();
+            GDN_PHASE(1)
+            ++prof_n;
+        }
+    } else if (role == 2) {
+        // ------------------------------- tiles and product of `item`; P of the one before, rows 0-31; T'' of the one before that, below the
+        //                                 diagonal blocks
+#pragma unroll 1
+        for (unsigned item = 0; item < count + 2; ++item) {
+            const bool more = item < count, one = item > 0 && item <= count;
+            const LeanItem &next = ps.item[item & 3], &x = ps.item[(item - 1) & 3], &y = ps.item[(item - 2) & 3];
+            if (one && !enter(item - 1)) break;
+            if (more && warp == 2 && elect_one()) load_k(next);
+            __syncwarp();
+            if (one) {
+                lean_mask_P(tables(item - 1), p.l2norm ? ps.prow[(item - 1) & 1] : nullptr, scale0, tmem + ((item - 1) & 1) * 64, 0, lane, x.valid, ptile);
+                tc_fence_before_sync();
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (elect_one()) {
+                    tma_store_2d(&tm_p, ptile, 0, static_cast<int>(x.tile * kChunk));
+                    tma_store_commit();
                 }
                 __syncwarp();
-                lean_invert_diag32(At, hwarp, lane);
-            } else {           // P = tril(scale * decay * Q K^T), bf16, into its staging tile in Q's place
-                lean_mask_row_P(ps, p.l2norm != 0, scale0, tmem_addr(acc, lane_base, 0), i, low_rows, cur.valid, ptile);
-                fence_proxy_async_smem();
-                named_bar_sync(3 + h, 64);
-                if (hwarp == 2 && elect_one()) {
-                    store_tri(&tm_p, ptile, tile);
+                if (item + 1 < count) look(item + 1);
+            }
+            if (item > 0) {
+                if (elect_one()) {
+                    tma_store_wait_read();           // (and T'' below the diagonal blocks of the item before that)
+                    mbar_arrive_a(cb(B_PAIR + h));
+                }
+                __syncwarp();
+                if (!wait(B_PAIR + h, item - 1)) break;
+            }
+            if (more && elect_one()) {
+                load_q_half(next, h);
+                if (HEADS == 1) load_q_half(next, 1);
+            }
+            __syncwarp();
+            if (item > 1) {
+                if (!wait(B_EXF + h, item - 2)) break;
+                if (ws.meta && lane == 0) {
+                    ws.meta[2 * y.tile] = y.decay;
+                    ws.meta[2 * y.tile + 1] = y.gates_ok ? fmaxf(ps.bound[item & 1][0], ps.bound[item & 1][1]) : INFINITY;
+                }
+                lean_below(ps.bet[(item - 2) & 3], 0, lane, ex, t2tile + 2048, cb(B_EXE + h));
+                if (!wait(B_LOW + h, item - 2)) break;
+                if (elect_one()) {
+                    tma_store_2d(&tm_t2, t2tile + 2048, 0, static_cast<int>(y.tile * kChunk) + 32);
                     tma_store_commit();
-                    if (more) {
-                        tma_store_wait_read();
-                        load_q_half(nxt, h);
-                        if (HEADS == 1) load_q_half(nxt, 1);
-                    }
                 }
                 __syncwarp();
             }
+            if (more) {
+                if (warp == 2) {
+                    if (one && !wait(B_ENT, item - 1)) break;   // (nobody reads the accumulator any more)
+                    if (!wait(B_K, item) || !wait(B_Q, item)) break;
+                    tc_fence_after_sync();
+                    if ((one || p.dbg != kDbgNoProduct) && elect_one()) issue_product(tmem + (item & 1) * 64);
+                    __syncwarp();
+                }
+                if (p.l2norm && !norms(item)) break;
+            }
         }
-        GDN_PHASE(2)
-        tc_fence_before_sync();
-        ctx.sync();
-        GDN_PHASE(3)
-        if (ws.meta && htid == 0) {
-            ws.meta[2 * tile] = ps.gam[kChunk - 1] * (1.f / kLog2e);
-            ws.meta[2 * tile + 1] = ps.gates_ok ? fmaxf(ps.bound[0], ps.bound[1]) : INFINITY;
+    } else {
+        // ------------------------------- gates and tables of `item`; P of the one before, rows 32-63; T'' of the one before that
+#pragma unroll 1
+        for (unsigned item = 0; item < count + 2; ++item) {
+            const bool more = item < count, one = item > 0 && item <= count;
+            LeanItem &next = ps.item[item & 3], &x = ps.item[(item - 1) & 3];
+            if (one && !enter(item - 1)) break;
+            LaneGates gates{0.f, 0.f, 0.f, 0.f};
+            if (more) gates = lean_load_gates<GATE_F32>(p, next.tok0, next.hv, next.valid, lane);
+            if (one) {
+                lean_mask_P(tables(item - 1), p.l2norm ? ps.prow[(item - 1) & 1] : nullptr, scale0, tmem + ((item - 1) & 1) * 64, 1, lane, x.valid, ptile);
+                tc_fence_before_sync();
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (elect_one()) {
+                    const int row = static_cast<int>(x.tile * kChunk) + 32;
+                    tma_store_2d(&tm_p, ptile + 2048, 0, row);
+                    tma_store_2d(&tm_p, ptile + 4096, 32, row);
+                    tma_store_commit();
+                    tma_store_wait_read();
+                }
+                __syncwarp();
+            }
+            if (item > 0 && lane == 0) mbar_arrive_a(cb(B_PAIR + h));
+            if (more) {
+                if (one && !wait(B_ENT, item - 1)) break;   // (nobody reads the tables any more)
+                lean_gates(ps, item, gates, p.gate_act != 0, scale0, p.l2norm ? nullptr : ws.vec + next.tile * 256, lane);
+                __syncwarp();
+                if (lane == 0) mbar_arrive_a(cb(p.l2norm ? B_SQ : B_TAB + h));
+            }
+            if (item > 0 && !wait(B_PAIR + h, item - 1)) break;   // (T'' below the diagonal blocks has left its place; what role 2 looked up)
+            if (item > 1) {
+                if (!wait(B_EXF + h, item - 2)) break;
+                lean_below(ps.bet[(item - 2) & 3], 1, lane, ex, t2tile + 2048, cb(B_EXE + h));
+                if (lane == 0) mbar_arrive_a(cb(B_LOW + h));
+            }
+            if (p.l2norm && more && !norms(item)) break;
         }
-        lean_finish_T2(At, ps.bet, t2tile, ctx);
-        GDN_PHASE(4)
-        if (warp == 3 && more) {   // the next item's product, into the other accumulator (read last an item ago)
-            ok = wait(&bar_tma, ph ^ 1, kDevTimeoutTma);
-            if (ok && elect_one()) issue_product(tmem + (ph ^ 1) * 64);
-            __syncwarp();
-        }
-        GDN_PHASE(5)
-        fence_proxy_async_smem();
-        ctx.sync();
-        if (hwarp == 0 && elect_one()) {
-            store_tri(&tm_t2, t2tile, tile);
-            tma_store_commit();
-        }
-        GDN_PHASE(6)
-        ++prof_n;
-        cur = nxt;
-        ph ^= 1;
     }
 #undef GDN_PHASE
     if (prof_on) {
@@ -270,7 +356,7 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     // Only now may the chain kernel's CTAs start (and set up while the last CTAs of this grid finish): let in earlier, they
     // pile up two to an SM on the SMs that this grid leaves first while others stay empty.
     grid_launch_dependents();
-    if ((hwarp & 1) == 0 && elect_one()) tma_store_wait_all();
+    if (elect_one()) tma_store_wait_all();
     tc_fence_before_sync();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, kLeanTmemCols);

@@ -404,6 +404,17 @@ __device__ __forceinline__ void tmem_ld_16x256b_x4(uint32_t taddr, uint32_t (&r)
         : "r"(taddr)
         : "memory");
 }
+__device__ __forceinline__ void tmem_ld_16x256b_x2(uint32_t taddr, uint32_t (&r)[8]) {   // two groups of 8 columns
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+// Four 8x8 matrices of 16-bit elements to shared memory: lanes 8 i .. 8 i + 7 give the rows' addresses of matrix i, whose register holds, in
+// lane l, elements (l / 4, 2 (l % 4)) and (l / 4, 2 (l % 4) + 1).
+__device__ __forceinline__ void stmatrix_x4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
 // Four 8x8 matrices of 16-bit elements, transposed on their way to shared memory: lanes 8 i .. 8 i + 7 give the rows' addresses of
 // matrix i, whose register holds, in lane l, elements (2 (l % 4), l / 4) and (2 (l % 4) + 1, l / 4).
 __device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
