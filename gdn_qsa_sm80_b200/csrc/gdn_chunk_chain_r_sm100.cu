@@ -120,7 +120,9 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                    const __grid_constant__ CUtensorMap tm_t2, const __grid_constant__ CUtensorMap tm_out, const __grid_constant__ Problem p,
                    const __grid_constant__ Workspace ws, const unsigned sms) {
     extern __shared__ uint8_t smem_raw[];
-    uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    // Rounded up as an offset: through an integer the pointer loses its address space, and every access by the roles becomes a generic one (us a call,
+    // before / after: 333 tokens 19.9 / 19.1, 2 x 1500 with 8 / 8 heads 28.2 / 27.0, 4 x 1999 82.1 / 80.4, 8192 83.1 / 82.0, 64 x 4096 2179 / 2143).
+    uint8_t* sm = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);
     const uint32_t sm_u32 = warp_uniform(smem_u32(sm));
     __shared__ __align__(8) uint64_t bars[kRBars];
     __shared__ uint32_t tmem_slot;
