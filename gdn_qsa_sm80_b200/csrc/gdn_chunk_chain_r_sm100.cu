@@ -455,22 +455,24 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             }
             if (!wait(R_QS, n - from)) break;
             tc_fence_after_sync();
-            const float* qf = reinterpret_cast<const float*>(sm + R_VEC + s * 1024) + kChunk;   // scale e^gamma_j
+            const float* qf = reinterpret_cast<const float*>(sm + R_VEC + s * 1024) + kChunk + 2 * (lane & 3);   // scale e^gamma_j
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                uint32_t x[8];
-                tmem_ld_x8(o_addr + 8 * u, x);
-                tmem_ld_wait();
+            for (int u = 0; u < 4; ++u) {                     // tokens [16 u, +16) of 16 value columns at a time
+                const float2 f[2] = {*reinterpret_cast<const float2*>(qf + 16 * u), *reinterpret_cast<const float2*>(qf + 16 * u + 8)};
 #pragma unroll
-                for (int j = 0; j < 8; j += 4) {
-                    const float4 f = *reinterpret_cast<const float4*>(qf + 8 * u + j);
-                    const float2 y = mul2(as_float2(x[j], x[j + 1]), make_float2(f.x, f.y)), z = mul2(as_float2(x[j + 2], x[j + 3]), make_float2(f.z, f.w));
-                    x[j] = __float_as_uint(y.x);
-                    x[j + 1] = __float_as_uint(y.y);
-                    x[j + 2] = __float_as_uint(z.x);
-                    x[j + 3] = __float_as_uint(z.y);
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t x[8];
+                    const uint32_t at = o_addr + (static_cast<uint32_t>(16 * h) << 16) + 16 * u;
+                    tmem_ld_16x256b_x2(at, x);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int e = 0; e < 8; e += 2) {
+                        const float2 y = mul2(as_float2(x[e], x[e + 1]), f[e >> 2]);
+                        x[e] = __float_as_uint(y.x);
+                        x[e + 1] = __float_as_uint(y.y);
+                    }
+                    tmem_st_16x256b_x2(at, x);
                 }
-                tmem_st_x8(o_addr + 8 * u, x);
             }
             tmem_st_wait();
             tc_fence_before_sync();
@@ -575,20 +577,21 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             if (!ok) break;
             tc_fence_after_sync();
             GDN_PHASE(0)
-            const float* vec = reinterpret_cast<const float*>(sm + R_VEC + s * 1024);
-            const float dC = vec[2 * kChunk];                 // exp(gamma_C); read now, the slot is released below
+            const float* vec = reinterpret_cast<const float*>(sm + R_VEC + s * 1024) + 32 * hf + 2 * (lane & 3);   // of this lane's columns
+            const float dC = *reinterpret_cast<const float*>(sm + R_VEC + s * 1024 + 8 * kChunk);   // exp(gamma_C); read now, the slot is released below
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {                     // X of tokens [32 hf + 8 u, +8)
-                uint32_t x[8], pk[4];
-                tmem_ld_x8(a_ks + 8 * u, x);
-                tmem_ld_wait();
+            for (int u = 0; u < 2; ++u) {                     // X of tokens [32 hf + 16 u, +16), 16 value columns at a time
+                const float2 f[2] = {*reinterpret_cast<const float2*>(vec + 3 * kChunk + 16 * u), *reinterpret_cast<const float2*>(vec + 3 * kChunk + 16 * u + 8)};
 #pragma unroll
-                for (int j = 0; j < 8; j += 4) {
-                    const float4 f = *reinterpret_cast<const float4*>(vec + 3 * kChunk + 32 * hf + 8 * u + j);
-                    pk[j / 2] = mul_bf16x2(as_float2(x[j], x[j + 1]), make_float2(f.x, f.y));
-                    pk[j / 2 + 1] = mul_bf16x2(as_float2(x[j + 2], x[j + 3]), make_float2(f.z, f.w));
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t x[8], pk[4];
+                    const uint32_t at = a_ks + (static_cast<uint32_t>(16 * h) << 16);
+                    tmem_ld_16x256b_x2(at + 16 * u, x);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) pk[c] = mul_bf16x2(as_float2(x[2 * c], x[2 * c + 1]), f[c >> 1]);
+                    tmem_st_16x128b_x2(at + 8 * u, pk);
                 }
-                tmem_st_x4(a_ks + 4 * u, pk);
             }
             tmem_st_wait();
             tc_fence_before_sync();
@@ -599,23 +602,24 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             if (!ok) break;
             tc_fence_after_sync();
             GDN_PHASE(2)
+#pragma unroll SPLIT ? 2 : 1                          // (unsplit and unrolled, eight registers more are spilled: 64 x 4096 1 % slower)
+            for (int u = 0; u < 2; ++u) {                     // v_new and v~ of tokens [32 hf + 16 u, +16)
+                const float2 f[2] = {*reinterpret_cast<const float2*>(vec + 16 * u), *reinterpret_cast<const float2*>(vec + 16 * u + 8)};   // exp(gamma_C - gamma_j)
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {                     // v_new and v~ of tokens [32 hf + 8 u, +8)
-                uint32_t x[8], pk[4];
-                tmem_ld_x8(tmem_addr(tmem, lane_base, C_VN + 32 * hf + 8 * u), x);
-                tmem_ld_wait();
-                if (n >= from) {
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t x[8], pk[4];
+                    const uint32_t l16 = lane_base + 16 * h;
+                    tmem_ld_16x256b_x2(tmem_addr(tmem, l16, C_VN + 32 * hf + 16 * u), x);
+                    tmem_ld_wait();
+                    if (n >= from) {
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) pk[c] = pack_bf16x2(__uint_as_float(x[2 * c]), __uint_as_float(x[2 * c + 1]));
-                    tmem_st_x4(tmem_addr(tmem, lane_base, C_VP + 16 * hf + 4 * u), pk);
+                        for (int c = 0; c < 4; ++c) pk[c] = pack_bf16x2(__uint_as_float(x[2 * c]), __uint_as_float(x[2 * c + 1]));
+                        tmem_st_16x128b_x2(tmem_addr(tmem, l16, C_VP + 16 * hf + 8 * u), pk);
+                    }
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) pk[c] = mul_bf16x2(as_float2(x[2 * c], x[2 * c + 1]), f[c >> 1]);
+                    tmem_st_16x128b_x2(tmem_addr(tmem, l16, C_VS + 16 * hf + 8 * u), pk);
                 }
-#pragma unroll
-                for (int c = 0; c < 4; c += 2) {
-                    const float4 f = *reinterpret_cast<const float4*>(vec + 32 * hf + 8 * u + 2 * c);   // exp(gamma_C - gamma_j)
-                    pk[c] = mul_bf16x2(as_float2(x[2 * c], x[2 * c + 1]), make_float2(f.x, f.y));
-                    pk[c + 1] = mul_bf16x2(as_float2(x[2 * c + 2], x[2 * c + 3]), make_float2(f.z, f.w));
-                }
-                tmem_st_x4(tmem_addr(tmem, lane_base, C_VS + 16 * hf + 4 * u), pk);
             }
             tmem_st_wait();
             tc_fence_before_sync();

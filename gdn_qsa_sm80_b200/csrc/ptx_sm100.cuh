@@ -443,6 +443,17 @@ __device__ __forceinline__ void tmem_st_x4(uint32_t taddr, const uint32_t (&r)[4
                  ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3])
                  : "memory");
 }
+// Fragments back: 16 lanes by two groups of 8 columns, as tmem_ld_16x256b_x2 reads them.
+__device__ __forceinline__ void tmem_st_16x256b_x2(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x2.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+// 16 lanes by two groups of 4 columns; thread l writes, of group k, column l % 4 of lane l / 4 from r[2 k] and of lane l / 4 + 8 from r[2 k + 1]: what a
+// fragment of 16-bit pairs made from tmem_ld_16x256b_x2's is.
+__device__ __forceinline__ void tmem_st_16x128b_x2(uint32_t taddr, const uint32_t (&r)[4]) {
+    asm volatile("tcgen05.st.sync.aligned.16x128b.x2.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
+}
 // All tcgen05.st of this thread have been performed.
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
