@@ -12,8 +12,8 @@
 // shuffles: no barrier.  With several tokens a tile what bounds it is the two warps' serial run through the tokens, not HBM (64 sequences
 // of 4: DRAM 40 % busy, issue slots 37 % with six compute warps an SM): two multiply-adds in one instruction (f32x2).  32 heads, before
 // and after: 8 sequences of 4 tokens 14.5 -> 12.7 us, 256 of 4 277 -> 241, 64 of 8 121 -> 111; 64 of one 47 us, 86 % of the copy bandwidth.
-//   GROUPS = 1: a CTA of two compute warps and a producer warp, four per SM (three from four tokens on, whose vectors take
-//   room in every stage); 32 states give 128 CTAs.
+//   GROUPS = 1: a CTA of two compute warps and a producer warp, four per SM (from five tokens on, whose vectors take room in every stage,
+//   three, or four with a ring of two: two_stages); 32 states give 128 CTAs.
 //   PACKED: the sequences of a packed batch that have at most kDecodeMaxTokens tokens, of any lengths, found through a table.
 //   GROUPS = 4: the four tiles of a state in one CTA, for the gated normalisation of the output rows (their sum of squares
 //   needs all 128 columns: one barrier a token), which then costs no launch and no pass over the rows of its own.  One token: a ring of
@@ -51,8 +51,9 @@ __device__ __forceinline__ float sum_rows(float x) {   // over the eight lanes t
     return x;
 }
 
-// bytes of the token area of one stage: k, q rows, 32 columns of v, g and beta
-__host__ __device__ constexpr uint32_t dec_token_bytes(int nt) { return (nt * (256 + 256 + 64) + 2 * kDecTokens * 4 + 127) & ~127u; }
+// bytes of the token area of one stage: k, q rows, 32 columns of v (a box's destination: a multiple of 128); g and beta, behind all of them
+__host__ __device__ constexpr uint32_t dec_token_bytes(int nt) { return (nt * (256 + 256 + 64) + 127) & ~127u; }
+constexpr uint32_t kDecGateBytes = 2 * kDecTokens * 4;
 
 // Where the vectors of several tokens come from: a box of nt rows each, three copies a tile instead of three a token, where a CTA has
 // more than one tile (32 heads, 18 sequences of 2 tokens 12.5 us, by rows 13.7; 32 of 2 22.0, 23.3; of 3 and more tokens the same within
@@ -87,6 +88,7 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
     // stage s of group g: the tile at (g * STAGES + s) * 16 KB; the token areas behind all tiles
     auto tile_of = [&](int g, int s) { return sm + (g * STAGES + s) * 16384; };
     auto tok_of = [&](int g, int s) { return sm + GROUPS * STAGES * 16384 + (g * STAGES + s) * tok_bytes; };
+    auto gates_of = [&](int g, int s) { return reinterpret_cast<float*>(sm + GROUPS * STAGES * (16384 + tok_bytes) + (g * STAGES + s) * kDecGateBytes); };
     const int rep = p.Hv / p.Hq;
 
     if (tid == 0) {
@@ -152,7 +154,7 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
                 x = dec_gate<GATE_F32>(lane < kDecTokens ? p.g : p.beta, (tok0 + (lane & 7)) * p.Hv + h);
             for (int g = 0; g < GROUPS; ++g) {
                 if (PACKED && lane == 0) seq_of[s] = seq;
-                if (lane < 2 * kDecTokens) *reinterpret_cast<float*>(tok_of(g, s) + nt * (256 + 256 + 64) + lane * 4) = x;
+                if (lane < 2 * kDecTokens) gates_of(g, s)[lane] = x;
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&full[g][s]);
             }
@@ -196,7 +198,7 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
                 st[i][0] = make_float2(x.x, x.y);
                 st[i][1] = make_float2(x.z, x.w);
             }
-            const float* gates = reinterpret_cast<const float*>(tk + nt * (256 + 256 + 64));
+            const float* gates = gates_of(g, s);
             for (int t = 0; t < tokens; ++t) {
                 const size_t tok = tok0 + t;
                 // this lane's rows of k and q, its four values, the gates
@@ -309,7 +311,7 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
             }
             named_bar_sync(2 + g, 64);
             if (half == 0 && elect_one()) {
-                if (p.hT && STAGES == 3) {
+                if (p.hT && STAGES > 1) {
                     tma_store_wait_read();                // tile n - 1's store has read its stage
                     if (n > 0) mbar_arrive(&empty[g][(n - 1) % STAGES]);
                     if (ok) tma_store_2d(&tm_out, tile_of(g, s), quarter * 32, state * kD);
@@ -349,6 +351,22 @@ bool two_gated_ctas(const Problem& p, long long states) {
     return 10 * rounds >= (p.S == 2 ? 19 : p.S == 3 ? 18 : 17) * pairs;
 }
 
+// Five to eight tokens: four CTAs per SM with a ring of two, or three with a ring of three?  What bounds these tiles is their warps' run through the tokens, so
+// four fill the SM's issue slots better, but a tile more at a time takes longer, and where the last round is not full three may have as many rounds.
+// In hundredths of a round of three: a round of four 126 (five tokens: 130), a last round of one tile 50, of more 100.  32 heads, states in and out, us per
+// call (three / two):
+//   sequences (tiles an SM)  3 (3)      4 (4)      5 (5)        6 (6)        8 (7)        10 (9)       13 (12)      24 (21)      64 (56)
+//   5 tokens                 6.3 / 7.0  8.2 / 6.9  10.1 / 8.6   10.2 / 10.4  14.5 / 11.9  14.9 / 15.8  18.7 / 17.1  30.9 / 31.8  76.3 / 76.9
+//   6 tokens                 6.9 / 7.6  9.2 / 7.5  11.3 / 9.6   11.4 / 11.7  16.4 / 13.1  16.7 / 17.5  21.2 / 19.0  35.1 / 35.4  87.8 / 84.7
+//   8 tokens                 8.2 / 8.8  11.1 / 8.8 13.8 / 11.5  13.8 / 13.8  20.2 / 15.6  20.5 / 21.2  26.3 / 22.7  44.1 / 43.2  112.0 / 100.2
+// (Packed batches keep three: where most of their sequences are single tokens a ring of two is 8 % slower, 128 sequences with one of 8 86.7 / 94.3.)
+bool two_stages(int tokens, long long tiles) {
+    if (tokens < 5) return false;
+    const long long t = (tiles + sm_count() - 1) / sm_count();
+    auto last = [](long long k) { return k == 0 ? 0 : k == 1 ? 50 : 100; };
+    return (tokens == 5 ? 130 : 126) * (t / 4) + last(t % 4) < 100 * (t / 3) + last(t % 3);
+}
+
 }  // namespace
 
 // `og`: gated normalisation applied to the output rows by the same kernel (null: none).
@@ -369,12 +387,12 @@ int launch_decode(const Problem& p, const OutputGate* og, cudaStream_t stream) {
     DecodeGate gate{};
     if (og) gate = DecodeGate{static_cast<const __nv_bfloat16*>(og->z), static_cast<const __nv_bfloat16*>(og->weight), og->eps};
     const bool gated = og && !p.pk_short;
-    const int groups = gated ? 4 : 1, stages = gated && two_gated_ctas(p, states) ? 1 : 3;
+    const long long items = p.pk_short ? 4ll * p.pk_shorts * p.Hv : gated ? states : states * 4;
+    const int groups = gated ? 4 : 1, stages = gated ? (two_gated_ctas(p, states) ? 1 : 3) : !p.pk_short && two_stages(p.S, items) ? 2 : 3;
     const int most = gated ? 4 : kDecTokens;                       // tokens whose vectors fit three stages of four groups
     const int nt = p.S < most ? p.S : most;
-    const long long items = p.pk_short ? 4ll * p.pk_shorts * p.Hv : gated ? states : states * 4;
-    const uint32_t smem = groups * stages * (16384 + dec_token_bytes(nt)) + 1024;
-    const int fit = static_cast<int>(228 * 1024 / (smem + 1536)), most_ctas = dec_ctas_per_sm(groups, stages), per_sm = fit > most_ctas ? most_ctas : fit;
+    const uint32_t smem = groups * stages * (16384 + dec_token_bytes(nt) + kDecGateBytes) + 1024;
+    const int fit = static_cast<int>(228 * 1024 / (smem + (groups == 1 ? 1088 : 1536))), most_ctas = dec_ctas_per_sm(groups, stages), per_sm = fit > most_ctas ? most_ctas : fit;
     const long long cap = static_cast<long long>(sm_count()) * per_sm;
     auto go = [&](auto kernel, const auto& maps) -> int {
         if (allow_smem(reinterpret_cast<const void*>(kernel), smem)) return GDN_ERR_CUDA;
@@ -402,6 +420,7 @@ int launch_decode(const Problem& p, const OutputGate* og, cudaStream_t stream) {
     }
     if (gated && stages == 3) return p.gate_f32 ? go(gdn_decode_kernel<4, true, false, 3, Fetch::BOXES>, maps) : go(gdn_decode_kernel<4, false, false, 3, Fetch::BOXES>, maps);
     if (gated) return p.gate_f32 ? go(gdn_decode_kernel<4, true, false, 1, Fetch::BOXES>, maps) : go(gdn_decode_kernel<4, false, false, 1, Fetch::BOXES>, maps);
+    if (stages == 2) return p.gate_f32 ? go(gdn_decode_kernel<1, true, false, 2, Fetch::BOXES>, maps) : go(gdn_decode_kernel<1, false, false, 2, Fetch::BOXES>, maps);
     return p.gate_f32 ? go(gdn_decode_kernel<1, true, false, 3, Fetch::BOXES>, maps) : go(gdn_decode_kernel<1, false, false, 3, Fetch::BOXES>, maps);
 }
 
