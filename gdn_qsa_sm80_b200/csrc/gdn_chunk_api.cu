@@ -318,12 +318,13 @@ int forward_device(const void* q, const void* k, const void* v, const void* g, c
     auto then_gate = [&](int st) -> int {
         if (st != GDN_OK || !gate) return st;
         const long long rows = static_cast<long long>(B) * S * Hv;
-        return launch_rmsnorm_gated(out, gate->z, gate->weight, out, rows, gate->eps, stream) == cudaSuccess ? GDN_OK
-                                                                                                          : GDN_ERR_CUDA;
+        const uintptr_t zb = reinterpret_cast<uintptr_t>(gate->z), ob = reinterpret_cast<uintptr_t>(out), bytes = static_cast<uintptr_t>(rows) * kD * 2;
+        const bool apart = zb + bytes <= ob || ob + bytes <= zb;   // (z is read before the forward pass has ended)
+        return launch_rmsnorm_gated(out, gate->z, gate->weight, out, rows, gate->eps, stream, apart) == cudaSuccess ? GDN_OK : GDN_ERR_CUDA;
     };
 
     // A few new tokens: the state read and write is all there is, and the decode kernel streams it, in exact fp32 (2048
-    // states: 47.8 us at one token = 5.6 TB/s, 65 at four, 112 at eight; the chunk kernels 93-94 whatever the number.  Fewer states
+    // states: 47.8 us at one token = 5.6 TB/s, 52 at four, 100 at eight; the chunk kernels 93-94 whatever the number.  Fewer states
     // favour it longer: the line lies where an eight-token chunk would be one eighth full).
     if (decode) return launch_decode(p, gate, stream);
     if (path == GDN_PATH_SIMT && !clear()) return GDN_ERR_CUDA;

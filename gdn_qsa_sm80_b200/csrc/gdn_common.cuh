@@ -153,8 +153,9 @@ inline int encode_tma_bf16(void* tmap_out, const void* base, int rank, const uns
 int encode_workspace_maps(const Problem& p, const Workspace& ws, void* tw, void* tp, void* tu_store, void* tu_load, int nv);
 // Number of SMs of the current device (cached per device).
 int sm_count();
+// z_ready: the kernel before it in the stream does not make z, and has waited for whatever did.
 cudaError_t launch_rmsnorm_gated(const void* y, const void* z, const void* weight, void* out, long long n_rows,
-                                 float eps, cudaStream_t stream);
+                                 float eps, cudaStream_t stream, bool z_ready);
 // The forward pass on device buffers (what gdn_chunk_fwd_sm100_ex does).  clear_status = false leaves the status
 // word at the start of `scratch` as it is, so that several launches can share one sticky word.
 // gate != nullptr: the output rows are replaced by rmsnorm_gated(row, z, weight), by the normalisation kernel
