@@ -361,6 +361,7 @@ int forward_device(const void* q, const void* k, const void* v, const void* g, c
         if (encode_tile_maps(p, ws, maps)) return GDN_ERR_DRIVER;
         int st = path == GDN_PATH_CHAIN_ONLY_T ? GDN_OK : launch_prepare_lean(p, ws, maps, stream);
         if (st != GDN_OK || prepare_only) return st;
+        p.behind_prepare = path != GDN_PATH_CHAIN_ONLY_T;
         return then_gate(launch_chain_r(p, ws, maps, stream));
     }
     if (path == GDN_PATH_CHAIN_ONLY) return then_gate(launch_chain(p, ws, nv, stream));   // workspace left by an earlier call

@@ -149,7 +149,11 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         tmem_alloc(&tmem_slot, kRTmemCols);
         tmem_relinquish();
     }
-    grid_dependency_wait();   // launched ahead of the end of the prepare kernel: nothing of the workspace is read above
+    // Launched ahead of the end of the prepare kernel.  What that one makes is read behind this wait, where sequences are split by every thread (the plan), else
+    // by the producer alone: the first tiles of K and V and the initial state are under way by then (whoever made them had ended when the prepare kernel's
+    // CTAs let this one start).  us a call, before / after: 9 tokens 10.04 / 9.47, 200 15.27 / 14.70, 333 18.59 / 18.02, 4 x 200 17.76 / 17.23.
+    const bool whole = SPLIT || p.pk_chunk || !p.behind_prepare;
+    if (whole) grid_dependency_wait();
 
     if (tid == 0) {   // which sequence: its tokens, chunks and workspace tiles
         int seq;
@@ -243,15 +247,17 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                     tma_load_4d_a(d + 8192, &tm_k, fb, 64, hq, s0, b);
                 }
             };
-            auto load_v = [&](int n) {
+            auto load_v = [&](int n, bool tile, bool factors) {
                 const uint32_t s = n & 1, fb = cb(R_VFULL + s);
                 const int t = work.t0 + n, s0 = work.s_first + t * kChunk, b = work.b;
                 const float* vec = ws.vec + (work.tile0 + t) * 256;
                 if (elect_one()) {
-                    mbar_arrive_expect_tx_a(fb, 16384 + 1024);
-                    tma_load_4d_a(sm_u32 + R_V + s * 16384, &tm_v, fb, 0, hv, s0, b);
-                    tma_load_4d_a(sm_u32 + R_V + s * 16384 + 8192, &tm_v, fb, 64, hv, s0, b);
-                    bulk_load_1d_a(sm_u32 + R_VEC + s * 1024, vec, 1024, fb);
+                    if (tile) {
+                        mbar_arrive_expect_tx_a(fb, 16384 + 1024);
+                        tma_load_4d_a(sm_u32 + R_V + s * 16384, &tm_v, fb, 0, hv, s0, b);
+                        tma_load_4d_a(sm_u32 + R_V + s * 16384 + 8192, &tm_v, fb, 64, hv, s0, b);
+                    }
+                    if (factors) bulk_load_1d_a(sm_u32 + R_VEC + s * 1024, vec, 1024, fb);
                 }
             };
             auto load_tri = [](uint32_t dst, const void* map, uint32_t bar, int row0) {
@@ -282,9 +288,17 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 const unsigned long long t0 = globaltimer_ns();
                 while (globaltimer_ns() - t0 < 20000ull) {}
             };
+            const bool tile = !HOOKS || p.dbg != kDbgNoTile;
             load_k(0);
-            load_t2(0);
-            if (!HOOKS || p.dbg != kDbgNoTile) load_v(0);
+            if (whole) {
+                load_t2(0);
+                if (tile) load_v(0, true, true);
+            } else {
+                if (tile) load_v(0, true, false);
+                grid_dependency_wait();
+                load_t2(0);
+                if (tile) load_v(0, false, true);
+            }
             // A slot's reload waits for the UMMA (or the epilogue) that read it, in the order in which those complete.  A wait names a parity,
             // so the next completion of its barrier has to need a tile that is loaded behind it.  In iteration n:
             //   R_S + slot of n - 1    next: E2 of n + 1, which needs K(n + 1), two lines below.  (One barrier for both slots would complete
@@ -338,7 +352,7 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                     dawdle();
                     if (n > 0 && !wait(R_VEMPTY + ((n + 1) & 1), ((n + 1) >> 1) - 1)) break;
                     if (n > from && !wait(R_OUT + ((n - 1) & 1), (n - from - 1) >> 1)) break;   // the outputs of chunk n - 1, staged in its V's place, have left
-                    load_v(n + 1);
+                    load_v(n + 1, true, true);
                 }
             }
         } else if (warp == 13) {
@@ -680,6 +694,7 @@ gdn_chain_r_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         }
     }
 
+    if (!whole) grid_dependency_wait();   // (of a CTA without chunks: it does not end before the prepare kernel has)
     tc_fence_before_sync();
     __syncthreads();
     if (work.late) {   // let copies that may still be in flight land before the CTA's memory is released

@@ -45,6 +45,7 @@ struct Problem {
     int gate_act;          // 1: g and beta hold raw values; the kernels apply g = -softplus(.), beta = sigmoid(.)
     int l2norm;            // 1: q and k are L2-normalised per head vector inside the kernels
     int clear_status;      // 1: the launch's first kernel clears the status word
+    int behind_prepare;    // 1: the residual-form chain is launched right behind the prepare kernel of the same call
     int dbg;               // test hook (environment variable GDN_CHUNK_DBG); 0 in production
     // Packed batch (residual-form kernels only; null / 0 otherwise): B = 1, S = all tokens, sequences laid end to end
     const int* pk_cu;      // [pk_n + 1] first token of each sequence
