@@ -17,8 +17,8 @@
 // All four at the same item, with barriers of the head between the phases, left a quarter of the warps' time at them.
 //
 // What bounds it: the shared-memory pipe (16 sequences of 2048 tokens: 56 % of the cycles for loads and stores, about 25 % for operands and copies), then HBM (29 KB
-// per chunk and head).  us alone, against the form that passed A and T through shared memory row by row and ran its phases in step: 16 x 2048 124 / 96, 8192 tokens
-// 36.3 / 29.8, 4 x 1999 36.3 / 29.6 (with L2 normalisation 41.8 / 38.9), 64 x 4096 941 / 744; 16 x 2048 with 16 / 16 heads 81.5 / 65.4.
+// per chunk and head).  us alone, against the form that passed A and T through shared memory row by row and ran its phases in step: 16 x 2048 124 / 95.8, 8192 tokens
+// 36.3 / 29.5, 4 x 1999 36.3 / 29.5 (with L2 normalisation 41.8 / 34.3), 64 x 4096 941 / 719; 16 x 2048 with 16 / 16 heads 81.5 / 66.0.
 // Stands in for the reference's gdn_prepare_kernel (csrc/gdn_chunk/gdn_kernel.cu:343-710).
 #include <cuda.h>
 
@@ -136,6 +136,17 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     auto load_q_half = [&](const LeanItem& x, int half) {
         tma_load_4d_a(sm_u32 + L::KQ + 8192 + half * 16384, &tm_q, cb(B_Q), 64 * half, x.hq, x.s0, x.b);
     };
+    // Rows of padding tokens count as zeros.  In a packed batch they are the next sequence's (elsewhere the copies leave zeros): cleared by one warp before the product
+    // (in the masks' registers instead, code that every role carried: 4 x 1999 tokens with L2 normalisation 35.6 us alone, now 34.3; 64 x 4096 726 / 719).
+    auto clear_tail = [&](int valid) {
+        uint32_t at = sm_u32 + L::KQ;
+        asm volatile("" : "+r"(at));              // (its addresses are computed here, not kept in registers across the items' loop)
+        at += ((lane >> 3) & 3) * 8192 + (lane & 7) * 16;
+#pragma unroll 1
+        for (int row = valid; row < kChunk; ++row) asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(at + row * 128), "r"(0) : "memory");
+        fence_proxy_async_smem();
+        __syncwarp();
+    };
     auto issue_product = [&](uint32_t d) {   // raw K K^T (lanes 0-63) and Q K^T (lanes 64-127), shared by the heads
         tc_fence_after_sync();
         constexpr uint32_t idesc = umma_idesc_bf16(128, 64, MAJOR_K, MAJOR_K);
@@ -177,8 +188,8 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         if (lane == 0) ps.item[item & 3] = x;
         __syncwarp();
     };
-    if (role == 3) look(0);
-    if (role == 2 && blockIdx.x + gridDim.x < num_items) look(1);
+    const unsigned count = (num_items - 1 - blockIdx.x) / gridDim.x + 1;
+    if (role == 3 || (role == 2 && count > 1)) look(3 - role);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -229,7 +240,6 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         return true;
     };
 
-    const unsigned count = (num_items - 1 - blockIdx.x) / gridDim.x + 1;
     if (role < 2) {
         // ------------------------------- diagonal blocks of the inverse --------------------------------------------------
         bool go = !p.l2norm || row_squares(0);
@@ -242,58 +252,75 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
             auto ready = [&]() {                           // (the next item's squares while the exchange is still read)
                 return (!p.l2norm || item + 1 == count || row_squares(item + 1)) && (item == 0 || wait(B_EXE + h, item - 1));
             };
-            go = lean_diagonal(tables(item), ps.bet[item & 3], p.l2norm != 0, ws.meta ? &ps.bound[buf][role] : nullptr, tmem + buf * 64, role, lane, x.valid, ex,
+            go = lean_diagonal(tables(item), ps.bet[item & 3], p.l2norm != 0, ws.meta ? &ps.bound[buf][role] : nullptr, tmem + buf * 64, role, lane, ex,
                                t2tile + 4096 * role, &tm_t2, static_cast<int>(x.tile * kChunk), cb(B_EXF + h), ready);
             tc_fence_before_sync();
             GDN_PHASE(1)
             ++prof_n;
         }
-    } else if (role == 2) {
-        // ------------------------------- tiles and product of `item`; P of the one before, rows 0-31; T'' of the one before that, below the
-        //                                 diagonal blocks
+    } else {
+        // ------------------------------- role 2: tiles and product of `item`, role 3: its gates and tables; P of the one before, rows 0-31 and 32-63; T'' of
+        //                                 the one before that, below the diagonal blocks, left and right half.  (One piece of code for both: what they share compiled
+        //                                 twice is 9 KB more for the instruction cache, 64 x 4096 tokens 744 us alone, now 726, 4 x 1999 with L2 normalisation 38.6, now 35.6.)
+        LaneGates gates{0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
         for (unsigned item = 0; item < count + 2; ++item) {
             const bool more = item < count, one = item > 0 && item <= count;
             const LeanItem &next = ps.item[item & 3], &x = ps.item[(item - 1) & 3], &y = ps.item[(item - 2) & 3];
             if (one && !enter(item - 1)) break;
-            if (more && warp == 2 && elect_one()) load_k(next);
+            if (more) {
+                if (role == 3) gates = lean_load_gates<GATE_F32>(p, next.tok0, next.hv, next.valid, lane);
+                else if (warp == 2 && elect_one()) load_k(next);
+            }
             __syncwarp();
             if (one) {
-                lean_mask_P(tables(item - 1), p.l2norm ? ps.prow[(item - 1) & 1] : nullptr, scale0, tmem + ((item - 1) & 1) * 64, 0, lane, x.valid, ptile);
+                lean_mask_P(tables(item - 1), p.l2norm ? ps.prow[(item - 1) & 1] : nullptr, scale0, tmem + ((item - 1) & 1) * 64, role - 2, lane, ptile);
                 tc_fence_before_sync();
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (elect_one()) {
-                    tma_store_2d(&tm_p, ptile, 0, static_cast<int>(x.tile * kChunk));
+                    const int row = static_cast<int>(x.tile * kChunk) + 32 * (role - 2);
+                    tma_store_2d(&tm_p, ptile + 2048 * (role - 2), 0, row);
+                    if (role == 3) tma_store_2d(&tm_p, ptile + 4096, 32, row);
                     tma_store_commit();
                 }
                 __syncwarp();
-                if (item + 1 < count) look(item + 1);
+                if (role == 2 && item + 1 < count) look(item + 1);
             }
             if (item > 0) {
                 if (elect_one()) {
-                    tma_store_wait_read();           // (and T'' below the diagonal blocks of the item before that)
+                    tma_store_wait_read();           // (role 2: and T'' below the diagonal blocks of the item before that)
                     mbar_arrive_a(cb(B_PAIR + h));
                 }
                 __syncwarp();
-                if (!wait(B_PAIR + h, item - 1)) break;
             }
-            if (more && elect_one()) {
+            if (role == 3 && more) {
+                if (one && !wait(B_ENT, item - 1)) break;   // (nobody reads the tables any more)
+                lean_gates(ps, item, gates, p.gate_act != 0, scale0, p.l2norm ? nullptr : ws.vec + next.tile * 256, lane);
+                __syncwarp();
+                if (lane == 0) mbar_arrive_a(cb(p.l2norm ? B_SQ : B_TAB + h));
+            }
+            if (item > 0 && !wait(B_PAIR + h, item - 1)) break;   // (T'' below the diagonal blocks has left its place; what role 2 looked up)
+            if (role == 2 && more && elect_one()) {
                 load_q_half(next, h);
                 if (HEADS == 1) load_q_half(next, 1);
             }
             __syncwarp();
             if (item > 1) {
                 if (!wait(B_EXF + h, item - 2)) break;
-                if (ws.meta && lane == 0) {
+                if (role == 2 && ws.meta && lane == 0) {
                     ws.meta[2 * y.tile] = y.decay;
                     ws.meta[2 * y.tile + 1] = y.gates_ok ? fmaxf(ps.bound[item & 1][0], ps.bound[item & 1][1]) : INFINITY;
                 }
-                lean_below(ps.bet[(item - 2) & 3], 0, lane, ex, t2tile + 2048, cb(B_EXE + h));
-                if (!wait(B_LOW + h, item - 2)) break;
-                if (elect_one()) {
-                    tma_store_2d(&tm_t2, t2tile + 2048, 0, static_cast<int>(y.tile * kChunk) + 32);
-                    tma_store_commit();
+                lean_below(ps.bet[(item - 2) & 3], role - 2, lane, ex, t2tile + 2048, cb(B_EXE + h));
+                if (role == 3) {
+                    if (lane == 0) mbar_arrive_a(cb(B_LOW + h));
+                } else {
+                    if (!wait(B_LOW + h, item - 2)) break;
+                    if (elect_one()) {
+                        tma_store_2d(&tm_t2, t2tile + 2048, 0, static_cast<int>(y.tile * kChunk) + 32);
+                        tma_store_commit();
+                    }
                 }
                 __syncwarp();
             }
@@ -301,50 +328,13 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                 if (warp == 2) {
                     if (one && !wait(B_ENT, item - 1)) break;   // (nobody reads the accumulator any more)
                     if (!wait(B_K, item) || !wait(B_Q, item)) break;
+                    if (p.pk_chunk && next.valid < kChunk) clear_tail(next.valid);
                     tc_fence_after_sync();
                     if ((one || p.dbg != kDbgNoProduct) && elect_one()) issue_product(tmem + (item & 1) * 64);
                     __syncwarp();
                 }
                 if (p.l2norm && !norms(item)) break;
             }
-        }
-    } else {
-        // ------------------------------- gates and tables of `item`; P of the one before, rows 32-63; T'' of the one before that
-#pragma unroll 1
-        for (unsigned item = 0; item < count + 2; ++item) {
-            const bool more = item < count, one = item > 0 && item <= count;
-            LeanItem &next = ps.item[item & 3], &x = ps.item[(item - 1) & 3];
-            if (one && !enter(item - 1)) break;
-            LaneGates gates{0.f, 0.f, 0.f, 0.f};
-            if (more) gates = lean_load_gates<GATE_F32>(p, next.tok0, next.hv, next.valid, lane);
-            if (one) {
-                lean_mask_P(tables(item - 1), p.l2norm ? ps.prow[(item - 1) & 1] : nullptr, scale0, tmem + ((item - 1) & 1) * 64, 1, lane, x.valid, ptile);
-                tc_fence_before_sync();
-                fence_proxy_async_smem();
-                __syncwarp();
-                if (elect_one()) {
-                    const int row = static_cast<int>(x.tile * kChunk) + 32;
-                    tma_store_2d(&tm_p, ptile + 2048, 0, row);
-                    tma_store_2d(&tm_p, ptile + 4096, 32, row);
-                    tma_store_commit();
-                    tma_store_wait_read();
-                }
-                __syncwarp();
-            }
-            if (item > 0 && lane == 0) mbar_arrive_a(cb(B_PAIR + h));
-            if (more) {
-                if (one && !wait(B_ENT, item - 1)) break;   // (nobody reads the tables any more)
-                lean_gates(ps, item, gates, p.gate_act != 0, scale0, p.l2norm ? nullptr : ws.vec + next.tile * 256, lane);
-                __syncwarp();
-                if (lane == 0) mbar_arrive_a(cb(p.l2norm ? B_SQ : B_TAB + h));
-            }
-            if (item > 0 && !wait(B_PAIR + h, item - 1)) break;   // (T'' below the diagonal blocks has left its place; what role 2 looked up)
-            if (item > 1) {
-                if (!wait(B_EXF + h, item - 2)) break;
-                lean_below(ps.bet[(item - 2) & 3], 1, lane, ex, t2tile + 2048, cb(B_EXE + h));
-                if (lane == 0) mbar_arrive_a(cb(B_LOW + h));
-            }
-            if (p.l2norm && more && !norms(item)) break;
         }
     }
 #undef GDN_PHASE

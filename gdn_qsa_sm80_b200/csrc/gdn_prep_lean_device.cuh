@@ -297,8 +297,7 @@ struct MaskTables {
 // lean_diagonal: one warp, the 32x32 diagonal block W from the accumulator's lanes 32 W .. + 31 (W = 1: also the mask of A21).  `stage`: its block of T'',
 // 2 KB, where the 8x8 blocks lie before that.  `wait`: for the exchange's readers of the item before.
 template <typename Wait>
-__device__ __forceinline__ bool lean_diagonal(const MaskTables& tab, const float* bet, bool l2norm, float* bound, uint32_t acc, int W, int lane, int valid,
-                                              LeanExchange& ex, uint8_t* stage, const void* map, int tile_row, uint32_t published, Wait&& wait) {
+__device__ __forceinline__ bool lean_diagonal(const MaskTables& tab, const float* bet, bool l2norm, float* bound, uint32_t acc, int W, int lane, LeanExchange& ex, uint8_t* stage, const void* map, int tile_row, uint32_t published, Wait&& wait) {
     asm volatile("" : "+r"(lane));   // (its addresses are computed here, not kept in registers across the items' loop)
     const int g = lane >> 2, t = lane & 3;
     const int R = 32 * W;            // first row, first column of the warp's diagonal block
@@ -320,14 +319,6 @@ __device__ __forceinline__ bool lean_diagonal(const MaskTables& tab, const float
             gj[r] = *reinterpret_cast<const float2*>(tab.gcol + R + 8 * r + 2 * t);
         }
         tmem_ld_wait();
-        if (valid < kChunk) {        // rows of padding tokens count as zeros whatever the tile holds there
-#pragma unroll
-            for (int e = 0; e < 8; ++e)
-                if (R + 4 * (e & 2) + g >= valid) x[e] = 0;
-#pragma unroll
-            for (int e = 0; e < 16; ++e)
-                if (R + 16 + 4 * (e & 2) + g >= valid) y[e] = 0;
-        }
         if (bound) {                 // max beta_i |k_i|^2; a key that is not a number counts as infinity (fmaxf would drop it)
             float m = 0.f;
             if (t == (g >> 1)) {
@@ -439,11 +430,6 @@ __device__ __forceinline__ bool lean_diagonal(const MaskTables& tab, const float
             uint32_t y[16];
             tmem_ld_16x256b_x4(tmem + ((16u * r) << 16), y);
             tmem_ld_wait();
-            if (valid < kChunk) {
-#pragma unroll
-                for (int e = 0; e < 16; ++e)
-                    if (32 + 16 * r + 4 * (e & 2) + g >= valid) y[e] = 0;
-            }
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const float2 col = *reinterpret_cast<const float2*>(tab.t32 + 8 * c + 2 * t);
@@ -520,7 +506,7 @@ __device__ __forceinline__ void lean_below(const float* bet, int b, int lane, co
 }
 
 // P = tril(scale * decay * Q K^T) as bf16 into its triangular tile, rows 32 W .. + 31, one warp.
-__device__ __forceinline__ void lean_mask_P(const MaskTables& tab, const float* prow, float scale0, uint32_t acc, int W, int lane, int valid, uint8_t* tile) {
+__device__ __forceinline__ void lean_mask_P(const MaskTables& tab, const float* prow, float scale0, uint32_t acc, int W, int lane, uint8_t* tile) {
     asm volatile("" : "+r"(lane));
     const int g = lane >> 2, t = lane & 3, R = 32 * W;
     const uint32_t tmem = tmem_addr(acc, 64 + R, 0), dst = smem_u32(tile) + 64 * R + tri_lane_offset(lane);   // (rows 32-63, columns 0-31 start at 2048)
@@ -528,13 +514,6 @@ __device__ __forceinline__ void lean_mask_P(const MaskTables& tab, const float* 
     float p[4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) p[r] = prow ? prow[R + 8 * r + g] : scale0;
-    auto clear = [&](uint32_t* y, int n, int row) {        // rows of padding tokens
-        if (valid < kChunk) {
-#pragma unroll
-            for (int e = 0; e < n; ++e)
-                if (row + 4 * (e & 2) + g >= valid) y[e] = 0;
-        }
-    };
     auto pack2 = [](float2 f, float2 col, const uint32_t* v) {
         const float2 x = mul2(mul2(f, col), floats(v[0], v[1]));
         return pack_bf16x2(x.x, x.y);
@@ -551,7 +530,6 @@ __device__ __forceinline__ void lean_mask_P(const MaskTables& tab, const float* 
             tmem_ld_16x256b_x4(tmem + ((16u * r) << 16), y);
             const float2 f0 = twice(p[2 * r] * tab.t32[32 + 16 * r + g]), f1 = twice(p[2 * r + 1] * tab.t32[40 + 16 * r + g]);
             tmem_ld_wait();
-            clear(y, 16, 32 + 16 * r);
             block(dst + 1024 * r, f0, f1, c0, c1, y);
             block((dst + 1024 * r) ^ 32, f0, f1, c2, c3, y + 8);
         }
@@ -568,8 +546,6 @@ __device__ __forceinline__ void lean_mask_P(const MaskTables& tab, const float* 
         gj[r] = column(tab.gcol + R, r);
     }
     tmem_ld_wait();
-    clear(x, 8, R);
-    clear(y, 16, R + 16);
     auto diag = [&](uint32_t at, int r, const uint32_t* v) {   // the 16x16 block of rows and columns 8 r ..
         const float2 a = mul2(mul2(decay2(twice(gi[r]), gj[r]), twice(p[r])), floats(v[0], v[1]));
         const float2 b = mul2(mul2(decay2(twice(gi[r + 1]), gj[r]), twice(p[r + 1])), floats(v[2], v[3]));
