@@ -51,9 +51,10 @@ __device__ __forceinline__ float sum_rows(float x) {   // over the eight lanes t
     return x;
 }
 
-// bytes of the token area of one stage: k, q rows, 32 columns of v (a box's destination: a multiple of 128); g and beta, behind all of them
-__host__ __device__ constexpr uint32_t dec_token_bytes(int nt) { return (nt * (256 + 256 + 64) + 127) & ~127u; }
+// bytes of the token area of one stage (a box's destination: a multiple of 128): k, q rows, 32 columns of v; g and beta there too, or, `apart`, behind all stages'
+// areas (four tokens: 128 bytes a stage less, which fits a fourth CTA; the other forms are 1 to 3 % faster with them inside)
 constexpr uint32_t kDecGateBytes = 2 * kDecTokens * 4;
+__host__ __device__ constexpr uint32_t dec_token_bytes(int nt, bool apart) { return (nt * (256 + 256 + 64) + (apart ? 0 : kDecGateBytes) + 127) & ~127u; }
 
 // Where the vectors of several tokens come from: a box of nt rows each, three copies a tile instead of three a token, where a CTA has
 // more than one tile (32 heads, 18 sequences of 2 tokens 12.5 us, by rows 13.7; 32 of 2 22.0, 23.3; of 3 and more tokens the same within
@@ -70,6 +71,7 @@ struct TokenMaps<Fetch::BOXES> {
     CUtensorMap q, k, v;
 };
 
+__host__ __device__ constexpr bool gates_apart(int groups, int stages, Fetch fetch) { return fetch == Fetch::BOXES && (groups == 1 || stages == 1); }
 __host__ __device__ constexpr int dec_ctas_per_sm(int groups, int stages) { return groups == 1 ? 4 : (stages == 3 ? 1 : 2); }
 
 template <int GROUPS, bool GATE_F32, bool PACKED, int STAGES, Fetch FETCH>
@@ -84,11 +86,14 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
     __shared__ int failed;
 
     const int tid = threadIdx.x, warp = static_cast<int>(warp_uniform(tid >> 5)), lane = tid & 31;
-    const uint32_t tok_bytes = dec_token_bytes(nt);
+    constexpr bool APART = gates_apart(GROUPS, STAGES, FETCH);
+    const uint32_t tok_bytes = dec_token_bytes(nt, APART);
     // stage s of group g: the tile at (g * STAGES + s) * 16 KB; the token areas behind all tiles
     auto tile_of = [&](int g, int s) { return sm + (g * STAGES + s) * 16384; };
     auto tok_of = [&](int g, int s) { return sm + GROUPS * STAGES * 16384 + (g * STAGES + s) * tok_bytes; };
-    auto gates_of = [&](int g, int s) { return reinterpret_cast<float*>(sm + GROUPS * STAGES * (16384 + tok_bytes) + (g * STAGES + s) * kDecGateBytes); };
+    auto gates_of = [&](int g, int s) {
+        return reinterpret_cast<float*>(APART ? sm + GROUPS * STAGES * (16384 + tok_bytes) + (g * STAGES + s) * kDecGateBytes : tok_of(g, s) + nt * (256 + 256 + 64));
+    };
     const int rep = p.Hv / p.Hq;
 
     if (tid == 0) {
@@ -360,9 +365,9 @@ bool two_gated_ctas(const Problem& p, long long states) {
 //   6 tokens                 6.9 / 7.6  9.2 / 7.5  11.3 / 9.6   11.4 / 11.7  16.4 / 13.1  16.7 / 17.5  21.2 / 19.0  35.1 / 35.4  87.8 / 84.7
 //   8 tokens                 8.2 / 8.8  11.1 / 8.8 13.8 / 11.5  13.8 / 13.8  20.2 / 15.6  20.5 / 21.2  26.3 / 22.7  44.1 / 43.2  112.0 / 100.2
 // (Packed batches keep three: where most of their sequences are single tokens a ring of two is 8 % slower, 128 sequences with one of 8 86.7 / 94.3.)
-bool two_stages(int tokens, long long tiles) {
+bool two_stages(int tokens, long long tiles, long long sms) {
     if (tokens < 5) return false;
-    const long long t = (tiles + sm_count() - 1) / sm_count();
+    const long long t = (tiles + sms - 1) / sms;
     auto last = [](long long k) { return k == 0 ? 0 : k == 1 ? 50 : 100; };
     return (tokens == 5 ? 130 : 126) * (t / 4) + last(t % 4) < 100 * (t / 3) + last(t % 3);
 }
@@ -387,13 +392,20 @@ int launch_decode(const Problem& p, const OutputGate* og, cudaStream_t stream) {
     DecodeGate gate{};
     if (og) gate = DecodeGate{static_cast<const __nv_bfloat16*>(og->z), static_cast<const __nv_bfloat16*>(og->weight), og->eps};
     const bool gated = og && !p.pk_short;
+    const long long sms = sm_count();
     const long long items = p.pk_short ? 4ll * p.pk_shorts * p.Hv : gated ? states : states * 4;
-    const int groups = gated ? 4 : 1, stages = gated ? (two_gated_ctas(p, states) ? 1 : 3) : !p.pk_short && two_stages(p.S, items) ? 2 : 3;
+    const int groups = gated ? 4 : 1, stages = gated ? (two_gated_ctas(p, states) ? 1 : 3) : !p.pk_short && two_stages(p.S, items, sms) ? 2 : 3;
     const int most = gated ? 4 : kDecTokens;                       // tokens whose vectors fit three stages of four groups
     const int nt = p.S < most ? p.S : most;
-    const uint32_t smem = groups * stages * (16384 + dec_token_bytes(nt) + kDecGateBytes) + 1024;
-    const int fit = static_cast<int>(228 * 1024 / (smem + (groups == 1 ? 1088 : 1536))), most_ctas = dec_ctas_per_sm(groups, stages), per_sm = fit > most_ctas ? most_ctas : fit;
-    const long long cap = static_cast<long long>(sm_count()) * per_sm;
+    auto bytes = [&](bool apart) { return groups * stages * (16384 + dec_token_bytes(nt, apart) + (apart ? kDecGateBytes : 0)) + 1024; };
+    auto resident = [&](uint32_t smem) {
+        const int fit = static_cast<int>(228 * 1024 / (smem + (groups == 1 ? 1088 : 1536))), most_ctas = dec_ctas_per_sm(groups, stages);
+        return sms * (fit > most_ctas ? most_ctas : fit);
+    };
+    // one tile a CTA: the host's time for three more maps is not hidden behind the kernel
+    const bool by_rows = p.pk_short || p.S == 1 || (!gated && p.S <= 4 && items <= resident(bytes(false)));
+    const uint32_t smem = bytes(!by_rows && gates_apart(groups, stages, Fetch::BOXES));
+    const long long cap = resident(smem);
     auto go = [&](auto kernel, const auto& maps) -> int {
         if (allow_smem(reinterpret_cast<const void*>(kernel), smem)) return GDN_ERR_CUDA;
         const unsigned grid = static_cast<unsigned>(items < cap ? items : cap);
@@ -406,8 +418,7 @@ int launch_decode(const Problem& p, const OutputGate* og, cudaStream_t stream) {
     if (p.pk_short) return p.gate_f32 ? go(gdn_decode_kernel<1, true, true, 3, Fetch::ROWS>, rows) : go(gdn_decode_kernel<1, false, true, 3, Fetch::ROWS>, rows);
     if (p.S == 1 && gated) return p.gate_f32 ? go(gdn_decode_kernel<4, true, false, 3, Fetch::ONE_ROW>, one) : go(gdn_decode_kernel<4, false, false, 3, Fetch::ONE_ROW>, one);
     if (p.S == 1) return p.gate_f32 ? go(gdn_decode_kernel<1, true, false, 3, Fetch::ONE_ROW>, one) : go(gdn_decode_kernel<1, false, false, 3, Fetch::ONE_ROW>, one);
-    // one tile a CTA: the host's time for three more maps is not hidden behind the kernel
-    if (!gated && p.S <= 4 && items <= cap)
+    if (by_rows)
         return p.gate_f32 ? go(gdn_decode_kernel<1, true, false, 3, Fetch::ROWS>, rows) : go(gdn_decode_kernel<1, false, false, 3, Fetch::ROWS>, rows);
     alignas(64) TokenMaps<Fetch::BOXES> maps;
     {
