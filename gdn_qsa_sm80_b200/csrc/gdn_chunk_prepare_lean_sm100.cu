@@ -16,7 +16,7 @@
 //   role 3      gates and tables of item i + 1; P, rows 32-63, of item i; T'' below the diagonal blocks, right half, of item i - 1
 // All four at the same item, with barriers of the head between the phases, left a quarter of the warps' time at them.
 //
-// What bounds it: the shared-memory pipe (16 sequences of 2048 tokens: 56 % of the cycles for loads and stores, about 25 % for operands and copies), then HBM (29 KB
+// What bounds it: the shared-memory pipe (16 sequences of 2048 tokens: 61 % of the cycles for loads and stores, about 25 % for operands and copies), then HBM (29 KB
 // per chunk and head).  us alone, against the form that passed A and T through shared memory row by row and ran its phases in step: 16 x 2048 124 / 95.8, 8192 tokens
 // 36.3 / 29.5, 4 x 1999 36.3 / 29.5 (with L2 normalisation 41.8 / 34.3), 64 x 4096 941 / 719; 16 x 2048 with 16 / 16 heads 81.5 / 66.0.
 // Stands in for the reference's gdn_prepare_kernel (csrc/gdn_chunk/gdn_kernel.cu:343-710).
