@@ -21,7 +21,7 @@ struct alignas(16) LeanScratch {
     float gam[2][kChunk];   // gamma_j * log2(e): inclusive cumsum of the log gate inside the chunk
     float bet[4][kChunk];   // beta_j (0 for padding tokens)
     float t16[2][kChunk];   // decay between a token and the last one of the first half of its 32 (t32: of the 64), times 1/|k_j| in the first half: the
-    float t32[2][kChunk];   // decay of a pair across that line is the product of its two entries, both at most 1
+    float t32[2][kChunk];   // decay of a pair across that line is the product of its two entries, both at most 1 (gates above zero: see lean_gates)
     float gcol[2][kChunk];  // with L2 normalisation: gamma_j - log2(1/|k_j|), the masks' column table
     float brow[2][kChunk];  // with L2 normalisation: beta_j / |k_j|, the row factors of A
     float prow[2][kChunk];  // with L2 normalisation: scale / |q_i|, the row factors of P
@@ -77,8 +77,22 @@ __device__ __forceinline__ void lean_gates(LeanScratch& ps, unsigned item, LaneG
     const float cC = __shfl_sync(0xffffffffu, c1, 31);
     *reinterpret_cast<float2*>(ps.gam[buf] + 2 * lane) = make_float2(c0, c1);
     *reinterpret_cast<float2*>(ps.bet[item & 3] + 2 * lane) = make_float2(x.b0, x.b1);
-    const float c16 = __shfl_sync(0xffffffffu, c1, (lane & 16) + 7), c32 = __shfl_sync(0xffffffffu, c1, 15);
+    float c16 = __shfl_sync(0xffffffffu, c1, (lane & 16) + 7), c32 = __shfl_sync(0xffffffffu, c1, 15);
     const float s16 = lane & 8 ? 1.f : -1.f, s32 = lane & 16 ? 1.f : -1.f;
+    if (!in_range) {
+        // Gates above zero: gamma can fall by 90 in front of a line and rise by 85 behind it, and the decay between the tokens before and after both is exp(-5), but
+        // exp(-90), what the line is from the first of them, is no fp32 number.  The tables then meet halfway between the smallest gamma before the line and the
+        // largest behind it: no entry is above the root of the largest decay across the line, and what is lost is below 2^-126 times that root.
+        auto halfway = [&](float s, int half, float line) {
+            float u = fmaxf(s * c0, s * c1);
+#pragma unroll 1
+            for (int o = half >> 1; o > 0; o >>= 1) u = fmaxf(u, __shfl_xor_sync(0xffffffffu, u, o));
+            const float v = __shfl_xor_sync(0xffffffffu, u, half);
+            return u + v < 250.f ? 0.5f * s * (u - v) : line;   // (not of a gate of +inf)
+        };
+        c16 = halfway(s16, 8, c16);
+        c32 = halfway(s32, 16, c32);
+    }
     *reinterpret_cast<float2*>(ps.t16[buf] + 2 * lane) = make_float2(fast_exp2(s16 * (c0 - c16)), fast_exp2(s16 * (c1 - c16)));
     *reinterpret_cast<float2*>(ps.t32[buf] + 2 * lane) = make_float2(fast_exp2(s32 * (c0 - c32)), fast_exp2(s32 * (c1 - c32)));
     if (lane == 0) {

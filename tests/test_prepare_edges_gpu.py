@@ -66,3 +66,25 @@ def test_fragments(B, S, Hq, Hv, l2norm):
     valid = S - 64 * (P.shape[2] - 1)
     assert np.abs(P[:, :, -1, valid:]).max(initial=0) == 0 and np.abs(T[:, :, -1, :, valid:]).max(initial=0) == 0
     assert O.rel_l2(vec[..., 192:], evec) < 1e-5
+
+
+@pytest.mark.parametrize("l2norm", [False, True])
+@pytest.mark.parametrize("Hq,Hv", [(1, 2), (3, 3)])
+@pytest.mark.parametrize("down,up", [(5, 12), (5, 20), (20, 40), (40, 52)])     # across a line of 8, 16, 32 and 16 tokens
+def test_gates_above_zero(down, up, Hq, Hv, l2norm):
+    """gamma falls by 90 and rises by 85 again inside a chunk: exp(-90) alone is no fp32 number, the decay between the tokens before and behind is exp(-5).  The
+    tokens between are not written (beta = 0)."""
+    B, S = 2, 120
+    gen = torch.Generator().manual_seed(down)
+    r = lambda *s: torch.randn(*s, generator=gen)
+    q, k = (t if l2norm else torch.nn.functional.normalize(t, dim=-1) for t in (r(B, S, Hq, 128), r(B, S, Hq, 128)))
+    g, beta = -0.01 * torch.rand(B, S, Hv, generator=gen), torch.sigmoid(r(B, S, Hv))
+    g[:, down], g[:, up], beta[:, down:up] = -90.0, 85.0, 0.0
+    d = [t.bfloat16().cuda() for t in (q, k, r(B, S, Hv, 128))] + [t.cuda() for t in (g, beta)]
+    gdn_chunk(*d, path="prepare_only_r", use_qk_l2norm_in_kernel=l2norm)
+    iface.check_device_status()
+    P, T, _ = workspace(B, S, Hq, Hv)
+    eP, eT, _ = exact(d[0], d[1], d[3], d[4], Hv, l2norm)
+    part = (slice(None), slice(None), 0, slice(up, None), slice(0, down))   # of the first chunk: rows behind the rise, columns before the fall
+    for got, want, limit in ((P, eP, 2.0 ** -8), (T, eT, 2.0 ** -8 + 8 * 2.0 ** -11)):
+        assert O.rel_l2(got[part], want[part]) < limit, O.rel_l2(got[part], want[part])
