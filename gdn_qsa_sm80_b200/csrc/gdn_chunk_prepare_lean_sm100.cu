@@ -22,6 +22,8 @@
 // Stands in for the reference's gdn_prepare_kernel (csrc/gdn_chunk/gdn_kernel.cu:343-710).
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "../../include/gdn_chunk_sm100.h"
 #include "gdn_common.cuh"
 #include "gdn_launch.cuh"
@@ -57,10 +59,11 @@ enum : uint32_t {
     B_EXF = B_PAIR + 2,  // + head: the exchange is full
     B_EXE = B_EXF + 2,   // + head: and has been read
     B_LOW = B_EXE + 2,   // + head: role 3's half of T'' below the diagonal blocks is there
-    B_BARS = B_LOW + 2
+    B_BARS = B_LOW + 2,
+    B_NEVER = B_BARS     // of a test hook: no arrival ever completes it
 };
 
-template <int HEADS, bool GATE_F32>
+template <int HEADS, bool GATE_F32, bool HOOKS>
 __global__ void __launch_bounds__(128 * HEADS, kLeanCtasPerSm<HEADS>)
 gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                         const __grid_constant__ CUtensorMap tm_p, const __grid_constant__ CUtensorMap tm_t2, Problem p,
@@ -69,7 +72,7 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);   // (an offset, so that the compiler knows the address space)
     const uint32_t sm_u32 = warp_uniform(smem_u32(sm));
-    __shared__ __align__(8) uint64_t bars[B_BARS];
+    __shared__ __align__(8) uint64_t bars[B_BARS + (HOOKS ? 1 : 0)];
     __shared__ uint32_t tmem_slot;
     __shared__ __align__(16) LeanScratch ps2[HEADS];
     __shared__ float squares[2][HEADS][128];      // with L2 normalisation: of the rows of [K;Q], per k-half
@@ -91,10 +94,13 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     // that share a qk head are prepared at about the same time.
     int late = 0;                                 // code of this thread's first wait that ran out
     auto wait = [&](uint32_t bar, uint32_t item) {
-        if (mbar_wait_compact(cb(bar), item & 1)) return true;
+        if (mbar_wait_compact(cb(HOOKS && p.dbg == kDbgLaneWaits && tid == 5 ? B_NEVER : bar), item & 1)) return true;
         if (late == 0) late = bar <= B_Q ? kDevTimeoutTma : kDevTimeoutMma;
         return false;
     };
+    // Each lane counts its own tries.  The warp goes on, or leaves, as one: a lane that left by itself would be at the CTA's last barrier while the others
+    // wait for it, without a limit, in the next instruction that needs the whole warp.
+    auto agreed = [](bool ok) { return __all_sync(0xffffffffu, ok) != 0; };
     auto decode = [&](unsigned n) {
         LeanItem x{};
         const unsigned c = n / groups, grp = n - c * groups;
@@ -174,6 +180,7 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                                    : i >= B_PAIR && i < B_LOW ? 2 : 1;
             mbar_init(&bars[i], count);
         }
+        if (HOOKS) mbar_init(&bars[B_NEVER], 1);
         fence_mbar_init();
     }
     if (warp == 0) {
@@ -194,16 +201,16 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = warp_uniform(tmem_slot);
-    if (p.dbg == kDbgLaneGivesUp && tid == 5) late = kDevTimeoutTma;
+    if (HOOKS && p.dbg == kDbgLaneGivesUp && tid == 5) late = kDevTimeoutTma;
 
     // Items of a CTA are counted from 0; `item & 1` names the buffer of its tables, its accumulator and the parity of its barriers.  A wait names a
     // parity, so the next completion of its barrier has to need something behind the wait: that of K, Q, MMA and TAB an arrival on ENT by each
     // warp that waits for them, the others an arrival by the one that waits.
     auto enter = [&](unsigned item) {
-        if (!wait(B_TAB + h, item) || !wait(B_MMA, item)) return false;
+        const bool ok = wait(B_TAB + h, item) && wait(B_MMA, item);
         tc_fence_after_sync();
-        if (lane == 0) mbar_arrive_a(cb(B_ENT));
-        return true;
+        if (ok && lane == 0) mbar_arrive_a(cb(B_ENT));
+        return agreed(ok);
     };
     auto tables = [&](unsigned item) {
         const uint32_t buf = item & 1;
@@ -212,7 +219,7 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     // L2 normalisation.  Squares of the next item's rows, of one k-half (of both where there is one head), by the warps of its head's diagonal blocks: role 0
     // K's, role 1 Q's.
     auto row_squares = [&](unsigned item) {
-        if (!wait(role == 0 ? B_K : B_Q, item)) return false;
+        if (!agreed(wait(role == 0 ? B_K : B_Q, item))) return false;
 #pragma unroll 1
         for (int e = 0; e < 2; ++e) {
             const int row = 64 * role + 32 * e + lane;
@@ -227,7 +234,7 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     // What is made of them behind role 3's gates: role 3 the keys' share of the tables, role 2 the queries'.
     auto norms = [&](unsigned item) {
         const uint32_t buf = item & 1;
-        if (!wait(B_SQ, item)) return false;
+        if (!agreed(wait(B_SQ, item))) return false;
         const LeanItem& x = ps.item[item & 3];
         float* vec = ws.vec + x.tile * 256;
 #pragma unroll 1
@@ -250,7 +257,7 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
             const uint32_t buf = item & 1;
             const LeanItem& x = ps.item[item & 3];
             auto ready = [&]() {                           // (the next item's squares while the exchange is still read)
-                return (!p.l2norm || item + 1 == count || row_squares(item + 1)) && (item == 0 || wait(B_EXE + h, item - 1));
+                return (!p.l2norm || item + 1 == count || row_squares(item + 1)) && (item == 0 || agreed(wait(B_EXE + h, item - 1)));
             };
             go = lean_diagonal(tables(item), ps.bet[item & 3], p.l2norm != 0, ws.meta ? &ps.bound[buf][role] : nullptr, tmem + buf * 64, role, lane, ex,
                                t2tile + 4096 * role, &tm_t2, static_cast<int>(x.tile * kChunk), cb(B_EXF + h), ready);
@@ -295,19 +302,18 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                 __syncwarp();
             }
             if (role == 3 && more) {
-                if (one && !wait(B_ENT, item - 1)) break;   // (nobody reads the tables any more)
+                if (one && !agreed(wait(B_ENT, item - 1))) break;   // (nobody reads the tables any more)
                 lean_gates(ps, item, gates, p.gate_act != 0, scale0, p.l2norm ? nullptr : ws.vec + next.tile * 256, lane);
                 __syncwarp();
                 if (lane == 0) mbar_arrive_a(cb(p.l2norm ? B_SQ : B_TAB + h));
             }
-            if (item > 0 && !wait(B_PAIR + h, item - 1)) break;   // (T'' below the diagonal blocks has left its place; what role 2 looked up)
+            if (item > 0 && !agreed(wait(B_PAIR + h, item - 1))) break;   // (T'' below the diagonal blocks has left its place; what role 2 looked up)
             if (role == 2 && more && elect_one()) {
                 load_q_half(next, h);
                 if (HEADS == 1) load_q_half(next, 1);
             }
-            __syncwarp();
             if (item > 1) {
-                if (!wait(B_EXF + h, item - 2)) break;
+                if (!agreed(wait(B_EXF + h, item - 2))) break;
                 if (role == 2 && ws.meta && lane == 0) {
                     ws.meta[2 * y.tile] = y.decay;
                     ws.meta[2 * y.tile + 1] = y.gates_ok ? fmaxf(ps.bound[item & 1][0], ps.bound[item & 1][1]) : INFINITY;
@@ -316,7 +322,7 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                 if (role == 3) {
                     if (lane == 0) mbar_arrive_a(cb(B_LOW + h));
                 } else {
-                    if (!wait(B_LOW + h, item - 2)) break;
+                    if (!agreed(wait(B_LOW + h, item - 2))) break;
                     if (elect_one()) {
                         tma_store_2d(&tm_t2, t2tile + 2048, 0, static_cast<int>(y.tile * kChunk) + 32);
                         tma_store_commit();
@@ -326,11 +332,11 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
             }
             if (more) {
                 if (warp == 2) {
-                    if (one && !wait(B_ENT, item - 1)) break;   // (nobody reads the accumulator any more)
-                    if (!wait(B_K, item) || !wait(B_Q, item)) break;
+                    // (ENT: nobody reads the accumulator any more)
+                    if (!agreed((!one || wait(B_ENT, item - 1)) && wait(B_K, item) && wait(B_Q, item))) break;
                     if (p.pk_chunk && next.valid < kChunk) clear_tail(next.valid);
                     tc_fence_after_sync();
-                    if ((one || p.dbg != kDbgNoProduct) && elect_one()) issue_product(tmem + (item & 1) * 64);
+                    if ((!HOOKS || one || p.dbg != kDbgNoProduct) && elect_one()) issue_product(tmem + (item & 1) * 64);
                     __syncwarp();
                 }
                 if (p.l2norm && !norms(item)) break;
@@ -368,12 +374,16 @@ int launch_prepare_lean(const Problem& p, const Workspace& ws, const TileMaps& m
                                                static_cast<unsigned>(NT), static_cast<unsigned>(items));
         return e == cudaSuccess ? GDN_OK : GDN_ERR_CUDA;
     };
-    if ((p.Hv / p.Hq) % 2 == 0) {
-        return p.gate_f32 ? go(gdn_prepare_lean_kernel<2, true>, 2, LeanSmem<2>::kDynamic, kLeanCtasPerSm<2>)
-                          : go(gdn_prepare_lean_kernel<2, false>, 2, LeanSmem<2>::kDynamic, kLeanCtasPerSm<2>);
-    }
-    return p.gate_f32 ? go(gdn_prepare_lean_kernel<1, true>, 1, LeanSmem<1>::kDynamic, kLeanCtasPerSm<1>)
-                      : go(gdn_prepare_lean_kernel<1, false>, 1, LeanSmem<1>::kDynamic, kLeanCtasPerSm<1>);
+    auto pick = [&](auto heads, auto hooks) -> int {
+        constexpr int H = decltype(heads)::value;
+        constexpr bool K = decltype(hooks)::value;
+        return p.gate_f32 ? go(gdn_prepare_lean_kernel<H, true, K>, H, LeanSmem<H>::kDynamic, kLeanCtasPerSm<H>)
+                          : go(gdn_prepare_lean_kernel<H, false, K>, H, LeanSmem<H>::kDynamic, kLeanCtasPerSm<H>);
+    };
+    using One = std::integral_constant<int, 1>;
+    using Two = std::integral_constant<int, 2>;
+    if ((p.Hv / p.Hq) % 2 == 0) return p.dbg ? pick(Two{}, std::true_type{}) : pick(Two{}, std::false_type{});
+    return p.dbg ? pick(One{}, std::true_type{}) : pick(One{}, std::false_type{});
 }
 
 }  // namespace gdn

@@ -21,13 +21,14 @@ constexpr int kD = 128;      // head dimension (keys and values)
 constexpr int kChunk = 64;   // tokens per chunk
 constexpr float kLog2e = 1.4426950408889634f;
 
-// Test hooks of Problem::dbg (7: gdn_chunk_coop_sm100.cu).  Those of the chain are compiled into instantiations of their own: a comparison
+// Test hooks of Problem::dbg (7: gdn_chunk_coop_sm100.cu).  Those of the two-kernel path are compiled into instantiations of their own: a comparison
 // in its loops made calls of a few tokens 0.3 to 1 % longer.
 constexpr int kDbgLateProducer = 8;    // residual-form chain: the TMA producer sleeps 20 us before it looks at a barrier
 constexpr int kDbgWarpGivesUp = 9;     // residual-form chain: one of the output warps waits for a barrier that nothing completes instead of the first outputs
 constexpr int kDbgNoTile = 10;         // residual-form chain: the first tile of V is never announced
 constexpr int kDbgNoProduct = 11;      // lean prepare: no CTA's first product is issued
 constexpr int kDbgLaneGivesUp = 12;    // lean prepare: one lane of each CTA that is not its warp's first has given up
+constexpr int kDbgLaneWaits = 13;      // lean prepare: the same lane waits for a barrier that nothing completes in place of its own
 
 struct Problem {
     const __nv_bfloat16* q;

@@ -458,6 +458,7 @@ __device__ __forceinline__ bool lean_diagonal(const MaskTables& tab, const float
     }
     __syncwarp();                    // (and the 8x8 blocks have been read)
     if (lane == 0) mbar_arrive_a(published);
+    __syncwarp();
     float2 be[4];
 #pragma unroll
     for (int n = 0; n < 4; ++n) be[n] = *reinterpret_cast<const float2*>(bet + R + 8 * n + 2 * t);
@@ -508,6 +509,7 @@ __device__ __forceinline__ void lean_below(const float* bet, int b, int lane, co
     }
     __syncwarp();
     if (lane == 0) mbar_arrive_a(taken);
+    __syncwarp();
     const uint32_t dst = (smem_u32(stage) + tri_lane_offset(lane)) ^ (32 * b);
     float2 be[2];
 #pragma unroll

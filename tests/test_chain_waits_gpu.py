@@ -12,7 +12,7 @@ from gdn_qsa_sm80_b200.synthetic import make_inputs
 
 pytestmark = pytest.mark.gpu
 
-LATE_PRODUCER, WARP_GIVES_UP, NO_TILE, NO_PRODUCT, LANE_GIVES_UP = "8", "9", "10", "11", "12"
+LATE_PRODUCER, WARP_GIVES_UP, NO_TILE, NO_PRODUCT, LANE_GIVES_UP, LANE_WAITS = "8", "9", "10", "11", "12", "13"
 
 
 def inputs(workload, **sizes):
@@ -85,7 +85,7 @@ def test_an_output_warp_that_gives_up_holds_up_the_others_for_a_limited_time(S, 
 
 @pytest.mark.parametrize("Hq,Hv", [(1, 2), (3, 3)])
 def test_a_single_lane_that_gave_up_is_reported(Hq, Hv, monkeypatch):
-    """Each lane counts its own tries; the prepare kernel's CTA leaves when any of them has run out."""
+    """Each lane counts its own tries; the code of any of them is reported."""
     d = inputs("default", S=40, Hq=Hq, Hv=Hv)
     monkeypatch.setenv("GDN_CHUNK_DBG", LANE_GIVES_UP)
     gdn_chunk(*d, path="prepare_only_t")
@@ -94,3 +94,22 @@ def test_a_single_lane_that_gave_up_is_reported(Hq, Hv, monkeypatch):
     monkeypatch.delenv("GDN_CHUNK_DBG")
     gdn_chunk(*d)
     check_device_status()
+
+
+@pytest.mark.parametrize("S", [40, 300])
+@pytest.mark.parametrize("Hq,Hv", [(1, 2), (3, 3)])
+def test_a_warp_leaves_when_one_of_its_lanes_has_given_up(Hq, Hv, S, monkeypatch):
+    """The other lanes of its warp have seen their barriers complete: had they gone on, they would wait without a limit for the lane that left."""
+    d = inputs("default", S=S, Hq=Hq, Hv=Hv)
+    out, st = gdn_chunk(*d)
+    check_device_status()
+    monkeypatch.setenv("GDN_CHUNK_DBG", LANE_WAITS)
+    t0 = time.time()
+    gdn_chunk(*d, path="prepare_only_t")
+    with pytest.raises(_lib.GdnLibraryError, match="0x102"):
+        check_device_status()
+    assert 1.5 < time.time() - t0 < 9.0      # its wait and those of the others for what its warp makes
+    monkeypatch.delenv("GDN_CHUNK_DBG")
+    again, st_again = gdn_chunk(*d)
+    check_device_status()
+    assert torch.equal(out, again) and torch.equal(st, st_again)
