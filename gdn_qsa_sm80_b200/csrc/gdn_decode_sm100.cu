@@ -74,6 +74,18 @@ struct TokenMaps<Fetch::BOXES> {
 __host__ __device__ constexpr bool gates_apart(int groups, int stages, Fetch fetch) { return fetch == Fetch::BOXES && (groups == 1 || stages == 1); }
 __host__ __device__ constexpr int dec_ctas_per_sm(int groups, int stages) { return groups == 1 ? 4 : (stages == 3 ? 1 : 2); }
 
+// Shared memory of a CTA, and the CTAs for which an SM's 228 KB suffice: each takes 1 KB more, and its own in steps of 128 bytes.
+constexpr uint32_t dec_static_bytes(int groups, int stages, bool packed) {
+    return (2 * 8 * groups * stages + (groups == 4 ? 64 : 0) + (packed ? 16 * stages : 0) + 4 + 15) & ~15;
+}
+constexpr uint32_t dec_dynamic_bytes(int groups, int stages, int nt, bool apart) {
+    return groups * stages * (16384 + dec_token_bytes(nt, apart) + (apart ? kDecGateBytes : 0)) + 1024;
+}
+constexpr int dec_fit(uint32_t dynamic_bytes, uint32_t static_bytes) {
+    return static_cast<int>(228 * 1024 / (((dynamic_bytes + static_bytes + 127) & ~127u) + 1024));
+}
+static_assert(dec_fit(dec_dynamic_bytes(1, 3, 4, true), dec_static_bytes(1, 3, false)) == 4, "four tokens: four CTAs of three stages an SM, to the byte");
+
 template <int GROUPS, bool GATE_F32, bool PACKED, int STAGES, Fetch FETCH>
 __global__ void __launch_bounds__(GROUPS * 64 + 32, dec_ctas_per_sm(GROUPS, STAGES))
 gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_out,
@@ -84,6 +96,8 @@ gdn_decode_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_consta
     __shared__ float ssq[2][GROUPS * 2];
     __shared__ int4 seq_of[PACKED ? STAGES : 1];   // (sequence, first token, tokens) of the stage's tile
     __shared__ int failed;
+    // (every variable above that the form uses counts: how many CTAs an SM holds goes by it)
+    static_assert(sizeof(full) + sizeof(empty) + (GROUPS == 4 ? sizeof(ssq) : 0) + (PACKED ? sizeof(seq_of) : 0) + sizeof(failed) <= dec_static_bytes(GROUPS, STAGES, PACKED));
 
     const int tid = threadIdx.x, warp = static_cast<int>(warp_uniform(tid >> 5)), lane = tid & 31;
     constexpr bool APART = gates_apart(GROUPS, STAGES, FETCH);
@@ -403,9 +417,9 @@ int launch_decode(const Problem& p, const OutputGate* og, cudaStream_t stream) {
     const int groups = gated ? 4 : 1, stages = gated ? (two_gated_ctas(p, states) ? 1 : 3) : !p.pk_short && two_stages(p, items, sms) ? 2 : 3;
     const int most = gated ? 4 : kDecTokens;                       // tokens whose vectors fit three stages of four groups
     const int nt = p.S < most ? p.S : most;
-    auto bytes = [&](bool apart) { return groups * stages * (16384 + dec_token_bytes(nt, apart) + (apart ? kDecGateBytes : 0)) + 1024; };
+    auto bytes = [&](bool apart) { return dec_dynamic_bytes(groups, stages, nt, apart); };
     auto resident = [&](uint32_t smem) {
-        const int fit = static_cast<int>(228 * 1024 / (smem + (groups == 1 ? 1088 : 1536))), most_ctas = dec_ctas_per_sm(groups, stages);
+        const int fit = dec_fit(smem, dec_static_bytes(groups, stages, p.pk_short != nullptr)), most_ctas = dec_ctas_per_sm(groups, stages);
         return sms * (fit > most_ctas ? most_ctas : fit);
     };
     // one tile a CTA: the host's time for three more maps is not hidden behind the kernel
