@@ -88,3 +88,52 @@ def test_gates_above_zero(down, up, Hq, Hv, l2norm):
     part = (slice(None), slice(None), 0, slice(up, None), slice(0, down))   # of the first chunk: rows behind the rise, columns before the fall
     for got, want, limit in ((P, eP, 2.0 ** -8), (T, eT, 2.0 ** -8 + 8 * 2.0 ** -11)):
         assert O.rel_l2(got[part], want[part]) < limit, O.rel_l2(got[part], want[part])
+
+
+def tf32(x):
+    """Rounded to the nearest number of 11 bits, halves to even."""
+    b = x.astype(np.float32).view(np.uint32).astype(np.uint64)
+    return ((b + 0xFFF + ((b >> 13) & 1)) & 0xFFFFE000).astype(np.uint32).view(np.float32).astype(np.float64)
+
+
+def rounded_inverse(A):
+    """(I + A)^-1 as the kernel rounds it: blocks of 16 exact, X21 = -X22 (A21 X11) of 32 and 64 with every factor a TF32 number."""
+    T = np.zeros_like(A)
+    for b in range(0, 64, 16):
+        T[..., b:b + 16, b:b + 16] = np.linalg.inv(np.eye(16) + A[..., b:b + 16, b:b + 16])
+    for s in (16, 32):
+        for b in range(0, 64, 2 * s):
+            lo, hi = slice(b, b + s), slice(b + s, b + 2 * s)
+            T[..., hi, lo] = -tf32(T[..., hi, hi]) @ tf32(tf32(A[..., hi, lo]) @ tf32(T[..., lo, lo]))
+    return T
+
+
+@pytest.mark.parametrize("decay,alike", [(0.3, False), (0.01, False), (2.0, False), (0.1, True), (0.0, True)])
+@pytest.mark.parametrize("Hq,Hv,l2norm", [(4, 8, False), (4, 8, True), (3, 3, True)])
+def test_error_before_the_last_rounding(decay, alike, Hq, Hv, l2norm):
+    """The rounding to bf16 hides what came before it but for the values it sends the other way, whose share grows with that error: of P (fp32 sums) next to none,
+    of T'' as many as the roundings of the inverse's TF32 factors give by themselves."""
+    B, S = 8, 640
+    gen = torch.Generator().manual_seed(5)
+    r = lambda *s: torch.randn(*s, generator=gen)
+    q, k = (t if l2norm else torch.nn.functional.normalize(t, dim=-1) for t in (r(B, S, Hq, 128), r(B, S, Hq, 128)))
+    if alike:
+        k = k[:, :1] + 1e-3 * k
+    g, beta = -torch.nn.functional.softplus(r(B, S, Hv)) * decay, torch.sigmoid(r(B, S, Hv))
+    d = [t.bfloat16().cuda() for t in (q, k, r(B, S, Hv, 128))] + [t.cuda() for t in (g, beta)]
+    gdn_chunk(*d, path="prepare_only_r", use_qk_l2norm_in_kernel=l2norm)
+    iface.check_device_status()
+    P, T, _ = workspace(B, S, Hq, Hv)
+    eP, eT, _ = exact(d[0], d[1], d[3], d[4], Hv, l2norm)
+    columns = np.moveaxis(beta.double().numpy(), 2, 1).reshape(B, Hv, -1, 1, 64)
+    bf16 = lambda x: torch.from_numpy(np.ascontiguousarray(x)).float().bfloat16().double().numpy()
+
+    def other_way(got, want):                # share of the values above a thousandth of the largest
+        return (got != bf16(want))[np.abs(want) > 1e-3 * np.abs(want).max()].mean()
+
+    expected = other_way(bf16(rounded_inverse(np.linalg.inv(eT / columns) - np.eye(64)) * columns), eT)
+    # P: sums of 128 products and a decay in fp32, a few 2^-21 of a typical value (exponents of a hundred lose some bits more), against steps of 2^-8: a share of 2^-11
+    # and less.  T'': some hundred (strong decay: 5e-4 of them are allowed for) to ten thousand values go the other way, so 15 % is outside their spread, and factors of
+    # one bit less would double the share.
+    assert other_way(P, eP) < 2.0 ** -10, other_way(P, eP)
+    assert other_way(T, eT) < 1.15 * expected + 5e-4, (other_way(T, eT), expected)
