@@ -532,89 +532,4 @@ __device__ __forceinline__ void prep_store_scaled_T_row(const float* Tm, const f
     }
 }
 
-// Columns [32 hh, 32 hh + 32) of row i of T, read once, as bf16 into BOTH consumers: T diag(fa) into row `dst_row` of
-// a 128-byte-swizzled K-major tile and T diag(fb) into a plain row of 64 values in global memory.  The block of T
-// above its two 32x32 diagonal blocks (rows 0-31, columns 32-63) is zero by definition and is not read, so that
-// part of `Tm` need not be defined.  hh and i < 32 must be uniform over a warp.
-__device__ __forceinline__ void prep_store_T_half_row_both(const float* Tm, const float* fa, const float* fb, int i, int hh,
-                                                           uint8_t* tile, uint32_t dst_row, __nv_bfloat16* grow) {
-    if (hh == 1 && i < 32) {
-#pragma unroll
-        for (int ch = 4; ch < 8; ++ch) {
-            *reinterpret_cast<uint4*>(tile + swz_chunk_offset<128>(dst_row, ch)) = make_uint4(0, 0, 0, 0);
-            *reinterpret_cast<uint4*>(grow + ch * 8) = make_uint4(0, 0, 0, 0);
-        }
-        return;
-    }
-#pragma unroll
-    for (int c4 = 0; c4 < 4; ++c4) {
-        const int ch = 4 * hh + c4;
-        const float4 t0 = *reinterpret_cast<const float4*>(Tm + i * kSolveStride + ch * 8);
-        const float4 t1 = *reinterpret_cast<const float4*>(Tm + i * kSolveStride + ch * 8 + 4);
-        const float4 a0 = *reinterpret_cast<const float4*>(fa + ch * 8), a1 = *reinterpret_cast<const float4*>(fa + ch * 8 + 4);
-        const float4 b0 = *reinterpret_cast<const float4*>(fb + ch * 8), b1 = *reinterpret_cast<const float4*>(fb + ch * 8 + 4);
-        uint4 pa, pb;
-        pa.x = pack_bf16x2(t0.x * a0.x, t0.y * a0.y);
-        pa.y = pack_bf16x2(t0.z * a0.z, t0.w * a0.w);
-        pa.z = pack_bf16x2(t1.x * a1.x, t1.y * a1.y);
-        pa.w = pack_bf16x2(t1.z * a1.z, t1.w * a1.w);
-        pb.x = pack_bf16x2(t0.x * b0.x, t0.y * b0.y);
-        pb.y = pack_bf16x2(t0.z * b0.z, t0.w * b0.w);
-        pb.z = pack_bf16x2(t1.x * b1.x, t1.y * b1.y);
-        pb.w = pack_bf16x2(t1.z * b1.z, t1.w * b1.w);
-        *reinterpret_cast<uint4*>(tile + swz_chunk_offset<128>(dst_row, ch)) = pa;
-        *reinterpret_cast<uint4*>(grow + ch * 8) = pb;
-    }
-}
-
-// The same with T diag(fb) into row `row_b` of a second 128-byte-swizzled tile in shared memory (a staging tile that a
-// TMA store takes to global memory: a row per thread written straight to global memory costs a wavefront per lane).
-__device__ __forceinline__ void prep_store_T_half_row_tiles(const float* Tm, const float* fa, const float* fb, int i, int hh,
-                                                            uint8_t* tile_a, uint32_t row_a, uint8_t* tile_b, uint32_t row_b) {
-    if (hh == 1 && i < 32) {
-#pragma unroll
-        for (int ch = 4; ch < 8; ++ch) {
-            *reinterpret_cast<uint4*>(tile_a + swz_chunk_offset<128>(row_a, ch)) = make_uint4(0, 0, 0, 0);
-            *reinterpret_cast<uint4*>(tile_b + swz_chunk_offset<128>(row_b, ch)) = make_uint4(0, 0, 0, 0);
-        }
-        return;
-    }
-#pragma unroll
-    for (int c4 = 0; c4 < 4; ++c4) {
-        const int ch = 4 * hh + c4;
-        const float4 t0 = *reinterpret_cast<const float4*>(Tm + i * kSolveStride + ch * 8);
-        const float4 t1 = *reinterpret_cast<const float4*>(Tm + i * kSolveStride + ch * 8 + 4);
-        const float4 a0 = *reinterpret_cast<const float4*>(fa + ch * 8), a1 = *reinterpret_cast<const float4*>(fa + ch * 8 + 4);
-        const float4 b0 = *reinterpret_cast<const float4*>(fb + ch * 8), b1 = *reinterpret_cast<const float4*>(fb + ch * 8 + 4);
-        uint4 pa, pb;
-        pa.x = pack_bf16x2(t0.x * a0.x, t0.y * a0.y);
-        pa.y = pack_bf16x2(t0.z * a0.z, t0.w * a0.w);
-        pa.z = pack_bf16x2(t1.x * a1.x, t1.y * a1.y);
-        pa.w = pack_bf16x2(t1.z * a1.z, t1.w * a1.w);
-        pb.x = pack_bf16x2(t0.x * b0.x, t0.y * b0.y);
-        pb.y = pack_bf16x2(t0.z * b0.z, t0.w * b0.w);
-        pb.z = pack_bf16x2(t1.x * b1.x, t1.y * b1.y);
-        pb.w = pack_bf16x2(t1.z * b1.z, t1.w * b1.w);
-        *reinterpret_cast<uint4*>(tile_a + swz_chunk_offset<128>(row_a, ch)) = pa;
-        *reinterpret_cast<uint4*>(tile_b + swz_chunk_offset<128>(row_b, ch)) = pb;
-    }
-}
-
-// Row `i` of  T diag(f)  as bf16 into a plain row-major row of 64 values in global memory (16-byte stores).
-__device__ __forceinline__ void prep_store_scaled_T_row_plain(const float* Tm, const float* f, int i, __nv_bfloat16* dst) {
-#pragma unroll
-    for (int ch = 0; ch < 8; ++ch) {
-        const float4 t0 = *reinterpret_cast<const float4*>(Tm + i * kSolveStride + ch * 8);
-        const float4 t1 = *reinterpret_cast<const float4*>(Tm + i * kSolveStride + ch * 8 + 4);
-        const float4 f0 = *reinterpret_cast<const float4*>(f + ch * 8);
-        const float4 f1 = *reinterpret_cast<const float4*>(f + ch * 8 + 4);
-        uint4 pk;
-        pk.x = pack_bf16x2(t0.x * f0.x, t0.y * f0.y);
-        pk.y = pack_bf16x2(t0.z * f0.z, t0.w * f0.w);
-        pk.z = pack_bf16x2(t1.x * f1.x, t1.y * f1.y);
-        pk.w = pack_bf16x2(t1.z * f1.z, t1.w * f1.w);
-        *reinterpret_cast<uint4*>(dst + ch * 8) = pk;
-    }
-}
-
 }  // namespace gdn
