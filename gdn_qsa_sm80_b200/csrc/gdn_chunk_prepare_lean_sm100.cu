@@ -350,7 +350,8 @@ gdn_prepare_lean_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     }
     if (late) atomicCAS(p.status, 0, late);       // (each lane counts its own tries)
     // Only now may the chain kernel's CTAs start (and set up while the last CTAs of this grid finish): let in earlier, they
-    // pile up two to an SM on the SMs that this grid leaves first while others stay empty.
+    // pile up two to an SM on the SMs that this grid leaves first while others stay empty.  (And never in front of this kernel's own wait: the chain
+    // reads K, V and the initial state as soon as it starts.)
     grid_launch_dependents();
     if (elect_one()) tma_store_wait_all();
     tc_fence_before_sync();

@@ -6,7 +6,8 @@
 // kernel is laid out for HBM.  The value columns of a state are independent, so the unit of work is a tile of
 // [128 rows][32 columns] (16 KB): two warps own one, 64 values per thread, and a persistent CTA streams tiles through a
 // ring of three TMA stages - the loads of the next tiles are in flight while this one is computed and the one before
-// leaves by TMA store, which the load-compute-store phases of one CTA per state could not do (75 % of the copy bandwidth).
+// leaves by TMA store, which the load-compute-store phases of one CTA per state could not do (75 % of the copy bandwidth).  (A ring of two that
+// writes states has no load in flight beside a computation: the next tile's place is the one whose store has to be read first.  The other CTAs of the SM fill that.)
 // The tile is 128-byte swizzled; a lane owns eight pairs of rows and the four columns of a chunk, so that a 16-byte access of eight
 // lanes covers all banks, a pair's two values of k arrive in one word, and the column sums a token needs (S^T k, S^T q) are three
 // shuffles: no barrier.  With several tokens a tile what bounds it is the two warps' serial run through the tokens, not HBM (64 sequences

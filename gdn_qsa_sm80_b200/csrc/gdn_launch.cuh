@@ -28,8 +28,10 @@ private:
 int allow_smem(const void* kernel, size_t bytes);
 
 // Launches with the programmatic-stream-serialization attribute: the CTAs may set up while the kernel before this one in the
-// stream drains (the kernel waits for it with grid_dependency_wait before it touches memory).  `pairs`: clusters of two CTAs
-// along x.  Where the context has neither, an ordinary launch, in which that wait is a no-op.
+// stream drains.  What that kernel makes is touched behind grid_dependency_wait only.  What is older may be read in front of it (the chain:
+// K, V and the initial state, Problem::behind_prepare; the normalisation: z, its z_ready), but only behind a kernel all of whose CTAs have
+// themselves waited before they trigger or end: a launch by this function says nothing about the kernels before the last one.
+// `pairs`: clusters of two CTAs along x.  Where the context has neither, an ordinary launch, in which that wait is a no-op.
 template <typename Kernel, typename... Args>
 inline cudaError_t launch_dependent(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool pairs, const Args&... args) {
     cudaLaunchConfig_t cfg = {};

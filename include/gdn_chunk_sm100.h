@@ -169,7 +169,7 @@ int gdn_rmsnorm_gated_sm100(const void* y, const void* z, const void* weight, vo
 /*
  * gdn_chunk_fwd_sm100_ex followed by the gated normalisation of its output, as one call: `out` receives
  * rmsnorm_gated(O, z, weight) with O the operator's output (z [B,S,Hv,128] bf16, weight [128] bf16).  The
- * normalisation runs right behind the forward pass on the same stream and in place, while O is still in L2.
+ * normalisation runs right behind the forward pass on the same stream and in place (of a few tokens: in the same kernel).
  * Stands in for the reference's sequence gdn_chunk -> rmsnorm_gated (README.md:127-139 and :184-190).
  */
 int gdn_chunk_fwd_gated_sm100(const void* q, const void* k, const void* v, const void* g, const void* beta,
