@@ -379,8 +379,9 @@ bool two_gated_ctas(const Problem& p, long long states) {
 //   5 tokens                 6.3 / 7.0  8.2 / 6.9  10.1 / 8.6   10.2 / 10.4  14.5 / 11.9  14.9 / 15.8  18.7 / 17.1  30.9 / 31.8  76.3 / 76.9
 //   6 tokens                 6.9 / 7.6  9.2 / 7.5  11.3 / 9.6   11.4 / 11.7  16.4 / 13.1  16.7 / 17.5  21.2 / 19.0  35.1 / 35.4  87.8 / 84.7
 //   8 tokens                 8.2 / 8.8  11.1 / 8.8 13.8 / 11.5  13.8 / 13.8  20.2 / 15.6  20.5 / 21.2  26.3 / 22.7  44.1 / 43.2  112.0 / 100.2
-// With states both in and out and many tiles an SM the three of a round run into the next round and its tiles' traffic counts: above 20 tiles, five tokens stay with three
-// (at 23 to 84 tiles 0.6 to 5 % faster, at 25, 28 and 173 it is two, by 0.6 to 1.7 %), six need two ahead by 3 % (21 tiles 35.2 / 35.9; left: 26 tiles 43.7 / 44.1).
+// With states both in and out and many tiles an SM a round's three run into the next round, the tiles' traffic counts and a last round of one costs the form of four more. Above
+// 20 tiles five tokens stay with three (21 to 84 tiles 0.6 to 5 % faster; two at 25, 28, 29 and 173 by 0.6 to 2 %); with six that last round counts 71 (21 tiles 35.3 / 35.8), and where two
+// are taken they are up to 5 % ahead at 22 to 65 tiles but at 26, 27, 30, 31, 34, 43 and 46 (0.7 to 1.8 % behind).
 // With one of them or neither two are ahead by 7 to 39 % wherever this rule takes them (64 sequences of 5 tokens: state in 71.2 / 55.2, out 73.4 / 66.6, neither 69.3 / 53.0).
 // (Packed batches keep three: where most of their sequences are single tokens a ring of two is 8 % slower, 128 sequences with one of 8 86.7 / 94.3.)
 bool two_stages(const Problem& p, long long tiles, long long sms) {
@@ -388,9 +389,8 @@ bool two_stages(const Problem& p, long long tiles, long long sms) {
     const long long t = (tiles + sms - 1) / sms;
     const bool many = p.h0 && p.hT && t > 20;
     if (many && p.S == 5) return false;
-    auto last = [](long long k) { return k == 0 ? 0 : k == 1 ? 50 : 100; };
-    const long long two = (p.S == 5 ? 130 : 126) * (t / 4) + last(t % 4), three = 100 * (t / 3) + last(t % 3);
-    return two * (many && p.S == 6 ? 103 : 100) < three * 100;
+    auto last = [](long long k, int one) { return k == 0 ? 0 : k == 1 ? one : 100; };
+    return (p.S == 5 ? 130 : 126) * (t / 4) + last(t % 4, many && p.S == 6 ? 71 : 50) < 100 * (t / 3) + last(t % 3, 50);
 }
 
 }  // namespace
